@@ -157,13 +157,19 @@ def _row_counts(case, seed):
     return torch.tensor(counts, dtype=torch.int64)
 
 
-def prepare(case, seed):
+def _drawn(case, seed):
+    r"""The layer with its weights, the input rows and the gradient that arrives at the output."""
     torch.manual_seed(seed)
     dtype = DTYPES[case["dtype"]]
     with torch.device("cuda"):
         layer = _layer(case).to(dtype)
         x = torch.randn(case["tokens"], case["d"]).to(dtype)
         gy = torch.randn(case["tokens"], case["h"] if case["kind"] == "linear" else case["d"]).to(dtype)
+    return layer, x, gy
+
+
+def prepare(case, seed):
+    layer, x, gy = _drawn(case, seed)
     layer.train(case["mode"] == "train")
     held = {"layer": layer, "gy": gy, "aux": case["gate"] != "naive"}
     if case["kind"] == "linear":
@@ -197,6 +203,65 @@ def _train(held, x):
 
 def run(state):
     return state["step"](state["x"])
+
+
+# ------------------------------------------------------------------------------ in 64 bits
+def _keep_within(ids, experts, cap):
+    r"""``ids`` with every slot beyond the first ``cap`` of its expert (in slot order) set to -1."""
+    one = nn.functional.one_hot(ids.reshape(-1), experts)
+    rank = (one.cumsum(0) * one).sum(1) - 1
+    return torch.where(rank < cap, ids.reshape(-1), -1).view_as(ids)
+
+
+def _exact_gate(case, x, w, b):
+    r"""Expert ids and scores ``[tokens, k]`` and the balance loss (or ``None``).  Which experts a
+    token goes to is decided on logits rounded to the layer's type, ties to the lower id, as any
+    implementation that holds them in that type does; the scores are those of the unrounded ones."""
+    n, experts, k, mode = case["tokens"], case["experts"], case["k"], case["mode"]
+    logits = x @ w.t() + b
+    rounded = logits.detach().to(DTYPES[case["dtype"]])
+    ids = rounded.sort(dim=1, descending=True, stable=True).indices[:, :k]
+    prob = torch.softmax(logits, dim=1)
+    if case["gate"] == "switch":
+        kept = _keep_within(ids, experts, math.ceil(CAPACITY[mode] * n / experts))
+        share = nn.functional.one_hot(kept[kept >= 0], experts).sum(0)
+        n_kept = share.sum().clamp(min=1)
+        return kept, prob.gather(1, ids), experts * ((share / n_kept) * (prob.sum(0) / n_kept)).sum()
+    score = torch.softmax(logits.gather(1, ids), dim=1)
+    if case["gate"] == "gshard":
+        share = nn.functional.one_hot(ids[:, 0], experts).sum(0) / n
+        loss = (share * prob.mean(0)).mean() * experts ** 2
+        return _keep_within(ids, experts, math.ceil(CAPACITY[mode] * n) * k // experts), score, loss
+    return ids, score, None
+
+
+def exact(case, seed):
+    layer, x, gy = _drawn(case, seed)
+    train, experts, kind = case["mode"] == "train", case["experts"], case["kind"]
+    par = {n: p.detach().double().requires_grad_(train) for n, p in layer.named_parameters()}
+    x, gy = x.double().requires_grad_(train), gy.double()
+    act = nn.functional.gelu if case["act"] == "gelu" else torch.relu
+    loss = None
+    if kind == "linear":
+        rows = x.split(_row_counts(case, seed).tolist())
+        y = torch.cat([r @ par["weight"][e].t() + par["bias"][e] for e, r in enumerate(rows)])
+    else:
+        ids, score, loss = _exact_gate(case, x, par["gate.gate.weight"], par["gate.gate.bias"])
+        y = torch.zeros_like(x)
+        for e in range(experts):
+            token, slot = (ids == e).nonzero(as_tuple=True)
+            if kind == "custom":
+                w1, b1, w2, b2 = (par["experts.%d.%s" % (e, n)] for n in
+                                  ("fc1.weight", "fc1.bias", "fc2.weight", "fc2.bias"))
+            else:
+                w1, b1, w2, b2 = (par["experts.%s" % n][e] for n in
+                                  ("htoh4.weight", "htoh4.bias", "h4toh.weight", "h4toh.bias"))
+            out = act(x[token] @ w1.t() + b1) @ w2.t() + b2
+            y = y.index_add(0, token, out * score[token, slot, None])
+    if not train:
+        return y
+    torch.autograd.backward([y] if loss is None else [y, loss], [gy] if loss is None else [gy, None])
+    return {"y": y.detach(), "dx": x.grad, "grads": {n: p.grad for n, p in par.items()}}
 
 
 # ------------------------------------------------------------------------------ what it needs
