@@ -1,7 +1,9 @@
-// Host side of the tcgen05 grouped GEMM: tensor-map construction and dispatch.  The kernel
-// lives in grouped_gemm_kernel.cuh and is instantiated per element type in
-// grouped_gemm_bf16.cu / grouped_gemm_f16.cu.
+// Host side of the tcgen05 grouped GEMM: tensor-map construction and dispatch.  The kernels live
+// in pair_gemm_kernel.cuh (CTA pairs; every launch without an exchange) and
+// grouped_gemm_kernel.cuh (row modes with rows arriving from or leaving for other GPUs) and are
+// instantiated per element type in pair_gemm_*.cu / grouped_gemm_*.cu.
 #include "grouped_gemm_kernel.cuh"
+#include "pair_gemm_kernel.cuh"
 
 namespace fmoe {
 using namespace gg;
@@ -54,25 +56,72 @@ bool grouped_gemm_supported(int mode, int m, int n, int k, int num_groups) {
   return k % 64 == 0 && k >= 64;
 }
 
-cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
-  if (!grouped_gemm_supported(a.mode, a.m, a.n, a.k, a.num_groups)) return cudaErrorInvalidValue;
+namespace {
+
+// The CTA-pair kernel takes every launch in which no rows arrive from or leave for other GPUs: it
+// was the faster one at every size measured, from 16 rows (8 experts, 1024 -> 4096, GELU: 22.7
+// against 25.2 us) to 22528 (8 experts, 512 -> 2048, GELU: 79.6 against 101.2 us).  The
+// single-CTA kernel keeps the exchange, whose flags and send units count 128-row blocks.
+bool pair_applies(const GroupedGemmArgs& a) {
+  if (a.mode == kWgrad) return true;
+  if (a.send.enabled || a.gate.flags != nullptr || a.push_meta != nullptr || a.trace != nullptr) return false;
+  if (a.mode == kRowsNT) return a.epi == kEpiBiasAct;
+  return a.bias == nullptr && a.pre_out == nullptr &&
+         (a.act == kActNone || (a.epi == kEpiDAct && a.aux != nullptr));
+}
+
+cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
   CUtensorMap ta, tb;
   bool ok = true;
   if (a.mode == kRowsNT) {
-    ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, BM) &&
-         make_map_2d(&tb, a.dtype, a.b, a.k, static_cast<uint64_t>(a.num_groups) * a.n, BK, BN);
+    ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, pg::CTA_M) &&
+         make_map_2d(&tb, a.dtype, a.b, a.k, static_cast<uint64_t>(a.num_groups) * a.n, BK, pg::CTA_N);
   } else if (a.mode == kRowsNN) {
-    ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, BM) &&
+    ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, pg::CTA_M) &&
          make_map_2d(&tb, a.dtype, a.b, a.n, static_cast<uint64_t>(a.num_groups) * a.k, 64, BK);
   } else {
     ok = make_map_2d(&ta, a.dtype, a.a, a.m, a.rows_cap, 64, BK) &&
          make_map_2d(&tb, a.dtype, a.b, a.n, a.rows_cap, 64, BK);
   }
   if (!ok) return cudaErrorInvalidValue;
+  pg::Params p;
+  p.num_groups = a.num_groups;
+  p.m = a.m;
+  p.n = a.n;
+  p.k = a.k;
+  p.offs = a.offs;
+  p.out = a.out;
+  p.pre_out = a.pre_out;
+  p.bias = a.bias;
+  p.aux = a.aux;
+  p.accumulate = a.accumulate;
+  p.out_fp32 = a.out_fp32;
+  p.psum = a.mode == kWgrad ? a.psum : nullptr;
+  p.psrc = a.a;
+  p.status = a.status;
+  const int grid = (a.num_sms > 1 ? a.num_sms : 148) & ~1;
+  return a.dtype == kBF16 ? pg::launch_bf16(a.mode, a.act, ta, tb, p, grid, a.stream)
+                          : pg::launch_f16(a.mode, a.act, ta, tb, p, grid, a.stream);
+}
+
+}  // namespace
+
+cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
+  if (!grouped_gemm_supported(a.mode, a.m, a.n, a.k, a.num_groups)) return cudaErrorInvalidValue;
+  if (pair_applies(a)) return launch_pair_gemm(a);
+  CUtensorMap ta, tb;
+  bool ok = true;
+  if (a.mode == kRowsNT) {
+    ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, BM) &&
+         make_map_2d(&tb, a.dtype, a.b, a.k, static_cast<uint64_t>(a.num_groups) * a.n, BK, BN);
+  } else {
+    ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, BM) &&
+         make_map_2d(&tb, a.dtype, a.b, a.n, static_cast<uint64_t>(a.num_groups) * a.k, 64, BK);
+  }
+  if (!ok) return cudaErrorInvalidValue;
 
   KernelParams kp;
   kp.num_groups = a.num_groups;
-  kp.m = a.m;
   kp.n = a.n;
   kp.k = a.k;
   kp.offs = a.offs;
@@ -82,10 +131,6 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
   kp.aux = a.aux;
   kp.act = a.act;
   kp.epi = a.epi;
-  kp.accumulate = a.accumulate;
-  kp.out_fp32 = a.out_fp32;
-  kp.psum = (a.mode == kWgrad) ? a.psum : nullptr;
-  kp.psrc = a.a;
   kp.status = a.status;
   kp.push_meta = a.push_meta;
   kp.push_dst = a.push_dst;
@@ -98,10 +143,6 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
   kp.send = a.send;
   kp.gate = a.gate;
   kp.trace = a.trace;
-  if (a.mode == kWgrad) {
-    kp.send.enabled = 0;
-    kp.gate.flags = nullptr;
-  }
   if (kp.send.enabled && (kp.send.d % 8 != 0 || kp.send.item_prefix == nullptr ||
                           kp.send.item_count == nullptr)) {
     return cudaErrorInvalidValue;

@@ -1,0 +1,11 @@
+// f16 instantiations of the paired grouped GEMM kernel.
+#include "pair_gemm_kernel.cuh"
+
+namespace fmoe {
+namespace pg {
+cudaError_t launch_f16(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int grid,
+                        cudaStream_t stream) {
+  return launch_for_type<__half>(mode, act, ta, tb, p, grid, stream);
+}
+}  // namespace pg
+}  // namespace fmoe
