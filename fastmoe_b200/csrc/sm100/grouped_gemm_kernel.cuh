@@ -428,32 +428,36 @@ __device__ __forceinline__ void epilogue_tile_rows(const RowTile& rt, Packed32& 
     ptx::tmem_ld_32x32(rt.t_row, ra);
 #pragma unroll 1
     for (int pair = 0; pair < CHUNKS_PER_WARP / 2; ++pair) {
-      const int i = 2 * pair;
-      if (i >= rt.n_chunks) break;
-      ptx::tmem_ld_wait();
-      if (i + 1 < rt.n_chunks) {
-        ptx::tmem_ld_32x32(rt.t_row + (i + 1) * 32, rb);
-        if (rt.use_aux) load_pre_chunk(rt.pre_tile, i + 1, lane, sb);
-      } else if (!released) {
-        ptx::tc_fence_before_sync();
-        ptx::mbar_arrive(rt.empty_bar);
-        released = true;
+      {
+        const int i = 2 * pair;
+        if (i >= rt.n_chunks) break;
+        ptx::tmem_ld_wait();
+        if (i + 1 < rt.n_chunks) {
+          ptx::tmem_ld_32x32(rt.t_row + (i + 1) * 32, rb);
+          if (rt.use_aux) load_pre_chunk(rt.pre_tile, i + 1, lane, sb);
+        } else if (!released) {
+          ptx::tc_fence_before_sync();
+          ptx::mbar_arrive(rt.empty_bar);
+          released = true;
+        }
+        rows_chunk<T, ACT>(rt, i, with_pre, ra, side_first);
+        rows_send(rt, i);
       }
-      rows_chunk<T, ACT>(rt, i, with_pre, ra, side_first);
-      rows_send(rt, i);
-      const int i = 2 * pair + 1;
-      if (i >= rt.n_chunks) break;
-      ptx::tmem_ld_wait();
-      if (i + 1 < rt.n_chunks) {
-        ptx::tmem_ld_32x32(rt.t_row + (i + 1) * 32, ra);
-        if (rt.use_aux) load_pre_chunk(rt.pre_tile, i + 1, lane, side_first);
-      } else if (!released) {
-        ptx::tc_fence_before_sync();
-        ptx::mbar_arrive(rt.empty_bar);
-        released = true;
+      {
+        const int i = 2 * pair + 1;
+        if (i >= rt.n_chunks) break;
+        ptx::tmem_ld_wait();
+        if (i + 1 < rt.n_chunks) {
+          ptx::tmem_ld_32x32(rt.t_row + (i + 1) * 32, ra);
+          if (rt.use_aux) load_pre_chunk(rt.pre_tile, i + 1, lane, side_first);
+        } else if (!released) {
+          ptx::tc_fence_before_sync();
+          ptx::mbar_arrive(rt.empty_bar);
+          released = true;
+        }
+        rows_chunk<T, ACT>(rt, i, with_pre, rb, sb);
+        rows_send(rt, i);
       }
-      rows_chunk<T, ACT>(rt, i, with_pre, rb, sb);
-      rows_send(rt, i);
     }
   }
   if (!released) {
