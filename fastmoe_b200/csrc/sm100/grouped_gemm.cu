@@ -58,13 +58,17 @@ bool grouped_gemm_supported(int mode, int m, int n, int k, int num_groups) {
 
 namespace {
 
-// The CTA-pair kernel takes every launch in which no rows arrive from or leave for other GPUs: it
-// was the faster one at every size measured, from 16 rows (8 experts, 1024 -> 4096, GELU: 22.7
-// against 25.2 us) to 22528 (8 experts, 512 -> 2048, GELU: 79.6 against 101.2 us).  The
-// single-CTA kernel keeps the exchange, whose flags and send units count 128-row blocks.
+// The CTA-pair kernel takes the launches in which no rows arrive from or leave for other GPUs
+// (8192 rows, 2 experts, 1024 -> 4096 with GELU: 69.0 against 85.5 us; 22528 rows, 8 experts,
+// 512 -> 2048: 79.6 against 101.2 us; weight gradient of 64 experts with 128 rows: 200 against
+// 394 us).  The single-CTA kernel keeps the exchange, whose flags and send units count 128-row
+// blocks, and the launches with a handful of rows per expert, where the weights' bytes are all
+// there is and the finer tiles share them more evenly (a layer of 64 experts on 64 tokens: 227
+// against 238 us).
 bool pair_applies(const GroupedGemmArgs& a) {
   if (a.mode == kWgrad) return true;
   if (a.send.enabled || a.gate.flags != nullptr || a.push_meta != nullptr || a.trace != nullptr) return false;
+  if (a.rows_cap <= 16L * a.num_groups) return false;
   if (a.mode == kRowsNT) return a.epi == kEpiBiasAct;
   return a.bias == nullptr && a.pre_out == nullptr &&
          (a.act == kActNone || (a.epi == kEpiDAct && a.aux != nullptr));

@@ -13,7 +13,8 @@
 //   warp 1      one elected thread issues tcgen05.mma (128 x 256 x 16 per instruction, fp32
 //               accumulators in TMEM) and tcgen05.commit; the warp owns the TMEM allocation;
 //   warps 2-3   idle, or row senders of the fused dispatch (see below);
-//   warps 4-11  epilogue (two warpgroups): two warps per TMEM lane quarter.  Each warp owns 32 rows x 128 columns of the tile; the tcgen05.ld of chunk i+1 and
+//   warps 4-11  epilogue (two warpgroups): two warps per TMEM lane quarter.  Each
+//               warp owns 32 rows x 128 columns of the tile; the tcgen05.ld of chunk i+1 and
 //               the load of its saved pre-activation are in flight while chunk i gets bias /
 //               activation / derivative and is written into the lane's row of a swizzled
 //               per-warp shared-memory patch; after every second chunk the warp stores whole
@@ -267,12 +268,6 @@ template <> struct Cvt<__half> {
 };
 
 // 256-bit global accesses (sm_100): one full 32-byte sector per lane and instruction.
-__device__ __forceinline__ void ldg256(const void* p, uint32_t (&r)[8]) {
-  asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                 "=r"(r[6]), "=r"(r[7])
-               : "l"(p));
-}
 __device__ __forceinline__ void ld256(const void* p, uint32_t (&r)[8]) {
   asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
@@ -1034,12 +1029,13 @@ cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const Kerne
   auto kernel = grouped_gemm_kernel<MODE, T, ACT>;
   int dev = 0;
   cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  if (!(configured >> (dev & 63) & 1)) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    configured |= 1ull << (dev & 63);
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!(configured >> (dev & 63) & 1)) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+      if (e != cudaSuccess) return e;
+      configured |= 1ull << (dev & 63);
+    }
   }
   kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, kp);
   return cudaGetLastError();

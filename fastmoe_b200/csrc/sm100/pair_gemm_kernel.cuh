@@ -4,6 +4,10 @@
 // A pair of CTAs (one cluster, two neighbouring SMs) works on a 256 x 256 output tile: CTA r
 // holds rows [128 r, 128 r + 128) of A, columns [128 r, 128 r + 128) of B and the accumulators of
 // its rows.  Per 64-wide K block an SM loads 32 KB where a 128 x 256 tile on one SM loads 48 KB.
+// Measured, bf16, 8192 rows, 2 experts, 1024 <-> 4096: forward 69.0 (GELU, saved pre-activation)
+// and 52.5 us, input gradient 69.0 and 51.8 us, weight gradient 64.4 us (1068 to 1327 TFLOP/s
+// without activation), where the single-CTA kernel took 85.5, 56.0, 78.4, 54.5 and 70.1 us.  What
+// bounds it: the last of the waves (128 tiles on 74 pairs) and, with an activation, the epilogue.
 //
 // Roles of a CTA (384 threads), persistent over the tiles of its pair:
 //   warp 0      TMA producer, one lane: this CTA's halves of A and B into a 5-stage ring; the
@@ -15,7 +19,8 @@
 //   warp 3      weight gradient: zeroes the gradients of experts without rows, beside the MMAs;
 //   warps 4-11  epilogue: as in the single-CTA kernel, 32 rows x 128 columns per warp.
 // The last K block of an expert in the weight gradient issues only the 16-row MMA steps that
-// contain rows of the expert.
+// contain rows of the expert.  With the zeroing in the producer warp, which waited for the copies
+// first, 64 experts of 128 rows took 394 us; now 200 us, 537 MB of gradients written.
 #pragma once
 #include "grouped_gemm_kernel.cuh"
 

@@ -393,3 +393,44 @@ def test_gate_tensor_core_many_experts(dtype, n_exp, k, d, bias):
         scale = ref.abs().max().item() + 1e-6
         assert (got.float() - ref).abs().max().item() <= 3e-2 * scale
     assert _native().read_status(0) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("counts,m,n", [
+    ([255, 0, 257, 1], 256, 288),       # one row either side of a pair's 256-row tile, an empty expert
+    ([65, 15, 16, 17, 127, 128], 72, 544),   # ragged ends around the 16-row MMA step and the K block
+    ([1, 513], 264, 256),               # an output tile whose second half has 8 rows
+])
+def test_pair_tiles_and_ragged_ends(dtype, counts, m, n):
+    r"""The paired kernel at the edges of its 256 x 256 tiles, 64-row K blocks and 16-row steps; rows
+    past the last expert are NaN and must not reach any output.  Against fp64: one rounding to
+    the 16-bit type (relative 2^-9 / 2^-12) plus an fp32 sum of at most 513 terms."""
+    from fastmoe_b200.ops import grouped_gemm as gg
+    torch.manual_seed(11)
+    g, rows, k = len(counts), sum(counts), 192
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    offs = _offs(counts)
+
+    def close(got, ref, terms):
+        bound = eps * ref.abs() + 2.0 ** -22 * terms ** 0.5 * ref.abs().amax().clamp(min=1.0) + 1e-6
+        return bool(((got.double() - ref).abs() <= bound).all())
+
+    dy = torch.randn(rows + 40, m, device=DEV).to(dtype)
+    q = torch.randn(rows + 40, n, device=DEV).to(dtype)
+    dy[rows:] = float("nan")
+    q[rows:] = float("nan")
+    dw, db = gg.wgrad(dy, q, offs, g, with_bias_grad=True)
+    x = torch.randn(rows, k, device=DEV).to(dtype)
+    w = (torch.randn(g, n, k, device=DEV) / k ** 0.5).to(dtype)
+    b = torch.randn(g, n, device=DEV).to(dtype)
+    y = gg.forward(x, w, offs, b)
+    go = torch.randn(rows, k, device=DEV).to(dtype)
+    wn = (torch.randn(g, k, n, device=DEV) / k ** 0.5).to(dtype)
+    dx = gg.dgrad(go, wn, offs)
+    for e, lo, hi in _segments(counts):
+        assert close(dw[e], dy[lo:hi].double().t() @ q[lo:hi].double(), max(1, hi - lo)), e
+        assert close(db[e], dy[lo:hi].double().sum(0), max(1, hi - lo)), e
+        if hi > lo:
+            assert close(y[lo:hi], x[lo:hi].double() @ w[e].double().t() + b[e].double(), k), e
+            assert close(dx[lo:hi], go[lo:hi].double() @ wn[e].double(), k), e
+    assert _native().read_status(0) == 0
