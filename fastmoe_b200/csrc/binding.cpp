@@ -302,8 +302,16 @@ bool grouped_gemm_supported(int64_t mode, int64_t m, int64_t n, int64_t k, int64
                                       static_cast<int>(groups));
 }
 
+// Whether the weight-gradient mode of simt_grouped_gemm can return the column sums of `a` too.
+bool simt_column_sums(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& out) {
+  return a.scalar_type() == torch::kFloat && a.is_contiguous() && b.is_contiguous() && out.is_contiguous() &&
+         fmoe::sgemm_applies(fmoe::kWgrad, static_cast<int>(out.size(0)), static_cast<int>(a.size(1)),
+                             static_cast<int>(b.size(1)), 0, a.data_ptr(), b.data_ptr(), nullptr, out.data_ptr());
+}
+
 void simt_grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor offs,
-                       torch::Tensor out, c10::optional<torch::Tensor> bias) {
+                       torch::Tensor out, c10::optional<torch::Tensor> bias,
+                       c10::optional<torch::Tensor> psum) {
   check_cuda_contig(a, "a");
   check_cuda_contig(b, "b");
   check_cuda_contig(out, "out");
@@ -319,6 +327,17 @@ void simt_grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Te
   }
   const void* bias_ptr = nullptr;
   if (bias.has_value() && bias->defined()) bias_ptr = bias->data_ptr();
+  if (psum.has_value() && psum->defined()) {
+    // the column sums of `a` come with the fp32 kernel: the caller asked simt_column_sums first
+    check_cuda_contig(*psum, "psum");
+    TORCH_CHECK(mode == fmoe::kWgrad && psum->scalar_type() == torch::kFloat &&
+                    psum->numel() == static_cast<int64_t>(groups) * m && simt_column_sums(a, b, out),
+                "simt_grouped_gemm: no column sums for these operands");
+    FMOE_CUDA_CHECK(fmoe::launch_sgemm(static_cast<int>(mode), groups, a.size(0), m, n, k, a.data_ptr<float>(),
+                                       b.data_ptr<float>(), offs.data_ptr<int>(), nullptr,
+                                       out.data_ptr<float>(), psum->data_ptr<float>(), cur_stream()));
+    return;
+  }
   FMOE_CUDA_CHECK(fmoe::launch_simt_grouped_gemm(static_cast<int>(mode), elem_code(a), groups,
                                                  a.size(0), m, n, k, a.data_ptr(), b.data_ptr(),
                                                  offs.data_ptr<int>(), bias_ptr, out.data_ptr(),
@@ -511,7 +530,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("accumulate") = false, py::arg("psum") = py::none());
   m.def("grouped_gemm_supported", &grouped_gemm_supported);
   m.def("simt_grouped_gemm", &simt_grouped_gemm, py::arg("mode"), py::arg("a"), py::arg("b"),
-        py::arg("offs"), py::arg("out"), py::arg("bias") = py::none());
+        py::arg("offs"), py::arg("out"), py::arg("bias") = py::none(), py::arg("psum") = py::none());
+  m.def("simt_column_sums", &simt_column_sums);
   m.def("scatter_rows", &scatter_rows, py::arg("src"), py::arg("idx"), py::arg("rank"),
         py::arg("base"), py::arg("scale"), py::arg("k"), py::arg("dst"),
         py::arg("row_slot") = py::none());

@@ -766,8 +766,8 @@ __device__ __forceinline__ int group_of_row(const int* offs, int num_groups, int
   return lo;
 }
 
-// Shared-memory tiled SIMT GEMM for the reference-precision types (fp32, fp64) and for 16-bit
-// shapes the tensor-core kernel does not take.  One CTA of 256 threads computes a 64 x 64 tile
+// Shared-memory tiled SIMT GEMM for fp64, for fp32 with rows that are not 16-byte aligned (sgemm.cu
+// takes the others) and for 16-bit shapes the tensor-core kernel does not take.  One CTA of 256 threads computes a 64 x 64 tile
 // of C = A B with a K step of 16; every thread owns a 4 x 4 block of the tile and accumulates in
 // fp32 (fp64 for doubles).  The three products of a grouped linear differ only in where A(i, kk)
 // and B(kk, j) live:
@@ -780,7 +780,7 @@ constexpr int kSimtK = 16;
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
-simt_tiled_kernel(int num_groups, int m, int n, int k, const T* __restrict__ a, const T* __restrict__ b,
+simt_tiled_kernel(int num_groups, long rows_cap, int m, int n, int k, const T* __restrict__ a, const T* __restrict__ b,
                   const int* __restrict__ offs, const T* __restrict__ bias, T* __restrict__ out) {
   using A = typename Acc<T>::type;
   __shared__ A As[kSimtK][kSimtTile + 4];
@@ -806,7 +806,17 @@ simt_tiled_kernel(int num_groups, int m, int n, int k, const T* __restrict__ a, 
       }
       piece -= pieces;
     }
-    if (!found) return;
+    if (!found) {
+      // no piece left: zero the rows past the last expert, so that what is applied to the whole
+      // buffer afterwards meets no stale bits
+      const long r0 = static_cast<long>(offs[num_groups]) + static_cast<long>(piece) * kSimtTile;
+      for (int it = threadIdx.x; it < kSimtTile * kSimtTile; it += blockDim.x) {
+        const long r = r0 + it / kSimtTile;
+        const int j = j0 + it % kSimtTile;
+        if (r < rows_cap && j < n) stv<T>(out, r * n + j, 0);
+      }
+      return;
+    }
     row_base = offs[g];
     i0 = piece * kSimtTile;
     rows_i = offs[g + 1] - row_base;
@@ -888,14 +898,14 @@ cudaError_t simt_typed(int mode, int num_groups, long rows_cap, int m, int n, in
   const unsigned nt = (n + kSimtTile - 1) / kSimtTile;
   if (mode == 2) {
     dim3 grid((m + kSimtTile - 1) / kSimtTile, nt, num_groups);
-    simt_tiled_kernel<T, 2><<<grid, 256, 0, stream>>>(num_groups, m, n, k, ap, bp, offs, biasp, op);
+    simt_tiled_kernel<T, 2><<<grid, 256, 0, stream>>>(num_groups, rows_cap, m, n, k, ap, bp, offs, biasp, op);
   } else {
     if (rows_cap == 0) return cudaSuccess;
     dim3 grid(static_cast<unsigned>((rows_cap + kSimtTile - 1) / kSimtTile + num_groups), nt);
     if (mode == 0) {
-      simt_tiled_kernel<T, 0><<<grid, 256, 0, stream>>>(num_groups, m, n, k, ap, bp, offs, biasp, op);
+      simt_tiled_kernel<T, 0><<<grid, 256, 0, stream>>>(num_groups, rows_cap, m, n, k, ap, bp, offs, biasp, op);
     } else {
-      simt_tiled_kernel<T, 1><<<grid, 256, 0, stream>>>(num_groups, m, n, k, ap, bp, offs, biasp, op);
+      simt_tiled_kernel<T, 1><<<grid, 256, 0, stream>>>(num_groups, rows_cap, m, n, k, ap, bp, offs, biasp, op);
     }
   }
   return cudaGetLastError();
@@ -1138,7 +1148,13 @@ cudaError_t launch_simt_grouped_gemm(int mode, int elem, int num_groups, long ro
   switch (elem) {
     case 0: return simt_typed<__nv_bfloat16>(mode, num_groups, rows_cap, m, n, k, a, b, offs, bias, out, stream);
     case 1: return simt_typed<__half>(mode, num_groups, rows_cap, m, n, k, a, b, offs, bias, out, stream);
-    case 2: return simt_typed<float>(mode, num_groups, rows_cap, m, n, k, a, b, offs, bias, out, stream);
+    case 2:
+      if (sgemm_applies(mode, num_groups, m, n, k, a, b, bias, out)) {
+        return launch_sgemm(mode, num_groups, rows_cap, m, n, k, static_cast<const float*>(a),
+                            static_cast<const float*>(b), offs, static_cast<const float*>(bias),
+                            static_cast<float*>(out), nullptr, stream);
+      }
+      return simt_typed<float>(mode, num_groups, rows_cap, m, n, k, a, b, offs, bias, out, stream);
     case 3: return simt_typed<double>(mode, num_groups, rows_cap, m, n, k, a, b, offs, bias, out, stream);
     default: return cudaErrorInvalidValue;
   }

@@ -82,9 +82,17 @@ cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, co
                             cudaStream_t stream);
 
 // Reference-precision grouped GEMM for fp32 / fp64 and for shapes the tensor-core kernel
-// does not take (elem: 0 bf16, 1 f16, 2 f32, 3 f64).  Same modes as the tcgen05 kernel.
+// does not take (elem: 0 bf16, 1 f16, 2 f32, 3 f64).  Same modes as the tcgen05 kernel; the row
+// modes zero the rows past the last expert.
 cudaError_t launch_simt_grouped_gemm(int mode, int elem, int num_groups, long rows_cap, int m, int n,
                                      int k, const void* a, const void* b, const int* offs,
                                      const void* bias, void* out, cudaStream_t stream);
+
+// fp32 with 16-byte aligned rows (see sgemm.cu).  `psum` (weight gradient, optional): fp32
+// [num_groups, m] column sums of `a` per group.
+bool sgemm_applies(int mode, int num_groups, int m, int n, int k, const void* a, const void* b, const void* bias,
+                   const void* out);
+cudaError_t launch_sgemm(int mode, int num_groups, long rows_cap, int m, int n, int k, const float* a, const float* b,
+                         const int* offs, const float* bias, float* out, float* psum, cudaStream_t stream);
 
 }  // namespace fmoe

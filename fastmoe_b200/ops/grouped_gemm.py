@@ -95,7 +95,6 @@ def forward(x, weight, offs, bias=None, act=None, want_pre=False):
             pre = out
     else:
         nat.simt_grouped_gemm(MODE_NT, x, weight, offs, out, bias)
-        _zero_tail(out, offs)
         if want_pre:
             pre = out
         if code != 0:
@@ -123,7 +122,6 @@ def dgrad(dy, weight, offs, pre=None, act=None):
         out = out * _torch_act_grad(pre, act)
     else:
         nat.simt_grouped_gemm(MODE_NN, dy, weight, offs, out, None)
-        _zero_tail(out, offs)
         if code:
             out = out * _torch_act_grad(pre, act)
     return out
@@ -139,7 +137,8 @@ def wgrad(dy, x, offs, groups, out=None, accumulate=False, with_bias_grad=False)
     """
     nat = native.get()
     m, n = dy.shape[1], x.shape[1]
-    if out is None:
+    fresh = out is None
+    if fresh:
         out = torch.empty(groups, m, n, dtype=dy.dtype, device=dy.device)
         accumulate = False
     db = None
@@ -149,13 +148,15 @@ def wgrad(dy, x, offs, groups, out=None, accumulate=False, with_bias_grad=False)
         nat.grouped_gemm(MODE_WGRAD, _aligned(dy), _aligned(x), offs, out, None, None, None, 0, 0,
                          accumulate, db)
     else:
-        tmp = torch.empty(groups, m, n, dtype=dy.dtype, device=dy.device)
-        nat.simt_grouped_gemm(MODE_WGRAD, dy, x, offs, tmp, None)
+        tmp = out if fresh else torch.empty(groups, m, n, dtype=dy.dtype, device=dy.device)
+        if with_bias_grad and nat.simt_column_sums(dy, x, tmp):
+            db = torch.empty(groups, m, dtype=dy.dtype, device=dy.device)
+        nat.simt_grouped_gemm(MODE_WGRAD, dy, x, offs, tmp, None, db)
         if accumulate:
             out += tmp
-        else:
+        elif not fresh:
             out.copy_(tmp)
-        if with_bias_grad:
+        if with_bias_grad and db is None:
             db = bias_grad(dy, offs)
     return (out, db) if with_bias_grad else out
 
@@ -177,8 +178,8 @@ def bias_grad(dy, offs, dtype=None):
 
 
 def _zero_tail(out, offs):
-    r"""The SIMT kernel leaves rows past the last expert segment unwritten (the buffer comes from
-    ``torch.empty``): zero them, without a host read, so that an activation applied to the whole
+    r"""The tensor-core kernel leaves rows past the last expert segment unwritten (the buffer comes
+    from ``torch.empty``): zero them, without a host read, so that what is applied to the whole
     buffer never meets NaN bit patterns."""
     rows = torch.arange(out.shape[0], device=out.device)
     out.masked_fill_((rows >= offs[-1])[:, None], 0)

@@ -434,3 +434,38 @@ def test_pair_tiles_and_ragged_ends(dtype, counts, m, n):
             assert close(y[lo:hi], x[lo:hi].double() @ w[e].double().t() + b[e].double(), k), e
             assert close(dx[lo:hi], go[lo:hi].double() @ wn[e].double(), k), e
     assert _native().read_status(0) == 0
+
+
+@pytest.mark.parametrize("counts,k,n", [([64, 0, 65, 1, 127], 20, 132), ([3], 4, 4), ([0, 0], 16, 128),
+                                        ([1] * 40 + [200], 36, 260), ([130, 70], 18, 128)])
+def test_fp32_tiles_tail_and_column_sums(counts, k, n):
+    r"""The aligned fp32 kernel (and, with k = 18, the general one) at the edges of its 64 x 128 x 16
+    tiles, with more experts than a warp has lanes, against fp64: an fp32 sum of t terms is off by
+    at most t * 2^-24 times the sum of the absolute products.  Rows past the last expert come back
+    zero although the buffers around them hold NaN."""
+    from fastmoe_b200.ops import grouped_gemm as gg
+    torch.manual_seed(12)
+    g, rows = len(counts), sum(counts)
+    offs = _offs(counts)
+    x = torch.randn(rows + 70, k, device=DEV)
+    go = torch.randn(rows + 70, n, device=DEV)
+    x[rows:] = float("nan")
+    go[rows:] = float("nan")
+    w, b = torch.randn(g, n, k, device=DEV), torch.randn(g, n, device=DEV)
+    torch.full((rows + 70, max(n, k)), float("nan"), device=DEV)   # stale bits for the allocator to hand out
+    y = gg.forward(x, w, offs, b)
+    dx = gg.dgrad(go, w, offs)
+    dw, db = gg.wgrad(go[:rows].contiguous(), x[:rows].contiguous(), offs, g, with_bias_grad=True)
+    assert not y[rows:].any() and not dx[rows:].any()
+
+    def close(got, a, bb, extra=0.0):
+        ref = a.double() @ bb.double() + extra
+        bound = (a.shape[1] + 2) * 2.0 ** -24 * (a.double().abs() @ bb.double().abs() + abs(extra)) + 1e-12
+        return bool(((got.double() - ref).abs() <= bound).all())
+
+    for e, lo, hi in _segments(counts):
+        if hi > lo:
+            assert close(y[lo:hi], x[lo:hi], w[e].t(), b[e].double()), e
+            assert close(dx[lo:hi], go[lo:hi], w[e]), e
+        assert close(dw[e], go[lo:hi].t(), x[lo:hi]), e
+        assert close(db[e][None], torch.ones(1, hi - lo, device=DEV), go[lo:hi]), e
