@@ -2,12 +2,18 @@
 // of fp32 (the tensor cores' tf32 would drop 13 bits of the inputs).
 //
 // One CTA of 128 threads computes a 64 x 128 tile with a K step of 16; a thread owns 8 x 8 outputs
-// and adds its products in ascending k, one fused multiply-add each.  Bound by the FMA pipe: 64
-// FMAs per thread and k against 4 shared-memory loads of 16 bytes; the next K step travels from
-// global memory to registers during the math and into the other of two buffers after it.  64 rows
-// per tile, and not 128, because an expert's last tile is ragged: 4096 rows on 8 experts with 512
-// outputs are 272 tiles for 148 SMs, with 128 x 128 they would be 144 and many nearly empty.
+// and adds its products in ascending k, one fused multiply-add each (packed two to an instruction:
+// every lane rounds like the scalar one).  Bound by the FMA pipe: 64 FMAs per thread and k against
+// 4 shared-memory loads of 16 bytes; the next K step travels from global memory to registers
+// during the math and into the other of two buffers after it.  64 rows per tile, and not 128,
+// because an expert's last tile is ragged: 4096 rows on 8 experts with 512 outputs are 272 tiles
+// for 148 SMs, with 128 x 128 they would be 144, many of them nearly empty.
+// Measured, 16384 rows, 4 experts, 1024 <-> 2048: 49 to 53 TFLOP/s (43 to 48 with scalar FMAs);
+// 4096 rows, 8 experts, 512 <-> 2048: forward 203 and 227, input gradient 192 and 218, weight
+// gradient with the bias gradient 171 us, where the general kernel took 437, 347 and 283 us on
+// average and the bias gradient a dozen more launches.
 // Operands need 16-byte aligned rows; the general kernel of routing.cu takes the rest.
+#include "ptx.cuh"
 #include "routing.cuh"
 
 namespace fmoe {
@@ -27,7 +33,7 @@ __device__ __forceinline__ float4 ld4(const float* p, bool ok) {
 // Modes as in GemmMode: 0 rows x weight^T, 1 rows x weight, 2 weight gradient (`psum`, optional:
 // [num_groups, m] column sums of `a` per group, formed by the CTAs of the first column block).
 template <int MODE>
-__global__ void __launch_bounds__(THREADS, 4)
+__global__ void __launch_bounds__(THREADS, MODE == 1 ? 4 : 3)   // 3: 168 registers, nothing spilled
 sgemm_kernel(int num_groups, long rows_cap, int m, int n, int k, const float* __restrict__ a, const float* __restrict__ b,
              const int* __restrict__ offs, const float* __restrict__ bias, float* __restrict__ out,
              float* __restrict__ psum) {
@@ -144,11 +150,11 @@ sgemm_kernel(int num_groups, long rows_cap, int m, int n, int k, const float* __
   };
 
   const int tx = tid & 15, ty = tid >> 4;   // columns tx * 4 and 64 + tx * 4, rows ty * 4 and 32 + ty * 4
-  float acc[8][8];
+  ptx::f32x2 acc[8][4];   // outputs in pairs of neighbouring columns
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
 #pragma unroll
-    for (int v = 0; v < 8; ++v) acc[u][v] = 0.f;
+    for (int v = 0; v < 4; ++v) acc[u][v] = 0ull;
   }
   const bool sums = MODE == 2 && psum != nullptr && blockIdx.y == 0;
   float col_sum = 0.f;   // of column i0 + tid (threads 0 .. 63), one partial sum per K step
@@ -164,15 +170,17 @@ sgemm_kernel(int num_groups, long rows_cap, int m, int n, int k, const float* __
     if (more) load(kk0 + TK);
 #pragma unroll
     for (int kk = 0; kk < TK; ++kk) {
-      float fa[8], fb[8];
-      *reinterpret_cast<float4*>(fa) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 4]);
-      *reinterpret_cast<float4*>(fa + 4) = *reinterpret_cast<const float4*>(&As[buf][kk][32 + ty * 4]);
-      *reinterpret_cast<float4*>(fb) = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 4]);
-      *reinterpret_cast<float4*>(fb + 4) = *reinterpret_cast<const float4*>(&Bs[buf][kk][64 + tx * 4]);
+      const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 4]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][kk][32 + ty * 4]);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&Bs[buf][kk][tx * 4]);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&Bs[buf][kk][64 + tx * 4]);
+      const float fa[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const ptx::f32x2 fb[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
+        const ptx::f32x2 aa = ptx::pack2(fa[u], fa[u]);
 #pragma unroll
-        for (int v = 0; v < 8; ++v) acc[u][v] = fmaf(fa[u], fb[v], acc[u][v]);
+        for (int v = 0; v < 4; ++v) acc[u][v] = ptx::fma2(aa, fb[v], acc[u][v]);
       }
     }
     if (sums && tid < TM) {
@@ -199,10 +207,12 @@ sgemm_kernel(int num_groups, long rows_cap, int m, int n, int k, const float* __
       if (i >= rows_i) continue;
       const long row = MODE == 2 ? static_cast<long>(g) * m + i : static_cast<long>(row_base) + i;
       float4 w;
-      w.x = acc[u][v4 * 4 + 0] + bv.x;
-      w.y = acc[u][v4 * 4 + 1] + bv.y;
-      w.z = acc[u][v4 * 4 + 2] + bv.z;
-      w.w = acc[u][v4 * 4 + 3] + bv.w;
+      ptx::unpack2(acc[u][v4 * 2], w.x, w.y);
+      ptx::unpack2(acc[u][v4 * 2 + 1], w.z, w.w);
+      w.x += bv.x;
+      w.y += bv.y;
+      w.z += bv.z;
+      w.w += bv.w;
       *reinterpret_cast<float4*>(out + row * n + j) = w;
     }
   }
