@@ -388,6 +388,87 @@ void combine_bwd(torch::Tensor dout, torch::Tensor rows, torch::Tensor idx, torc
                                            dscore.data_ptr(), cur_stream()));
 }
 
+// ------------------------------------------------------------------------------ whole layer
+// One GPU, both expert linears with a fused activation: the launches of a layer's forward, and of
+// its backward, issued by one call each.  For a small layer the calls from Python between the
+// kernels, and not the kernels, were what a training step waited for.
+torch::Tensor aligned32(const torch::Tensor& t) {
+  torch::Tensor c = t.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 32 == 0 ? c : c.clone();
+}
+
+bool moe_mlp_supported(int64_t experts, int64_t d, int64_t h) {
+  const int g = static_cast<int>(experts), id = static_cast<int>(d), ih = static_cast<int>(h);
+  return d % 64 == 0 && h % 64 == 0 && fmoe::grouped_gemm_supported(fmoe::kRowsNT, 0, ih, id, g) &&
+         fmoe::grouped_gemm_supported(fmoe::kRowsNT, 0, id, ih, g);
+}
+
+// {out, xs, pre (empty when not kept), a, ys, rank, offs, score in the layer's type, idx}
+std::vector<torch::Tensor> moe_mlp_forward(torch::Tensor x_in, torch::Tensor idx_in, torch::Tensor score_in,
+                                           torch::Tensor w1_in, torch::Tensor b1_in, torch::Tensor w2_in,
+                                           torch::Tensor b2_in, int64_t act, bool keep) {
+  c10::cuda::CUDAGuard guard(x_in.device());
+  const torch::Tensor x = x_in.contiguous();
+  const torch::Tensor idx = idx_in.contiguous().view({-1});
+  const torch::Tensor score = score_in.reshape({-1}).to(x.scalar_type()).contiguous();
+  const torch::Tensor w1 = aligned32(w1_in), b1 = aligned32(b1_in), w2 = aligned32(w2_in), b2 = aligned32(b2_in);
+  const int64_t groups = w1.size(0), h = w1.size(1), d = w1.size(2), rows = idx.numel(), k = rows / x.size(0);
+  auto r = route(idx, groups, true);
+  const torch::Tensor rank = r[1], offs = r[2];
+  auto xs = torch::empty({rows, d}, x.options());
+  scatter_rows(x, idx, rank, offs, c10::nullopt, k, xs, c10::nullopt);
+  auto a = torch::empty({rows, h}, x.options());
+  c10::optional<torch::Tensor> pre;
+  if (keep && act != fmoe::kActNone) {
+    pre = torch::empty({((rows + 127) / 128 + groups) * ((h + 255) / 256) * (128 * 256)}, x.options());
+  }
+  grouped_gemm(fmoe::kRowsNT, xs, w1, offs, a, b1, pre, c10::nullopt, act, fmoe::kEpiBiasAct, false, c10::nullopt);
+  auto ys = torch::empty({rows, d}, x.options());
+  grouped_gemm(fmoe::kRowsNT, a, w2, offs, ys, b2, c10::nullopt, c10::nullopt, fmoe::kActNone, fmoe::kEpiBiasAct,
+               false, c10::nullopt);
+  auto out = torch::empty_like(x);
+  gather_combine(ys, idx, rank, offs, score, k, out);
+  return {out, xs, pre.has_value() ? *pre : torch::Tensor(), a, ys, rank, offs, score, idx};
+}
+
+// {dx, dscore, dw1, db1, dw2, db2}; what `need_*` leaves out is empty.
+std::vector<torch::Tensor> moe_mlp_backward(torch::Tensor dout_in, torch::Tensor xs, c10::optional<torch::Tensor> pre,
+                                            torch::Tensor a, torch::Tensor ys, torch::Tensor rank, torch::Tensor offs,
+                                            torch::Tensor score, torch::Tensor idx, torch::Tensor w1_in,
+                                            torch::Tensor w2_in, int64_t act, bool need_dx, bool need_w1, bool need_w2) {
+  c10::cuda::CUDAGuard guard(xs.device());
+  const torch::Tensor dout = dout_in.contiguous();
+  const torch::Tensor w1 = aligned32(w1_in), w2 = aligned32(w2_in);
+  const int64_t groups = w1.size(0), h = w1.size(1), d = w1.size(2), n_tok = dout.size(0), k = idx.numel() / n_tok;
+  auto dys = torch::empty_like(ys);
+  auto dscore = torch::empty_like(score);
+  combine_bwd(dout, ys, idx, rank, offs, score, k, dys, dscore);
+  torch::Tensor dw1, db1, dw2, db2, dx;
+  if (need_w2) {
+    dw2 = torch::empty({groups, d, h}, xs.options());
+    db2 = torch::empty({groups, d}, xs.options());
+    grouped_gemm(fmoe::kWgrad, dys, a, offs, dw2, c10::nullopt, c10::nullopt, c10::nullopt, 0, 0, false, db2);
+  }
+  if (need_dx || need_w1) {
+    auto da = torch::empty_like(a);
+    grouped_gemm(fmoe::kRowsNN, dys, w2, offs, da, c10::nullopt, c10::nullopt, pre, pre.has_value() ? act : 0,
+                 pre.has_value() ? fmoe::kEpiDAct : fmoe::kEpiBiasAct, false, c10::nullopt);
+    if (need_w1) {
+      dw1 = torch::empty({groups, h, d}, xs.options());
+      db1 = torch::empty({groups, h}, xs.options());
+      grouped_gemm(fmoe::kWgrad, da, xs, offs, dw1, c10::nullopt, c10::nullopt, c10::nullopt, 0, 0, false, db1);
+    }
+    if (need_dx) {
+      auto dxs = torch::empty_like(xs);
+      grouped_gemm(fmoe::kRowsNN, da, w1, offs, dxs, c10::nullopt, c10::nullopt, c10::nullopt, 0, fmoe::kEpiBiasAct,
+                   false, c10::nullopt);
+      dx = torch::empty({n_tok, d}, xs.options());
+      gather_combine(dxs, idx, rank, offs, c10::nullopt, k, dx);
+    }
+  }
+  return {dx, dscore, dw1, db1, dw2, db2};
+}
+
 torch::Tensor colsum(torch::Tensor x, torch::Tensor offs) {
   check_cuda_contig(x, "x");
   c10::cuda::CUDAGuard guard(x.device());
@@ -538,6 +619,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gather_combine", &gather_combine);
   m.def("combine_bwd", &combine_bwd);
   m.def("colsum", &colsum);
+  m.def("moe_mlp_supported", &moe_mlp_supported);
+  m.def("moe_mlp_forward", &moe_mlp_forward);
+  m.def("moe_mlp_backward", &moe_mlp_backward);
   m.def("gate_topk_softmax", &gate_topk_softmax);
   m.def("gate_topk_softmax_bwd", &gate_topk_softmax_bwd);
   m.def("gate_fused_supported", &gate_fused_supported);

@@ -172,12 +172,54 @@ def moe_mlp_local(x, gate_idx, gate_score, w1, b1, w2, b2, activation):
     return _Combine.apply(ys, score, idx, rank, offs, k)
 
 
+class _MoEMLP(Function):
+    r"""The whole single-GPU layer behind the gate as one node: :class:`_Dispatch`,
+    :class:`_ExpertMLP` and :class:`_Combine` with their launches issued by one native call per
+    direction.  With ``keep`` false (nothing will be differentiated) the pre-activation is not
+    written."""
+
+    @staticmethod
+    def forward(ctx, x, score, w1, b1, w2, b2, idx, act, keep):
+        out, xs, pre, a, ys, rank, offs, score16, slots = native.get().moe_mlp_forward(
+            x, idx, score, w1, b1, w2, b2, act, keep)
+        if keep:
+            ctx.save_for_backward(xs, pre, a, ys, rank, offs, score16, slots, w1, w2)
+        ctx.act = act
+        ctx.score_like = score.shape, score.dtype
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        xs, pre, a, ys, rank, offs, score16, slots, w1, w2 = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        dx, dscore, dw1, db1, dw2, db2 = native.get().moe_mlp_backward(
+            dout, xs, pre, a, ys, rank, offs, score16, slots, w1, w2, ctx.act,
+            need[0], need[2] or need[3], need[4] or need[5])
+        shape, dtype = ctx.score_like
+        return (dx, dscore.to(dtype).view(shape) if need[1] else None, dw1, db1, dw2, db2, None, None, None)
+
+
+def _native_layer_ok(layer, x, gate_idx):
+    r"""Whether :class:`_MoEMLP` takes the call: an activation the GEMM epilogue knows, shapes of the
+    tensor-core kernel, at least one row, and nobody who wants to look between the launches."""
+    act = activation_kind(layer.experts.activation)
+    return (act is not None and x.dim() == 2 and x.shape[0] > 0 and gate_idx.shape[1] > 0
+            and gate_idx.shape[0] == x.shape[0] and gate_idx.dtype == torch.int64
+            and not config.nvtx_enabled() and not config.debug_bounds()
+            and native.get().moe_mlp_supported(layer.num_expert, layer.d_model, layer.d_hidden))
+
+
 def moe_mlp_forward(layer, x, gate_idx, gate_score):
     r"""``[B, d] → [B, d]`` for one ``FMoETransformerMLP`` call on the GPU."""
     if layer.world_size > 1 or _forced_ep():
         from ..parallel import symm
         return symm.moe_mlp_forward(layer, x, gate_idx, gate_score)
     nat = native.get()
+    if _native_layer_ok(layer, x, gate_idx):
+        e = layer.experts
+        args = (x, gate_score, e.htoh4.weight, e.htoh4.bias, e.h4toh.weight, e.h4toh.bias)
+        keep = torch.is_grad_enabled() and any(t.requires_grad for t in args)
+        return _MoEMLP.apply(*args, gate_idx, gg.ACT_CODES[activation_kind(e.activation)], keep)
     k = gate_idx.shape[1]
     idx = gate_idx.contiguous().view(-1)
     score = gate_score.reshape(-1).to(x.dtype)
