@@ -6,14 +6,19 @@
 // All kernels are deterministic: no result depends on the order in which atomics land.
 #include "routing.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 namespace fmoe {
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kRouteThreads = 1024;
 constexpr int kRouteSmemLimit = 200 * 1024;
+constexpr int kRouteCluster = 8;
+constexpr int kRouteClusterSlots = 65536;
 
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
@@ -24,16 +29,21 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // CTA b owns the contiguous slot range [b * cta_slots, (b + 1) * cta_slots), warp w of it the
 // sub-range [w * chunk, (w + 1) * chunk): pass 1 builds per-warp histograms, the CTA turns them
 // into exclusive prefixes over warps, pass 2 hands every slot its rank.  Within a warp slots
-// are visited in order, 32 at a time.  One CTA does everything in one launch.  For many slots
-// the work is spread over several CTAs and two launches: the first (`part_out`) only writes
-// every CTA's per-expert totals, the second (`part_in`) starts each CTA's prefixes at the sum
-// of the totals of the CTAs before it, so ranks stay those of a single ordered scan.
+// are visited in order, 32 at a time.  The chain of these steps is what bounds the kernel (a
+// match of 32 keys and an update of shared memory that the next step waits for), so up to
+// kRouteClusterSlots slots are spread over a cluster of eight CTAs, which exchange their
+// per-expert totals through distributed shared memory in the one launch: 16384 slots took 19 us
+// on one CTA.  For more slots the work is spread over more CTAs and two launches: the first
+// (`part_out`) only writes every CTA's per-expert totals, the second (`part_in`) starts each CTA's
+// prefixes at the sum of the totals of the CTAs before it.  Ranks are always those of a single
+// ordered scan.
 __global__ void __launch_bounds__(kRouteThreads, 1)
-route_kernel(const int64_t* __restrict__ idx, int n_slots, int tot, int nw, int cta_slots,
+route_kernel(const int64_t* __restrict__ idx, int n_slots, int tot, int nw, int cta_slots, int in_cluster,
              const int* __restrict__ part_in, int* __restrict__ part_out, int* __restrict__ counts,
              int* __restrict__ rank, int* __restrict__ offs, int* __restrict__ pos) {
-  extern __shared__ int hist[];  // [nw][tot], then [tot + 1] expert offsets when `pos` is wanted
+  extern __shared__ int hist[];  // [nw][tot], [tot + 1] expert offsets; in a cluster [tot] totals of this CTA
   int* eoff = hist + nw * tot;
+  int* mine = in_cluster ? eoff + tot + 1 : eoff + 1;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < nw * tot; i += blockDim.x) hist[i] = 0;
@@ -59,15 +69,24 @@ route_kernel(const int64_t* __restrict__ idx, int n_slots, int tot, int nw, int 
     }
   }
   __syncthreads();
-  if (part_out != nullptr) {
-    // first launch of the multi-CTA scheme: this CTA's totals, nothing else
-    for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-      int run = 0;
-      for (int w = 0; w < nw; ++w) run += hist[w * tot + e];
-      part_out[blockIdx.x * tot + e] = run;
+  // exclusive prefixes over the warps, and this CTA's totals
+  for (int e = threadIdx.x; e < tot; e += blockDim.x) {
+    int run = 0;
+    for (int w0 = 0; w0 < nw; w0 += 8) {
+      int t[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t[i] = w0 + i < nw ? hist[(w0 + i) * tot + e] : 0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (w0 + i < nw) hist[(w0 + i) * tot + e] = run;
+        run += t[i];
+      }
     }
-    return;
+    mine[e] = run;
+    if (part_out != nullptr) part_out[blockIdx.x * tot + e] = run;
   }
+  if (part_out != nullptr) return;   // first launch of the two-launch scheme: totals, nothing else
+  if (in_cluster) cg::this_cluster().sync(); else __syncthreads();
   for (int e = threadIdx.x; e < tot; e += blockDim.x) {
     int run = 0, total = 0;
     if (part_in != nullptr) {
@@ -76,25 +95,38 @@ route_kernel(const int64_t* __restrict__ idx, int n_slots, int tot, int nw, int 
         if (b < static_cast<int>(blockIdx.x)) run += t;
         total += t;
       }
+    } else if (in_cluster) {
+#pragma unroll
+      for (int b = 0; b < kRouteCluster; ++b) {
+        const int t = *cg::this_cluster().map_shared_rank(mine + e, b);
+        if (b < static_cast<int>(blockIdx.x)) run += t;
+        total += t;
+      }
+    } else {
+      total = mine[e];
     }
-    for (int w = 0; w < nw; ++w) {
-      const int t = hist[w * tot + e];
-      hist[w * tot + e] = run;
-      run += t;
+    if (run != 0) {
+      for (int w = 0; w < nw; ++w) hist[w * tot + e] += run;
     }
-    if (part_in == nullptr) total = run;
     if (blockIdx.x == 0) counts[e] = total;
-    if (pos != nullptr || offs != nullptr) eoff[e + 1] = total;
+    eoff[e + 1] = total;
   }
-  __syncthreads();
+  if (in_cluster) cg::this_cluster().sync(); else __syncthreads();   // nobody reads `mine` any more
   if (pos != nullptr || offs != nullptr) {
     // exclusive prefix of the counts: where the slots of every expert start in `pos`
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
       int run = 0;
-      eoff[0] = 0;
-      for (int e = 0; e < tot; ++e) {
-        run += eoff[e + 1];
-        eoff[e + 1] = run;
+      if (lane == 0) eoff[0] = 0;
+      for (int e0 = 0; e0 < tot; e0 += 32) {
+        const int e = e0 + lane;
+        int v = e < tot ? eoff[e + 1] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int up = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += up;
+        }
+        if (e < tot) eoff[e + 1] = run + v;
+        run += __shfl_sync(0xffffffffu, v, 31);
       }
     }
     __syncthreads();
@@ -618,119 +650,253 @@ gate_linear_topk_kernel(const T* __restrict__ x, const T* __restrict__ w, const 
   }
 }
 
+// The same result for R tokens per warp, TOT <= 8 and R * TOT <= 32: a slice of W is loaded and
+// unpacked once for R tokens, and the R * TOT sums over the lanes are formed together (each
+// exchange step halves the number of values a lane still holds; the additions are those of the
+// one-token kernel, in the same tree).  With one token per warp the kernel spent its time on
+// re-reading W: 8192 tokens, d = 2048, 8 experts took 34 us for 32 MB of input.
+template <typename T, int TOT, int R>
+__global__ void __launch_bounds__(256)
+gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias,
+                             int n_rows, int d, int tot, int k, T* __restrict__ logits,
+                             int64_t* __restrict__ idx, T* __restrict__ prob) {
+  constexpr int V = R * TOT;
+  const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
+  const int lane = threadIdx.x & 31;
+  if (row0 >= n_rows) return;
+  float acc[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) acc[v] = 0.f;
+  const int nv = d >> 3;
+  const uint4* xr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) xr[r] = reinterpret_cast<const uint4*>(x + static_cast<long>(min(row0 + r, n_rows - 1)) * d);
+#pragma unroll 2
+  for (int i = lane; i < nv; i += 32) {
+    uint4 xv[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) xv[r] = __ldg(xr[r] + i);
+    uint4 wv[TOT];
+#pragma unroll
+    for (int e = 0; e < TOT; ++e) {
+      wv[e] = e < tot ? __ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(e) * d) + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    float xf[R][8];
+#pragma unroll
+    for (int r = 0; r < R; ++r) unpack8<T>(xv[r], xf[r]);
+#pragma unroll
+    for (int e = 0; e < TOT; ++e) {
+      float wf[8];
+      unpack8<T>(wv[e], wf);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[r * TOT + e] = fmaf(xf[r][q], wf[q], acc[r * TOT + e]);
+      }
+    }
+  }
+  // value v of the warp ends in the lanes whose low bits, read from 16 down, spell v
+  int held = V, at = 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (held > 1) {
+      held >>= 1;
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int v = 0; v < V / 2; ++v) {
+        if (v < held) {
+          const float send = up ? acc[v] : acc[v + held];
+          const float keep = up ? acc[v + held] : acc[v];
+          acc[v] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+      if (up) at += held;
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+    }
+  }
+  const int r = at / TOT, e_of = at % TOT;
+  float mine = acc[0];
+  if (e_of < tot && bias != nullptr) mine += V2<T>::to_f(bias[e_of]);
+  mine = V2<T>::to_f(V2<T>::from_f(mine));   // ids and probabilities follow the rounded logits
+  constexpr int kStep = 32 / V;                 // lanes that hold the same value
+  const bool row_ok = row0 + r < n_rows;
+  if (row_ok && e_of < tot && (lane & (kStep - 1)) == 0) {
+    logits[static_cast<long>(row0 + r) * tot + e_of] = V2<T>::from_f(mine);
+  }
+  float all[TOT];
+  const int base = lane & ~(TOT * kStep - 1);   // first lane of this token's group
+#pragma unroll
+  for (int e = 0; e < TOT; ++e) all[e] = __shfl_sync(0xffffffffu, mine, base + e * kStep);
+  if (lane == base && row_ok) {
+    float sel_v[kMaxK];
+    int sel_i[kMaxK];
+    unsigned taken = 0u;
+    for (int j = 0; j < k; ++j) {
+      float best = -INFINITY;
+      int best_i = -1;
+#pragma unroll
+      for (int e = 0; e < TOT; ++e) {
+        if (e < tot && !((taken >> e) & 1u) && (best_i < 0 || all[e] > best)) {
+          best = all[e];
+          best_i = e;
+        }
+      }
+      taken |= 1u << best_i;
+      sel_v[j] = best;
+      sel_i[j] = best_i;
+    }
+    float den = 0.f, ex[kMaxK];
+    for (int j = 0; j < k; ++j) {
+      ex[j] = __expf(sel_v[j] - sel_v[0]);
+      den += ex[j];
+    }
+    const long o = static_cast<long>(row0 + r) * k;
+    for (int j = 0; j < k; ++j) {
+      idx[o + j] = sel_i[j];
+      prob[o + j] = V2<T>::from_f(ex[j] / den);
+    }
+  }
+}
+
 // dl[t, e] = softmax backward of the selected logits scattered to their experts, plus the
 // gradient that reached the logits directly (may be null).  dx[t, :] = sum_e dl[t, e] W[e, :].
-// dl is written out (fp32) for the weight-gradient kernel.  One warp per token.
-template <typename T, int TOT>
+// dl is written out (fp32) for the weight-gradient kernel.  R tokens per warp share every slice
+// of W that is loaded and unpacked (one token per warp: 37 us for 8192 tokens, d = 2048, 8 experts).
+template <typename T, int TOT, int R>
 __global__ void __launch_bounds__(256)
 gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
                    const T* __restrict__ prob, const T* __restrict__ dlogits_in,
                    const T* __restrict__ w, int n_rows, int d, int tot, int k,
                    float* __restrict__ dl_out, T* __restrict__ dx) {
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
   const int lane = threadIdx.x & 31;
-  if (row >= n_rows) return;
-  float dl[TOT];
+  if (row0 >= n_rows) return;
+  float dl[R][TOT];
 #pragma unroll
-  for (int e = 0; e < TOT; ++e) {
-    dl[e] = (e < tot && dlogits_in != nullptr)
-                ? V2<T>::to_f(dlogits_in[static_cast<long>(row) * tot + e]) : 0.f;
-  }
-  if (dprob != nullptr) {
-    float g[kMaxK], pj[kMaxK];
-    int id[kMaxK];
-    float dotp = 0.f;
-    for (int j = 0; j < k; ++j) {
-      g[j] = V2<T>::to_f(dprob[static_cast<long>(row) * k + j]);
-      pj[j] = V2<T>::to_f(prob[static_cast<long>(row) * k + j]);
-      id[j] = static_cast<int>(idx[static_cast<long>(row) * k + j]);
-      dotp += g[j] * pj[j];
-    }
-    for (int j = 0; j < k; ++j) {
-      const float v = pj[j] * (g[j] - dotp);
-#pragma unroll
-      for (int e = 0; e < TOT; ++e) {
-        if (e == id[j]) dl[e] += v;
-      }
-    }
-  }
-  if (lane == 0) {
+  for (int r = 0; r < R; ++r) {
+    const long row = row0 + r;
+    const bool ok = row < n_rows;
 #pragma unroll
     for (int e = 0; e < TOT; ++e) {
-      if (e < tot) dl_out[static_cast<long>(row) * tot + e] = dl[e];
+      dl[r][e] = (ok && e < tot && dlogits_in != nullptr) ? V2<T>::to_f(dlogits_in[row * tot + e]) : 0.f;
     }
-  }
-  if (dx != nullptr) {
-    uint4* out = reinterpret_cast<uint4*>(dx + static_cast<long>(row) * d);
-    const int nv = d >> 3;
-#pragma unroll 4
-    for (int i = lane; i < nv; i += 32) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (ok && dprob != nullptr) {
+      float g[kMaxK], pj[kMaxK];
+      int id[kMaxK];
+      float dotp = 0.f;
+      for (int j = 0; j < k; ++j) {
+        g[j] = V2<T>::to_f(dprob[row * k + j]);
+        pj[j] = V2<T>::to_f(prob[row * k + j]);
+        id[j] = static_cast<int>(idx[row * k + j]);
+        dotp += g[j] * pj[j];
+      }
+      for (int j = 0; j < k; ++j) {
+        const float v = pj[j] * (g[j] - dotp);
 #pragma unroll
-      for (int e = 0; e < TOT; ++e) {
-        if (e < tot && dl[e] != 0.f) {
-          float wf[8];
-          unpack8<T>(__ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(e) * d) + i), wf);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) acc[q] = fmaf(dl[e], wf[q], acc[q]);
+        for (int e = 0; e < TOT; ++e) {
+          if (e == id[j]) dl[r][e] += v;
         }
       }
-      out[i] = pack8<T>(acc);
+    }
+    if (ok && lane == 0) {
+#pragma unroll
+      for (int e = 0; e < TOT; ++e) {
+        if (e < tot) dl_out[row * tot + e] = dl[r][e];
+      }
+    }
+  }
+  if (dx == nullptr) return;
+  const int nv = d >> 3;
+#pragma unroll 2
+  for (int i = lane; i < nv; i += 32) {
+    float acc[R][8];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[r][q] = 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < TOT; ++e) {
+      if (e < tot) {
+        float wf[8];
+        unpack8<T>(__ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(e) * d) + i), wf);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if (dl[r][e] != 0.f) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[r][q] = fmaf(dl[r][e], wf[q], acc[r][q]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (row0 + r < n_rows) reinterpret_cast<uint4*>(dx + static_cast<long>(row0 + r) * d)[i] = pack8<T>(acc[r]);
     }
   }
 }
 
 // dW[e, c] += sum_t dl[t, e] x[t, c] and db[e] += sum_t dl[t, e] (fp32, pre-zeroed).  A block
-// takes a 64-column strip and one of `gridDim.y` token ranges; a lane owns two columns.
+// takes a 256-column strip and one of `gridDim.y` token ranges; a lane owns eight columns, so that
+// a token is one 16-byte load per lane (with two columns per lane and 64-column strips the loads
+// were too small to keep the memory busy: 40 us for 8192 tokens, d = 2048, 8 experts).
 template <typename T, int TOT>
 __global__ void __launch_bounds__(256)
 gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_rows, int d, int tot,
                    float* __restrict__ dw, float* __restrict__ db) {
-  __shared__ float red[8][TOT][64 + 1];
+  __shared__ float red[8][256 + 8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = blockIdx.x * 64 + lane * 2;
+  const int col = blockIdx.x * 256 + lane * 8;
   const int per = (n_rows + gridDim.y - 1) / gridDim.y;
   const int t0 = blockIdx.y * per, t1 = min(n_rows, t0 + per);
-  float a0[TOT], a1[TOT], bsum[TOT];
+  const bool sums = db != nullptr && blockIdx.x == 0;
+  float acc[TOT][8], bsum[TOT];
 #pragma unroll
-  for (int e = 0; e < TOT; ++e) a0[e] = a1[e] = bsum[e] = 0.f;
-#pragma unroll 4
-  for (int t = t0 + warp; t < t1; t += 8) {
-    float x0 = 0.f, x1 = 0.f;
-    if (col < d) {
-      const typename V2<T>::type v = *reinterpret_cast<const typename V2<T>::type*>(x + static_cast<long>(t) * d + col);
-      const float2 f = V2<T>::to_f2(v);
-      x0 = f.x;
-      x1 = f.y;
+  for (int e = 0; e < TOT; ++e) {
+    bsum[e] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[e][q] = 0.f;
+  }
+  constexpr int U = 4;
+  for (int t = t0 + warp; t < t1; t += 8 * U) {
+    uint4 xv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      xv[u] = (t + 8 * u < t1 && col < d) ? __ldg(reinterpret_cast<const uint4*>(x + static_cast<long>(t + 8 * u) * d + col))
+                                          : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
-    for (int e = 0; e < TOT; ++e) {
-      if (e < tot) {
-        const float g = __ldg(dl + static_cast<long>(t) * tot + e);
-        a0[e] = fmaf(g, x0, a0[e]);
-        a1[e] = fmaf(g, x1, a1[e]);
-        bsum[e] += g;
+    for (int u = 0; u < U; ++u) {
+      if (t + 8 * u >= t1) break;
+      float xf[8];
+      unpack8<T>(xv[u], xf);
+#pragma unroll
+      for (int e = 0; e < TOT; ++e) {
+        if (e < tot) {
+          const float g = __ldg(dl + static_cast<long>(t + 8 * u) * tot + e);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[e][q] = fmaf(g, xf[q], acc[e][q]);
+          if (sums) bsum[e] += g;
+        }
       }
     }
   }
 #pragma unroll
   for (int e = 0; e < TOT; ++e) {
-    red[warp][e][lane * 2] = a0[e];
-    red[warp][e][lane * 2 + 1] = a1[e];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < tot * 64; i += blockDim.x) {
-    const int e = i / 64, c = i % 64;
-    float s = 0.f;
+    if (e >= tot) break;
+    __syncthreads();
 #pragma unroll
-    for (int wv = 0; wv < 8; ++wv) s += red[wv][e][c];
-    if (blockIdx.x * 64 + c < d) atomicAdd(dw + static_cast<long>(e) * d + blockIdx.x * 64 + c, s);
-  }
-  if (db != nullptr && blockIdx.x == 0 && lane == 0) {
+    for (int q = 0; q < 8; ++q) red[warp][lane * 8 + q] = acc[e][q];
+    __syncthreads();
+    const int c = blockIdx.x * 256 + threadIdx.x;
+    if (c < d) {
+      float s = 0.f;
 #pragma unroll
-    for (int e = 0; e < TOT; ++e) {
-      if (e < tot) atomicAdd(db + e, bsum[e]);
+      for (int wv = 0; wv < 8; ++wv) s += red[wv][threadIdx.x];
+      atomicAdd(dw + static_cast<long>(e) * d + c, s);
     }
+    if (sums && lane == 0) atomicAdd(db + e, bsum[e]);
   }
 }
 
@@ -915,8 +1081,8 @@ cudaError_t simt_typed(int mode, int num_groups, long rows_cap, int m, int n, in
 
 // ------------------------------------------------------------------------------ launchers
 int route_blocks(int n_slots) {
-  // one CTA up to 32 K slots (a single launch, about 8 us); beyond that 16 K slots per CTA
-  if (n_slots <= 32768) return 1;
+  // one launch (a CTA or a cluster) up to kRouteClusterSlots; beyond that 16 K slots per CTA
+  if (n_slots <= kRouteClusterSlots) return 1;
   int nb = (n_slots + 16383) / 16384;
   return nb > 148 ? 148 : nb;
 }
@@ -928,24 +1094,43 @@ cudaError_t launch_route(const int64_t* idx, int n_slots, int tot, int* counts, 
   if (nw < 1) return cudaErrorInvalidValue;
   if (nw > 32) nw = 32;
   const int nb = part != nullptr ? route_blocks(n_slots) : 1;
-  int cta_slots = (n_slots + nb - 1) / nb;
+  // below 1 K slots one CTA has at most one step per warp and pass: nothing to spread; with very
+  // many experts the histograms of fewer warps fit beside the cluster's totals
+  const bool cluster = nb == 1 && n_slots > 1024 && tot <= 1024;
+  const int ctas = cluster ? kRouteCluster : nb;
+  int cta_slots = (n_slots + ctas - 1) / ctas;
   cta_slots = (cta_slots + 31) & ~31;
   if (cta_slots < 32) cta_slots = 32;
   const int by_work = (cta_slots + 31) / 32;
   if (nw > by_work) nw = by_work > 0 ? by_work : 1;
-  const size_t smem = static_cast<size_t>(nw) * tot * 4 + static_cast<size_t>(tot + 1) * 4;
+  const size_t smem = static_cast<size_t>(nw) * tot * 4 + static_cast<size_t>(cluster ? 2 * tot + 1 : tot + 1) * 4;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kRouteSmemLimit);
     if (e != cudaSuccess) return e;
   }
   if (nb > 1) {
-    route_kernel<<<nb, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, nullptr, part,
+    route_kernel<<<nb, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, 0, nullptr, part,
                                                      counts, rank, offs, pos);
-    route_kernel<<<nb, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, part, nullptr,
+    route_kernel<<<nb, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, 0, part, nullptr,
                                                      counts, rank, offs, pos);
+  } else if (cluster) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kRouteCluster);
+    cfg.blockDim = dim3(kRouteThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kRouteCluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, route_kernel, idx, n_slots, tot, nw, cta_slots, 1,
+                              static_cast<const int*>(nullptr), static_cast<int*>(nullptr), counts, rank, offs, pos);
   } else {
-    route_kernel<<<1, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, nullptr, nullptr,
+    route_kernel<<<1, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, 0, nullptr, nullptr,
                                                     counts, rank, offs, pos);
   }
   return cudaGetLastError();
@@ -1086,10 +1271,7 @@ cudaError_t launch_gate_topk_softmax_bwd(int logit_dtype, const void* dprob, con
 }
 
 #define FMOE_GATE_TOT(tot, ...)                          \
-  if ((tot) <= 2) { constexpr int TOT = 2; __VA_ARGS__; }       \
-  else if ((tot) <= 4) { constexpr int TOT = 4; __VA_ARGS__; }  \
-  else if ((tot) <= 8) { constexpr int TOT = 8; __VA_ARGS__; }  \
-  else if ((tot) <= 16) { constexpr int TOT = 16; __VA_ARGS__; } \
+  if ((tot) <= 16) { constexpr int TOT = 16; __VA_ARGS__; } \
   else if ((tot) <= 32) { constexpr int TOT = 32; __VA_ARGS__; } \
   else { constexpr int TOT = 64; __VA_ARGS__; }
 
@@ -1097,12 +1279,35 @@ bool gate_fused_supported(int tot, int d, int k) {
   return tot >= 1 && tot <= kGateMaxExperts && d % 8 == 0 && k >= 1 && k <= kMaxK && k <= tot;
 }
 
+// Tokens per warp: as many as leave every SM eight warps, up to what registers hold (measured with
+// d = 2048, 8 experts: see the kernels).
+int gate_rows_per_warp(int n_rows, int tot) {
+  if (tot > 8 || n_rows < 148 * 8 * 2) return 1;
+  return n_rows < 148 * 8 * 4 ? 2 : 4;
+}
+
 cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, const void* bias,
                                     int n_rows, int d, int tot, int k, void* logits, int64_t* idx,
                                     void* prob, cudaStream_t stream) {
   if (n_rows == 0) return cudaSuccess;
   if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
-  const int grid = (n_rows + 7) / 8;
+  const int per = gate_rows_per_warp(n_rows, tot);
+  const int grid = (n_rows + 8 * per - 1) / (8 * per);
+#define FMOE_GATE_ROWS(TOT, R)                                                                          \
+  FMOE_DISPATCH_16(dtype, (gate_linear_topk_rows_kernel<T, TOT, R><<<grid, 256, 0, stream>>>(           \
+      static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,  \
+      k, static_cast<T*>(logits), idx, static_cast<T*>(prob))))
+  if (tot <= 8) {
+    if (tot <= 2) {
+      if (per == 1) { FMOE_GATE_ROWS(2, 1); } else if (per == 2) { FMOE_GATE_ROWS(2, 2); } else { FMOE_GATE_ROWS(2, 4); }
+    } else if (tot <= 4) {
+      if (per == 1) { FMOE_GATE_ROWS(4, 1); } else if (per == 2) { FMOE_GATE_ROWS(4, 2); } else { FMOE_GATE_ROWS(4, 4); }
+    } else {
+      if (per == 1) { FMOE_GATE_ROWS(8, 1); } else if (per == 2) { FMOE_GATE_ROWS(8, 2); } else { FMOE_GATE_ROWS(8, 4); }
+    }
+    return cudaGetLastError();
+  }
+#undef FMOE_GATE_ROWS
   FMOE_DISPATCH_16(dtype, FMOE_GATE_TOT(tot, (gate_linear_topk_kernel<T, TOT><<<grid, 256, 0, stream>>>(
       static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,
       k, static_cast<T*>(logits), idx, static_cast<T*>(prob)))));
@@ -1115,20 +1320,36 @@ cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, co
                             cudaStream_t stream) {
   if (n_rows == 0) return cudaSuccess;
   if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
-  const int grid = (n_rows + 7) / 8;
-  FMOE_DISPATCH_16(dtype, FMOE_GATE_TOT(tot, (gate_bwd_dx_kernel<T, TOT><<<grid, 256, 0, stream>>>(
-      static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in),
-      static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx)))));
+  const int per = gate_rows_per_warp(n_rows, tot);
+  const int grid = (n_rows + 8 * per - 1) / (8 * per);
+#define FMOE_GATE_DX(TOT, R)                                                                             \
+  FMOE_DISPATCH_16(dtype, (gate_bwd_dx_kernel<T, TOT, R><<<grid, 256, 0, stream>>>(                      \
+      static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in), \
+      static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx))))
+  if (tot <= 2) {
+    if (per == 1) { FMOE_GATE_DX(2, 1); } else if (per == 2) { FMOE_GATE_DX(2, 2); } else { FMOE_GATE_DX(2, 4); }
+  } else if (tot <= 4) {
+    if (per == 1) { FMOE_GATE_DX(4, 1); } else if (per == 2) { FMOE_GATE_DX(4, 2); } else { FMOE_GATE_DX(4, 4); }
+  } else if (tot <= 8) {
+    if (per == 1) { FMOE_GATE_DX(8, 1); } else if (per == 2) { FMOE_GATE_DX(8, 2); } else { FMOE_GATE_DX(8, 4); }
+  } else if (tot <= 16) {
+    FMOE_GATE_DX(16, 1);
+  } else if (tot <= 32) {
+    FMOE_GATE_DX(32, 1);
+  } else {
+    FMOE_GATE_DX(64, 1);
+  }
+#undef FMOE_GATE_DX
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   if (dw == nullptr) return cudaSuccess;
   if (tot > 16) return cudaErrorInvalidValue;
-  // Each warp walks its token range serially (one dependent load chain), so the ranges are
-  // kept short: many blocks, a few tokens per warp, partial sums merged with atomics.
-  int splits = n_rows / 64;
-  if (splits < 1) splits = 1;
-  if (splits > 64) splits = 64;
-  dim3 g2((d + 63) / 64, splits);
+  // two blocks per SM over the strips and token ranges, a warp at least four tokens; the partial
+  // sums of the ranges are merged with atomics
+  const int strips = (d + 255) / 256;
+  int splits = (2 * 148 + strips - 1) / strips;
+  if (splits > (n_rows + 31) / 32) splits = (n_rows + 31) / 32;
+  dim3 g2(strips, splits);
   if (tot <= 2) {
     FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 2><<<g2, 256, 0, stream>>>(
         dl_scratch, static_cast<const T*>(x), n_rows, d, tot, dw, db)));

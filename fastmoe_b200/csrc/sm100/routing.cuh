@@ -10,7 +10,7 @@ namespace fmoe {
 // rank: pos[offs[e] + rank[s]] = s; entries past offs[tot] are not written).  Deterministic:
 // slots of one expert are ranked by slot id.
 // `part` (optional): int32 scratch of route_blocks(n_slots) * tot entries; with it, more than
-// 32 K slots are ranked by several CTAs in two launches instead of by one CTA.
+// 64 K slots are ranked by many CTAs in two launches instead of by one cluster.
 int route_blocks(int n_slots);
 cudaError_t launch_route(const int64_t* idx, int n_slots, int tot, int* counts, int* rank,
                          int* offs, int* pos, int* part, cudaStream_t stream);

@@ -469,3 +469,56 @@ def test_fp32_tiles_tail_and_column_sums(counts, k, n):
             assert close(dx[lo:hi], go[lo:hi], w[e]), e
         assert close(dw[e], go[lo:hi].t(), x[lo:hi]), e
         assert close(db[e][None], torch.ones(1, hi - lo, device=DEV), go[lo:hi]), e
+
+
+@pytest.mark.parametrize("n_slots,tot", [(1024, 8), (1025, 8), (22528, 8), (16384, 2), (16385, 64), (65536, 1),
+                                         (65537, 3), (40000, 1024), (40000, 1025), (1, 1), (5000, 20000)])
+def test_route_at_the_lines_between_cta_cluster_and_grid(n_slots, tot):
+    r"""Counts, ranks, offsets and slot list where the routing kernel changes its split of the work,
+    with a third of the slots dropped and one expert holding most of the others."""
+    torch.manual_seed(14)
+    idx = torch.randint(0, tot, (n_slots,))
+    idx[torch.rand(n_slots) < 0.5] = tot // 2
+    idx[torch.rand(n_slots) < 0.3] = -1
+    counts, rank, offs, pos = (t.cpu().long() for t in _native().route_pos(idx.to(DEV), tot))
+    kept = idx >= 0
+    want = torch.bincount(idx[kept], minlength=tot)
+    assert torch.equal(counts, want)
+    assert torch.equal(offs, torch.cat([torch.zeros(1, dtype=torch.long), want.cumsum(0)]))
+    order = torch.argsort(torch.where(kept, idx, tot), stable=True)[:int(kept.sum())]
+    assert torch.equal(pos[:order.numel()], order)
+    want_rank = torch.full((n_slots,), -1)
+    want_rank[order] = torch.arange(order.numel()) - offs[idx[order]]
+    assert torch.equal(rank, want_rank)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,tot,k,d", [(2367, 8, 2, 136), (2368, 7, 8, 264), (2369, 2, 1, 128), (4735, 3, 2, 64),
+                                          (4736, 8, 2, 1024), (4739, 2, 2, 512), (9001, 5, 4, 520), (1, 1, 1, 8)])
+def test_gate_rows_per_warp(dtype, rows, tot, k, d):
+    r"""The fused gate on both sides of the lines where a warp takes one, two or four tokens, against
+    fp64 on the same 16-bit inputs: logits to one rounding plus an fp32 sum of d terms, ids by the
+    returned logits (ties to the lower id), gradients to one rounding plus a sum of tot, k or rows
+    terms."""
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(15)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    x = torch.randn(rows, d, device=DEV).to(dtype).requires_grad_(True)
+    w = (torch.randn(tot, d, device=DEV) / d ** 0.5).to(dtype).requires_grad_(True)
+    b = torch.randn(tot, device=DEV).to(dtype).requires_grad_(True)
+    logits, idx, prob = gating.linear_topk_softmax(x, w, b, k)
+    ref = x.double() @ w.double().t() + b.double()
+    assert ((logits.double() - ref).abs() <= eps * ref.abs() + d * 2.0 ** -23).all()
+    assert torch.equal(idx, logits.double().sort(dim=1, descending=True, stable=True).indices[:, :k])
+    gl, gp = torch.randn_like(logits), torch.randn_like(prob)
+    torch.autograd.backward([logits, prob], [gl, gp])
+    p64, g64 = prob.detach().double(), gp.double()
+    dl = gl.double().scatter_add(1, idx, p64 * (g64 - (p64 * g64).sum(1, keepdim=True)))
+
+    def close(got, a, m):
+        r = a @ m
+        return bool(((got.double() - r).abs() <= eps * r.abs() + (a.shape[1] + 16) * 2.0 ** -22 * (a.abs() @ m.abs()) + 1e-7).all())
+
+    assert close(x.grad, dl, w.detach().double())
+    assert close(w.grad, dl.t(), x.detach().double())
+    assert close(b.grad[None], torch.ones(1, rows, device=DEV, dtype=torch.float64), dl)

@@ -146,3 +146,53 @@ def test_gates_run_on_gpu(gate_name):
 def test_smoke_entry():
     import __graft_entry__ as entry
     entry.smoke()
+
+
+@pytest.mark.parametrize("case", ["plain", "strided", "scores_fp32", "frozen_weights", "frozen_input", "no_grad",
+                                  "unaligned", "dropped"])
+@pytest.mark.parametrize("act", [torch.nn.GELU(), torch.nn.Identity()])
+def test_native_layer_call_equals_separate_launches(case, act, monkeypatch):
+    r"""One native call per direction against the route / dispatch / experts / combine functions (taken
+    when the bounds checks look between the launches): the same kernels, so the same bits."""
+    from fastmoe_b200 import FMoETransformerMLP
+    from fastmoe_b200.ops import fused
+    torch.manual_seed(13)
+    layer = FMoETransformerMLP(num_expert=5, d_model=128, d_hidden=192, top_k=2, activation=act).cuda().bfloat16()
+    x = torch.randn(77, 128, device="cuda").bfloat16()
+    score = torch.rand(77, 2, device="cuda").to(torch.float32 if case == "scores_fp32" else torch.bfloat16)
+    idx = torch.randint(0, 5, (77, 2), device="cuda")
+    if case == "strided":
+        x = torch.randn(128, 77, device="cuda").bfloat16().t()
+        score = torch.rand(2, 77, device="cuda").bfloat16().t()
+        idx = torch.randint(0, 5, (2, 77), device="cuda").t()
+    if case == "dropped":
+        idx[::3, 1] = -1
+        idx[5] = -1
+    if case == "frozen_weights":
+        layer.experts.requires_grad_(False)
+    if case == "unaligned":
+        for lin in (layer.experts.htoh4, layer.experts.h4toh):
+            flat = torch.empty(lin.weight.numel() + 1, device="cuda", dtype=torch.bfloat16)
+            flat[1:] = lin.weight.detach().view(-1)
+            lin.weight = torch.nn.Parameter(flat[1:].view_as(lin.weight))
+    gy = torch.randn(77, 128, device="cuda").bfloat16()
+
+    def run():
+        layer.zero_grad(set_to_none=True)
+        xi = x.detach().requires_grad_(case != "frozen_input")
+        si = score.detach().requires_grad_(True)
+        if case == "no_grad":
+            with torch.no_grad():
+                return [fused.moe_mlp_forward(layer, xi, idx, si)]
+        y = fused.moe_mlp_forward(layer, xi, idx, si)
+        y.backward(gy)
+        return [y, xi.grad, si.grad] + [p.grad for p in layer.experts.parameters()]
+
+    got = run()
+    monkeypatch.setenv("FMOE_DEBUG_BOUNDS", "1")
+    want = run()
+    assert len(got) == len(want)
+    for a, b in zip(got, want):
+        assert (a is None) == (b is None)
+        if a is not None:
+            assert a.dtype == b.dtype and torch.equal(a, b)
