@@ -555,20 +555,23 @@ std::vector<torch::Tensor> gate_linear_topk_bwd(c10::optional<torch::Tensor> dpr
   auto dl = torch::empty({rows, tot}, f32);
   torch::Tensor dx = need_dx ? torch::empty_like(x) : torch::Tensor();
   const bool fused_dw = tot <= 16;
-  // one zero-filled buffer for dW and db so that a single fill and a single cast serve both
-  torch::Tensor acc = fused_dw ? torch::zeros({static_cast<long>(tot) * d + tot}, f32) : torch::Tensor();
+  torch::Tensor part, dw_db;
+  if (fused_dw) {
+    const long elems = static_cast<long>(tot) * d + tot;
+    // without rows nothing is launched: the sums over no tokens are zero
+    dw_db = rows > 0 ? torch::empty({elems}, x.options()) : torch::zeros({elems}, x.options());
+    part = torch::empty({fmoe::gate_bwd_ranges(rows, d) * elems}, f32);
+  }
   FMOE_CUDA_CHECK(fmoe::launch_gate_bwd(
       dtype16(x), dprob.has_value() ? dprob->data_ptr() : nullptr, idx.data_ptr<int64_t>(),
       prob.data_ptr(), dlogits.has_value() ? dlogits->data_ptr() : nullptr, x.data_ptr(),
       w.data_ptr(), rows, d, tot, k, dl.data_ptr<float>(), need_dx ? dx.data_ptr() : nullptr,
-      fused_dw ? acc.data_ptr<float>() : nullptr,
-      fused_dw ? acc.data_ptr<float>() + static_cast<long>(tot) * d : nullptr, cur_stream()));
+      fused_dw ? part.data_ptr<float>() : nullptr, fused_dw ? dw_db.data_ptr() : nullptr, cur_stream()));
   torch::Tensor dw, db;
   if (fused_dw) {
-    g_launches.fetch_add(1, std::memory_order_relaxed);  // the weight-gradient kernel
-    auto cast = acc.to(x.scalar_type());
-    dw = cast.narrow(0, 0, static_cast<long>(tot) * d).view({tot, d});
-    if (need_db) db = cast.narrow(0, static_cast<long>(tot) * d, tot);
+    g_launches.fetch_add(2, std::memory_order_relaxed);  // the weight-gradient and merge kernels
+    dw = dw_db.narrow(0, 0, static_cast<long>(tot) * d).view({tot, d});
+    if (need_db) db = dw_db.narrow(0, static_cast<long>(tot) * d, tot);
   } else {
     auto dl16 = dl.to(x.scalar_type());
     dw = dl16.t().matmul(x);

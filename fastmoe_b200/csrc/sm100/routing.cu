@@ -729,10 +729,13 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
 #pragma unroll
   for (int e = 0; e < TOT; ++e) all[e] = __shfl_sync(0xffffffffu, mine, base + e * kStep);
   if (lane == base && row_ok) {
-    float sel_v[kMaxK];
-    int sel_i[kMaxK];
+    // constant bounds keep the selection in registers (TOT <= kMaxK, k <= tot)
+    float sel_v[TOT];
+    int sel_i[TOT];
     unsigned taken = 0u;
-    for (int j = 0; j < k; ++j) {
+#pragma unroll
+    for (int j = 0; j < TOT; ++j) {
+      if (j >= k) break;
       float best = -INFINITY;
       int best_i = -1;
 #pragma unroll
@@ -746,13 +749,17 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
       sel_v[j] = best;
       sel_i[j] = best_i;
     }
-    float den = 0.f, ex[kMaxK];
-    for (int j = 0; j < k; ++j) {
+    float den = 0.f, ex[TOT];
+#pragma unroll
+    for (int j = 0; j < TOT; ++j) {
+      if (j >= k) break;
       ex[j] = __expf(sel_v[j] - sel_v[0]);
       den += ex[j];
     }
     const long o = static_cast<long>(row0 + r) * k;
-    for (int j = 0; j < k; ++j) {
+#pragma unroll
+    for (int j = 0; j < TOT; ++j) {
+      if (j >= k) break;
       idx[o + j] = sel_i[j];
       prob[o + j] = V2<T>::from_f(ex[j] / den);
     }
@@ -761,96 +768,77 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
 
 // dl[t, e] = softmax backward of the selected logits scattered to their experts, plus the
 // gradient that reached the logits directly (may be null).  dx[t, :] = sum_e dl[t, e] W[e, :].
-// dl is written out (fp32) for the weight-gradient kernel.  R tokens per warp share every slice
-// of W that is loaded and unpacked (one token per warp: 37 us for 8192 tokens, d = 2048, 8 experts).
-template <typename T, int TOT, int R>
+// dl is written out (fp32) for the weight-gradient kernel.  One warp per token; every lane forms
+// the dl of one expert and the warp shares them: with all lanes walking the k choices of the
+// token 8192 tokens (d = 2048, 8 experts) took 37 us, now 21.
+template <typename T, int TOT>
 __global__ void __launch_bounds__(256)
 gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
                    const T* __restrict__ prob, const T* __restrict__ dlogits_in,
                    const T* __restrict__ w, int n_rows, int d, int tot, int k,
                    float* __restrict__ dl_out, T* __restrict__ dx) {
-  const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (row0 >= n_rows) return;
-  float dl[R][TOT];
+  if (row >= n_rows) return;
+  float dl[TOT];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const long row = row0 + r;
-    const bool ok = row < n_rows;
-#pragma unroll
-    for (int e = 0; e < TOT; ++e) {
-      dl[r][e] = (ok && e < tot && dlogits_in != nullptr) ? V2<T>::to_f(dlogits_in[row * tot + e]) : 0.f;
-    }
-    if (ok && dprob != nullptr) {
-      float g[kMaxK], pj[kMaxK];
-      int id[kMaxK];
-      float dotp = 0.f;
-      for (int j = 0; j < k; ++j) {
-        g[j] = V2<T>::to_f(dprob[row * k + j]);
-        pj[j] = V2<T>::to_f(prob[row * k + j]);
-        id[j] = static_cast<int>(idx[row * k + j]);
-        dotp += g[j] * pj[j];
-      }
-      for (int j = 0; j < k; ++j) {
-        const float v = pj[j] * (g[j] - dotp);
-#pragma unroll
-        for (int e = 0; e < TOT; ++e) {
-          if (e == id[j]) dl[r][e] += v;
+  for (int e0 = 0; e0 < TOT; e0 += 32) {
+    const int e = e0 + lane;
+    float mine = 0.f;
+    if (e < tot) {
+      if (dlogits_in != nullptr) mine = V2<T>::to_f(dlogits_in[static_cast<long>(row) * tot + e]);
+      if (dprob != nullptr) {
+        const T* g = dprob + static_cast<long>(row) * k;
+        const T* p = prob + static_cast<long>(row) * k;
+        const int64_t* id = idx + static_cast<long>(row) * k;
+        float dotp = 0.f;
+        for (int j = 0; j < k; ++j) dotp += V2<T>::to_f(g[j]) * V2<T>::to_f(p[j]);
+        for (int j = 0; j < k; ++j) {
+          if (id[j] == e) mine += V2<T>::to_f(p[j]) * (V2<T>::to_f(g[j]) - dotp);
         }
       }
+      dl_out[static_cast<long>(row) * tot + e] = mine;
     }
-    if (ok && lane == 0) {
 #pragma unroll
-      for (int e = 0; e < TOT; ++e) {
-        if (e < tot) dl_out[row * tot + e] = dl[r][e];
-      }
+    for (int u = 0; u < 32; ++u) {
+      if (e0 + u < TOT) dl[e0 + u] = __shfl_sync(0xffffffffu, mine, u);
     }
   }
   if (dx == nullptr) return;
+  uint4* out = reinterpret_cast<uint4*>(dx + static_cast<long>(row) * d);
   const int nv = d >> 3;
-#pragma unroll 2
+#pragma unroll 4
   for (int i = lane; i < nv; i += 32) {
-    float acc[R][8];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-#pragma unroll
-      for (int q = 0; q < 8; ++q) acc[r][q] = 0.f;
-    }
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int e = 0; e < TOT; ++e) {
-      if (e < tot) {
+      if (e < tot && dl[e] != 0.f) {
         float wf[8];
         unpack8<T>(__ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(e) * d) + i), wf);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (dl[r][e] != 0.f) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) acc[r][q] = fmaf(dl[r][e], wf[q], acc[r][q]);
-          }
-        }
+        for (int q = 0; q < 8; ++q) acc[q] = fmaf(dl[e], wf[q], acc[q]);
       }
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (row0 + r < n_rows) reinterpret_cast<uint4*>(dx + static_cast<long>(row0 + r) * d)[i] = pack8<T>(acc[r]);
-    }
+    out[i] = pack8<T>(acc);
   }
 }
 
-// dW[e, c] += sum_t dl[t, e] x[t, c] and db[e] += sum_t dl[t, e] (fp32, pre-zeroed).  A block
-// takes a 256-column strip and one of `gridDim.y` token ranges; a lane owns eight columns, so that
-// a token is one 16-byte load per lane (with two columns per lane and 64-column strips the loads
-// were too small to keep the memory busy: 40 us for 8192 tokens, d = 2048, 8 experts).
+// Partial sums of dW[e, c] = sum_t dl[t, e] x[t, c] and db[e] = sum_t dl[t, e] over one of
+// `gridDim.y` token ranges: part[range][tot * d + tot] in fp32.  A block takes a 256-column strip;
+// a lane owns eight columns, so that a token is one 16-byte load per lane (two columns per lane,
+// as before, kept too few bytes in flight).  The ranges used to be merged with atomics on a
+// zeroed buffer: 296 additions per address took most of the 20 us of 16384 tokens with d = 256.
 template <typename T, int TOT>
 __global__ void __launch_bounds__(256)
 gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_rows, int d, int tot,
-                   float* __restrict__ dw, float* __restrict__ db) {
+                   float* __restrict__ part) {
   __shared__ float red[8][256 + 8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 256 + lane * 8;
   const int per = (n_rows + gridDim.y - 1) / gridDim.y;
   const int t0 = blockIdx.y * per, t1 = min(n_rows, t0 + per);
-  const bool sums = db != nullptr && blockIdx.x == 0;
+  const bool sums = blockIdx.x == 0;
+  float* mine = part + static_cast<long>(blockIdx.y) * (static_cast<long>(tot) * d + tot);
   float acc[TOT][8], bsum[TOT];
 #pragma unroll
   for (int e = 0; e < TOT; ++e) {
@@ -888,15 +876,44 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < 8; ++q) red[warp][lane * 8 + q] = acc[e][q];
+    if (sums && lane == 0) red[warp][256] = bsum[e];
     __syncthreads();
     const int c = blockIdx.x * 256 + threadIdx.x;
     if (c < d) {
       float s = 0.f;
 #pragma unroll
       for (int wv = 0; wv < 8; ++wv) s += red[wv][threadIdx.x];
-      atomicAdd(dw + static_cast<long>(e) * d + c, s);
+      mine[static_cast<long>(e) * d + c] = s;
     }
-    if (sums && lane == 0) atomicAdd(db + e, bsum[e]);
+    if (sums && threadIdx.x == 0) {
+      float s = 0.f;
+#pragma unroll
+      for (int wv = 0; wv < 8; ++wv) s += red[wv][256];
+      mine[static_cast<long>(tot) * d + e] = s;
+    }
+  }
+}
+
+// out[i] = sum over the ranges of part[range][i], in a fixed order, in the layer's type: eight
+// lanes of ranges per 32 elements.
+template <typename T>
+__global__ void __launch_bounds__(256)
+gate_bwd_merge_kernel(const float* __restrict__ part, int ranges, long elems, T* __restrict__ out) {
+  __shared__ float red[8][33];
+  const int sub = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long i = static_cast<long>(blockIdx.x) * 32 + lane;
+  float s = 0.f;
+  if (i < elems) {
+#pragma unroll 4
+    for (int r = sub; r < ranges; r += 8) s += __ldg(part + static_cast<long>(r) * elems + i);
+  }
+  red[sub][lane] = s;
+  __syncthreads();
+  if (sub == 0 && i < elems) {
+    float total = 0.f;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) total += red[u][lane];
+    out[i] = V2<T>::from_f(total);
   }
 }
 
@@ -921,15 +938,6 @@ template <> __device__ __forceinline__ void stv<__nv_bfloat16>(__nv_bfloat16* p,
 }
 template <> __device__ __forceinline__ void stv<__half>(__half* p, long i, float v) {
   p[i] = __float2half(v);
-}
-
-__device__ __forceinline__ int group_of_row(const int* offs, int num_groups, int row) {
-  int lo = 0, hi = num_groups;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (offs[mid] <= row) lo = mid; else hi = mid;
-  }
-  return lo;
 }
 
 // Shared-memory tiled SIMT GEMM for fp64, for fp32 with rows that are not 16-byte aligned (sgemm.cu
@@ -1271,7 +1279,10 @@ cudaError_t launch_gate_topk_softmax_bwd(int logit_dtype, const void* dprob, con
 }
 
 #define FMOE_GATE_TOT(tot, ...)                          \
-  if ((tot) <= 16) { constexpr int TOT = 16; __VA_ARGS__; } \
+  if ((tot) <= 2) { constexpr int TOT = 2; __VA_ARGS__; }       \
+  else if ((tot) <= 4) { constexpr int TOT = 4; __VA_ARGS__; }  \
+  else if ((tot) <= 8) { constexpr int TOT = 8; __VA_ARGS__; }  \
+  else if ((tot) <= 16) { constexpr int TOT = 16; __VA_ARGS__; } \
   else if ((tot) <= 32) { constexpr int TOT = 32; __VA_ARGS__; } \
   else { constexpr int TOT = 64; __VA_ARGS__; }
 
@@ -1314,52 +1325,46 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
   return cudaGetLastError();
 }
 
+int gate_bwd_ranges(int n_rows, int d) {
+  // a block per SM over the strips and token ranges, a warp at least four tokens
+  const int strips = (d + 255) / 256;
+  int ranges = (148 + strips - 1) / strips;
+  if (ranges > (n_rows + 31) / 32) ranges = (n_rows + 31) / 32;
+  return ranges > 0 ? ranges : 1;
+}
+
 cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, const void* prob,
                             const void* dlogits_in, const void* x, const void* w, int n_rows, int d,
-                            int tot, int k, float* dl_scratch, void* dx, float* dw, float* db,
+                            int tot, int k, float* dl_scratch, void* dx, float* part, void* dw_db,
                             cudaStream_t stream) {
   if (n_rows == 0) return cudaSuccess;
   if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
-  const int per = gate_rows_per_warp(n_rows, tot);
-  const int grid = (n_rows + 8 * per - 1) / (8 * per);
-#define FMOE_GATE_DX(TOT, R)                                                                             \
-  FMOE_DISPATCH_16(dtype, (gate_bwd_dx_kernel<T, TOT, R><<<grid, 256, 0, stream>>>(                      \
-      static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in), \
-      static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx))))
-  if (tot <= 2) {
-    if (per == 1) { FMOE_GATE_DX(2, 1); } else if (per == 2) { FMOE_GATE_DX(2, 2); } else { FMOE_GATE_DX(2, 4); }
-  } else if (tot <= 4) {
-    if (per == 1) { FMOE_GATE_DX(4, 1); } else if (per == 2) { FMOE_GATE_DX(4, 2); } else { FMOE_GATE_DX(4, 4); }
-  } else if (tot <= 8) {
-    if (per == 1) { FMOE_GATE_DX(8, 1); } else if (per == 2) { FMOE_GATE_DX(8, 2); } else { FMOE_GATE_DX(8, 4); }
-  } else if (tot <= 16) {
-    FMOE_GATE_DX(16, 1);
-  } else if (tot <= 32) {
-    FMOE_GATE_DX(32, 1);
-  } else {
-    FMOE_GATE_DX(64, 1);
-  }
-#undef FMOE_GATE_DX
+  const int grid = (n_rows + 7) / 8;
+  FMOE_DISPATCH_16(dtype, FMOE_GATE_TOT(tot, (gate_bwd_dx_kernel<T, TOT><<<grid, 256, 0, stream>>>(
+      static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in),
+      static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx)))));
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  if (dw == nullptr) return cudaSuccess;
+  if (part == nullptr) return cudaSuccess;
   if (tot > 16) return cudaErrorInvalidValue;
-  // two blocks per SM over the strips and token ranges, a warp at least four tokens; the partial
-  // sums of the ranges are merged with atomics
-  const int strips = (d + 255) / 256;
-  int splits = (2 * 148 + strips - 1) / strips;
-  if (splits > (n_rows + 31) / 32) splits = (n_rows + 31) / 32;
-  dim3 g2(strips, splits);
+  const int ranges = gate_bwd_ranges(n_rows, d);
+  dim3 g2((d + 255) / 256, ranges);
   if (tot <= 2) {
     FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 2><<<g2, 256, 0, stream>>>(
-        dl_scratch, static_cast<const T*>(x), n_rows, d, tot, dw, db)));
+        dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
+  } else if (tot <= 4) {
+    FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 4><<<g2, 256, 0, stream>>>(
+        dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   } else if (tot <= 8) {
     FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 8><<<g2, 256, 0, stream>>>(
-        dl_scratch, static_cast<const T*>(x), n_rows, d, tot, dw, db)));
+        dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   } else {
     FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 16><<<g2, 256, 0, stream>>>(
-        dl_scratch, static_cast<const T*>(x), n_rows, d, tot, dw, db)));
+        dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   }
+  const long elems = static_cast<long>(tot) * d + tot;
+  FMOE_DISPATCH_16(dtype, (gate_bwd_merge_kernel<T><<<static_cast<unsigned>((elems + 31) / 32), 256, 0, stream>>>(
+      part, ranges, elems, static_cast<T*>(dw_db))));
   return cudaGetLastError();
 }
 

@@ -72,13 +72,14 @@ bool gate_fused_supported(int tot, int d, int k);
 cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, const void* bias,
                                     int n_rows, int d, int tot, int k, void* logits, int64_t* idx,
                                     void* prob, cudaStream_t stream);
-// Backward of the fused gate.  dl_scratch: fp32 [n_rows, tot]; dx (optional) [n_rows, d];
-// dw fp32 [tot, d] and db fp32 [tot] (optional) must be zero on entry (accumulated with
-// atomics).  The weight gradient kernel covers tot <= 16: pass dw = nullptr above that and
-// form dW = dl^T x from dl_scratch with a library GEMM.
+// Backward of the fused gate.  dl_scratch: fp32 [n_rows, tot]; dx (optional) [n_rows, d].
+// part (optional, tot <= 16): fp32 scratch of gate_bwd_ranges() * (tot * d + tot) entries; with it
+// dw_db receives dW [tot, d] followed by db [tot] in the layer's type.  Above 16 experts pass
+// part = nullptr and form dW = dl^T x from dl_scratch with a library GEMM.
+int gate_bwd_ranges(int n_rows, int d);
 cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, const void* prob,
                             const void* dlogits_in, const void* x, const void* w, int n_rows, int d,
-                            int tot, int k, float* dl_scratch, void* dx, float* dw, float* db,
+                            int tot, int k, float* dl_scratch, void* dx, float* part, void* dw_db,
                             cudaStream_t stream);
 
 // Reference-precision grouped GEMM for fp32 / fp64 and for shapes the tensor-core kernel
