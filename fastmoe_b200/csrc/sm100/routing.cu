@@ -671,7 +671,7 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
   const uint4* xr[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) xr[r] = reinterpret_cast<const uint4*>(x + static_cast<long>(min(row0 + r, n_rows - 1)) * d);
-#pragma unroll 2
+#pragma unroll 1
   for (int i = lane; i < nv; i += 32) {
     uint4 xv[R];
 #pragma unroll
@@ -724,45 +724,28 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
   if (row_ok && e_of < tot && (lane & (kStep - 1)) == 0) {
     logits[static_cast<long>(row0 + r) * tot + e_of] = V2<T>::from_f(mine);
   }
-  float all[TOT];
+  // Every lane ranks its logit among those of its token (ties to the lower id, NaN last) and writes
+  // the entry of that rank: a handful of instructions where a selection loop unrolled into
+  // registers was long enough to be bound by instruction fetch (8 tokens: 17 us).
   const int base = lane & ~(TOT * kStep - 1);   // first lane of this token's group
+  const float key = (e_of < tot && mine == mine) ? mine : -INFINITY;
+  int pos = 0;
+  float top = -INFINITY;
 #pragma unroll
-  for (int e = 0; e < TOT; ++e) all[e] = __shfl_sync(0xffffffffu, mine, base + e * kStep);
-  if (lane == base && row_ok) {
-    // constant bounds keep the selection in registers (TOT <= kMaxK, k <= tot)
-    float sel_v[TOT];
-    int sel_i[TOT];
-    unsigned taken = 0u;
+  for (int e = 0; e < TOT; ++e) {
+    const float other = __shfl_sync(0xffffffffu, key, base + e * kStep);
+    pos += (other > key || (other == key && e < e_of)) ? 1 : 0;
+    top = fmaxf(top, other);
+  }
+  const bool chosen = e_of < tot && pos < k;
+  const float ex = chosen ? __expf(mine - top) : 0.f;
+  float den = ex;
 #pragma unroll
-    for (int j = 0; j < TOT; ++j) {
-      if (j >= k) break;
-      float best = -INFINITY;
-      int best_i = -1;
-#pragma unroll
-      for (int e = 0; e < TOT; ++e) {
-        if (e < tot && !((taken >> e) & 1u) && (best_i < 0 || all[e] > best)) {
-          best = all[e];
-          best_i = e;
-        }
-      }
-      taken |= 1u << best_i;
-      sel_v[j] = best;
-      sel_i[j] = best_i;
-    }
-    float den = 0.f, ex[TOT];
-#pragma unroll
-    for (int j = 0; j < TOT; ++j) {
-      if (j >= k) break;
-      ex[j] = __expf(sel_v[j] - sel_v[0]);
-      den += ex[j];
-    }
-    const long o = static_cast<long>(row0 + r) * k;
-#pragma unroll
-    for (int j = 0; j < TOT; ++j) {
-      if (j >= k) break;
-      idx[o + j] = sel_i[j];
-      prob[o + j] = V2<T>::from_f(ex[j] / den);
-    }
+  for (int o = kStep; o < TOT * kStep; o <<= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+  if (row_ok && chosen && (lane & (kStep - 1)) == 0) {
+    const long o = static_cast<long>(row0 + r) * k + pos;
+    idx[o] = e_of;
+    prob[o] = V2<T>::from_f(ex / den);
   }
 }
 
@@ -829,7 +812,7 @@ gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
 // as before, kept too few bytes in flight).  The ranges used to be merged with atomics on a
 // zeroed buffer: 296 additions per address took most of the 20 us of 16384 tokens with d = 256.
 template <typename T, int TOT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, TOT <= 8 ? 2 : 1)
 gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_rows, int d, int tot,
                    float* __restrict__ part) {
   __shared__ float red[8][256 + 8];
@@ -1326,9 +1309,9 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
 }
 
 int gate_bwd_ranges(int n_rows, int d) {
-  // a block per SM over the strips and token ranges, a warp at least four tokens
+  // two blocks per SM over the strips and token ranges, a warp at least four tokens
   const int strips = (d + 255) / 256;
-  int ranges = (148 + strips - 1) / strips;
+  int ranges = (2 * 148 + strips - 1) / strips;
   if (ranges > (n_rows + 31) / 32) ranges = (n_rows + 31) / 32;
   return ranges > 0 ? ranges : 1;
 }
