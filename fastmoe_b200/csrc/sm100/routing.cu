@@ -671,7 +671,7 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
   const uint4* xr[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) xr[r] = reinterpret_cast<const uint4*>(x + static_cast<long>(min(row0 + r, n_rows - 1)) * d);
-#pragma unroll 1
+#pragma unroll(R == 1 ? 4 : 2)
   for (int i = lane; i < nv; i += 32) {
     uint4 xv[R];
 #pragma unroll
@@ -679,7 +679,8 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
     uint4 wv[TOT];
 #pragma unroll
     for (int e = 0; e < TOT; ++e) {
-      wv[e] = e < tot ? __ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(e) * d) + i) : make_uint4(0u, 0u, 0u, 0u);
+      // (past the last expert the last one again, for nothing: the loads need no predicate)
+      wv[e] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(min(e, tot - 1)) * d) + i);
     }
     float xf[R][8];
 #pragma unroll
