@@ -32,8 +32,8 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // are visited in order, 32 at a time.  The chain of these steps is what bounds the kernel (a
 // match of 32 keys and an update of shared memory that the next step waits for), so up to
 // kRouteClusterSlots slots are spread over a cluster of eight CTAs, which exchange their
-// per-expert totals through distributed shared memory in the one launch: 16384 slots took 19 us
-// on one CTA.  For more slots the work is spread over more CTAs and two launches: the first
+// per-expert totals through distributed shared memory in the one launch: 16384 slots on 8 experts
+// 19 -> 6.8 us, 8192 slots on 64 experts 17.9 -> 6.4 us.  For more slots the work is spread over more CTAs and two launches: the first
 // (`part_out`) only writes every CTA's per-expert totals, the second (`part_in`) starts each CTA's
 // prefixes at the sum of the totals of the CTAs before it.  Ranks are always those of a single
 // ordered scan.
@@ -793,29 +793,6 @@ gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
   if (dx == nullptr) return;
   uint4* out = reinterpret_cast<uint4*>(dx + static_cast<long>(row) * d);
   const int nv = d >> 3;
-  if (TOT <= 8 && dlogits_in != nullptr) {
-    // every expert has a gradient: loads without a predicate, which are all in flight at once
-#pragma unroll 2
-    for (int i = lane; i < nv; i += 32) {
-      uint4 wv[TOT];
-#pragma unroll
-      for (int e = 0; e < TOT; ++e) {
-        wv[e] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(min(e, tot - 1)) * d) + i);
-      }
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int e = 0; e < TOT; ++e) {
-        if (e < tot && dl[e] != 0.f) {
-          float wf[8];
-          unpack8<T>(wv[e], wf);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) acc[q] = fmaf(dl[e], wf[q], acc[q]);
-        }
-      }
-      out[i] = pack8<T>(acc);
-    }
-    return;
-  }
 #pragma unroll 4
   for (int i = lane; i < nv; i += 32) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -836,7 +813,9 @@ gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
 // `gridDim.y` token ranges: part[range][tot * d + tot] in fp32.  A block takes a 256-column strip;
 // a lane owns eight columns, so that a token is one 16-byte load per lane (two columns per lane,
 // as before, kept too few bytes in flight).  The ranges used to be merged with atomics on a
-// zeroed buffer: 296 additions per address took most of the 20 us of 16384 tokens with d = 256.
+// zeroed buffer: 296 additions per address took most of the 20 us of 16384 tokens with d = 256,
+// which take 6 us now and 5 in the merge; 8192 tokens, d = 2048, 8 experts 40 -> 18 us, 11264 tokens,
+// d = 512 19 -> 10 us.  Two blocks per SM; with one 29 and 13 us.
 template <typename T, int TOT>
 __global__ void __launch_bounds__(256, TOT <= 8 ? 2 : 1)
 gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_rows, int d, int tot,
@@ -855,19 +834,13 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
 #pragma unroll
     for (int q = 0; q < 8; ++q) acc[e][q] = 0.f;
   }
-  constexpr int U = TOT <= 8 ? 4 : 2;
+  constexpr int U = 4;
   for (int t = t0 + warp; t < t1; t += 8 * U) {
     uint4 xv[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       xv[u] = (t + 8 * u < t1 && col < d) ? __ldg(reinterpret_cast<const uint4*>(x + static_cast<long>(t + 8 * u) * d + col))
                                           : make_uint4(0u, 0u, 0u, 0u);
-    }
-    float gv[U][TOT];   // unconditional loads (of valid entries): predicated ones were issued one by one
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-#pragma unroll
-      for (int e = 0; e < TOT; ++e) gv[u][e] = __ldg(dl + static_cast<long>(min(t + 8 * u, t1 - 1)) * tot + min(e, tot - 1));
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -877,7 +850,7 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
 #pragma unroll
       for (int e = 0; e < TOT; ++e) {
         if (e < tot) {
-          const float g = gv[u][e];
+          const float g = __ldg(dl + static_cast<long>(t + 8 * u) * tot + e);
 #pragma unroll
           for (int q = 0; q < 8; ++q) acc[e][q] = fmaf(g, xf[q], acc[e][q]);
           if (sums) bsum[e] += g;

@@ -20,14 +20,25 @@ from .ops import api as _ops
 from .parallel.comm import ensure_comm, get_moe_group  # noqa: F401  (re-exported)
 
 
-def count_by_gate(gate, num_expert, world_size, require_pos=True):
+def count_by_gate(gate, num_expert, world_size, require_pos=True, cut_pos=True):
     r"""Routing summary ``(pos, local_expert_count, global_expert_count)``.
 
     ``pos`` lists the kept slots grouped by ascending global expert id (ascending slot id
-    inside a group); the counts are int64 tensors on the device of ``gate``.
+    inside a group); the counts are int64 tensors on the device of ``gate``.  With ``cut_pos``
+    false ``pos`` may be longer than the number of kept slots (entries past it are undefined).
     """
     with torch.no_grad():
         tot = num_expert * world_size
+        if require_pos and gate.is_cuda:
+            # counts and the sorted slot list from one launch; the list comes at full length and is
+            # cut to the kept slots by whoever knows their number (`prepare_forward`)
+            counts, pos, n_kept = _ops.route_pos(gate, tot)
+            local_expert_count = counts.long()
+            if world_size > 1:
+                global_expert_count = _ops.expert_exchange(local_expert_count, num_expert, world_size)
+            else:
+                global_expert_count = local_expert_count
+            return pos[:n_kept()] if cut_pos else pos, local_expert_count, global_expert_count
         counts, rank = _ops.route(gate, tot)
         local_expert_count = counts.long()
         if world_size > 1:
@@ -41,8 +52,6 @@ def count_by_gate(gate, num_expert, world_size, require_pos=True):
         kept = flat >= 0
         dest = starts[flat.clamp(min=0)] + rank.long()
         slots = torch.arange(flat.numel(), device=flat.device)
-        # Boolean indexing sizes its result from device data: this is the one host read of
-        # the general path, shared with the counts copy below in `prepare_forward`.
         pos = torch.empty(int(kept.sum()), dtype=torch.long, device=flat.device)
         pos[dest[kept]] = slots[kept]
     return pos, local_expert_count, global_expert_count
@@ -50,10 +59,15 @@ def count_by_gate(gate, num_expert, world_size, require_pos=True):
 
 def prepare_forward(gate, num_expert, world_size):
     r"""``(pos, lec_cpu, gec_cpu, fwd_expert_count_cpu, fwd_batch_size)`` for one layer call."""
-    pos, lec, gec = count_by_gate(gate, num_expert, world_size)
+    pos, lec, gec = count_by_gate(gate, num_expert, world_size, cut_pos=False)
     with torch.no_grad():
-        both = torch.stack([lec, gec]).cpu()
-        lec_cpu, gec_cpu = both[0], both[1]
+        # the one device -> host read of the general path
+        if gec is lec:
+            lec_cpu = gec_cpu = lec.cpu()
+        else:
+            both = torch.stack([lec, gec]).cpu()
+            lec_cpu, gec_cpu = both[0], both[1]
+        pos = pos[:int(lec_cpu.sum())]
         fwd_expert_count = gec_cpu.view(world_size, num_expert).sum(dim=0)
         fwd_batch_size = int(fwd_expert_count.sum())
     return pos, lec_cpu, gec_cpu, fwd_expert_count, fwd_batch_size
@@ -64,12 +78,12 @@ def _local_scatter(inp, pos):
 
 
 def _local_gather(inp, pos, out_batch_size, maybe_overlap=True):
-    out = torch.zeros((out_batch_size,) + tuple(inp.shape[1:]), dtype=inp.dtype, device=inp.device)
+    shape = (out_batch_size,) + tuple(inp.shape[1:])
     if maybe_overlap:
-        out.index_add_(0, pos, inp)
-    else:
-        out.index_copy_(0, pos, inp)
-    return out
+        return torch.zeros(shape, dtype=inp.dtype, device=inp.device).index_add_(0, pos, inp)
+    # distinct positions: without a dropped slot every row is written and none has to be zeroed
+    alloc = torch.empty if pos.shape[0] == out_batch_size else torch.zeros
+    return alloc(shape, dtype=inp.dtype, device=inp.device).index_copy_(0, pos, inp)
 
 
 class MOEScatter(Function):

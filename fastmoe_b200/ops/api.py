@@ -56,6 +56,14 @@ def route(gate_idx, tot_expert):
     return cnt, rank
 
 
+def route_pos(gate_idx, tot_expert):
+    r"""``(counts int32[tot], pos int64[n_slots], n_kept)`` of a CUDA ``gate_idx`` from one launch:
+    ``pos`` lists the kept slots by expert, then slot id; ``n_kept()`` reads their number on the
+    host, and entries of ``pos`` past it are undefined."""
+    counts, _rank, offs, pos = native.get().route_pos(gate_idx.contiguous().view(-1), int(tot_expert))
+    return counts, pos[:gate_idx.numel()].long(), lambda: int(offs[-1])
+
+
 def limit_by_capacity(expert_count_w, capacity, n_expert, n_worker):
     if expert_count_w.is_cuda:
         return native.get().limit_by_capacity(expert_count_w, capacity, int(n_expert), int(n_worker))
