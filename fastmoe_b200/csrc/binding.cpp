@@ -514,6 +514,75 @@ torch::Tensor gate_topk_softmax_bwd(torch::Tensor dprob, torch::Tensor idx, torc
   return dlogits;
 }
 
+// ------------------------------------------------------------------------------ balanced gates
+bool balance_supported(int64_t tot) { return fmoe::balance_supported(static_cast<int>(tot)); }
+
+// Slots of every expert beyond the first `cap` (in slot order) become -1.
+torch::Tensor prune_gate_scalar(torch::Tensor idx, int64_t cap, int64_t tot) {
+  check_cuda_contig(idx, "gate_idx");
+  auto flat = idx.view({-1});
+  auto res = route(flat, tot, false);
+  c10::cuda::CUDAGuard guard(idx.device());
+  auto out = torch::empty_like(idx);
+  FMOE_CUDA_CHECK(fmoe::launch_prune_scalar(flat.data_ptr<int64_t>(), res[1].data_ptr<int>(),
+                                            static_cast<int>(std::min<int64_t>(cap, INT32_MAX)),
+                                            static_cast<int>(flat.numel()), static_cast<int>(tot),
+                                            out.data_ptr<int64_t>(), cur_stream()));
+  return out;
+}
+
+void check_logits(const torch::Tensor& logits) {
+  TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1 && logits.size(0) > 0,
+              "logits must be a non-empty CUDA matrix with contiguous rows");
+}
+
+// {loss, weight}: see routing.cuh.  `ids` is [n, ...]: its first column counts.
+std::vector<torch::Tensor> balance_loss(torch::Tensor logits, torch::Tensor ids, bool is_switch, double scale) {
+  check_logits(logits);
+  check_cuda_contig(ids, "ids");
+  TORCH_CHECK(ids.scalar_type() == torch::kLong && ids.size(0) == logits.size(0), "ids must be int64 [n, k]");
+  c10::cuda::CUDAGuard guard(logits.device());
+  const int n = static_cast<int>(logits.size(0)), tot = static_cast<int>(logits.size(1));
+  auto f32 = torch::dtype(torch::kFloat).device(logits.device());
+  auto part = torch::empty({static_cast<long>(fmoe::balance_blocks(n)) * 2 * tot}, f32);
+  auto loss = torch::empty({}, f32);
+  auto weight = torch::empty({tot}, f32);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  FMOE_CUDA_CHECK(fmoe::launch_balance_loss(logit_code(logits), logits.data_ptr(), logits.stride(0),
+                                            ids.data_ptr<int64_t>(), static_cast<int>(ids.numel() / n), n, tot,
+                                            is_switch, static_cast<float>(scale), part.data_ptr<float>(),
+                                            loss.data_ptr<float>(), weight.data_ptr<float>(), cur_stream()));
+  return {loss, weight};
+}
+
+torch::Tensor balance_bwd(torch::Tensor logits, torch::Tensor weight, c10::optional<torch::Tensor> dloss,
+                          c10::optional<torch::Tensor> win, c10::optional<torch::Tensor> dscore) {
+  check_logits(logits);
+  c10::cuda::CUDAGuard guard(logits.device());
+  const int n = static_cast<int>(logits.size(0)), tot = static_cast<int>(logits.size(1));
+  TORCH_CHECK(!dloss.has_value() || (dloss->scalar_type() == torch::kFloat && dloss->numel() == 1), "dloss");
+  TORCH_CHECK(!dscore.has_value() || (dscore->scalar_type() == logits.scalar_type() && dscore->numel() == n &&
+                                      dscore->is_contiguous() && win.has_value()), "dscore");
+  auto dlogits = torch::empty({n, tot}, logits.options());
+  FMOE_CUDA_CHECK(fmoe::launch_balance_bwd(
+      logit_code(logits), logits.data_ptr(), logits.stride(0), weight.data_ptr<float>(),
+      dloss.has_value() ? dloss->data_ptr<float>() : nullptr, win.has_value() ? win->data_ptr<int64_t>() : nullptr,
+      dscore.has_value() ? dscore->data_ptr() : nullptr, n, tot, dlogits.data_ptr(), cur_stream()));
+  return dlogits;
+}
+
+std::vector<torch::Tensor> switch_top1(torch::Tensor logits) {
+  check_logits(logits);
+  check_cuda_contig(logits, "logits");
+  c10::cuda::CUDAGuard guard(logits.device());
+  const int n = static_cast<int>(logits.size(0)), tot = static_cast<int>(logits.size(1));
+  auto win = torch::empty({n, 1}, torch::dtype(torch::kLong).device(logits.device()));
+  auto score = torch::empty({n, 1}, logits.options());
+  FMOE_CUDA_CHECK(fmoe::launch_switch_top1(logit_code(logits), logits.data_ptr(), n, tot, win.data_ptr<int64_t>(),
+                                           score.data_ptr(), cur_stream()));
+  return {win, score};
+}
+
 bool gate_fused_supported(int64_t tot, int64_t d, int64_t k) {
   return fmoe::gate_fused_supported(static_cast<int>(tot), static_cast<int>(d), static_cast<int>(k));
 }
@@ -627,6 +696,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_mlp_backward", &moe_mlp_backward);
   m.def("gate_topk_softmax", &gate_topk_softmax);
   m.def("gate_topk_softmax_bwd", &gate_topk_softmax_bwd);
+  m.def("balance_supported", &balance_supported);
+  m.def("prune_gate_scalar", &prune_gate_scalar);
+  m.def("balance_loss", &balance_loss);
+  m.def("balance_bwd", &balance_bwd);
+  m.def("switch_top1", &switch_top1);
   m.def("gate_fused_supported", &gate_fused_supported);
   m.def("gate_linear_topk", &gate_linear_topk);
   m.def("gate_linear_topk_bwd", &gate_linear_topk_bwd);

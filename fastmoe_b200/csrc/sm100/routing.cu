@@ -562,6 +562,146 @@ __global__ void gate_topk_softmax_bwd_kernel(const T* __restrict__ dprob,
   }
 }
 
+// ------------------------------------------------------------------------------ balance losses
+// GShard: loss = mean_e(c_e m_e) scale, c_e = share of the tokens whose first choice is e, m_e = mean
+// softmax probability; Switch: loss = scale sum_e (f_e / K) (P_e / K) with f_e the kept tokens of e,
+// P_e the sum of its probabilities and K = max(1, kept).  Both are  factor * sum_e count_e P_e  with
+// a factor that only depends on the counts.  As PyTorch operations a loss and its gradient were
+// about 25 launches of 1 to 17 us; here: partial sums per block, one block that adds them in order,
+// and one pass for the gradient.  One thread per token, tot <= kBalanceMaxExperts, sums in fp32.
+constexpr int kBalanceMaxExperts = 64;
+constexpr int kBalanceThreads = 128;
+
+// softmax(logits[row])_e = exp(l_e - mx) / den
+template <typename T>
+__device__ __forceinline__ void row_softmax(const T* in, int tot, float& mx, float& inv_den) {
+  mx = -INFINITY;
+  for (int e = 0; e < tot; ++e) mx = fmaxf(mx, Ld<T>::get(in, e));
+  float den = 0.f;
+  for (int e = 0; e < tot; ++e) den += __expf(Ld<T>::get(in, e) - mx);
+  inv_den = 1.f / den;
+}
+
+// part[block][2 * tot]: kept tokens and probability sums of the block's tokens per expert.
+template <typename T>
+__global__ void __launch_bounds__(kBalanceThreads)
+balance_sums_kernel(const T* __restrict__ logits, long pitch, const int64_t* __restrict__ ids, int id_stride, int n,
+                    int tot, float* __restrict__ part) {
+  __shared__ float red[kBalanceThreads / 32][2 * kBalanceMaxExperts];
+  const int t = blockIdx.x * kBalanceThreads + threadIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const T* in = logits + static_cast<long>(min(t, n - 1)) * pitch;
+  const long id = t < n ? ids[static_cast<long>(t) * id_stride] : -1;
+  float mx, inv;
+  row_softmax<T>(in, tot, mx, inv);
+  for (int e = 0; e < tot; ++e) {
+    float p = t < n ? __expf(Ld<T>::get(in, e) - mx) * inv : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+    const int c = __popc(__ballot_sync(0xffffffffu, id == e));
+    if (lane == 0) {
+      red[warp][e] = static_cast<float>(c);
+      red[warp][tot + e] = p;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * tot; i += kBalanceThreads) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < kBalanceThreads / 32; ++w) s += red[w][i];
+    part[static_cast<long>(blockIdx.x) * 2 * tot + i] = s;
+  }
+}
+
+// One block: adds the blocks' sums; `weight` [tot] receives d loss / d P_e.
+__global__ void __launch_bounds__(1024)
+balance_finish_kernel(const float* __restrict__ part, int blocks, int n, int tot, int is_switch, float scale,
+                      float* __restrict__ loss, float* __restrict__ weight) {
+  __shared__ float red[32][2 * kBalanceMaxExperts];
+  __shared__ float total[2 * kBalanceMaxExperts];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = lane; i < 2 * tot; i += 32) {
+    float s = 0.f;
+    for (int b = warp; b < blocks; b += 32) s += part[static_cast<long>(b) * 2 * tot + i];
+    red[warp][i] = s;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * tot; i += blockDim.x) {
+    float s = 0.f;
+    for (int w = 0; w < 32; ++w) s += red[w][i];
+    total[i] = s;
+  }
+  __syncthreads();
+  float kept = 0.f;
+  for (int e = 0; e < tot; ++e) kept += total[e];
+  kept = fmaxf(kept, 1.f);
+  const float factor = is_switch ? scale / (kept * kept) : scale / (static_cast<float>(tot) * n * n);
+  if (threadIdx.x == 0) {
+    float s = 0.f;
+    for (int e = 0; e < tot; ++e) s += total[e] * total[tot + e];
+    *loss = s * factor;
+  }
+  for (int e = threadIdx.x; e < tot; e += blockDim.x) weight[e] = total[e] * factor;
+}
+
+// dlogits[t, e] = p_e (g_e - sum_i g_i p_i) with g_e = dloss * weight_e, and, for a score that is
+// the probability of expert win[t], dscore[t] added to g of that expert (win / dscore may be null).
+template <typename T>
+__global__ void __launch_bounds__(kBalanceThreads)
+balance_bwd_kernel(const T* __restrict__ logits, long pitch, const float* __restrict__ weight,
+                   const float* __restrict__ dloss, const int64_t* __restrict__ win, const T* __restrict__ dscore,
+                   int n, int tot, T* __restrict__ dlogits) {
+  const int t = blockIdx.x * kBalanceThreads + threadIdx.x;
+  if (t >= n) return;
+  const T* in = logits + static_cast<long>(t) * pitch;
+  float mx, inv;
+  row_softmax<T>(in, tot, mx, inv);
+  const float gl = dloss != nullptr ? *dloss : 0.f;
+  const float gs = dscore != nullptr ? Ld<T>::get(dscore, t) : 0.f;
+  const long w = win != nullptr ? win[t] : -1;
+  float dot = 0.f;
+  for (int e = 0; e < tot; ++e) {
+    const float p = __expf(Ld<T>::get(in, e) - mx) * inv;
+    dot += p * (gl * weight[e] + (e == w ? gs : 0.f));
+  }
+  for (int e = 0; e < tot; ++e) {
+    const float p = __expf(Ld<T>::get(in, e) - mx) * inv;
+    Ld<T>::put(dlogits, static_cast<long>(t) * tot + e, p * (gl * weight[e] + (e == w ? gs : 0.f) - dot));
+  }
+}
+
+// Switch: the most probable expert (the lower id wins a tie) and its softmax probability.
+template <typename T>
+__global__ void __launch_bounds__(kBalanceThreads)
+switch_top1_kernel(const T* __restrict__ logits, int n, int tot, int64_t* __restrict__ win, T* __restrict__ score) {
+  const int t = blockIdx.x * kBalanceThreads + threadIdx.x;
+  if (t >= n) return;
+  const T* in = logits + static_cast<long>(t) * tot;
+  float mx, inv;
+  row_softmax<T>(in, tot, mx, inv);
+  // as torch.max over the probabilities: NaN counts as the largest, the first of equals wins
+  int best = 0;
+  float best_p = __expf(Ld<T>::get(in, 0) - mx) * inv;
+  for (int e = 1; e < tot; ++e) {
+    const float p = __expf(Ld<T>::get(in, e) - mx) * inv;
+    if (p > best_p || (p != p && best_p == best_p)) {
+      best = e;
+      best_p = p;
+    }
+  }
+  win[t] = best;
+  Ld<T>::put(score, t, best_p);
+}
+
+// new_idx[s] = idx[s] when fewer than `cap` slots of its expert come before it, else -1
+__global__ void prune_scalar_kernel(const int64_t* __restrict__ idx, const int* __restrict__ rank, int cap, int n_slots,
+                                    int tot, int64_t* __restrict__ out) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n_slots) return;
+  const long e = idx[s];
+  out[s] = (e >= 0 && e < tot && rank[s] < cap) ? e : -1;
+}
+
 // ------------------------------------------------------------------------------ fused gate
 // logits = x W^T + b for a handful of experts (tot <= kGateMaxExperts), top-k and softmax of the
 // selected logits, one warp per token: x is read once, W comes from L1/L2, nothing but the
@@ -1263,6 +1403,50 @@ cudaError_t launch_gate_topk_softmax_bwd(int logit_dtype, const void* dprob, con
         static_cast<const float*>(dprob), idx, static_cast<const float*>(prob), n_rows, n_experts,
         k, static_cast<float*>(dlogits));
   }
+  return cudaGetLastError();
+}
+
+#define FMOE_DISPATCH_LOGITS(code, ...)                                   \
+  if ((code) == 0) { using T = __nv_bfloat16; __VA_ARGS__; }              \
+  else if ((code) == 1) { using T = __half; __VA_ARGS__; }                \
+  else { using T = float; __VA_ARGS__; }
+
+bool balance_supported(int tot) { return tot >= 1 && tot <= kBalanceMaxExperts; }
+int balance_blocks(int n) { return (n + kBalanceThreads - 1) / kBalanceThreads; }
+
+cudaError_t launch_balance_loss(int code, const void* logits, long pitch, const int64_t* ids, int id_stride, int n,
+                                int tot, bool is_switch, float scale, float* part, float* loss, float* weight,
+                                cudaStream_t stream) {
+  if (n < 1 || !balance_supported(tot)) return cudaErrorInvalidValue;
+  const int blocks = balance_blocks(n);
+  FMOE_DISPATCH_LOGITS(code, (balance_sums_kernel<T><<<blocks, kBalanceThreads, 0, stream>>>(
+      static_cast<const T*>(logits), pitch, ids, id_stride, n, tot, part)));
+  balance_finish_kernel<<<1, 1024, 0, stream>>>(part, blocks, n, tot, is_switch ? 1 : 0, scale, loss, weight);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_balance_bwd(int code, const void* logits, long pitch, const float* weight, const float* dloss,
+                               const int64_t* win, const void* dscore, int n, int tot, void* dlogits,
+                               cudaStream_t stream) {
+  if (n < 1 || !balance_supported(tot)) return cudaErrorInvalidValue;
+  FMOE_DISPATCH_LOGITS(code, (balance_bwd_kernel<T><<<balance_blocks(n), kBalanceThreads, 0, stream>>>(
+      static_cast<const T*>(logits), pitch, weight, dloss, win, static_cast<const T*>(dscore), n, tot,
+      static_cast<T*>(dlogits))));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_switch_top1(int code, const void* logits, int n, int tot, int64_t* win, void* score,
+                               cudaStream_t stream) {
+  if (n < 1 || !balance_supported(tot)) return cudaErrorInvalidValue;
+  FMOE_DISPATCH_LOGITS(code, (switch_top1_kernel<T><<<balance_blocks(n), kBalanceThreads, 0, stream>>>(
+      static_cast<const T*>(logits), n, tot, win, static_cast<T*>(score))));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_prune_scalar(const int64_t* idx, const int* rank, int cap, int n_slots, int tot, int64_t* new_idx,
+                                cudaStream_t stream) {
+  if (n_slots == 0) return cudaSuccess;
+  prune_scalar_kernel<<<(n_slots + 255) / 256, 256, 0, stream>>>(idx, rank, cap, n_slots, tot, new_idx);
   return cudaGetLastError();
 }
 

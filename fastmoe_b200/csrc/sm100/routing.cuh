@@ -66,6 +66,26 @@ cudaError_t launch_gate_topk_softmax_bwd(int logit_dtype, const void* dprob, con
                                          const void* prob, int n_rows, int n_experts, int k,
                                          void* dlogits, cudaStream_t stream);
 
+// Balance losses of the capacity-limited gates and Switch's choice (logit_dtype as above, `pitch`
+// elements between rows of logits, tot <= 64, n >= 1).  part: fp32 [balance_blocks(n)][2 * tot];
+// loss fp32 scalar; weight fp32 [tot], handed to the backward.  ids[t * id_stride] is the expert a
+// token counts for (-1: none).  The backward takes dloss (device scalar or null) and, for a score
+// that is the softmax probability of expert win[t], dscore (or null); dlogits is [n, tot].
+bool balance_supported(int tot);
+int balance_blocks(int n);
+cudaError_t launch_balance_loss(int logit_dtype, const void* logits, long pitch, const int64_t* ids, int id_stride, int n,
+                                int tot, bool is_switch, float scale, float* part, float* loss, float* weight,
+                                cudaStream_t stream);
+cudaError_t launch_balance_bwd(int logit_dtype, const void* logits, long pitch, const float* weight, const float* dloss,
+                               const int64_t* win, const void* dscore, int n, int tot, void* dlogits,
+                               cudaStream_t stream);
+cudaError_t launch_switch_top1(int logit_dtype, const void* logits, int n, int tot, int64_t* win, void* score,
+                               cudaStream_t stream);
+
+// new_idx[s] = (idx[s] in range && rank[s] < cap) ? idx[s] : -1
+cudaError_t launch_prune_scalar(const int64_t* idx, const int* rank, int cap, int n_slots, int tot, int64_t* new_idx,
+                                cudaStream_t stream);
+
 // Fused gate: logits = x W^T + b (tot <= 64 experts, 16-bit types), top-k ids (descending) and
 // softmax over the selected logits; one pass over x.
 bool gate_fused_supported(int tot, int d, int k);

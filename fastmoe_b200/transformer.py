@@ -37,7 +37,27 @@ def activation_kind(act):
         return "gelu"
     if act is torch.nn.functional.relu or act is torch.relu:
         return "relu"
+    if type(act) is nn.Sequential and not _hooked(act):
+        # a chain whose other members do nothing in this call: the Transformer-XL block's
+        # ReLU -> Dropout at evaluation, or with p = 0
+        live = [m for m in act if not _does_nothing(m)]
+        if not live:
+            return "identity"
+        if len(live) == 1 and not _hooked(live[0]):
+            return activation_kind(live[0])
     return None
+
+
+def _hooked(module):
+    r"""Whether somebody watches calls of ``module``, which a fused activation would not make."""
+    return any(getattr(module, name, None) for name in
+               ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks"))
+
+
+def _does_nothing(module):
+    inert = type(module) is nn.Identity or (
+        type(module) is nn.Dropout and (module.p == 0 or not module.training))
+    return inert and not _hooked(module)
 
 
 class _Expert(nn.Module):
