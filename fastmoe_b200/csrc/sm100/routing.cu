@@ -578,7 +578,7 @@ __device__ __forceinline__ void row_softmax(const T* in, int tot, float& mx, flo
   mx = -INFINITY;
   for (int e = 0; e < tot; ++e) mx = fmaxf(mx, Ld<T>::get(in, e));
   float den = 0.f;
-  for (int e = 0; e < tot; ++e) den += __expf(Ld<T>::get(in, e) - mx);
+  for (int e = 0; e < tot; ++e) den += expf(Ld<T>::get(in, e) - mx);
   inv_den = 1.f / den;
 }
 
@@ -595,7 +595,7 @@ balance_sums_kernel(const T* __restrict__ logits, long pitch, const int64_t* __r
   float mx, inv;
   row_softmax<T>(in, tot, mx, inv);
   for (int e = 0; e < tot; ++e) {
-    float p = t < n ? __expf(Ld<T>::get(in, e) - mx) * inv : 0.f;
+    float p = t < n ? expf(Ld<T>::get(in, e) - mx) * inv : 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
     const int c = __popc(__ballot_sync(0xffffffffu, id == e));
@@ -661,11 +661,11 @@ balance_bwd_kernel(const T* __restrict__ logits, long pitch, const float* __rest
   const long w = win != nullptr ? win[t] : -1;
   float dot = 0.f;
   for (int e = 0; e < tot; ++e) {
-    const float p = __expf(Ld<T>::get(in, e) - mx) * inv;
+    const float p = expf(Ld<T>::get(in, e) - mx) * inv;
     dot += p * (gl * weight[e] + (e == w ? gs : 0.f));
   }
   for (int e = 0; e < tot; ++e) {
-    const float p = __expf(Ld<T>::get(in, e) - mx) * inv;
+    const float p = expf(Ld<T>::get(in, e) - mx) * inv;
     Ld<T>::put(dlogits, static_cast<long>(t) * tot + e, p * (gl * weight[e] + (e == w ? gs : 0.f) - dot));
   }
 }
@@ -681,9 +681,9 @@ switch_top1_kernel(const T* __restrict__ logits, int n, int tot, int64_t* __rest
   row_softmax<T>(in, tot, mx, inv);
   // as torch.max over the probabilities: NaN counts as the largest, the first of equals wins
   int best = 0;
-  float best_p = __expf(Ld<T>::get(in, 0) - mx) * inv;
+  float best_p = expf(Ld<T>::get(in, 0) - mx) * inv;
   for (int e = 1; e < tot; ++e) {
-    const float p = __expf(Ld<T>::get(in, e) - mx) * inv;
+    const float p = expf(Ld<T>::get(in, e) - mx) * inv;
     if (p > best_p || (p != p && best_p == best_p)) {
       best = e;
       best_p = p;

@@ -8,7 +8,7 @@ import torch
 import torch.nn.functional as F
 
 from .naive_gate import NaiveGate
-from ..ops import api as _ops
+from ..ops import api as _ops, gating
 
 
 def gshard_balance_loss(logits, top1_idx, tot_expert, num_expert):
@@ -41,14 +41,20 @@ class GShardGate(NaiveGate):
         self.random_routing = random_routing
 
     def forward(self, x):
-        topk_idx, topk_val, logits = super().forward(x, return_all_scores=True)
-        logits = logits.view(-1, self.tot_expert)
-        self.set_loss(gshard_balance_loss(logits, topk_idx[:, 0], self.tot_expert, self.num_expert))
-
+        logits, topk_idx, topk_val = self._choose(x)
         rate = self.capacity[0 if self.training else 1]
         cap = math.ceil(rate * x.shape[0]) * self.top_k // self.tot_expert
-        cap_t = torch.full((self.tot_expert,), cap, dtype=torch.int32, device=topk_idx.device)
-        topk_idx = _ops.prune_gate_by_capacity(topk_idx, cap_t, self.num_expert, self.world_size)
+        if gating.balance_native(logits):
+            self.set_loss(gating.gshard_loss(
+                logits, topk_idx, self.num_expert ** 2,
+                lambda l, ids: gshard_balance_loss(l, ids[:, 0], self.tot_expert, self.num_expert)))
+        else:
+            self.set_loss(gshard_balance_loss(logits, topk_idx[:, 0], self.tot_expert, self.num_expert))
+        if topk_idx.is_cuda and topk_idx.numel() > 0:
+            topk_idx = gating.prune_to_capacity(topk_idx, cap, self.tot_expert)
+        else:
+            cap_t = torch.full((self.tot_expert,), cap, dtype=torch.int32, device=topk_idx.device)
+            topk_idx = _ops.prune_gate_by_capacity(topk_idx, cap_t, self.num_expert, self.world_size)
 
         if self.random_routing:
             topk_idx = drop_second_expert_randomly(topk_idx, topk_val)

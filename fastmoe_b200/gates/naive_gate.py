@@ -19,9 +19,12 @@ class NaiveGate(BaseGate):
         self.gate = nn.Linear(d_model, self.tot_expert, bias=gate_bias)
         self.top_k = top_k
 
-    def forward(self, inp, return_all_scores=False):
-        logits, idx, score = gating.linear_topk_softmax(
+    def _choose(self, inp):
+        return gating.linear_topk_softmax(
             inp.reshape(-1, inp.shape[-1]), self.gate.weight, self.gate.bias, self.top_k)
+
+    def forward(self, inp, return_all_scores=False):
+        logits, idx, score = self._choose(inp)
         logits = logits.view(*inp.shape[:-1], self.tot_expert)
         # The reference installs a zero "dummy" loss so that callers can always add it.
         self.set_loss(torch.zeros(1, device=inp.device, requires_grad=True))

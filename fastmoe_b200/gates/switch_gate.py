@@ -15,6 +15,7 @@ import torch
 
 from .naive_gate import NaiveGate
 from .utils import limit_by_capacity
+from ..ops import gating
 
 
 class SwitchGate(NaiveGate):
@@ -46,11 +47,21 @@ class SwitchGate(NaiveGate):
         share.scatter_add_(0, ids.clamp(min=0), kept)
         return self.tot_expert * ((share / n_kept) * (prob.sum(dim=0) / n_kept)).sum()
 
+    def _score_and_loss(self, logits, chosen, winner):
+        r"""The score of the experts ``chosen`` and the loss for the kept ones ``winner``."""
+        prob = torch.softmax(logits.float(), dim=-1)
+        return prob.gather(1, chosen).to(logits.dtype), self._balance_loss(prob, winner)
+
     def forward(self, inp):
-        prob = torch.softmax(self._jitter(self.gate(inp)).float(), dim=-1)
+        logits = self._jitter(self.gate(inp))
+        cap = self._slots_per_expert(inp.shape[0])
+        if self.world_size == 1 and logits.dtype == inp.dtype and gating.balance_native(logits):
+            winner, score, loss = gating.switch_route(logits, cap, self._score_and_loss)
+            self.set_loss(loss)
+            return winner, score
+        prob = torch.softmax(logits.float(), dim=-1)
         score, winner = prob.max(dim=-1, keepdim=True)
-        _, _, winner = limit_by_capacity(winner, self.num_expert, self.world_size,
-                                         self._slots_per_expert(inp.shape[0]),
+        _, _, winner = limit_by_capacity(winner, self.num_expert, self.world_size, cap,
                                          group=getattr(self, "moe_group", None))
         self.set_loss(self._balance_loss(prob, winner))
         return winner, score.to(inp.dtype)

@@ -168,3 +168,84 @@ def linear_topk_softmax(x, weight, bias, k):
     logits = torch.nn.functional.linear(x, weight, bias)
     idx, prob = topk_softmax(logits, k)
     return logits, idx, prob
+
+
+# ------------------------------------------------------------------ capacity-limited gates
+def balance_native(logits):
+    r"""Whether the balance-loss kernels take these logits (a non-empty CUDA matrix, 16 or 32 bits, at
+    most 64 experts)."""
+    return (logits.is_cuda and logits.dim() == 2 and logits.shape[0] > 0 and logits.stride(1) == 1
+            and logits.dtype in (torch.float32, torch.bfloat16, torch.float16)
+            and native.get().balance_supported(logits.shape[1]))
+
+
+def prune_to_capacity(idx, cap, tot_expert):
+    r"""``idx`` with the slots of every expert beyond its first ``cap`` (slot order) set to -1."""
+    return native.get().prune_gate_scalar(idx.contiguous(), int(cap), int(tot_expert))
+
+
+class _BalanceLoss(Function):
+    r"""``reference(logits, ids)`` — GShard's loss — from two launches, its gradient from one."""
+
+    @staticmethod
+    def forward(ctx, logits, ids, scale, reference):
+        loss, weight = native.get().balance_loss(logits, ids, False, float(scale))
+        ctx.save_for_backward(logits, ids, weight)
+        ctx.reference = reference
+        return loss
+
+    @staticmethod
+    def backward(ctx, grad):
+        logits, ids, weight = ctx.saved_tensors
+        if torch.is_grad_enabled():   # a gradient of the gradient is wanted
+            with torch.enable_grad():
+                (dl,) = torch.autograd.grad(ctx.reference(logits, ids), logits, grad, create_graph=True)
+        else:
+            dl = native.get().balance_bwd(logits, weight, grad.contiguous(), None, None)
+        return dl, None, None, None
+
+
+def gshard_loss(logits, ids, scale, reference):
+    return _BalanceLoss.apply(logits, ids.contiguous(), scale, reference)
+
+
+class _SwitchRoute(Function):
+    r"""Switch's choice, capacity limit and balance loss of one rank: ``(ids [n, 1], score [n, 1],
+    loss)``.  ``reference(logits, ids)`` gives ``(score, loss)`` in PyTorch operations for the
+    given pruned ids and winners."""
+
+    @staticmethod
+    def forward(ctx, logits, cap, reference):
+        nat = native.get()
+        tot = logits.shape[1]
+        win, score = nat.switch_top1(logits)
+        kept = nat.prune_gate_scalar(win, cap, tot)
+        loss, weight = nat.balance_loss(logits, kept, True, float(tot))
+        ctx.save_for_backward(logits, win, kept, weight)
+        ctx.reference = reference
+        ctx.mark_non_differentiable(kept)
+        ctx.set_materialize_grads(False)
+        return kept, score, loss
+
+    @staticmethod
+    def backward(ctx, _grad_kept, grad_score, grad_loss):
+        logits, win, kept, weight = ctx.saved_tensors
+        if grad_score is None and grad_loss is None:
+            return None, None, None
+        if torch.is_grad_enabled():   # a gradient of the gradient is wanted
+            with torch.enable_grad():
+                outs, grads = [], []
+                for out, grad in zip(ctx.reference(logits, win, kept), (grad_score, grad_loss)):
+                    if grad is not None:
+                        outs.append(out)
+                        grads.append(grad)
+                (dl,) = torch.autograd.grad(outs, logits, grads, create_graph=True)
+        else:
+            dl = native.get().balance_bwd(logits, weight, None if grad_loss is None else grad_loss.contiguous(),
+                                          None if grad_score is None else win,
+                                          None if grad_score is None else grad_score.contiguous())
+        return dl, None, None
+
+
+def switch_route(logits, cap, reference):
+    return _SwitchRoute.apply(logits.contiguous(), int(min(cap, 2 ** 31 - 1)), reference)

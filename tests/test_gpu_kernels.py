@@ -522,3 +522,65 @@ def test_gate_rows_per_warp(dtype, rows, tot, k, d):
     assert close(x.grad, dl, w.detach().double())
     assert close(w.grad, dl.t(), x.detach().double())
     assert close(b.grad[None], torch.ones(1, rows, device=DEV, dtype=torch.float64), dl)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("kind", ["gshard", "switch"])
+@pytest.mark.parametrize("n,tot", [(1, 2), (127, 3), (129, 64), (5000, 8), (40000, 2)])
+def test_balanced_gates_native_loss(dtype, kind, n, tot, monkeypatch):
+    r"""Ids, scores, loss and gradients of the capacity-limited gates with the balance-loss kernels
+    against the PyTorch operations, which run in 64 bits on the same logits: one rounding to the
+    layer's type, fp32 sums over the tokens and experts."""
+    from fastmoe_b200.gates import GShardGate, SwitchGate
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(16)
+    d = 64
+    gate = (GShardGate(d, tot, 1, random_routing=False) if kind == "gshard" else
+            SwitchGate(d, tot, 1, switch_eps=0.0)).to(DEV).to(dtype)
+    x = torch.randn(n, d, device=DEV).to(dtype)
+    idx, score = gate(x)
+    loss = gate.get_loss()
+    gs = torch.randn_like(score)
+    torch.autograd.backward([score, loss], [gs, None])
+    grads = [p.grad.double() for p in gate.parameters()]
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -20}[dtype]
+
+    gate.zero_grad()
+    monkeypatch.setattr(gating, "balance_native", lambda logits: False)
+    want_idx, want_score = gate(x)
+    want_loss = gate.get_loss()
+    assert torch.equal(idx, want_idx)
+    assert torch.allclose(score.double(), want_score.double(), rtol=2 * eps, atol=1e-6)
+    assert loss.dim() == 0 and loss.dtype == want_loss.dtype
+    # GShard's reference rounds the probabilities and their mean to the layer's type
+    assert torch.allclose(loss.double(), want_loss.double(), rtol=4 * eps + 1e-5)
+    torch.autograd.backward([want_score, want_loss], [gs, None])
+    for g, p in zip(grads, gate.parameters()):
+        scale = p.grad.double().abs().max().clamp(min=1e-6)
+        assert ((g - p.grad.double()).abs() <= (4 * eps + 1e-5 * n ** 0.5) * scale).all()
+
+
+def test_balance_loss_second_derivative():
+    r"""A gradient of the gradient goes through the PyTorch operations."""
+    from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(17)
+    logits = torch.randn(50, 4, device=DEV, requires_grad=True)
+    ids = torch.randint(0, 4, (50, 2), device=DEV)
+    ref = lambda l, i: gshard_balance_loss(l, i[:, 0], 4, 4)   # noqa: E731
+    got = []
+    for loss in (gating.gshard_loss(logits, ids, 16, ref), ref(logits, ids)):
+        (g,) = torch.autograd.grad(loss, logits, create_graph=True)
+        got.append((g, torch.autograd.grad(g.pow(2).sum(), logits)[0]))
+    for a, b in zip(*got):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-9)
+
+
+def test_inert_dropout_is_fused_and_live_dropout_is_not():
+    from fastmoe_b200.transformer import activation_kind
+    seq = torch.nn.Sequential(torch.nn.ReLU(), torch.nn.Dropout(0.5))
+    assert activation_kind(seq) is None and activation_kind(seq.eval()) == "relu"
+    assert activation_kind(torch.nn.Sequential(torch.nn.ReLU(), torch.nn.Dropout(0.0))) == "relu"
+    assert activation_kind(torch.nn.Sequential(torch.nn.ReLU(), torch.nn.Tanh()).eval()) is None
+    seq[0].register_forward_hook(lambda *a: None)
+    assert activation_kind(seq) is None
