@@ -36,16 +36,16 @@ constexpr int TILE_N = 256;
 constexpr int CTA_N = TILE_N / 2;           // columns of B per CTA
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int STAGES = 4;
+constexpr int STAGES = 5;
 constexpr int BOX_BYTES = 64 * BK * 2;      // one 64-wide MN-major box
 constexpr int A_BYTES = CTA_M * BK * 2;
 constexpr int B_BYTES = CTA_N * BK * 2;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int MAX_GROUPS = gg::MAX_GROUPS;
-constexpr int NUM_EPI_WARPS = 16;
-constexpr int FIRST_EPI_WARP = 4;
-constexpr int NUM_THREADS = (FIRST_EPI_WARP + NUM_EPI_WARPS) * 32;
-constexpr int EPI_COLS = TILE_N / 4;        // columns per epilogue warp: one 128-byte line of outputs
+constexpr int NUM_EPI_WARPS = gg::NUM_EPI_WARPS;
+constexpr int FIRST_EPI_WARP = gg::FIRST_EPI_WARP;
+constexpr int NUM_THREADS = gg::NUM_THREADS;
+constexpr int EPI_COLS = TILE_N / 2;        // columns per epilogue warp
 constexpr int EPI_CHUNKS = EPI_COLS / 32;
 constexpr int TMEM_COLS = 512;
 
@@ -173,13 +173,13 @@ template <int ACT> __device__ __forceinline__ void act_grad2(float x0, float x1,
 struct EpiTile {
   uint32_t t_row;           // TMEM address: this warp's lane quarter, first column of its span
   int lane;
-  int n_chunks;             // valid 32-column chunks of the span (0..2)
+  int n_chunks;             // valid 32-column chunks of the span (0..4)
   int warp_valid;           // valid rows of the warp's 32
   uint8_t* patch;
   const uint8_t* bias;      // shared memory: the span's bias values, or null
   uint8_t* out;             // first row, first column of the span
   long out_pitch;
-  uint8_t* pre_tile;        // this warp's 2 x 2 KB of the tile-blocked pre-activation, or null
+  uint8_t* pre_tile;        // this warp's 4 x 2 KB of the tile-blocked pre-activation, or null
   uint32_t empty_bar;       // CTA 0's accumulator-free barrier
 };
 
@@ -229,22 +229,23 @@ __device__ __forceinline__ void finish_chunk(const EpiTile& et, int i, const uin
         *reinterpret_cast<uint4*>(pd + 512) = make_uint4(wp[4], wp[5], wp[6], wp[7]);
       }
     }
-    const int c = i * 4 + q * 2;
+    const int c = (i & 1) * 4 + q * 2;
     *reinterpret_cast<uint4*>(gg::patch_piece(et.patch, et.lane, c)) = make_uint4(wo[0], wo[1], wo[2], wo[3]);
     *reinterpret_cast<uint4*>(gg::patch_piece(et.patch, et.lane, c + 1)) = make_uint4(wo[4], wo[5], wo[6], wo[7]);
   }
 }
 
-// Whole 128-byte lines (64 bytes where the matrix ends), 8 lanes per row.
-__device__ __forceinline__ void send_lines(const EpiTile& et) {
+// After an odd chunk (or the last one): whole 128-byte lines, 8 lanes per row.
+__device__ __forceinline__ void send_lines(const EpiTile& et, int i) {
+  if (!(i + 1 == et.n_chunks || (i & 1))) return;
+  const int bytes = ((i & 1) + 1) * 64;
   const int sub = et.lane & 7;
-  const bool on = sub < et.n_chunks * 4;
-  uint8_t* dst = et.out + sub * 16 + (et.lane >> 3) * et.out_pitch;
+  uint8_t* dst = et.out + (i & ~1) * 64 + sub * 16 + (et.lane >> 3) * et.out_pitch;
   __syncwarp();
 #pragma unroll
   for (int it = 0; it < 8; ++it) {
     const int row = 4 * it + (et.lane >> 3);
-    if (row < et.warp_valid && on) {
+    if (row < et.warp_valid && sub * 16 < bytes) {
       *reinterpret_cast<uint4*>(dst + it * 4 * et.out_pitch) =
           *reinterpret_cast<const uint4*>(gg::patch_piece(et.patch, row, sub));
     }
@@ -258,26 +259,42 @@ __device__ __forceinline__ void release_accumulator(const EpiTile& et) {
   if (et.lane == 0) ptx::mbar_arrive_cluster(et.empty_bar);
 }
 
-// One tile for one epilogue warp.  The chunks are taken one after the other; the other three
-// epilogue warps of the scheduler fill the waits.
+// One tile for one epilogue warp: the tcgen05.ld of chunk i + 1 (and the load of its saved
+// pre-activation) is in flight while chunk i is finished.
 template <typename T, int ACT, bool DACT>
-__device__ __forceinline__ void epilogue_tile(const EpiTile& et, Packed32& side) {
+__device__ __forceinline__ void epilogue_tile(const EpiTile& et, Packed32& side_a) {
+  uint32_t ra[32], rb[32];
+  Packed32 side_b;
+  bool released = false;
   if (et.n_chunks > 0 && et.warp_valid > 0) {
-#pragma unroll
-    for (int i = 0; i < EPI_CHUNKS; ++i) {
-      if (i < et.n_chunks) {
-        uint32_t r[32];
-        ptx::tmem_ld_32x32(et.t_row + i * 32, r);
-        ptx::tmem_ld_wait();
-        if (i + 1 == et.n_chunks) release_accumulator(et);
-        finish_chunk<T, ACT, DACT>(et, i, r, side);
-        if (DACT && i + 1 < et.n_chunks) gg::load_pre_chunk(et.pre_tile, i + 1, et.lane, side);
+    ptx::tmem_ld_32x32(et.t_row, ra);
+#pragma unroll 1
+    for (int i = 0; i < et.n_chunks; i += 2) {
+      ptx::tmem_ld_wait();
+      const bool second = i + 1 < et.n_chunks;
+      if (second) {
+        ptx::tmem_ld_32x32(et.t_row + (i + 1) * 32, rb);
+        if (DACT) gg::load_pre_chunk(et.pre_tile, i + 1, et.lane, side_b);
+      } else {
+        release_accumulator(et);
+        released = true;
       }
+      finish_chunk<T, ACT, DACT>(et, i, ra, side_a);
+      send_lines(et, i);
+      if (!second) break;
+      ptx::tmem_ld_wait();
+      if (i + 2 < et.n_chunks) {
+        ptx::tmem_ld_32x32(et.t_row + (i + 2) * 32, ra);
+        if (DACT) gg::load_pre_chunk(et.pre_tile, i + 2, et.lane, side_a);
+      } else {
+        release_accumulator(et);
+        released = true;
+      }
+      finish_chunk<T, ACT, DACT>(et, i + 1, rb, side_b);
+      send_lines(et, i + 1);
     }
-    send_lines(et);
-  } else {
-    release_accumulator(et);
   }
+  if (!released) release_accumulator(et);
 }
 
 // Weight gradient into an fp32 buffer, or added to the old gradient: the sum is formed in fp32
@@ -346,17 +363,16 @@ __device__ __forceinline__ void column_sums(const Params& p, uint8_t* patches, c
   };
   if (col < p.m) {
     const T* src = static_cast<const T*>(p.psrc) + col;
-    constexpr int kStep = 2 * NUM_EPI_WARPS;   // rows taken by all warps at once
     int r = c.row_begin + ew * 2 + (lane >> 4);
-    constexpr int kUnroll = 8;
-    for (; r + kStep * (kUnroll - 1) < row_end; r += kStep * kUnroll) {
+    constexpr int kUnroll = 16;
+    for (; r + 16 * (kUnroll - 1) < row_end; r += 16 * kUnroll) {
       uint4 v[kUnroll];
 #pragma unroll
-      for (int i = 0; i < kUnroll; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<long>(r + kStep * i) * p.m));
+      for (int i = 0; i < kUnroll; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<long>(r + 16 * i) * p.m));
 #pragma unroll
       for (int i = 0; i < kUnroll; ++i) add(v[i]);
     }
-    for (; r < row_end; r += kStep) add(__ldg(reinterpret_cast<const uint4*>(src + static_cast<long>(r) * p.m)));
+    for (; r < row_end; r += 16) add(__ldg(reinterpret_cast<const uint4*>(src + static_cast<long>(r) * p.m)));
   }
   float* mine = reinterpret_cast<float*>(patches + ew * PATCH_BYTES);
 #pragma unroll
@@ -369,7 +385,7 @@ __device__ __forceinline__ void column_sums(const Params& p, uint8_t* patches, c
   if (tid < CTA_M && col0 + tid < p.m) {
     float total = 0.f;
 #pragma unroll
-    for (int w = 0; w < NUM_EPI_WARPS; ++w) total += reinterpret_cast<const float*>(patches + w * PATCH_BYTES)[tid];
+    for (int w8 = 0; w8 < NUM_EPI_WARPS; ++w8) total += reinterpret_cast<const float*>(patches + w8 * PATCH_BYTES)[tid];
     T* dst = static_cast<T*>(p.psum) + static_cast<long>(c.group) * p.m + col0 + tid;
     if (p.accumulate) total += Cvt<T>::to_f(*dst);
     *dst = Cvt<T>::from_f(total);
@@ -614,30 +630,30 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
     }
   } else {
-    // ============================================================== epilogue (warps 4..19)
-    const int part = warp & 3;                          // TMEM lane quarter this warp may read
-    const int quarter = (warp - FIRST_EPI_WARP) >> 2;   // which 64 accumulator columns
+    // ============================================================== epilogue (warps 4..11)
+    const int part = warp & 3;                       // TMEM lane quarter this warp may read
+    const int half = (warp - FIRST_EPI_WARP) >> 2;   // which half of the accumulator columns
     const int ew = warp - FIRST_EPI_WARP;
     uint8_t* patches = smem + PATCH_OFF;
     uint8_t* bias_sm = smem + BIAS_OFF + ew * BIAS_BYTES;
     const bool has_bias = MODE == kRowsNT && p.bias != nullptr;
-    // this lane's two bias values of a tile, loaded one tile ahead
-    auto load_bias = [&](int tile) -> uint32_t {
-      uint32_t v = 0u;
+    // this lane's four bias values of a tile, loaded one tile ahead
+    auto load_bias = [&](int tile) -> uint2 {
+      uint2 v = make_uint2(0u, 0u);
       if (has_bias && tile < total) {
         const Tile c = decode(sh, p.num_groups, n_tiles, tile);
-        const int col = c.n_tile * TILE_N + quarter * EPI_COLS + lane * 2;
-        if (col < p.n) v = __ldg(reinterpret_cast<const uint32_t*>(static_cast<const T*>(p.bias) + static_cast<long>(c.group) * p.n + col));
+        const int col = c.n_tile * TILE_N + half * EPI_COLS + lane * 4;
+        if (col < p.n) v = __ldg(reinterpret_cast<const uint2*>(static_cast<const T*>(p.bias) + static_cast<long>(c.group) * p.n + col));
       }
       return v;
     };
-    uint32_t bias_next = load_bias(pair);
+    uint2 bias_next = load_bias(pair);
     int iter = 0;
     bool dead = false;   // a wait ran out: walk the remaining tiles' barriers, touch nothing else
     for (int tile = pair; tile < total; tile += num_pairs, ++iter) {
       const Tile c = decode(sh, p.num_groups, n_tiles, tile);
       const int acc = iter & 1;
-      const int col_first = c.n_tile * TILE_N + quarter * EPI_COLS;
+      const int col_first = c.n_tile * TILE_N + half * EPI_COLS;
       const int m0 = c.m_tile * TILE_M + rank * CTA_M + part * 32;
       EpiTile et;
       et.lane = lane;
@@ -648,7 +664,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       et.out_pitch = static_cast<long>(p.n) * 2;
       et.pre_tile = nullptr;
       et.empty_bar = ptx::mapa(&sh->tmem_empty[acc], 0);
-      et.t_row = tmem_base + (static_cast<uint32_t>(part * 32) << 16) + acc * TILE_N + quarter * EPI_COLS;
+      et.t_row = tmem_base + (static_cast<uint32_t>(part * 32) << 16) + acc * TILE_N + half * EPI_COLS;
       const long first_elem = ((MODE == kWgrad) ? static_cast<long>(c.group) * p.m + m0 : static_cast<long>(c.row_begin) + m0) * p.n + col_first;
       et.out = static_cast<uint8_t*>(p.out) + first_elem * 2;
       Packed32 side;
@@ -659,29 +675,28 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       } else {
         const void* pre = (MODE == kRowsNN) ? p.aux : p.pre_out;
         if (ACT != kActNone && pre != nullptr) {
-          // the tile-blocked layout counts 128 x 256 blocks, groups in order; inside a block it goes
-          // by 32 x 128 spans of four chunks, of which this warp has two
-          const int in_block = ((quarter >> 1) * 4 + part) * gg::CHUNKS_PER_WARP + (quarter & 1) * EPI_CHUNKS;
+          // the tile-blocked layout counts 128 x 256 blocks, groups in order
           const long blk = (static_cast<long>(sh->blocks[c.group]) + c.m_tile * 2 + rank) * n_tiles + c.n_tile;
           et.pre_tile = const_cast<uint8_t*>(static_cast<const uint8_t*>(pre)) + blk * gg::PRE_TILE_BYTES +
-                        in_block * gg::PRE_CHUNK_BYTES;
+                        ew * (gg::CHUNKS_PER_WARP * gg::PRE_CHUNK_BYTES);
           if (MODE == kRowsNN && et.n_chunks > 0 && et.warp_valid > 0) {
             // it does not depend on the accumulator: fetch the first chunk before the wait, and
-            // pull the next tile's chunks of this warp (4 KB, one line per lane) into L2
+            // pull the next tile's chunks of this warp (8 KB, two lines per lane) into L2
             gg::load_pre_chunk(et.pre_tile, 0, lane, side);
             if (tile + num_pairs < total) {
               const Tile cn = decode(sh, p.num_groups, n_tiles, tile + num_pairs);
               if (cn.m_tile * TILE_M + rank * CTA_M < cn.rows) {
                 const long nb = (static_cast<long>(sh->blocks[cn.group]) + cn.m_tile * 2 + rank) * n_tiles + cn.n_tile;
                 const uint8_t* nx = static_cast<const uint8_t*>(pre) + nb * gg::PRE_TILE_BYTES +
-                                    in_block * gg::PRE_CHUNK_BYTES + lane * 128;
+                                    ew * (gg::CHUNKS_PER_WARP * gg::PRE_CHUNK_BYTES) + lane * 256;
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(nx));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + 128));
               }
             }
           }
         }
         if (has_bias) {
-          *reinterpret_cast<uint32_t*>(bias_sm + lane * 4) = bias_next;
+          *reinterpret_cast<uint2*>(bias_sm + lane * 8) = bias_next;
           __syncwarp();
           bias_next = load_bias(tile + num_pairs);
         }
