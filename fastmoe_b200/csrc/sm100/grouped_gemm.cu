@@ -3,6 +3,7 @@
 // grouped_gemm_kernel.cuh (row modes with rows arriving from or leaving for other GPUs) and are
 // instantiated per element type in pair_gemm_*.cu / grouped_gemm_*.cu.
 #include "grouped_gemm_kernel.cuh"
+#include "narrow_gemm.cuh"
 #include "pair_gemm_kernel.cuh"
 
 namespace fmoe {
@@ -74,6 +75,29 @@ bool pair_applies(const GroupedGemmArgs& a) {
          (a.act == kActNone || (a.epi == kEpiDAct && a.aux != nullptr));
 }
 
+// A handful of rows per expert and nothing saved for a backward: the weights' bytes are the work.
+bool narrow_applies(const GroupedGemmArgs& a) {
+  return a.mode == kRowsNT && a.epi == kEpiBiasAct && a.pre_out == nullptr && a.rows_cap <= 16L * a.num_groups &&
+         !a.send.enabled && a.gate.flags == nullptr && a.push_meta == nullptr && a.trace == nullptr;
+}
+
+cudaError_t launch_narrow_gemm(const GroupedGemmArgs& a) {
+  CUtensorMap tw, tx;
+  if (!make_map_2d(&tw, a.dtype, a.b, a.k, static_cast<uint64_t>(a.num_groups) * a.n, ng::BK, ng::TILE_N) ||
+      !make_map_2d(&tx, a.dtype, a.a, a.k, a.rows_cap, ng::BK, ng::TILE_ROWS)) {
+    return cudaErrorInvalidValue;
+  }
+  ng::Params p;
+  p.num_groups = a.num_groups;
+  p.n = a.n;
+  p.k = a.k;
+  p.offs = a.offs;
+  p.bias = a.bias;
+  p.out = a.out;
+  p.status = a.status;
+  return ng::launch(a.dtype, a.act, tw, tx, p, a.num_sms > 0 ? a.num_sms : 148, a.stream);
+}
+
 cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
   CUtensorMap ta, tb;
   bool ok = true;
@@ -112,6 +136,7 @@ cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
 
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
   if (!grouped_gemm_supported(a.mode, a.m, a.n, a.k, a.num_groups)) return cudaErrorInvalidValue;
+  if (narrow_applies(a)) return launch_narrow_gemm(a);
   if (pair_applies(a)) return launch_pair_gemm(a);
   CUtensorMap ta, tb;
   bool ok = true;

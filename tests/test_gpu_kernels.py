@@ -584,3 +584,35 @@ def test_inert_dropout_is_fused_and_live_dropout_is_not():
     assert activation_kind(torch.nn.Sequential(torch.nn.ReLU(), torch.nn.Tanh()).eval()) is None
     seq[0].register_forward_hook(lambda *a: None)
     assert activation_kind(seq) is None
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("act", [None, "gelu", "relu", "gelu_tanh"])
+@pytest.mark.parametrize("counts,k,n", [
+    ([1, 0, 2, 0, 0, 0], 64, 32),              # one K block, a quarter of a tile's columns
+    ([0] * 6 + [32, 0], 128, 288),             # exactly one tile of rows, a ragged last column tile
+    ([33, 0, 0, 31] + [0] * 60, 1024, 416),    # a second row tile with one row, ring longer than the K blocks
+    ([65] + [0] * 9, 4096, 128),               # three row tiles of one expert
+])
+def test_narrow_kernel(dtype, act, counts, k, n):
+    r"""A handful of rows per expert, nothing saved: against fp64, one rounding to the 16-bit type, an
+    fp32 sum of k terms and, for the tanh form, the hardware tanh (2^-10.9)."""
+    from fastmoe_b200.ops import grouped_gemm as gg
+    torch.manual_seed(18)
+    g, rows = len(counts), sum(counts)
+    assert rows <= 16 * g
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    offs = _offs(counts)
+    x = torch.randn(rows, k, device=DEV).to(dtype)
+    w = (torch.randn(g, n, k, device=DEV) / k ** 0.5).to(dtype)
+    b = torch.randn(g, n, device=DEV).to(dtype)
+    fn = {None: lambda t: t, "relu": torch.relu, "gelu": torch.nn.functional.gelu,
+          "gelu_tanh": lambda t: torch.nn.functional.gelu(t, approximate="tanh")}[act]
+    for bias in (b, None):
+        y = gg.forward(x, w, offs, bias, act=act)
+        for e, lo, hi in _segments(counts):
+            pre = x[lo:hi].double() @ w[e].double().t() + (0 if bias is None else bias[e].double())
+            ref = fn(pre)
+            bound = eps * ref.abs() + 2.0 ** -22 * k ** 0.5 * 8 + (2.0 ** -11 * pre.abs() if act == "gelu_tanh" else 0) + 1e-6
+            assert ((y[lo:hi].double() - ref).abs() <= bound).all(), e
+    assert _native().read_status(0) == 0
