@@ -1,7 +1,7 @@
 // Host side of the tcgen05 grouped GEMM: tensor-map construction and dispatch.  The kernels live
-// in pair_gemm_kernel.cuh (CTA pairs; every launch without an exchange) and
-// grouped_gemm_kernel.cuh (row modes with rows arriving from or leaving for other GPUs) and are
-// instantiated per element type in pair_gemm_*.cu / grouped_gemm_*.cu.
+// in pair_gemm_kernel.cuh (CTA pairs: most launches), grouped_gemm_kernel.cuh (row modes with rows
+// arriving from or leaving for other GPUs) — instantiated per element type in pair_gemm_*.cu /
+// grouped_gemm_*.cu — and narrow_gemm.cu (decoding).
 #include "grouped_gemm_kernel.cuh"
 #include "narrow_gemm.cuh"
 #include "pair_gemm_kernel.cuh"
@@ -63,9 +63,9 @@ namespace {
 // (8192 rows, 2 experts, 1024 -> 4096 with GELU: 69.0 against 85.5 us; 22528 rows, 8 experts,
 // 512 -> 2048: 79.6 against 101.2 us; weight gradient of 64 experts with 128 rows: 200 against
 // 394 us).  The single-CTA kernel keeps the exchange, whose flags and send units count 128-row
-// blocks, and the launches with a handful of rows per expert, where the weights' bytes are all
-// there is and the finer tiles share them more evenly (a layer of 64 experts on 64 tokens: 227
-// against 238 us).
+// blocks, and the launches with at most 16 rows per expert that narrow_applies leaves, where the
+// weights' bytes are most of the work and the finer tiles share them more evenly (a layer of 64
+// experts on 64 tokens: 227 against 238 us).
 bool pair_applies(const GroupedGemmArgs& a) {
   if (a.mode == kWgrad) return true;
   if (a.send.enabled || a.gate.flags != nullptr || a.push_meta != nullptr || a.trace != nullptr) return false;
@@ -75,9 +75,13 @@ bool pair_applies(const GroupedGemmArgs& a) {
          (a.act == kActNone || (a.epi == kEpiDAct && a.aux != nullptr));
 }
 
-// A handful of rows per expert and nothing saved for a backward: the weights' bytes are the work.
+// A handful of rows per expert and nothing saved for a backward: the weights' bytes are the work
+// (64 experts, 128 rows, 1024 <-> 4096: 74 and 74 us against 85 and 82 of the single-CTA kernel; 8
+// experts, 16 rows: 15 and 23 against 22 and 27).  Up to 256 rows in all: with 1024 rows that go to
+// two of 64 experts every 32-row tile reads the weights again, 43 against 19 us.
 bool narrow_applies(const GroupedGemmArgs& a) {
-  return a.mode == kRowsNT && a.epi == kEpiBiasAct && a.pre_out == nullptr && a.rows_cap <= 16L * a.num_groups &&
+  return a.mode == kRowsNT && a.epi == kEpiBiasAct && a.pre_out == nullptr && a.rows_cap <= 256 &&
+         a.rows_cap <= 16L * a.num_groups &&
          !a.send.enabled && a.gate.flags == nullptr && a.push_meta == nullptr && a.trace == nullptr;
 }
 
