@@ -12,6 +12,7 @@
 // Roles of a CTA (192 threads, persistent over tiles): warp 0 loads (TMA), warp 1 issues the MMAs
 // and owns the TMEM, warps 2-5 finish 32 output columns x 32 rows each: lane = output column.
 #include "grouped_gemm_kernel.cuh"
+#include "launch.cuh"
 #include "narrow_gemm.cuh"
 
 namespace fmoe {
@@ -92,6 +93,7 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     ptx::tmem_alloc(&sh->tmem_base, TMEM_COLS);
     ptx::tmem_relinquish();
   }
+  ptx::chain_begin();   // nothing an earlier kernel writes is read above
   if (warp == 2) {
     int run = 0;
     if (lane == 0) {
@@ -246,8 +248,7 @@ cudaError_t launch_one(const CUtensorMap& tw, const CUtensorMap& tx, const Param
       configured |= 1ull << (dev & 63);
     }
   }
-  kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tw, tx, p);
-  return cudaGetLastError();
+  return launch_chained(kernel, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, tw, tx, p);
 }
 
 template <typename T>

@@ -23,6 +23,7 @@
 // first, 64 experts of 128 rows took 394 us; now 200 us, 537 MB of gradients written.
 #pragma once
 #include "grouped_gemm_kernel.cuh"
+#include "launch.cuh"
 
 namespace fmoe {
 namespace pg {
@@ -427,6 +428,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     ptx::prefetch_tmap(&tm_b);
   }
   if (warp == 1) ptx::tmem_alloc_pair(&sh->tmem_base, TMEM_COLS);
+  ptx::chain_begin();   // nothing an earlier kernel writes is read above
   if (warp == 2) {
     // offsets and the prefixes of tiles and blocks; an expert without rows has no tile
     int run = 0, run_b = 0;
@@ -752,8 +754,7 @@ cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const Param
       configured |= 1ull << (dev & 63);
     }
   }
-  kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(ta, tb, p);
-  return cudaGetLastError();
+  return launch_chained(kernel, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, ta, tb, p);
 }
 
 template <int MODE, typename T>

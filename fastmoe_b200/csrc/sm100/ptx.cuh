@@ -39,6 +39,19 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ----------------------------------------------------------------------------- kernel chains
+// Kernels launched through launch_chained (launch.cuh) may start while the kernel before them in
+// the stream still runs.  Every thread of each of them executes chain_begin() before it touches
+// what an earlier kernel wrote (or that one still reads): everything before it is complete and
+// visible then.  Only after that may the next kernel of the chain be scheduled: no more than two of
+// a chain run at a time, and what a kernel finds in an SM's L1 was loaded after everything but its
+// direct predecessor had ended.  (A kernel that returned without waiting would let its successor
+// pass the kernel before it.)
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -4,6 +4,8 @@
 // (limit_by_capacity, prune_gate_by_capacity), cuda/parallel_linear.cuh:8-53 (column_reduce)
 // and the ATen index_select / index_copy_ / bmm / topk / softmax calls of the reference's layer.
 // All kernels are deterministic: no result depends on the order in which atomics land.
+#include "launch.cuh"
+#include "ptx.cuh"
 #include "routing.cuh"
 
 #include <cooperative_groups.h>
@@ -41,6 +43,7 @@ __global__ void __launch_bounds__(kRouteThreads, 1)
 route_kernel(const int64_t* __restrict__ idx, int n_slots, int tot, int nw, int cta_slots, int in_cluster,
              const int* __restrict__ part_in, int* __restrict__ part_out, int* __restrict__ counts,
              int* __restrict__ rank, int* __restrict__ offs, int* __restrict__ pos) {
+  ptx::chain_begin();
   extern __shared__ int hist[];  // [nw][tot], [tot + 1] expert offsets; in a cluster [tot] totals of this CTA
   int* eoff = hist + nw * tot;
   int* mine = in_cluster ? eoff + tot + 1 : eoff + 1;
@@ -270,6 +273,7 @@ __global__ void scatter_rows_kernel(const T* __restrict__ src, const int64_t* __
                                     const int* __restrict__ rank, const int* __restrict__ base,
                                     const T* __restrict__ scale, int n_slots, int k, int d,
                                     T* __restrict__ dst, int* __restrict__ row_slot) {
+  ptx::chain_begin();
   const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (s >= n_slots) return;
@@ -311,6 +315,7 @@ __global__ void __launch_bounds__(256, 4) gather_combine_kernel(const T* __restr
                                       const int* __restrict__ rank, const int* __restrict__ base,
                                       const T* __restrict__ weight, int n_tokens, int k, int d,
                                       T* __restrict__ out) {
+  ptx::chain_begin();
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (t >= n_tokens) return;
@@ -390,6 +395,7 @@ __global__ void combine_bwd_kernel(const T* __restrict__ dout, const T* __restri
                                    const int* __restrict__ base, const T* __restrict__ weight,
                                    int n_slots, int k, int d, T* __restrict__ drows,
                                    T* __restrict__ dscore) {
+  ptx::chain_begin();
   const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (s >= n_slots) return;
@@ -488,6 +494,7 @@ constexpr int kMaxK = 8;
 template <typename T>
 __global__ void gate_topk_softmax_kernel(const T* __restrict__ logits, int n_rows, int n_experts,
                                          int k, int64_t* __restrict__ idx, T* __restrict__ prob) {
+  ptx::chain_begin();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= n_rows) return;
@@ -802,6 +809,7 @@ __global__ void __launch_bounds__(256)
 gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias,
                              int n_rows, int d, int tot, int k, T* __restrict__ logits,
                              int64_t* __restrict__ idx, T* __restrict__ prob) {
+  ptx::chain_begin();
   constexpr int V = R * TOT;
   const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
   const int lane = threadIdx.x & 31;
@@ -903,6 +911,7 @@ gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
                    const T* __restrict__ prob, const T* __restrict__ dlogits_in,
                    const T* __restrict__ w, int n_rows, int d, int tot, int k,
                    float* __restrict__ dl_out, T* __restrict__ dx) {
+  ptx::chain_begin();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= n_rows) return;
@@ -960,6 +969,7 @@ template <typename T, int TOT>
 __global__ void __launch_bounds__(256, TOT <= 8 ? 2 : 1)
 gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_rows, int d, int tot,
                    float* __restrict__ part) {
+  ptx::chain_begin();
   __shared__ float red[8][256 + 8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 256 + lane * 8;
@@ -1027,6 +1037,7 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
 template <typename T>
 __global__ void __launch_bounds__(256)
 gate_bwd_merge_kernel(const float* __restrict__ part, int ranges, long elems, T* __restrict__ out) {
+  ptx::chain_begin();
   __shared__ float red[8][33];
   const int sub = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long i = static_cast<long>(blockIdx.x) * 32 + lane;
@@ -1245,31 +1256,37 @@ cudaError_t launch_route(const int64_t* idx, int n_slots, int tot, int* counts, 
                                          kRouteSmemLimit);
     if (e != cudaSuccess) return e;
   }
+  const int* none_in = nullptr;
+  int* none_out = nullptr;
   if (nb > 1) {
-    route_kernel<<<nb, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, 0, nullptr, part,
-                                                     counts, rank, offs, pos);
-    route_kernel<<<nb, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, 0, part, nullptr,
-                                                     counts, rank, offs, pos);
-  } else if (cluster) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kRouteCluster);
-    cfg.blockDim = dim3(kRouteThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kRouteCluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, route_kernel, idx, n_slots, tot, nw, cta_slots, 1,
-                              static_cast<const int*>(nullptr), static_cast<int*>(nullptr), counts, rank, offs, pos);
-  } else {
-    route_kernel<<<1, kRouteThreads, smem, stream>>>(idx, n_slots, tot, nw, cta_slots, 0, nullptr, nullptr,
-                                                    counts, rank, offs, pos);
+    const cudaError_t e = launch_chained(route_kernel, dim3(nb), dim3(kRouteThreads), smem, stream, idx, n_slots, tot, nw,
+                                         cta_slots, 0, none_in, part, counts, rank, offs, pos);
+    if (e != cudaSuccess) return e;
+    return launch_chained(route_kernel, dim3(nb), dim3(kRouteThreads), smem, stream, idx, n_slots, tot, nw, cta_slots, 0,
+                          static_cast<const int*>(part), none_out, counts, rank, offs, pos);
   }
-  return cudaGetLastError();
+  if (!cluster) {
+    return launch_chained(route_kernel, dim3(1), dim3(kRouteThreads), smem, stream, idx, n_slots, tot, nw, cta_slots, 0,
+                          none_in, none_out, counts, rank, offs, pos);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kRouteCluster);
+  cfg.blockDim = dim3(kRouteThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kRouteCluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, route_kernel, idx, n_slots, tot, nw, cta_slots, 1, none_in, none_out,
+                                           counts, rank, offs, pos);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_swipe_mark(const int64_t* idx, const int* rank, const int* quota, int n,
@@ -1315,39 +1332,42 @@ cudaError_t launch_fill_pos(const int64_t* idx, const int* rank, const int* cum_
 cudaError_t launch_scatter_rows(int dtype, const void* src, const int64_t* idx, const int* rank,
                                 const int* base, const void* scale, int n_slots, int k, int d,
                                 void* dst, int* row_slot, cudaStream_t stream) {
+  cudaError_t chained = cudaSuccess;
   if (n_slots == 0) return cudaSuccess;
   if (d % 8 != 0) return cudaErrorInvalidValue;
   const int wpb = 8;
-  FMOE_DISPATCH_16(dtype, (scatter_rows_kernel<T><<<(n_slots + wpb - 1) / wpb, wpb * 32, 0, stream>>>(
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(scatter_rows_kernel<T>, dim3((n_slots + wpb - 1) / wpb), dim3(wpb * 32), 0, stream,
       static_cast<const T*>(src), idx, rank, base, static_cast<const T*>(scale), n_slots, k, d,
       static_cast<T*>(dst), row_slot)));
-  return cudaGetLastError();
+  return chained;
 }
 
 cudaError_t launch_gather_combine(int dtype, const void* rows, const int64_t* idx, const int* rank,
                                   const int* base, const void* weight, int n_tokens, int k, int d,
                                   void* out, cudaStream_t stream) {
+  cudaError_t chained = cudaSuccess;
   if (n_tokens == 0) return cudaSuccess;
   if (d % 8 != 0) return cudaErrorInvalidValue;
   const int wpb = 8;
-  FMOE_DISPATCH_16(dtype, (gather_combine_kernel<T><<<(n_tokens + wpb - 1) / wpb, wpb * 32, 0, stream>>>(
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gather_combine_kernel<T>, dim3((n_tokens + wpb - 1) / wpb), dim3(wpb * 32), 0, stream,
       static_cast<const T*>(rows), idx, rank, base, static_cast<const T*>(weight), n_tokens, k, d,
       static_cast<T*>(out))));
-  return cudaGetLastError();
+  return chained;
 }
 
 cudaError_t launch_combine_bwd(int dtype, const void* dout, const void* rows, const int64_t* idx,
                                const int* rank, const int* base, const void* weight, int n_tokens,
                                int k, int d, void* drows, void* dscore, cudaStream_t stream) {
+  cudaError_t chained = cudaSuccess;
   const int n_slots = n_tokens * k;
   if (n_slots == 0) return cudaSuccess;
   if (d % 8 != 0) return cudaErrorInvalidValue;
   const int wpb = 8;
-  FMOE_DISPATCH_16(dtype, (combine_bwd_kernel<T><<<(n_slots + wpb - 1) / wpb, wpb * 32, 0, stream>>>(
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(combine_bwd_kernel<T>, dim3((n_slots + wpb - 1) / wpb), dim3(wpb * 32), 0, stream,
       static_cast<const T*>(dout), static_cast<const T*>(rows), idx, rank, base,
       static_cast<const T*>(weight), n_slots, k, d, static_cast<T*>(drows),
       static_cast<T*>(dscore))));
-  return cudaGetLastError();
+  return chained;
 }
 
 cudaError_t launch_colsum(int dtype, const void* x, const int* offs, int num_groups, long rows_cap,
@@ -1365,22 +1385,23 @@ cudaError_t launch_colsum(int dtype, const void* x, const int* offs, int num_gro
 
 cudaError_t launch_gate_topk_softmax(int logit_dtype, const void* logits, int n_rows, int n_experts,
                                      int k, int64_t* idx, void* prob, cudaStream_t stream) {
+  cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
   if (k < 1 || k > kMaxK || k > n_experts) return cudaErrorInvalidValue;
   const int wpb = 8;
   const int grid = (n_rows + wpb - 1) / wpb;
   if (logit_dtype == 0) {
-    gate_topk_softmax_kernel<__nv_bfloat16><<<grid, wpb * 32, 0, stream>>>(
+    chained = launch_chained(gate_topk_softmax_kernel<__nv_bfloat16>, dim3(grid), dim3(wpb * 32), 0, stream,
         static_cast<const __nv_bfloat16*>(logits), n_rows, n_experts, k, idx,
         static_cast<__nv_bfloat16*>(prob));
   } else if (logit_dtype == 1) {
-    gate_topk_softmax_kernel<__half><<<grid, wpb * 32, 0, stream>>>(
+    chained = launch_chained(gate_topk_softmax_kernel<__half>, dim3(grid), dim3(wpb * 32), 0, stream,
         static_cast<const __half*>(logits), n_rows, n_experts, k, idx, static_cast<__half*>(prob));
   } else {
-    gate_topk_softmax_kernel<float><<<grid, wpb * 32, 0, stream>>>(
+    chained = launch_chained(gate_topk_softmax_kernel<float>, dim3(grid), dim3(wpb * 32), 0, stream,
         static_cast<const float*>(logits), n_rows, n_experts, k, idx, static_cast<float*>(prob));
   }
-  return cudaGetLastError();
+  return chained;
 }
 
 cudaError_t launch_gate_topk_softmax_bwd(int logit_dtype, const void* dprob, const int64_t* idx,
@@ -1472,12 +1493,13 @@ int gate_rows_per_warp(int n_rows, int tot) {
 cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, const void* bias,
                                     int n_rows, int d, int tot, int k, void* logits, int64_t* idx,
                                     void* prob, cudaStream_t stream) {
+  cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
   if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
   const int per = gate_rows_per_warp(n_rows, tot);
   const int grid = (n_rows + 8 * per - 1) / (8 * per);
 #define FMOE_GATE_ROWS(TOT, R)                                                                          \
-  FMOE_DISPATCH_16(dtype, (gate_linear_topk_rows_kernel<T, TOT, R><<<grid, 256, 0, stream>>>(           \
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_linear_topk_rows_kernel<T, TOT, R>, dim3(grid), dim3(256), 0, stream,  \
       static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,  \
       k, static_cast<T*>(logits), idx, static_cast<T*>(prob))))
   if (tot <= 8) {
@@ -1488,7 +1510,7 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
     } else {
       if (per == 1) { FMOE_GATE_ROWS(8, 1); } else if (per == 2) { FMOE_GATE_ROWS(8, 2); } else { FMOE_GATE_ROWS(8, 4); }
     }
-    return cudaGetLastError();
+    return chained;
   }
 #undef FMOE_GATE_ROWS
   FMOE_DISPATCH_16(dtype, FMOE_GATE_TOT(tot, (gate_linear_topk_kernel<T, TOT><<<grid, 256, 0, stream>>>(
@@ -1509,35 +1531,36 @@ cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, co
                             const void* dlogits_in, const void* x, const void* w, int n_rows, int d,
                             int tot, int k, float* dl_scratch, void* dx, float* part, void* dw_db,
                             cudaStream_t stream) {
+  cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
   if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
   const int grid = (n_rows + 7) / 8;
-  FMOE_DISPATCH_16(dtype, FMOE_GATE_TOT(tot, (gate_bwd_dx_kernel<T, TOT><<<grid, 256, 0, stream>>>(
+  FMOE_DISPATCH_16(dtype, FMOE_GATE_TOT(tot, (chained = launch_chained(gate_bwd_dx_kernel<T, TOT>, dim3(grid), dim3(256), 0, stream,
       static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in),
       static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx)))));
-  cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess) return err;
+  if (chained != cudaSuccess) return chained;
   if (part == nullptr) return cudaSuccess;
   if (tot > 16) return cudaErrorInvalidValue;
   const int ranges = gate_bwd_ranges(n_rows, d);
   dim3 g2((d + 255) / 256, ranges);
   if (tot <= 2) {
-    FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 2><<<g2, 256, 0, stream>>>(
+    FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 2>, g2, dim3(256), 0, stream,
         dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   } else if (tot <= 4) {
-    FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 4><<<g2, 256, 0, stream>>>(
+    FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 4>, g2, dim3(256), 0, stream,
         dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   } else if (tot <= 8) {
-    FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 8><<<g2, 256, 0, stream>>>(
+    FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 8>, g2, dim3(256), 0, stream,
         dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   } else {
-    FMOE_DISPATCH_16(dtype, (gate_bwd_dw_kernel<T, 16><<<g2, 256, 0, stream>>>(
+    FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 16>, g2, dim3(256), 0, stream,
         dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   }
+  if (chained != cudaSuccess) return chained;
   const long elems = static_cast<long>(tot) * d + tot;
-  FMOE_DISPATCH_16(dtype, (gate_bwd_merge_kernel<T><<<static_cast<unsigned>((elems + 31) / 32), 256, 0, stream>>>(
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_merge_kernel<T>, dim3(static_cast<unsigned>((elems + 31) / 32)), dim3(256), 0, stream,
       part, ranges, elems, static_cast<T*>(dw_db))));
-  return cudaGetLastError();
+  return chained;
 }
 
 cudaError_t launch_simt_grouped_gemm(int mode, int elem, int num_groups, long rows_cap, int m, int n,
