@@ -10,8 +10,8 @@ class NaiveGate(BaseGate):
     r"""``Linear(d_model → tot_expert)``, top-k of the logits, softmax over the k selected logits.
 
     State-dict keys: ``gate.weight [tot_expert, d_model]``, ``gate.bias [tot_expert]``.
-    On a GPU with 16-bit parameters and at most 64 experts the linear layer, the top-k and the
-    softmax are one kernel (two in backward); otherwise the top-k + softmax are.
+    On a GPU with 16-bit parameters and at most 8 experts the linear layer, the top-k and the
+    softmax are one kernel (three in backward); otherwise the top-k + softmax are.
     """
 
     def __init__(self, d_model, num_expert, world_size, top_k=2, gate_bias=True):

@@ -9,8 +9,8 @@ Jacobian in backward and scatters the result into the dense logits gradient.
 ``linear_topk_softmax`` goes one step further for the plain linear gate
 (``fmoe/gates/naive_gate.py:24-38``: ``nn.Linear`` → ``topk`` → ``softmax``): with at most 64
 experts the logits of a token fit in registers, so one kernel reads the token once and writes
-logits, ids and probabilities, and the backward is two kernels (softmax Jacobian + ``dx``;
-``dW`` and ``db``) instead of the six of the ATen sequence.
+logits, ids and probabilities, and the backward is three kernels (softmax Jacobian + ``dx``; partial
+sums of ``dW`` and ``db``; their merge) instead of the six of the ATen sequence.
 """
 import torch
 from torch.autograd import Function
@@ -144,9 +144,9 @@ def linear_topk_softmax(x, weight, bias, k):
     r"""``(logits [B,E], idx int64 [B,k], prob [B,k])`` of a linear gate over 2-D ``x``.
 
     Uses the single-pass kernel when the shape allows it (16-bit types on a GPU, ``d_model`` a
-    multiple of 8) and the expert count is small enough for its one-warp-per-token SIMT dot
-    products to beat a library GEMM (measured on B200 with 4096 tokens, ``d_model`` 1024:
-    30.6 vs 35.5 µs forward + backward at 2 experts, 52 vs 37 µs at 16).  Above that the
+    multiple of 8) and the expert count is small enough for its SIMT dot products to beat a GEMM
+    (with one token per warp, 4096 tokens, ``d_model`` 1024: 30.6 vs 35.5 µs forward + backward at 2
+    experts, 52 vs 37 µs at 16; up to 8 experts warps take several tokens, 17.5 µs at 2).  Above that the
     product runs on the tcgen05 grouped-GEMM kernel with a single group (:class:`_GateGemm`),
     followed by :func:`topk_softmax`; only 32-/64-bit inputs, CPU tensors and odd ``d_model``
     take the ``linear`` → :func:`topk_softmax` sequence of PyTorch ops.
