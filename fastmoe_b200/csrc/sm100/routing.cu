@@ -1513,9 +1513,18 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
     return chained;
   }
 #undef FMOE_GATE_ROWS
-  FMOE_DISPATCH_16(dtype, FMOE_GATE_TOT(tot, (gate_linear_topk_kernel<T, TOT><<<grid, 256, 0, stream>>>(
-      static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,
-      k, static_cast<T*>(logits), idx, static_cast<T*>(prob)))));
+#define FMOE_GATE_WIDE(TOT)                                                                             \
+  FMOE_DISPATCH_16(dtype, (gate_linear_topk_kernel<T, TOT><<<grid, 256, 0, stream>>>(                   \
+      static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,  \
+      k, static_cast<T*>(logits), idx, static_cast<T*>(prob))))
+  if (tot <= 16) {
+    FMOE_GATE_WIDE(16);
+  } else if (tot <= 32) {
+    FMOE_GATE_WIDE(32);
+  } else {
+    FMOE_GATE_WIDE(64);
+  }
+#undef FMOE_GATE_WIDE
   return cudaGetLastError();
 }
 
