@@ -556,18 +556,20 @@ std::vector<torch::Tensor> balance_loss(torch::Tensor logits, torch::Tensor ids,
 }
 
 torch::Tensor balance_bwd(torch::Tensor logits, torch::Tensor weight, c10::optional<torch::Tensor> dloss,
-                          c10::optional<torch::Tensor> win, c10::optional<torch::Tensor> dscore) {
+                          c10::optional<torch::Tensor> win, c10::optional<torch::Tensor> dscore, bool is_switch,
+                          double scale) {
   check_logits(logits);
   c10::cuda::CUDAGuard guard(logits.device());
   const int n = static_cast<int>(logits.size(0)), tot = static_cast<int>(logits.size(1));
   TORCH_CHECK(!dloss.has_value() || (dloss->scalar_type() == torch::kFloat && dloss->numel() == 1), "dloss");
   TORCH_CHECK(!dscore.has_value() || (dscore->scalar_type() == logits.scalar_type() && dscore->numel() == n &&
-                                      dscore->is_contiguous() && win.has_value()), "dscore");
+                                      dscore->is_contiguous() && win.has_value() && is_switch), "dscore");
   auto dlogits = torch::empty({n, tot}, logits.options());
   FMOE_CUDA_CHECK(fmoe::launch_balance_bwd(
       logit_code(logits), logits.data_ptr(), logits.stride(0), weight.data_ptr<float>(),
       dloss.has_value() ? dloss->data_ptr<float>() : nullptr, win.has_value() ? win->data_ptr<int64_t>() : nullptr,
-      dscore.has_value() ? dscore->data_ptr() : nullptr, n, tot, dlogits.data_ptr(), cur_stream()));
+      dscore.has_value() ? dscore->data_ptr() : nullptr, n, tot, is_switch, static_cast<float>(scale),
+      dlogits.data_ptr(), cur_stream()));
   return dlogits;
 }
 

@@ -572,25 +572,34 @@ __global__ void gate_topk_softmax_bwd_kernel(const T* __restrict__ dprob,
 // ------------------------------------------------------------------------------ balance losses
 // GShard: loss = mean_e(c_e m_e) scale, c_e = share of the tokens whose first choice is e, m_e = mean
 // softmax probability; Switch: loss = scale sum_e (f_e / K) (P_e / K) with f_e the kept tokens of e,
-// P_e the sum of its probabilities and K = max(1, kept).  Both are  factor * sum_e count_e P_e  with
-// a factor that only depends on the counts.  As PyTorch operations a loss and its gradient were
-// about 25 launches of 1 to 17 us; here: partial sums per block, one block that adds them in order,
-// and one pass for the gradient.  One thread per token, tot <= kBalanceMaxExperts, sums in fp32.
+// P_e the sum of its probabilities and K = max(1, kept).  As PyTorch operations a loss and its
+// gradient were about 25 launches of 1 to 17 us; here: partial sums per block, one block that adds
+// them in order, and one pass for the gradient.  One thread per token, tot <= kBalanceMaxExperts.
+// Sums are formed in fp32.  Switch holds everything else in fp32 too, as its PyTorch operations do;
+// GShard's operations hold the probabilities, their mean and the gradients of both in the type T of
+// the logits, and the kernels round where they round: with two experts in fp16 a gradient without
+// those roundings moves the gate's bias gradient by up to 1e-2.
 constexpr int kBalanceMaxExperts = 64;
 constexpr int kBalanceThreads = 128;
 
+// `v` as a tensor of type T holds it
+template <typename T> __device__ __forceinline__ float rounded(float v) {
+  T t;
+  Ld<T>::put(&t, 0, v);
+  return Ld<T>::get(&t, 0);
+}
+
 // softmax(logits[row])_e = exp(l_e - mx) / den
 template <typename T>
-__device__ __forceinline__ void row_softmax(const T* in, int tot, float& mx, float& inv_den) {
+__device__ __forceinline__ void row_softmax(const T* in, int tot, float& mx, float& den) {
   mx = -INFINITY;
   for (int e = 0; e < tot; ++e) mx = fmaxf(mx, Ld<T>::get(in, e));
-  float den = 0.f;
+  den = 0.f;
   for (int e = 0; e < tot; ++e) den += expf(Ld<T>::get(in, e) - mx);
-  inv_den = 1.f / den;
 }
 
 // part[block][2 * tot]: kept tokens and probability sums of the block's tokens per expert.
-template <typename T>
+template <typename T, bool SWITCH>
 __global__ void __launch_bounds__(kBalanceThreads)
 balance_sums_kernel(const T* __restrict__ logits, long pitch, const int64_t* __restrict__ ids, int id_stride, int n,
                     int tot, float* __restrict__ part) {
@@ -599,10 +608,12 @@ balance_sums_kernel(const T* __restrict__ logits, long pitch, const int64_t* __r
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const T* in = logits + static_cast<long>(min(t, n - 1)) * pitch;
   const long id = t < n ? ids[static_cast<long>(t) * id_stride] : -1;
-  float mx, inv;
-  row_softmax<T>(in, tot, mx, inv);
+  float mx, den;
+  row_softmax<T>(in, tot, mx, den);
   for (int e = 0; e < tot; ++e) {
-    float p = t < n ? expf(Ld<T>::get(in, e) - mx) * inv : 0.f;
+    float p = expf(Ld<T>::get(in, e) - mx) / den;
+    if (!SWITCH) p = rounded<T>(p);
+    if (t >= n) p = 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
     const int c = __popc(__ballot_sync(0xffffffffu, id == e));
@@ -620,9 +631,11 @@ balance_sums_kernel(const T* __restrict__ logits, long pitch, const int64_t* __r
   }
 }
 
-// One block: adds the blocks' sums; `weight` [tot] receives d loss / d P_e.
+// One block: adds the blocks' sums.  `weight` [tot] receives d loss / d P_e of Switch, the shares
+// c_e of GShard.
+template <typename T, bool SWITCH>
 __global__ void __launch_bounds__(1024)
-balance_finish_kernel(const float* __restrict__ part, int blocks, int n, int tot, int is_switch, float scale,
+balance_finish_kernel(const float* __restrict__ part, int blocks, int n, int tot, float scale,
                       float* __restrict__ loss, float* __restrict__ weight) {
   __shared__ float red[32][2 * kBalanceMaxExperts];
   __shared__ float total[2 * kBalanceMaxExperts];
@@ -639,41 +652,64 @@ balance_finish_kernel(const float* __restrict__ part, int blocks, int n, int tot
     total[i] = s;
   }
   __syncthreads();
-  float kept = 0.f;
-  for (int e = 0; e < tot; ++e) kept += total[e];
-  kept = fmaxf(kept, 1.f);
-  const float factor = is_switch ? scale / (kept * kept) : scale / (static_cast<float>(tot) * n * n);
+  const float inv_n = 1.f / static_cast<float>(n);
+  float factor = inv_n;
+  if (SWITCH) {
+    float kept = 0.f;
+    for (int e = 0; e < tot; ++e) kept += total[e];
+    kept = fmaxf(kept, 1.f);
+    factor = scale / (kept * kept);
+  }
   if (threadIdx.x == 0) {
     float s = 0.f;
-    for (int e = 0; e < tot; ++e) s += total[e] * total[tot + e];
-    *loss = s * factor;
+    for (int e = 0; e < tot; ++e) {
+      s += SWITCH ? total[e] * total[tot + e] : total[e] * inv_n * rounded<T>(total[tot + e] * inv_n);
+    }
+    *loss = SWITCH ? s * factor : s * (1.f / static_cast<float>(tot)) * scale;
   }
   for (int e = threadIdx.x; e < tot; e += blockDim.x) weight[e] = total[e] * factor;
 }
 
-// dlogits[t, e] = p_e (g_e - sum_i g_i p_i) with g_e = dloss * weight_e, and, for a score that is
-// the probability of expert win[t], dscore[t] added to g of that expert (win / dscore may be null).
-template <typename T>
+// Switch: dlogits[t, e] = p_e (g_e - sum_i g_i p_i) with g_e = dloss * weight_e, and, for a score
+// that is the probability of expert win[t], dscore[t] added to g of that expert (win / dscore may
+// be null).  GShard: the same with g_e = dloss scale / tot c_e / n, in the steps and roundings of
+// the operations' backwards (mean, product, cast, mean over the tokens, softmax).
+template <typename T, bool SWITCH>
 __global__ void __launch_bounds__(kBalanceThreads)
 balance_bwd_kernel(const T* __restrict__ logits, long pitch, const float* __restrict__ weight,
                    const float* __restrict__ dloss, const int64_t* __restrict__ win, const T* __restrict__ dscore,
-                   int n, int tot, T* __restrict__ dlogits) {
+                   float scale, int n, int tot, T* __restrict__ dlogits) {
   const int t = blockIdx.x * kBalanceThreads + threadIdx.x;
   if (t >= n) return;
   const T* in = logits + static_cast<long>(t) * pitch;
-  float mx, inv;
-  row_softmax<T>(in, tot, mx, inv);
-  const float gl = dloss != nullptr ? *dloss : 0.f;
+  T* out = dlogits + static_cast<long>(t) * tot;
+  float mx, den;
+  row_softmax<T>(in, tot, mx, den);
+  float gl = dloss != nullptr ? *dloss : 0.f;
+  if (!SWITCH) {
+    gl = gl * scale * (1.f / static_cast<float>(tot));
+    const float inv_n = 1.f / static_cast<float>(n);
+    float sum = 0.f;
+    for (int e = 0; e < tot; ++e) {
+      const float p = rounded<T>(expf(Ld<T>::get(in, e) - mx) / den);
+      sum += rounded<T>(rounded<T>(rounded<T>(gl * weight[e]) * inv_n) * p);
+    }
+    for (int e = 0; e < tot; ++e) {
+      const float p = rounded<T>(expf(Ld<T>::get(in, e) - mx) / den);
+      Ld<T>::put(out, e, rounded<T>(rounded<T>(rounded<T>(gl * weight[e]) * inv_n) * p) - p * sum);
+    }
+    return;
+  }
   const float gs = dscore != nullptr ? Ld<T>::get(dscore, t) : 0.f;
   const long w = win != nullptr ? win[t] : -1;
   float dot = 0.f;
   for (int e = 0; e < tot; ++e) {
-    const float p = expf(Ld<T>::get(in, e) - mx) * inv;
+    const float p = expf(Ld<T>::get(in, e) - mx) / den;
     dot += p * (gl * weight[e] + (e == w ? gs : 0.f));
   }
   for (int e = 0; e < tot; ++e) {
-    const float p = expf(Ld<T>::get(in, e) - mx) * inv;
-    Ld<T>::put(dlogits, static_cast<long>(t) * tot + e, p * (gl * weight[e] + (e == w ? gs : 0.f) - dot));
+    const float p = expf(Ld<T>::get(in, e) - mx) / den;
+    Ld<T>::put(out, e, p * (gl * weight[e] + (e == w ? gs : 0.f) - dot));
   }
 }
 
@@ -684,8 +720,9 @@ switch_top1_kernel(const T* __restrict__ logits, int n, int tot, int64_t* __rest
   const int t = blockIdx.x * kBalanceThreads + threadIdx.x;
   if (t >= n) return;
   const T* in = logits + static_cast<long>(t) * tot;
-  float mx, inv;
-  row_softmax<T>(in, tot, mx, inv);
+  float mx, den;
+  row_softmax<T>(in, tot, mx, den);
+  const float inv = 1.f / den;
   // as torch.max over the probabilities: NaN counts as the largest, the first of equals wins
   int best = 0;
   float best_p = expf(Ld<T>::get(in, 0) - mx) * inv;
@@ -1435,24 +1472,30 @@ cudaError_t launch_gate_topk_softmax_bwd(int logit_dtype, const void* dprob, con
 bool balance_supported(int tot) { return tot >= 1 && tot <= kBalanceMaxExperts; }
 int balance_blocks(int n) { return (n + kBalanceThreads - 1) / kBalanceThreads; }
 
+#define FMOE_DISPATCH_BALANCE(code, is_switch, ...)                                                       \
+  if (is_switch) { constexpr bool SWITCH = true; FMOE_DISPATCH_LOGITS(code, __VA_ARGS__) }               \
+  else { constexpr bool SWITCH = false; FMOE_DISPATCH_LOGITS(code, __VA_ARGS__) }
+
 cudaError_t launch_balance_loss(int code, const void* logits, long pitch, const int64_t* ids, int id_stride, int n,
                                 int tot, bool is_switch, float scale, float* part, float* loss, float* weight,
                                 cudaStream_t stream) {
   if (n < 1 || !balance_supported(tot)) return cudaErrorInvalidValue;
   const int blocks = balance_blocks(n);
-  FMOE_DISPATCH_LOGITS(code, (balance_sums_kernel<T><<<blocks, kBalanceThreads, 0, stream>>>(
-      static_cast<const T*>(logits), pitch, ids, id_stride, n, tot, part)));
-  balance_finish_kernel<<<1, 1024, 0, stream>>>(part, blocks, n, tot, is_switch ? 1 : 0, scale, loss, weight);
+  FMOE_DISPATCH_BALANCE(code, is_switch,
+      (balance_sums_kernel<T, SWITCH><<<blocks, kBalanceThreads, 0, stream>>>(
+           static_cast<const T*>(logits), pitch, ids, id_stride, n, tot, part),
+       balance_finish_kernel<T, SWITCH><<<1, 1024, 0, stream>>>(part, blocks, n, tot, scale, loss, weight)));
   return cudaGetLastError();
 }
 
 cudaError_t launch_balance_bwd(int code, const void* logits, long pitch, const float* weight, const float* dloss,
-                               const int64_t* win, const void* dscore, int n, int tot, void* dlogits,
-                               cudaStream_t stream) {
+                               const int64_t* win, const void* dscore, int n, int tot, bool is_switch, float scale,
+                               void* dlogits, cudaStream_t stream) {
   if (n < 1 || !balance_supported(tot)) return cudaErrorInvalidValue;
-  FMOE_DISPATCH_LOGITS(code, (balance_bwd_kernel<T><<<balance_blocks(n), kBalanceThreads, 0, stream>>>(
-      static_cast<const T*>(logits), pitch, weight, dloss, win, static_cast<const T*>(dscore), n, tot,
-      static_cast<T*>(dlogits))));
+  FMOE_DISPATCH_BALANCE(code, is_switch,
+      (balance_bwd_kernel<T, SWITCH><<<balance_blocks(n), kBalanceThreads, 0, stream>>>(
+           static_cast<const T*>(logits), pitch, weight, dloss, win, static_cast<const T*>(dscore), scale, n, tot,
+           static_cast<T*>(dlogits))));
   return cudaGetLastError();
 }
 

@@ -68,17 +68,18 @@ cudaError_t launch_gate_topk_softmax_bwd(int logit_dtype, const void* dprob, con
 
 // Balance losses of the capacity-limited gates and Switch's choice (logit_dtype as above, `pitch`
 // elements between rows of logits, tot <= 64, n >= 1).  part: fp32 [balance_blocks(n)][2 * tot];
-// loss fp32 scalar; weight fp32 [tot], handed to the backward.  ids[t * id_stride] is the expert a
-// token counts for (-1: none).  The backward takes dloss (device scalar or null) and, for a score
-// that is the softmax probability of expert win[t], dscore (or null); dlogits is [n, tot].
+// loss fp32 scalar; weight fp32 [tot], handed to the backward with the same is_switch and scale.
+// ids[t * id_stride] is the expert a token counts for (-1: none).  The backward takes dloss (device
+// scalar or null) and, for a score that is the softmax probability of expert win[t], dscore (or
+// null; Switch only); dlogits is [n, tot].
 bool balance_supported(int tot);
 int balance_blocks(int n);
 cudaError_t launch_balance_loss(int logit_dtype, const void* logits, long pitch, const int64_t* ids, int id_stride, int n,
                                 int tot, bool is_switch, float scale, float* part, float* loss, float* weight,
                                 cudaStream_t stream);
 cudaError_t launch_balance_bwd(int logit_dtype, const void* logits, long pitch, const float* weight, const float* dloss,
-                               const int64_t* win, const void* dscore, int n, int tot, void* dlogits,
-                               cudaStream_t stream);
+                               const int64_t* win, const void* dscore, int n, int tot, bool is_switch, float scale,
+                               void* dlogits, cudaStream_t stream);
 cudaError_t launch_switch_top1(int logit_dtype, const void* logits, int n, int tot, int64_t* win, void* score,
                                cudaStream_t stream);
 

@@ -44,7 +44,8 @@ class GShardGate(NaiveGate):
         logits, topk_idx, topk_val = self._choose(x)
         rate = self.capacity[0 if self.training else 1]
         cap = math.ceil(rate * x.shape[0]) * self.top_k // self.tot_expert
-        if gating.balance_native(logits):
+        # (under autocast the operations hold the probabilities in fp32: the kernels do not)
+        if gating.balance_native(logits) and not torch.is_autocast_enabled():
             self.set_loss(gating.gshard_loss(
                 logits, topk_idx, self.num_expert ** 2,
                 lambda l, ids: gshard_balance_loss(l, ids[:, 0], self.tot_expert, self.num_expert)))

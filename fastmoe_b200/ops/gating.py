@@ -185,13 +185,14 @@ def prune_to_capacity(idx, cap, tot_expert):
 
 
 class _BalanceLoss(Function):
-    r"""``reference(logits, ids)`` — GShard's loss — from two launches, its gradient from one."""
+    r"""``reference(logits, ids)`` — GShard's loss — from two launches, its gradient from one.  Both
+    round to the type of the logits where the PyTorch operations do (without autocast)."""
 
     @staticmethod
     def forward(ctx, logits, ids, scale, reference):
         loss, weight = native.get().balance_loss(logits, ids, False, float(scale))
         ctx.save_for_backward(logits, ids, weight)
-        ctx.reference = reference
+        ctx.reference, ctx.scale = reference, float(scale)
         return loss
 
     @staticmethod
@@ -201,7 +202,7 @@ class _BalanceLoss(Function):
             with torch.enable_grad():
                 (dl,) = torch.autograd.grad(ctx.reference(logits, ids), logits, grad, create_graph=True)
         else:
-            dl = native.get().balance_bwd(logits, weight, grad.contiguous(), None, None)
+            dl = native.get().balance_bwd(logits, weight, grad.contiguous(), None, None, False, ctx.scale)
         return dl, None, None, None
 
 
@@ -243,7 +244,8 @@ class _SwitchRoute(Function):
         else:
             dl = native.get().balance_bwd(logits, weight, None if grad_loss is None else grad_loss.contiguous(),
                                           None if grad_score is None else win,
-                                          None if grad_score is None else grad_score.contiguous())
+                                          None if grad_score is None else grad_score.contiguous(),
+                                          True, float(logits.shape[1]))
         return dl, None, None
 
 

@@ -560,6 +560,38 @@ def test_balanced_gates_native_loss(dtype, kind, n, tot, monkeypatch):
         assert ((g - p.grad.double()).abs() <= (4 * eps + 1e-5 * n ** 0.5) * scale).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n,tot", [(1, 2), (127, 3), (1000, 2), (4096, 2), (5000, 8), (9001, 64)])
+def test_gshard_loss_rounds_like_its_operations(dtype, n, tot):
+    r"""GShard's loss by itself: the PyTorch operations hold the probabilities, their mean and the
+    gradients of both in the logits' type, and so do the kernels.  The same fp32 values are rounded,
+    up to a few units of fp32, so that about 2^-11 (fp16) or 2^-14 (bf16) of the roundings go the
+    other way: one element in a hundred may differ, by a few units of the type of the largest term
+    of its sum.  Unrounded, a fifth to a half of them would."""
+    from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(19)
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -22}[dtype]
+    wide = torch.randn(n, tot + 6, device=DEV).to(dtype)   # rows with a pitch, as the padded gate has them
+    ids = wide[:, :tot].topk(2, dim=1).indices
+    ref = lambda l, i: gshard_balance_loss(l, i[:, 0], tot, tot)   # noqa: E731
+    losses, grads = [], []
+    for fn in (lambda l: gating.gshard_loss(l, ids, tot ** 2, ref), lambda l: ref(l, ids)):
+        w = wide.clone().requires_grad_(True)
+        loss = fn(w[:, :tot])
+        losses.append(loss.detach())
+        grads.append(torch.autograd.grad(loss, w, torch.full_like(loss, 3.0))[0][:, :tot].double())
+    assert losses[0].dtype == losses[1].dtype and losses[0].shape == losses[1].shape
+    assert torch.allclose(losses[0], losses[1], rtol=eps + 1e-5)
+    p = torch.softmax(wide[:, :tot].double(), 1)
+    c = torch.bincount(ids[:, 0], minlength=tot).double() / n
+    term = 3.0 * tot / n * c * p
+    bound = 4 * eps * (term + p * term.sum(1, keepdim=True)) + (2.0 ** -23 if dtype == torch.float16 else 1e-12)
+    assert ((grads[0] - grads[1]).abs() <= bound).all()
+    if dtype != torch.float32 and n > 1:
+        assert (grads[0] != grads[1]).double().mean() <= 0.01
+
+
 def test_balance_loss_second_derivative():
     r"""A gradient of the gradient goes through the PyTorch operations."""
     from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
