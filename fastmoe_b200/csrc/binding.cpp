@@ -201,23 +201,26 @@ torch::Tensor swipe_reassign(torch::Tensor idx, torch::Tensor quota, int64_t n_e
 }
 
 // ------------------------------------------------------------------------------ grouped GEMM
-// Generic entry: see sm100/grouped_gemm.cuh for the meaning of mode / act / epi.
-void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor offs,
+// Generic entry: see sm100/grouped_gemm.cuh for the meaning of mode / act / epi.  Without `offs`
+// there is one group, which all rows belong to.
+void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, c10::optional<torch::Tensor> offs,
                   torch::Tensor out, c10::optional<torch::Tensor> bias,
                   c10::optional<torch::Tensor> pre_out, c10::optional<torch::Tensor> aux,
                   int64_t act, int64_t epi, bool accumulate,
                   c10::optional<torch::Tensor> psum) {
   check_cuda_contig(a, "a");
   check_cuda_contig(b, "b");
-  check_cuda_contig(offs, "offs");
   check_cuda_contig(out, "out");
-  TORCH_CHECK(offs.scalar_type() == torch::kInt, "offs must be int32");
+  if (offs.has_value()) {
+    check_cuda_contig(*offs, "offs");
+    TORCH_CHECK(offs->scalar_type() == torch::kInt, "offs must be int32");
+  }
   c10::cuda::CUDAGuard guard(a.device());
   fmoe::GroupedGemmArgs g;
   g.mode = static_cast<int>(mode);
   g.dtype = dtype16(a);
   TORCH_CHECK(b.scalar_type() == a.scalar_type(), "operand dtypes differ");
-  g.num_groups = static_cast<int>(offs.numel() - 1);
+  g.num_groups = offs.has_value() ? static_cast<int>(offs->numel() - 1) : 1;
   g.rows_cap = a.size(0);
   if (mode == fmoe::kWgrad) {
     // a = P [rows, m], b = Q [rows, n], out [G, m, n]
@@ -248,7 +251,7 @@ void grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor 
               "grouped_gemm: operands must be 32-byte aligned");
   g.a = a.data_ptr();
   g.b = b.data_ptr();
-  g.offs = offs.data_ptr<int>();
+  g.offs = offs.has_value() ? offs->data_ptr<int>() : nullptr;
   g.out = out.data_ptr();
   if (bias.has_value() && bias->defined()) {
     check_cuda_contig(*bias, "bias");

@@ -85,6 +85,12 @@ bool narrow_applies(const GroupedGemmArgs& a) {
          !a.send.enabled && a.gate.flags == nullptr && a.push_meta == nullptr && a.trace == nullptr;
 }
 
+template <typename P> void set_offsets(P& p, const GroupedGemmArgs& a) {
+  p.offs = a.offs;
+  p.one_group[0] = 0;
+  p.one_group[1] = static_cast<int>(a.rows_cap);
+}
+
 cudaError_t launch_narrow_gemm(const GroupedGemmArgs& a) {
   CUtensorMap tw, tx;
   if (!make_map_2d(&tw, a.dtype, a.b, a.k, static_cast<uint64_t>(a.num_groups) * a.n, ng::BK, ng::TILE_N) ||
@@ -95,7 +101,7 @@ cudaError_t launch_narrow_gemm(const GroupedGemmArgs& a) {
   p.num_groups = a.num_groups;
   p.n = a.n;
   p.k = a.k;
-  p.offs = a.offs;
+  set_offsets(p, a);
   p.bias = a.bias;
   p.out = a.out;
   p.status = a.status;
@@ -121,7 +127,7 @@ cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
   p.m = a.m;
   p.n = a.n;
   p.k = a.k;
-  p.offs = a.offs;
+  set_offsets(p, a);
   p.out = a.out;
   p.pre_out = a.pre_out;
   p.bias = a.bias;
@@ -140,6 +146,7 @@ cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
 
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
   if (!grouped_gemm_supported(a.mode, a.m, a.n, a.k, a.num_groups)) return cudaErrorInvalidValue;
+  if (a.offs == nullptr && a.num_groups != 1) return cudaErrorInvalidValue;
   if (narrow_applies(a)) return launch_narrow_gemm(a);
   if (pair_applies(a)) return launch_pair_gemm(a);
   CUtensorMap ta, tb;
@@ -157,7 +164,7 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
   kp.num_groups = a.num_groups;
   kp.n = a.n;
   kp.k = a.k;
-  kp.offs = a.offs;
+  set_offsets(kp, a);
   kp.out = a.out;
   kp.pre_out = a.pre_out;
   kp.bias = a.bias;

@@ -81,7 +81,8 @@ struct GroupedGemmArgs {
   int k = 0;
   const void* a = nullptr;       // A (row modes) or P (wgrad)
   const void* b = nullptr;       // weights (row modes) or Q (wgrad)
-  const int* offs = nullptr;     // device, [num_groups + 1] exclusive row offsets
+  // device, [num_groups + 1] exclusive row offsets; null with one group: all rows_cap rows are its
+  const int* offs = nullptr;
   void* out = nullptr;
   void* pre_out = nullptr;       // optional, row modes only
   const void* bias = nullptr;    // optional [num_groups, n]

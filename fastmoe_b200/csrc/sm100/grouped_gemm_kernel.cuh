@@ -114,7 +114,8 @@ struct KernelParams {
   int num_groups;
   int n;
   int k;
-  const int* offs;
+  const int* offs;       // null: `one_group` instead
+  int one_group[2];
   void* out;
   void* pre_out;
   const void* bias;
@@ -143,6 +144,10 @@ struct TileCoord {
   int row_end;    // one past the last row of the group
 };
 
+__device__ __forceinline__ const int* row_offsets(const KernelParams& p) {
+  return p.offs != nullptr ? p.offs : p.one_group;
+}
+
 __device__ __forceinline__ int tiles_of_group(const KernelParams& p, int rows) {
   return ((rows + BM - 1) / BM) * ((p.n + BN - 1) / BN);
 }
@@ -158,8 +163,8 @@ __device__ __forceinline__ TileCoord decode_tile(const KernelParams& p, const Sh
     c.group = min(packed >> BLK_ORDER_SHIFT, p.num_groups - 1);
     c.m_tile = packed & ((1 << BLK_ORDER_SHIFT) - 1);
     c.n_tile = tile - i * n_tiles;
-    c.row_begin = p.offs[c.group];
-    c.row_end = p.offs[c.group + 1];
+    c.row_begin = row_offsets(p)[c.group];
+    c.row_end = row_offsets(p)[c.group + 1];
     return c;
   }
   // Binary search of the group whose tile range contains `tile`.
@@ -172,8 +177,8 @@ __device__ __forceinline__ TileCoord decode_tile(const KernelParams& p, const Sh
   const int local = tile - aux->tile_prefix[lo];
   c.m_tile = local / n_tiles;
   c.n_tile = local - c.m_tile * n_tiles;
-  c.row_begin = p.offs[lo];
-  c.row_end = p.offs[lo + 1];
+  c.row_begin = row_offsets(p)[lo];
+  c.row_end = row_offsets(p)[lo + 1];
   return c;
 }
 
@@ -721,7 +726,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_a,
     ptx::prefetch_tmap(&tm_b);
   }
   for (int g = threadIdx.x; g < p.num_groups; g += NUM_THREADS) {
-    aux->tile_prefix[g + 1] = tiles_of_group(p, p.offs[g + 1] - p.offs[g]);
+    aux->tile_prefix[g + 1] = tiles_of_group(p, row_offsets(p)[g + 1] - row_offsets(p)[g]);
   }
   if (warp == 1) {
     ptx::tmem_alloc(&aux->tmem_base, TMEM_COLS);

@@ -95,17 +95,18 @@ narrow_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
   ptx::chain_begin();   // nothing an earlier kernel writes is read above
   if (warp == 2) {
+    const int* offs = p.offs != nullptr ? p.offs : p.one_group;
     int run = 0;
     if (lane == 0) {
       sh->tiles[0] = 0;
-      sh->offs[0] = p.offs[0];
+      sh->offs[0] = offs[0];
     }
     for (int g0 = 0; g0 < p.num_groups; g0 += 32) {
       const int g = g0 + lane;
       int end = 0, t = 0;
       if (g < p.num_groups) {
-        end = p.offs[g + 1];
-        t = (end - p.offs[g] + TILE_ROWS - 1) / TILE_ROWS * n_tiles;
+        end = offs[g + 1];
+        t = (end - offs[g] + TILE_ROWS - 1) / TILE_ROWS * n_tiles;
       }
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {

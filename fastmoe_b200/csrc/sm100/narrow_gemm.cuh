@@ -14,7 +14,8 @@ struct Params {
   int num_groups;
   int n;
   int k;
-  const int* offs;
+  const int* offs;      // null: `one_group` instead
+  int one_group[2];
   const void* bias;   // optional [num_groups, n]
   void* out;
   int* status;

@@ -76,7 +76,8 @@ struct Params {
   int m;   // weight gradient only
   int n;
   int k;   // row modes only
-  const int* offs;
+  const int* offs;       // null: `one_group` instead
+  int one_group[2];
   void* out;
   void* pre_out;
   const void* bias;
@@ -431,18 +432,19 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   ptx::chain_begin();   // nothing an earlier kernel writes is read above
   if (warp == 2) {
     // offsets and the prefixes of tiles and blocks; an expert without rows has no tile
+    const int* offs = p.offs != nullptr ? p.offs : p.one_group;
     int run = 0, run_b = 0;
     if (lane == 0) {
       sh->tiles[0] = 0;
       sh->blocks[0] = 0;
-      sh->offs[0] = p.offs[0];
+      sh->offs[0] = offs[0];
     }
     for (int g0 = 0; g0 < p.num_groups; g0 += 32) {
       const int g = g0 + lane;
       int rows = 0, end = 0;
       if (g < p.num_groups) {
-        end = p.offs[g + 1];
-        rows = end - p.offs[g];
+        end = offs[g + 1];
+        rows = end - offs[g];
       }
       int t = (MODE == kWgrad) ? (rows > 0 ? m_tiles_w * n_tiles : 0) : (rows + TILE_M - 1) / TILE_M * n_tiles;
       int b = (rows + CTA_M - 1) / CTA_M;

@@ -78,22 +78,11 @@ class _LinearTopkSoftmax(Function):
 
 
 _PAD_BIAS = -30000.0   # bias of the padding columns: representable in bf16 and fp16, never selected
-_OFFS_CACHE = {}
-
-
-def _one_group_offs(rows, device):
-    key = (rows, device)
-    offs = _OFFS_CACHE.get(key)
-    if offs is None:
-        # built from device ops only, so that a first call inside a graph capture is legal
-        offs = (torch.arange(2, device=device, dtype=torch.int32) * rows).contiguous()
-        _OFFS_CACHE[key] = offs
-    return offs
 
 
 class _GateGemm(Function):
-    r"""``logits = x W^T + b`` on the tcgen05 grouped-GEMM kernel (one group), for any number of
-    experts.  The expert dimension is padded to a multiple of 64 — the padding columns get a
+    r"""``logits = x W^T + b`` on the tcgen05 grouped-GEMM kernel (one group, whose row count goes
+    with the launch: no offsets on the device), for any number of experts.  The expert dimension is padded to a multiple of 64 — the padding columns get a
     large negative bias, so a top-k over the padded logits never selects them — and the
     backward products ``dx = dl W`` and ``dW = dl^T x`` (with ``db`` from the same launch) run on
     the same kernel's input-gradient and weight-gradient modes."""
@@ -109,9 +98,8 @@ class _GateGemm(Function):
             bp[0, :tot] = bias
         else:
             bp[0, :tot] = 0
-        offs = _one_group_offs(x.shape[0], x.device)
-        logits = gg.forward(x, wp, offs, bp)
-        ctx.save_for_backward(x, wp, offs)
+        logits = gg.forward(x, wp, None, bp)
+        ctx.save_for_backward(x, wp)
         ctx.tot = tot
         ctx.has_bias = bias is not None
         return logits
@@ -119,12 +107,12 @@ class _GateGemm(Function):
     @staticmethod
     def backward(ctx, dl):
         from . import grouped_gemm as gg
-        x, wp, offs = ctx.saved_tensors
+        x, wp = ctx.saved_tensors
         dl = dl.contiguous()
-        dx = gg.dgrad(dl, wp, offs) if ctx.needs_input_grad[0] else None
+        dx = gg.dgrad(dl, wp, None) if ctx.needs_input_grad[0] else None
         dw = db = None
         if ctx.needs_input_grad[1] or (ctx.has_bias and ctx.needs_input_grad[2]):
-            dwp, dbp = gg.wgrad(dl, x, offs, 1, with_bias_grad=True)
+            dwp, dbp = gg.wgrad(dl, x, None, 1, with_bias_grad=True)
             dw = dwp[0, :ctx.tot]
             db = dbp[0, :ctx.tot] if ctx.has_bias else None
         return dx, dw, db

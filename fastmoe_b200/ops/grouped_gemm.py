@@ -6,7 +6,8 @@ The three products of a grouped linear — forward ``Y_e = X_e W_e^T (+b_e)``, i
 124-147`` in the reference, one cuBLAS call each per expert) — are single launches of the
 tcgen05 kernel for bf16/fp16 with tensor-core-friendly shapes, and of the reference-precision
 SIMT kernel for fp32/fp64 or odd shapes.  Row offsets are an int32 device tensor
-``offs[E+1]``; only the compatibility entry points below take host counts.
+``offs[E+1]`` (``None`` for a single group of all rows, tensor-core shapes only); only the
+compatibility entry points below take host counts.
 """
 import torch
 

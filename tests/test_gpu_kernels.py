@@ -592,6 +592,45 @@ def test_gshard_loss_rounds_like_its_operations(dtype, n, tot):
         assert (grads[0] != grads[1]).double().mean() <= 0.01
 
 
+@pytest.mark.parametrize("rows", [9, 300, 777])
+def test_wide_gate_first_called_under_capture(rows):
+    r"""The tensor-core gate (12 experts) called for a row count first inside a graph that has not
+    been replayed, then eagerly, on another stream, and by the replay: nothing of one call is
+    left for the next.  9 rows take the narrow kernel and, in backward, the single-CTA one."""
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(20)
+    dtype, eps = torch.bfloat16, 2.0 ** -8
+
+    def make(n):
+        x = torch.randn(n, 128, device=DEV).to(dtype).requires_grad_(True)
+        w = (torch.randn(12, 128, device=DEV) / 128 ** 0.5).to(dtype).requires_grad_(True)
+        return x, w, torch.randn(12, device=DEV).to(dtype).requires_grad_(True)
+
+    def close(got, ref):
+        return bool(((got.double() - ref).abs() <= eps * ref.abs() + 1e-4 * ref.abs().max()).all())
+
+    gating.linear_topk_softmax(*make(64), 2)   # the library's own lazy set-up, for another row count
+    xg, wg, bg = (t.detach() for t in make(rows))
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        captured = gating.linear_topk_softmax(xg, wg, bg, 2)[0]
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            x, w, b = make(rows)
+            logits, _idx, _prob = gating.linear_topk_softmax(x, w, b, 2)
+            gl = torch.randn_like(logits)
+            logits.backward(gl)
+        torch.cuda.synchronize()
+        x64, w64, g64 = x.detach().double(), w.detach().double(), gl.double()
+        assert close(logits, x64 @ w64.t() + b.detach().double())
+        assert close(x.grad, g64 @ w64) and close(w.grad, g64.t() @ x64) and close(b.grad, g64.sum(0))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert close(captured, xg.double() @ wg.double().t() + bg.double())
+
+
 def test_balance_loss_second_derivative():
     r"""A gradient of the gradient goes through the PyTorch operations."""
     from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
