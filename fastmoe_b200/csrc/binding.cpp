@@ -64,6 +64,13 @@ void check_cuda_contig(const torch::Tensor& t, const char* name) {
   TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
 }
 
+// For kernels that read or write rows 16 bytes at a time: a contiguous view into a flat buffer may
+// start anywhere.
+void check_rows(const torch::Tensor& t, const char* name) {
+  check_cuda_contig(t, name);
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, name, " must be 16-byte aligned");
+}
+
 // One int32 status word per device; kernels write a non-zero code when a bounded wait ran out.
 std::mutex g_status_mu;
 std::map<int, torch::Tensor> g_status;
@@ -351,8 +358,8 @@ void simt_grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Te
 void scatter_rows(torch::Tensor src, torch::Tensor idx, torch::Tensor rank, torch::Tensor base,
                   c10::optional<torch::Tensor> scale, int64_t k, torch::Tensor dst,
                   c10::optional<torch::Tensor> row_slot) {
-  check_cuda_contig(src, "src");
-  check_cuda_contig(dst, "dst");
+  check_rows(src, "src");
+  check_rows(dst, "dst");
   c10::cuda::CUDAGuard guard(src.device());
   const void* sc = (scale.has_value() && scale->defined()) ? scale->data_ptr() : nullptr;
   int* rs = (row_slot.has_value() && row_slot->defined()) ? row_slot->data_ptr<int>() : nullptr;
@@ -365,8 +372,8 @@ void scatter_rows(torch::Tensor src, torch::Tensor idx, torch::Tensor rank, torc
 
 void gather_combine(torch::Tensor rows, torch::Tensor idx, torch::Tensor rank, torch::Tensor base,
                     c10::optional<torch::Tensor> weight, int64_t k, torch::Tensor out) {
-  check_cuda_contig(rows, "rows");
-  check_cuda_contig(out, "out");
+  check_rows(rows, "rows");
+  check_rows(out, "out");
   c10::cuda::CUDAGuard guard(rows.device());
   const void* w = (weight.has_value() && weight->defined()) ? weight->data_ptr() : nullptr;
   FMOE_CUDA_CHECK(fmoe::launch_gather_combine(dtype16(rows), rows.data_ptr(),
@@ -380,8 +387,9 @@ void gather_combine(torch::Tensor rows, torch::Tensor idx, torch::Tensor rank, t
 void combine_bwd(torch::Tensor dout, torch::Tensor rows, torch::Tensor idx, torch::Tensor rank,
                  torch::Tensor base, torch::Tensor weight, int64_t k, torch::Tensor drows,
                  torch::Tensor dscore) {
-  check_cuda_contig(dout, "dout");
-  check_cuda_contig(rows, "rows");
+  check_rows(dout, "dout");
+  check_rows(rows, "rows");
+  check_rows(drows, "drows");
   c10::cuda::CUDAGuard guard(dout.device());
   FMOE_CUDA_CHECK(fmoe::launch_combine_bwd(dtype16(dout), dout.data_ptr(), rows.data_ptr(),
                                            idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
@@ -395,10 +403,11 @@ void combine_bwd(torch::Tensor dout, torch::Tensor rows, torch::Tensor idx, torc
 // One GPU, both expert linears with a fused activation: the launches of a layer's forward, and of
 // its backward, issued by one call each.  For a small layer the calls from Python between the
 // kernels, and not the kernels, were what a training step waited for.
-torch::Tensor aligned32(const torch::Tensor& t) {
+torch::Tensor aligned(const torch::Tensor& t, uintptr_t bytes) {
   torch::Tensor c = t.contiguous();
-  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 32 == 0 ? c : c.clone();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % bytes == 0 ? c : c.clone();
 }
+torch::Tensor aligned32(const torch::Tensor& t) { return aligned(t, 32); }
 
 bool moe_mlp_supported(int64_t experts, int64_t d, int64_t h) {
   const int g = static_cast<int>(experts), id = static_cast<int>(d), ih = static_cast<int>(h);
@@ -411,7 +420,7 @@ std::vector<torch::Tensor> moe_mlp_forward(torch::Tensor x_in, torch::Tensor idx
                                            torch::Tensor w1_in, torch::Tensor b1_in, torch::Tensor w2_in,
                                            torch::Tensor b2_in, int64_t act, bool keep) {
   c10::cuda::CUDAGuard guard(x_in.device());
-  const torch::Tensor x = x_in.contiguous();
+  const torch::Tensor x = aligned(x_in, 16);
   const torch::Tensor idx = idx_in.contiguous().view({-1});
   const torch::Tensor score = score_in.reshape({-1}).to(x.scalar_type()).contiguous();
   const torch::Tensor w1 = aligned32(w1_in), b1 = aligned32(b1_in), w2 = aligned32(w2_in), b2 = aligned32(b2_in);
@@ -440,7 +449,7 @@ std::vector<torch::Tensor> moe_mlp_backward(torch::Tensor dout_in, torch::Tensor
                                             torch::Tensor score, torch::Tensor idx, torch::Tensor w1_in,
                                             torch::Tensor w2_in, int64_t act, bool need_dx, bool need_w1, bool need_w2) {
   c10::cuda::CUDAGuard guard(xs.device());
-  const torch::Tensor dout = dout_in.contiguous();
+  const torch::Tensor dout = aligned(dout_in, 16);
   const torch::Tensor w1 = aligned32(w1_in), w2 = aligned32(w2_in);
   const int64_t groups = w1.size(0), h = w1.size(1), d = w1.size(2), n_tok = dout.size(0), k = idx.numel() / n_tok;
   auto dys = torch::empty_like(ys);
@@ -473,7 +482,7 @@ std::vector<torch::Tensor> moe_mlp_backward(torch::Tensor dout_in, torch::Tensor
 }
 
 torch::Tensor colsum(torch::Tensor x, torch::Tensor offs) {
-  check_cuda_contig(x, "x");
+  check_rows(x, "x");
   c10::cuda::CUDAGuard guard(x.device());
   const int groups = static_cast<int>(offs.numel() - 1);
   auto out = torch::zeros({groups, x.size(1)}, torch::dtype(torch::kFloat).device(x.device()));
@@ -595,8 +604,8 @@ bool gate_fused_supported(int64_t tot, int64_t d, int64_t k) {
 // logits [B, tot], idx [B, k] and prob [B, k] of a linear gate in one pass over x.
 std::vector<torch::Tensor> gate_linear_topk(torch::Tensor x, torch::Tensor w,
                                             c10::optional<torch::Tensor> bias, int64_t k) {
-  check_cuda_contig(x, "x");
-  check_cuda_contig(w, "w");
+  check_rows(x, "x");
+  check_rows(w, "w");
   TORCH_CHECK(x.scalar_type() == w.scalar_type(), "gate input and weight dtypes differ");
   c10::cuda::CUDAGuard guard(x.device());
   const int rows = static_cast<int>(x.size(0));
@@ -618,8 +627,8 @@ std::vector<torch::Tensor> gate_linear_topk_bwd(c10::optional<torch::Tensor> dpr
                                                 c10::optional<torch::Tensor> dlogits,
                                                 torch::Tensor x, torch::Tensor w, bool need_dx,
                                                 bool need_db) {
-  check_cuda_contig(x, "x");
-  check_cuda_contig(w, "w");
+  check_rows(x, "x");
+  check_rows(w, "w");
   c10::cuda::CUDAGuard guard(x.device());
   const int rows = static_cast<int>(x.size(0));
   const int d = static_cast<int>(x.size(1));

@@ -34,6 +34,12 @@ int dtype16(const torch::Tensor& t) {
   return 1;
 }
 
+// Rows that a kernel reads 16 bytes at a time: a contiguous view into a flat buffer may start anywhere.
+void check_rows(const torch::Tensor& t, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, name,
+              " must be a contiguous, 16-byte aligned CUDA tensor");
+}
+
 class ExchangeContext {
  public:
   ExchangeContext(std::vector<int64_t> flag_ptrs, torch::Tensor epoch, int64_t me, int64_t world,
@@ -116,6 +122,7 @@ class ExchangeContext {
                      std::vector<int64_t> meta_ptrs, int64_t n_expert, int64_t k,
                      int64_t capacity_rows) {
     c10::cuda::CUDAGuard guard(x.device());
+    check_rows(x, "dispatch_push: x");
     const void* sc = (scale.has_value() && scale->defined()) ? scale->data_ptr() : nullptr;
     FMOE_P2P_CHECK(fmoe::launch_dispatch_push(
         ctx_, dtype16(x), x.data_ptr(), idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
@@ -145,6 +152,7 @@ class ExchangeContext {
   void return_push(torch::Tensor rows, torch::Tensor meta, torch::Tensor total_rows,
                    std::vector<int64_t> ret_ptrs, int64_t ret_slots) {
     c10::cuda::CUDAGuard guard(rows.device());
+    check_rows(rows, "return_push: rows");
     FMOE_P2P_CHECK(fmoe::launch_return_push(ctx_, dtype16(rows), rows.data_ptr(),
                                             meta.data_ptr<int64_t>(), total_rows.data_ptr<int>(),
                                             to_ptrs(ret_ptrs), static_cast<int>(rows.size(1)),
@@ -395,6 +403,8 @@ class ExchangeContext {
 void slot_dot(torch::Tensor dout, torch::Tensor y, torch::Tensor idx, int64_t k,
               torch::Tensor dscore) {
   c10::cuda::CUDAGuard guard(dout.device());
+  check_rows(dout, "slot_dot: dout");
+  check_rows(y, "slot_dot: y");
   fmoe_count_launch();
   FMOE_P2P_CHECK(fmoe::launch_slot_dot(dtype16(dout), dout.data_ptr(), y.data_ptr(),
                                        idx.data_ptr<int64_t>(), static_cast<int>(idx.numel()),

@@ -58,7 +58,7 @@ class _Dispatch(Function):
     def forward(ctx, x, idx, rank, offs, k):
         nat = native.get()
         xs = torch.empty(idx.numel(), x.shape[1], dtype=x.dtype, device=x.device)
-        nat.scatter_rows(x, idx, rank, offs, None, k, xs, None)
+        nat.scatter_rows(gg.aligned(x, 16), idx, rank, offs, None, k, xs, None)
         ctx.save_for_backward(idx, rank, offs)
         ctx.k = k
         ctx.n_tok = x.shape[0]
@@ -68,7 +68,7 @@ class _Dispatch(Function):
     def backward(ctx, dxs):
         idx, rank, offs = ctx.saved_tensors
         dx = torch.empty(ctx.n_tok, dxs.shape[1], dtype=dxs.dtype, device=dxs.device)
-        native.get().gather_combine(dxs.contiguous(), idx, rank, offs, None, ctx.k, dx)
+        native.get().gather_combine(gg.aligned(dxs, 16), idx, rank, offs, None, ctx.k, dx)
         return dx, None, None, None, None
 
 
@@ -89,7 +89,7 @@ class _Combine(Function):
         ys, score, idx, rank, offs = ctx.saved_tensors
         dys = torch.empty_like(ys)
         dscore = torch.empty_like(score)
-        native.get().combine_bwd(dout.contiguous(), ys, idx, rank, offs, score, ctx.k, dys, dscore)
+        native.get().combine_bwd(gg.aligned(dout, 16), ys, idx, rank, offs, score, ctx.k, dys, dscore)
         return dys, dscore, None, None, None, None
 
 

@@ -57,6 +57,8 @@ class _LinearTopkSoftmax(Function):
 
     @staticmethod
     def forward(ctx, x, weight, bias, k):
+        from .grouped_gemm import aligned
+        x, weight = aligned(x, 16), aligned(weight, 16)   # 16-byte loads
         logits, idx, prob = native.get().gate_linear_topk(x, weight, bias, int(k))
         ctx.save_for_backward(x, weight, idx, prob)
         ctx.has_bias = bias is not None

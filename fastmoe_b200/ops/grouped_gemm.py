@@ -32,14 +32,15 @@ def _tc_ok(t, mode, m, n, k, groups):
     return t.dtype in _TC and native.get().grouped_gemm_supported(mode, m, n, k, groups)
 
 
-def _aligned(t):
-    r"""The tensor-core kernel wants 32-byte aligned, contiguous operands.  Views into flat
-    buffers (e.g. the replicas ``nn.DataParallel`` broadcasts) may not be: copy those."""
+def aligned(t, to=32):
+    r"""The tensor-core kernel wants 32-byte aligned, contiguous operands, the kernels that move and
+    combine rows 16-byte aligned ones.  Views into flat buffers (e.g. the replicas
+    ``nn.DataParallel`` broadcasts) may not be: copy those."""
     if t is None:
         return None
-    if not t.is_contiguous() or t.data_ptr() % 32 != 0:
-        return t.contiguous().clone() if t.data_ptr() % 32 != 0 and t.is_contiguous() else t.contiguous()
-    return t
+    if not t.is_contiguous():
+        return t.contiguous()
+    return t if t.data_ptr() % to == 0 else t.clone()
 
 
 TILE_M, TILE_N = 128, 256
@@ -90,7 +91,7 @@ def forward(x, weight, offs, bias=None, act=None, want_pre=False):
     if _tc_ok(x, MODE_NT, 0, n, k, groups):
         if want_pre and code != 0:
             pre = pre_buffer(x.shape[0], n, groups, x.dtype, x.device)
-        nat.grouped_gemm(MODE_NT, _aligned(x), _aligned(weight), offs, out, _aligned(bias), pre, None,
+        nat.grouped_gemm(MODE_NT, aligned(x), aligned(weight), offs, out, aligned(bias), pre, None,
                          code, EPI_BIAS_ACT, False)
         if want_pre and pre is None:
             pre = out
@@ -113,11 +114,11 @@ def dgrad(dy, weight, offs, pre=None, act=None):
     if dy.shape[0] == 0:
         return out
     if _tc_ok(dy, MODE_NN, 0, n, k, groups) and (not code or pre.dim() == 1):
-        nat.grouped_gemm(MODE_NN, _aligned(dy), _aligned(weight), offs, out, None, None,
+        nat.grouped_gemm(MODE_NN, aligned(dy), aligned(weight), offs, out, None, None,
                          pre if code else None, code, EPI_DACT if code else EPI_BIAS_ACT, False)
     elif _tc_ok(dy, MODE_NN, 0, n, k, groups):
         # a row-major pre-activation: plain tensor-core product, derivative as a PyTorch op
-        nat.grouped_gemm(MODE_NN, _aligned(dy), _aligned(weight), offs, out, None, None, None, 0,
+        nat.grouped_gemm(MODE_NN, aligned(dy), aligned(weight), offs, out, None, None, None, 0,
                          EPI_BIAS_ACT, False)
         _zero_tail(out, offs)
         out = out * _torch_act_grad(pre, act)
@@ -146,7 +147,7 @@ def wgrad(dy, x, offs, groups, out=None, accumulate=False, with_bias_grad=False)
     if _tc_ok(dy, MODE_WGRAD, m, n, 0, groups) and out.data_ptr() % 32 == 0:
         if with_bias_grad:
             db = torch.empty(groups, m, dtype=dy.dtype, device=dy.device)
-        nat.grouped_gemm(MODE_WGRAD, _aligned(dy), _aligned(x), offs, out, None, None, None, 0, 0,
+        nat.grouped_gemm(MODE_WGRAD, aligned(dy), aligned(x), offs, out, None, None, None, 0, 0,
                          accumulate, db)
     else:
         tmp = out if fresh else torch.empty(groups, m, n, dtype=dy.dtype, device=dy.device)
@@ -165,7 +166,7 @@ def wgrad(dy, x, offs, groups, out=None, accumulate=False, with_bias_grad=False)
 def bias_grad(dy, offs, dtype=None):
     r"""Column sums of ``dy`` per expert → ``[E, n]`` (fp32 accumulation)."""
     if dy.dtype in _TC and dy.shape[1] % 8 == 0:
-        out = native.get().colsum(dy, offs)
+        out = native.get().colsum(aligned(dy, 16), offs)
     else:
         groups = offs.numel() - 1
         rows = torch.arange(dy.shape[0], device=dy.device)

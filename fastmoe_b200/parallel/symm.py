@@ -354,13 +354,14 @@ class _DispatchP2P(Function):
 
     @staticmethod
     def forward(ctx, x, idx, rank, lec, ws, n_expert, k, capacity, budget):
+        from ..ops import grouped_gemm as gg
         nat = native.get()
         d = x.shape[1]
         dev = x.device
         tb = _Tables(ws, lec, n_expert, capacity)
         stage_rows, rows_ptrs = ws.buffer("rows", capacity * d * x.element_size())
         stage_meta, meta_ptrs = ws.buffer("meta", capacity * 8)
-        ws.ctx.dispatch_push(x, idx, rank, tb.dst_base, None, rows_ptrs, meta_ptrs, n_expert, k, capacity)
+        ws.ctx.dispatch_push(gg.aligned(x, 16), idx, rank, tb.dst_base, None, rows_ptrs, meta_ptrs, n_expert, k, capacity)
         xs = torch.empty(capacity, d, dtype=x.dtype, device=dev)
         meta = torch.empty(capacity, dtype=torch.int64, device=dev)
         ws.ctx.wait_copy(nat.P2P_CHAN_DISPATCH, stage_rows, stage_meta.view(torch.int64), tb.total, xs, meta)
@@ -375,9 +376,10 @@ class _DispatchP2P(Function):
 
     @staticmethod
     def backward(ctx, dxs, _g1, _g2, _g3, _g4):
+        from ..ops import grouped_gemm as gg
         idx, meta, total, rank, dst_base = ctx.saved_tensors
         ws = ctx.ws
-        dxs = dxs.contiguous()
+        dxs = gg.aligned(dxs, 16)
         d = dxs.shape[1]
         stage_ret, ret_ptrs = ws.buffer("ret", ctx.budget * ctx.k * d * dxs.element_size())
         ws.ctx.return_push(dxs, meta, total, ret_ptrs, ctx.budget * ctx.k)
@@ -408,11 +410,12 @@ class _CombineP2P(Function):
 
     @staticmethod
     def backward(ctx, dout):
+        from ..ops import grouped_gemm as gg
         nat = native.get()
         y_slots, score, idx, rank, dst_base, total = ctx.saved_tensors
         n_expert, k, capacity = ctx.args
         ws = ctx.ws
-        dout = dout.contiguous()
+        dout = gg.aligned(dout, 16)
         d = dout.shape[1]
         dscore = torch.empty_like(score)
         nat.slot_dot(dout, y_slots, idx, k, dscore)
@@ -443,6 +446,7 @@ class _FusedEPMLP(Function):
     def forward(ctx, x, score, w1, b1, w2, b2, idx, rank, lec, my_offs, pos, ws, n_expert, k,
                 capacity, budget, act):
         from ..ops import grouped_gemm as gg
+        x = gg.aligned(x, 16)
         d = x.shape[1]
         h = w1.shape[1]
         dev = x.device
@@ -494,7 +498,7 @@ class _FusedEPMLP(Function):
         n_expert, k, capacity, budget, act, n_tok = ctx.args
         tb = ctx.tables
         ws = ctx.ws
-        dout = dout.contiguous()
+        dout = gg.aligned(dout, 16)
         d = dout.shape[1]
         h = w1.shape[1]
         es = dout.element_size()

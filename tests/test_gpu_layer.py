@@ -196,3 +196,81 @@ def test_native_layer_call_equals_separate_launches(case, act, monkeypatch):
         assert (a is None) == (b is None)
         if a is not None:
             assert a.dtype == b.dtype and torch.equal(a, b)
+
+
+def _shifted(t):
+    r"""The same values as a contiguous view that starts one element after an allocation."""
+    flat = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+    flat[1:] = t.detach().reshape(-1)
+    view = flat[1:].view_as(t)
+    assert view.is_contiguous() and view.data_ptr() % 16 != 0
+    return view
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("act", [nn.GELU(), nn.Tanh()])
+@pytest.mark.parametrize("experts", [5, 12])
+def test_rows_that_start_anywhere(dtype, act, experts, monkeypatch):
+    r"""Input, output gradient and gate weight inside flat buffers, for a fused and for a user's
+    activation, with the gate in one kernel (5 experts) and on the tensor cores (12), and with the
+    bounds checks on (separate launches): the bits of aligned operands."""
+    from fastmoe_b200 import FMoETransformerMLP
+    torch.manual_seed(21)
+    layer = FMoETransformerMLP(num_expert=experts, d_model=128, d_hidden=192, top_k=2, activation=act).to(DEV).to(dtype)
+    x = torch.randn(77, 128, device=DEV).to(dtype)
+    gy = torch.randn(77, 128, device=DEV).to(dtype)
+
+    def run(x, gy):
+        layer.zero_grad(set_to_none=True)
+        xi = x.detach().requires_grad_(True)
+        y = layer(xi)
+        y.backward(gy)
+        return [y, xi.grad] + [p.grad for p in layer.parameters()]
+
+    want = run(x, gy)
+    layer.gate.gate.weight = nn.Parameter(_shifted(layer.gate.gate.weight))
+    for checks in ("0", "1"):
+        monkeypatch.setenv("FMOE_DEBUG_BOUNDS", checks)
+        for a, b in zip(run(_shifted(x), _shifted(gy)), want):
+            assert torch.equal(a, b)
+
+
+def test_native_calls_refuse_unaligned_rows():
+    r"""The kernels with 16-byte accesses are not launched on rows that start elsewhere."""
+    from fastmoe_b200.ops import native
+    nat = native.get()
+    rows = torch.zeros(8, 64, device=DEV, dtype=torch.bfloat16)
+    bad = _shifted(rows)
+    idx = torch.zeros(8, device=DEV, dtype=torch.int64)
+    _counts, rank, offs = nat.route_offs(idx, 1)
+    score = torch.ones(8, device=DEV, dtype=torch.bfloat16)
+    w = torch.zeros(2, 64, device=DEV, dtype=torch.bfloat16)
+    for call in (lambda: nat.scatter_rows(bad, idx, rank, offs, None, 1, rows, None),
+                 lambda: nat.scatter_rows(rows, idx, rank, offs, None, 1, bad, None),
+                 lambda: nat.gather_combine(bad, idx, rank, offs, None, 1, rows),
+                 lambda: nat.combine_bwd(bad, rows, idx, rank, offs, score, 1, rows.clone(), score.clone()),
+                 lambda: nat.colsum(bad, offs), lambda: nat.slot_dot(bad, rows, idx, 1, score),
+                 lambda: nat.gate_linear_topk(bad, w, None, 1), lambda: nat.gate_linear_topk(rows, _shifted(w), None, 1)):
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            call()
+
+
+@pytest.mark.parametrize("shape", [(64, 128), (64, 72)])
+def test_grouped_linear_of_unaligned_rows(shape):
+    r"""``FMoELinear`` on the tensor cores and (72 columns) on the general kernels, whose bias gradient
+    is a kernel of its own."""
+    from fastmoe_b200 import FMoELinear
+    torch.manual_seed(22)
+    layer = FMoELinear(3, *shape).to(DEV).bfloat16()
+    counts = torch.tensor([20, 0, 13])
+    x = torch.randn(33, shape[0], device=DEV).bfloat16()
+    gy = torch.randn(33, shape[1], device=DEV).bfloat16()
+    got = []
+    for a, g in ((x, gy), (_shifted(x), _shifted(gy))):
+        layer.zero_grad(set_to_none=True)
+        a = a.detach().requires_grad_(True)
+        y = layer(a, counts)
+        y.backward(g)
+        got.append([y, a.grad, layer.weight.grad, layer.bias.grad])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
