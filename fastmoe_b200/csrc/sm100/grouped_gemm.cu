@@ -147,6 +147,14 @@ cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
 cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
   if (!grouped_gemm_supported(a.mode, a.m, a.n, a.k, a.num_groups)) return cudaErrorInvalidValue;
   if (a.offs == nullptr && a.num_groups != 1) return cudaErrorInvalidValue;
+  if (a.rows_cap == 0) {
+    // no rows: no tensor map has an extent of 0.  The weight gradient is the empty sum.
+    if (a.mode != kWgrad || a.accumulate) return cudaSuccess;
+    const size_t width = static_cast<size_t>(a.num_groups) * a.m;
+    const cudaError_t e = cudaMemsetAsync(a.out, 0, width * a.n * (a.out_fp32 ? 4 : 2), a.stream);
+    if (e != cudaSuccess || a.psum == nullptr) return e;
+    return cudaMemsetAsync(a.psum, 0, width * 2, a.stream);
+  }
   if (narrow_applies(a)) return launch_narrow_gemm(a);
   if (pair_applies(a)) return launch_pair_gemm(a);
   CUtensorMap ta, tb;

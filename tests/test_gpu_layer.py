@@ -274,3 +274,31 @@ def test_grouped_linear_of_unaligned_rows(shape):
         got.append([y, a.grad, layer.weight.grad, layer.bias.grad])
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("act", [nn.GELU(), nn.Tanh()])
+def test_no_rows_at_all(dtype, act):
+    r"""Forward and backward of the layer without tokens and of ``FMoELinear`` without rows: empty
+    outputs and input gradients, zero parameter gradients."""
+    from fastmoe_b200 import FMoELinear, FMoETransformerMLP
+    layer = FMoETransformerMLP(num_expert=4, d_model=64, d_hidden=128, top_k=2, activation=act).to(DEV).to(dtype)
+    linear = FMoELinear(3, 64, 128).to(DEV).to(dtype)
+    torch.full((4, 128, 64), float("nan"), device=DEV, dtype=dtype)   # stale bits for the allocator to hand out
+    for module, args, width in ((layer, (), 64), (linear, (torch.zeros(3, dtype=torch.int64),), 128)):
+        x = torch.empty(0, 64, device=DEV, dtype=dtype, requires_grad=True)
+        y = module(x, *args)
+        assert y.shape == (0, width)
+        y.backward(torch.empty_like(y))
+        assert x.grad.shape == (0, 64)
+        for name, p in module.named_parameters():
+            assert p.grad is not None and not p.grad.any(), name
+
+
+def test_no_rows_leave_an_accumulated_gradient_alone():
+    from fastmoe_b200.ops import grouped_gemm as gg
+    out = torch.ones(2, 64, 32, device=DEV, dtype=torch.bfloat16)
+    offs = torch.zeros(3, dtype=torch.int32, device=DEV)
+    empty = [torch.empty(0, n, device=DEV, dtype=torch.bfloat16) for n in (64, 32)]
+    assert (gg.wgrad(*empty, offs, 2, out=out, accumulate=True) == 1).all()
+    assert not gg.wgrad(*empty, offs, 2, out=out).any()
