@@ -912,8 +912,8 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
   if (row_ok && e_of < tot && (lane & (kStep - 1)) == 0) {
     logits[static_cast<long>(row0 + r) * tot + e_of] = V2<T>::from_f(mine);
   }
-  // Every lane ranks its logit among those of its token (ties to the lower id, NaN last) and writes
-  // the entry of that rank: a handful of instructions where a selection loop unrolled into
+  // Every lane ranks its logit among those of its token (ties to the lower id) and writes the
+  // entry of that rank: a handful of instructions where a selection loop unrolled into
   // registers was long enough to be bound by instruction fetch (8 tokens: 17 us).
   const int base = lane & ~(TOT * kStep - 1);   // first lane of this token's group
   const float key = (e_of < tot && mine == mine) ? mine : -INFINITY;
@@ -924,6 +924,30 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
     const float other = __shfl_sync(0xffffffffu, key, base + e * kStep);
     pos += (other > key || (other == key && e < e_of)) ? 1 : 0;
     top = fmaxf(top, other);
+  }
+  if (__any_sync(0xffffffffu, e_of < tot && mine != mine)) {
+    // With a NaN the choice is what k scans over the experts left give, in which only a greater
+    // logit replaces the first one: a NaN that comes first is chosen and shows in every score.
+    bool taken = false;
+    pos = TOT;
+#pragma unroll 1
+    for (int j = 0; j < k; ++j) {
+      float best = 0.f;
+      int best_e = -1;
+#pragma unroll 1
+      for (int e = 0; e < tot; ++e) {
+        const float other = __shfl_sync(0xffffffffu, mine, base + e * kStep);
+        const int gone = __shfl_sync(0xffffffffu, static_cast<int>(taken), base + e * kStep);
+        if (gone == 0 && (best_e < 0 || other > best)) {
+          best = other;
+          best_e = e;
+        }
+      }
+      if (best_e == e_of) {
+        taken = true;
+        pos = j;
+      }
+    }
   }
   const bool chosen = e_of < tot && pos < k;
   const float ex = chosen ? __expf(mine - top) : 0.f;

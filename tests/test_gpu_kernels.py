@@ -524,6 +524,36 @@ def test_gate_rows_per_warp(dtype, rows, tot, k, d):
     assert close(b.grad[None], torch.ones(1, rows, device=DEV, dtype=torch.float64), dl)
 
 
+@pytest.mark.parametrize("rows,tot,k", [(5, 2, 1), (5, 8, 2), (2400, 3, 2), (2400, 7, 7), (4800, 8, 4), (4800, 2, 2)])
+def test_gate_with_nan_logits(rows, tot, k):
+    r"""NaN in one expert's weights, or in some tokens, with one, two and four tokens per warp: the
+    choice is that of k scans in which only a greater logit replaces the first expert left, and a
+    chosen NaN makes all scores of its token NaN."""
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(23)
+    nan = float("nan")
+    for bad in range(-1, tot):
+        x = torch.randn(rows, 64, device=DEV).bfloat16()
+        w = torch.randn(tot, 64, device=DEV).bfloat16()
+        if bad < 0:
+            x[::3] = nan
+        else:
+            w[bad] = nan
+        logits, idx, prob = (t.cpu() for t in gating.linear_topk_softmax(x, w, None, k))
+        v = logits.double()
+        left = torch.ones(rows, tot, dtype=torch.bool)
+        for j in range(k):
+            first = left.double().argmax(1, keepdim=True)       # the lowest id left
+            seen = torch.where(left, v, -float("inf")).nan_to_num(nan=-float("inf"))
+            best = seen.argmax(1, keepdim=True)                 # the greatest, the lowest id of equals
+            choice = torch.where(v.gather(1, first).isnan(), first, best)
+            assert torch.equal(idx[:, j:j + 1], choice), (bad, j)
+            left.scatter_(1, choice, False)
+        want = torch.softmax(v.gather(1, idx), 1)
+        assert torch.equal(prob.isnan(), want.isnan())
+        assert torch.allclose(prob.double().nan_to_num(), want.nan_to_num(), atol=2.0 ** -8)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("kind", ["gshard", "switch"])
 @pytest.mark.parametrize("n,tot", [(1, 2), (127, 3), (129, 64), (5000, 8), (40000, 2)])
