@@ -15,6 +15,7 @@ sums of ``dW`` and ``db``; their merge) instead of the six of the ATen sequence.
 import torch
 from torch.autograd import Function
 
+from . import grouped_gemm as gg
 from . import native
 
 MAX_FUSED_K = 8
@@ -57,8 +58,8 @@ class _LinearTopkSoftmax(Function):
 
     @staticmethod
     def forward(ctx, x, weight, bias, k):
-        from .grouped_gemm import aligned
-        x, weight = aligned(x, 16), aligned(weight, 16)   # 16-byte loads
+        if (x.data_ptr() | weight.data_ptr()) % 16 != 0:   # the kernels load 16 bytes at a time
+            x, weight = gg.aligned(x, 16), gg.aligned(weight, 16)
         logits, idx, prob = native.get().gate_linear_topk(x, weight, bias, int(k))
         ctx.save_for_backward(x, weight, idx, prob)
         ctx.has_bias = bias is not None
@@ -91,7 +92,6 @@ class _GateGemm(Function):
 
     @staticmethod
     def forward(ctx, x, weight, bias):
-        from . import grouped_gemm as gg
         tot, d = weight.shape
         pad = (-tot) % 64
         wp = torch.nn.functional.pad(weight, (0, 0, 0, pad)).unsqueeze(0).contiguous()
@@ -108,7 +108,6 @@ class _GateGemm(Function):
 
     @staticmethod
     def backward(ctx, dl):
-        from . import grouped_gemm as gg
         x, wp = ctx.saved_tensors
         dl = dl.contiguous()
         dx = gg.dgrad(dl, wp, None) if ctx.needs_input_grad[0] else None
@@ -121,7 +120,6 @@ class _GateGemm(Function):
 
 
 def _gate_gemm_ok(x, weight, bias):
-    from . import grouped_gemm as gg
     return (x.is_cuda and x.dim() == 2 and x.dtype in (torch.bfloat16, torch.float16)
             and weight.dtype == x.dtype and (bias is None or bias.dtype == x.dtype)
             and x.shape[1] % 64 == 0 and x.shape[0] > 0 and not torch.is_autocast_enabled()
