@@ -119,7 +119,7 @@ std::vector<torch::Tensor> route(torch::Tensor idx, int64_t tot, bool want_offs,
   }
   torch::Tensor part;
   int* part_ptr = nullptr;
-  const int nb = fmoe::route_blocks(n_slots);
+  const int nb = fmoe::route_blocks(n_slots, static_cast<int>(tot));
   if (nb > 1) {
     part = torch::empty({static_cast<int64_t>(nb) * tot}, opt);
     part_ptr = part.data_ptr<int>();

@@ -21,6 +21,8 @@ constexpr int kRouteThreads = 1024;
 constexpr int kRouteSmemLimit = 200 * 1024;
 constexpr int kRouteCluster = 8;
 constexpr int kRouteClusterSlots = 65536;
+constexpr int kRouteClusterExperts = 1024;
+constexpr int kRouteCtaSlots = 32768;
 
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;
@@ -1288,9 +1290,11 @@ cudaError_t simt_typed(int mode, int num_groups, long rows_cap, int m, int n, in
 }  // namespace
 
 // ------------------------------------------------------------------------------ launchers
-int route_blocks(int n_slots) {
-  // one launch (a CTA or a cluster) up to kRouteClusterSlots; beyond that 16 K slots per CTA
-  if (n_slots <= kRouteClusterSlots) return 1;
+int route_blocks(int n_slots, int tot) {
+  // one launch up to what a cluster, or a single CTA where the cluster does not apply, holds; beyond
+  // that 16 K slots per CTA (1025 experts: 40000 slots 58 us on three CTAs, 97 on one; 65536 slots 67
+  // and 154; 65536 slots on 1024 experts 28 on the cluster)
+  if (n_slots <= (tot <= kRouteClusterExperts ? kRouteClusterSlots : kRouteCtaSlots)) return 1;
   int nb = (n_slots + 16383) / 16384;
   return nb > 148 ? 148 : nb;
 }
@@ -1301,10 +1305,10 @@ cudaError_t launch_route(const int64_t* idx, int n_slots, int tot, int* counts, 
   int nw = (kRouteSmemLimit - 4 * (tot + 1)) / (4 * tot);
   if (nw < 1) return cudaErrorInvalidValue;
   if (nw > 32) nw = 32;
-  const int nb = part != nullptr ? route_blocks(n_slots) : 1;
+  const int nb = part != nullptr ? route_blocks(n_slots, tot) : 1;
   // below 1 K slots one CTA has at most one step per warp and pass: nothing to spread; with very
   // many experts the histograms of fewer warps fit beside the cluster's totals
-  const bool cluster = nb == 1 && n_slots > 1024 && tot <= 1024;
+  const bool cluster = nb == 1 && n_slots > 1024 && tot <= kRouteClusterExperts;
   const int ctas = cluster ? kRouteCluster : nb;
   int cta_slots = (n_slots + ctas - 1) / ctas;
   cta_slots = (cta_slots + 31) & ~31;

@@ -9,9 +9,10 @@ namespace fmoe {
 // (exclusive prefix of counts) and optional pos[n_slots] (slot ids sorted by expert, then by
 // rank: pos[offs[e] + rank[s]] = s; entries past offs[tot] are not written).  Deterministic:
 // slots of one expert are ranked by slot id.
-// `part` (optional): int32 scratch of route_blocks(n_slots) * tot entries; with it, more than
-// 64 K slots are ranked by many CTAs in two launches instead of by one cluster.
-int route_blocks(int n_slots);
+// `part` (optional): int32 scratch of route_blocks(n_slots, tot) * tot entries; with it, more than
+// 64 K slots (32 K with more experts than the cluster takes) are ranked by many CTAs in two
+// launches instead of by one cluster or CTA.
+int route_blocks(int n_slots, int tot);
 cudaError_t launch_route(const int64_t* idx, int n_slots, int tot, int* counts, int* rank,
                          int* offs, int* pos, int* part, cudaStream_t stream);
 

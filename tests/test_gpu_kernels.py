@@ -492,6 +492,17 @@ def test_route_at_the_lines_between_cta_cluster_and_grid(n_slots, tot):
     assert torch.equal(rank, want_rank)
 
 
+@pytest.mark.parametrize("n_slots,tot,launches", [(32768, 1025, 1), (32769, 1025, 2), (65536, 5000, 2), (65536, 1024, 1),
+                                                  (65537, 1024, 2)])
+def test_route_launches(n_slots, tot, launches):
+    r"""One launch while a cluster, or with more than 1024 experts a CTA, holds the slots; then two on
+    many CTAs."""
+    idx = torch.zeros(n_slots, dtype=torch.int64, device=DEV)
+    before = _native().launch_count()
+    _native().route_pos(idx, tot)
+    assert _native().launch_count() - before == launches
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows,tot,k,d", [(2367, 8, 2, 136), (2368, 7, 7, 264), (2369, 2, 1, 128), (4735, 3, 2, 64),
                                           (4736, 8, 2, 1024), (4739, 2, 2, 512), (9001, 5, 4, 520), (1, 1, 1, 8)])
