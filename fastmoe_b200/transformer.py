@@ -22,6 +22,7 @@ import torch.nn as nn
 from .layers import FMoE
 from .linear import FMoELinear
 
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
 _PER_EXPERT_KEY = re.compile(r"^(.*experts\.)(\d+)\.(htoh4|h4toh)\.(weight|bias)$")
 
 
@@ -37,7 +38,7 @@ def activation_kind(act):
         return "gelu"
     if act is torch.nn.functional.relu or act is torch.relu:
         return "relu"
-    if type(act) is nn.Sequential and not _hooked(act):
+    if type(act) is nn.Sequential and not _hooked(act) and not _hooked_globally():
         # a chain whose other members do nothing in this call: the Transformer-XL block's
         # ReLU -> Dropout at evaluation, or with p = 0
         live = [m for m in act if not _does_nothing(m)]
@@ -49,9 +50,14 @@ def activation_kind(act):
 
 
 def _hooked(module):
-    r"""Whether somebody watches calls of ``module``, which a fused activation would not make."""
-    return any(getattr(module, name, None) for name in
-               ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks"))
+    r"""Whether somebody watches calls of ``module``, or has put another ``forward`` into the instance:
+    a fused activation would not make the call."""
+    return "forward" in vars(module) or any(getattr(module, name, None) for name in _HOOKS)
+
+
+def _hooked_globally():
+    r"""Whether somebody watches the calls of all modules (``register_module_forward_hook`` and the like)."""
+    return any(getattr(nn.modules.module, "_global" + name, None) for name in _HOOKS)
 
 
 def _does_nothing(module):

@@ -468,3 +468,27 @@ def test_scatter_gather_rows_and_gradients():
     assert torch.equal(back[pos], y.detach()) and float(back[1 * k + 0].abs().sum()) == 0.0
     assert torch.autograd.gradcheck(
         lambda t: MOEGather.apply(t, pos, lec, gec, n_tok * k, 1), (y,))
+
+
+def test_watched_activation_chain_is_not_fused():
+    r"""A chain is only replaced by a fused activation while nobody watches its members: hooks of a
+    member, hooks of all modules, or another ``forward`` put into an instance."""
+    from fastmoe_b200.transformer import activation_kind
+    seq = nn.Sequential(nn.ReLU(), nn.Dropout(0.0))
+    assert activation_kind(seq) == "relu"
+    everywhere = nn.modules.module
+    for watch in (lambda: everywhere.register_module_forward_hook(lambda m, i, o: None),
+                  lambda: everywhere.register_module_forward_pre_hook(lambda m, i: None),
+                  lambda: everywhere.register_module_full_backward_hook(lambda m, i, o: None),
+                  lambda: everywhere.register_module_full_backward_pre_hook(lambda m, o: None),
+                  lambda: seq[1].register_forward_hook(lambda m, i, o: None),
+                  lambda: seq.register_full_backward_hook(lambda m, i, o: None)):
+        handle = watch()
+        assert activation_kind(seq) is None
+        handle.remove()
+        assert activation_kind(seq) == "relu"
+    for module in (seq, seq[0], seq[1]):
+        module.forward = type(module).forward.__get__(module)
+        assert activation_kind(seq) is None
+        del module.forward
+        assert activation_kind(seq) == "relu"
