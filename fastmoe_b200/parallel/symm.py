@@ -552,7 +552,8 @@ def moe_mlp_forward(layer, x, gate_idx, gate_score):
         from ..utils.profiling import check_routing
         check_routing(idx, rank, lec, n_expert * ws.world)
     capacity = receive_capacity(budget, k, ws.world)
-    act = activation_kind(layer.experts.activation)
+    # which exchange runs must not depend on hooks, which one rank may have and another not
+    act = activation_kind(layer.experts.activation, chains=False)
     if act is not None:
         e = layer.experts
         return _FusedEPMLP.apply(x.contiguous(), score, e.htoh4.weight, e.htoh4.bias, e.h4toh.weight,

@@ -26,8 +26,12 @@ _HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_
 _PER_EXPERT_KEY = re.compile(r"^(.*experts\.)(\d+)\.(htoh4|h4toh)\.(weight|bias)$")
 
 
-def activation_kind(act):
-    r"""Name of an activation the fused GEMM epilogue implements, or ``None``."""
+def activation_kind(act, chains=True):
+    r"""Name of an activation the fused GEMM epilogue implements, or ``None``.
+
+    With ``chains`` a ``Sequential`` whose other members do nothing in this call counts as the one
+    that does.  That depends on who watches the modules in this process, so what all ranks have
+    to decide alike is decided without."""
     if isinstance(act, nn.GELU):
         return "gelu_tanh" if getattr(act, "approximate", "none") == "tanh" else "gelu"
     if isinstance(act, nn.ReLU):
@@ -38,7 +42,7 @@ def activation_kind(act):
         return "gelu"
     if act is torch.nn.functional.relu or act is torch.relu:
         return "relu"
-    if type(act) is nn.Sequential and not _hooked(act) and not _hooked_globally():
+    if chains and type(act) is nn.Sequential and not _hooked(act) and not _hooked_globally():
         # a chain whose other members do nothing in this call: the Transformer-XL block's
         # ReLU -> Dropout at evaluation, or with p = 0
         live = [m for m in act if not _does_nothing(m)]

@@ -492,3 +492,30 @@ def test_watched_activation_chain_is_not_fused():
         assert activation_kind(seq) is None
         del module.forward
         assert activation_kind(seq) == "relu"
+
+
+@pytest.mark.parametrize("act,exchange", [(nn.ReLU(), "fused"), (nn.Sequential(nn.ReLU(), nn.Dropout(0.0)), "plain")])
+def test_hooks_do_not_choose_the_exchange(act, exchange, monkeypatch):
+    r"""Under expert parallelism all ranks have to run the same exchange, whoever has a hook."""
+    from fastmoe_b200.ops import fused, native
+    from fastmoe_b200.parallel import symm
+    taken = []
+
+    def record(name, result):
+        return types.SimpleNamespace(apply=lambda *a: (taken.append(name), result)[1])
+
+    monkeypatch.setattr(native, "get", lambda: types.SimpleNamespace(route_pos=lambda idx, tot: (None,) * 4))
+    monkeypatch.setattr(symm, "get_workspace", lambda comm, device: types.SimpleNamespace(world=2, token_budget=lambda n: n))
+    monkeypatch.setattr(symm, "_layer_group", lambda layer: None)
+    monkeypatch.setattr(symm, "_FusedEPMLP", record("fused", None))
+    monkeypatch.setattr(symm, "_DispatchP2P", record("plain", (None,) * 5))
+    monkeypatch.setattr(symm, "_CombineP2P", record("combine", None))
+    monkeypatch.setattr(fused, "expert_mlp", lambda layer, xs, offs: None)
+    lin = types.SimpleNamespace(weight=None, bias=None)
+    layer = types.SimpleNamespace(num_expert=2, experts=types.SimpleNamespace(htoh4=lin, h4toh=lin, activation=act))
+    args = layer, torch.zeros(3, 4), torch.zeros(3, 1, dtype=torch.long), torch.ones(3, 1)
+    symm.moe_mlp_forward(*args)
+    handle = act.register_forward_hook(lambda m, i, o: None)
+    symm.moe_mlp_forward(*args)
+    handle.remove()
+    assert [t for t in taken if t != "combine"] == [exchange] * 2
