@@ -63,7 +63,8 @@ def prepare_forward(gate, num_expert, world_size):
     with torch.no_grad():
         # the one device -> host read of the general path
         if gec is lec:
-            lec_cpu = gec_cpu = lec.cpu()
+            lec_cpu = lec.cpu()
+            gec_cpu = lec_cpu.clone()   # two tensors: a caller may change one of them
         else:
             both = torch.stack([lec, gec]).cpu()
             lec_cpu, gec_cpu = both[0], both[1]

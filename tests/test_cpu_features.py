@@ -519,3 +519,12 @@ def test_hooks_do_not_choose_the_exchange(act, exchange, monkeypatch):
     symm.moe_mlp_forward(*args)
     handle.remove()
     assert [t for t in taken if t != "combine"] == [exchange] * 2
+
+
+def test_prepared_counts_are_separate_tensors():
+    from fastmoe_b200.functions import prepare_forward
+    _pos, lec, gec, fwd, _n = prepare_forward(torch.tensor([[0], [1], [1]]), 2, 1)
+    lec.zero_()
+    assert gec.tolist() == [1, 2] and fwd.tolist() == [1, 2]
+    gec.zero_()
+    assert fwd.tolist() == [1, 2]
