@@ -47,6 +47,10 @@ class SwitchGate(NaiveGate):
         share.scatter_add_(0, ids.clamp(min=0), kept)
         return self.tot_expert * ((share / n_kept) * (prob.sum(dim=0) / n_kept)).sum()
 
+    def _usual_loss(self):
+        r"""Whether the balance loss is this class's own, the one the kernels compute."""
+        return type(self)._balance_loss is SwitchGate._balance_loss and "_balance_loss" not in vars(self)
+
     def _score_and_loss(self, logits, chosen, winner):
         r"""The score of the experts ``chosen`` and the loss for the kept ones ``winner``."""
         prob = torch.softmax(logits.float(), dim=-1)
@@ -55,7 +59,8 @@ class SwitchGate(NaiveGate):
     def forward(self, inp):
         logits = self._jitter(self.gate(inp))
         cap = self._slots_per_expert(inp.shape[0])
-        if self.world_size == 1 and logits.dtype == inp.dtype and gating.balance_native(logits):
+        if (self.world_size == 1 and logits.dtype == inp.dtype and gating.balance_native(logits)
+                and self._usual_loss()):
             winner, score, loss = gating.switch_route(logits, cap, self._score_and_loss)
             self.set_loss(loss)
             return winner, score

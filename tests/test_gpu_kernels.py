@@ -672,6 +672,22 @@ def test_wide_gate_first_called_under_capture(rows):
     assert close(captured, xg.double() @ wg.double().t() + bg.double())
 
 
+def test_switch_gate_with_its_own_loss():
+    r"""A subclass, or an instance, with another balance loss is asked for it."""
+    from fastmoe_b200.gates import SwitchGate
+
+    class Summed(SwitchGate):
+        def _balance_loss(self, prob, winner):
+            return prob.sum() + (winner >= 0).sum()
+
+    x = torch.randn(40, 64, device=DEV)
+    patched = SwitchGate(64, 4, 1).to(DEV)
+    patched._balance_loss = lambda prob, winner: prob.sum() + (winner >= 0).sum()
+    for gate in (Summed(64, 4, 1).to(DEV), patched):
+        idx, _score = gate(x)
+        assert abs(float(gate.get_loss()) - 40 - int((idx >= 0).sum())) < 1e-3
+
+
 def test_balance_loss_second_derivative():
     r"""A gradient of the gradient goes through the PyTorch operations."""
     from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
