@@ -12,6 +12,7 @@ dropped with id -1) and the same balance loss
 import math
 
 import torch
+from torch.autograd import forward_ad
 
 from .naive_gate import NaiveGate
 from .utils import limit_by_capacity
@@ -60,7 +61,7 @@ class SwitchGate(NaiveGate):
         logits = self._jitter(self.gate(inp))
         cap = self._slots_per_expert(inp.shape[0])
         if (self.world_size == 1 and logits.dtype == inp.dtype and gating.balance_native(logits)
-                and self._usual_loss()):
+                and self._usual_loss() and forward_ad.unpack_dual(logits).tangent is None):
             winner, score, loss = gating.switch_route(logits, cap, self._score_and_loss)
             self.set_loss(loss)
             return winner, score

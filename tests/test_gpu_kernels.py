@@ -688,6 +688,34 @@ def test_switch_gate_with_its_own_loss():
         assert abs(float(gate.get_loss()) - 40 - int((idx >= 0).sum())) < 1e-3
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_switch_gate_in_forward_mode(dtype):
+    r"""Directional derivatives of Switch's scores and loss, in 64 bits up to the type's rounding (the
+    derivative of a softmax over 4 entries is a sum of 4 products of numbers of order one)."""
+    import torch.autograd.forward_ad as forward_ad
+    from fastmoe_b200.gates import SwitchGate
+    torch.manual_seed(24)
+    gate = SwitchGate(64, 4, 1).to(DEV).to(dtype).eval()
+    x, dx = (torch.randn(50, 64, device=DEV).to(dtype) for _ in range(2))
+    with forward_ad.dual_level():
+        idx, score = gate(forward_ad.make_dual(x, dx))
+        dscore = forward_ad.unpack_dual(score).tangent
+        dloss = forward_ad.unpack_dual(gate.get_loss()).tangent
+        logits, tangent = forward_ad.unpack_dual(gate.gate(forward_ad.make_dual(x, dx)))
+    assert (idx >= 0).all()   # nothing is dropped at 2.4 times the even share
+    l64 = logits.detach().double().requires_grad_(True)
+    p = torch.softmax(l64, 1)
+    share = torch.bincount(idx.view(-1), minlength=4).double() / 50
+
+    def along(y):   # d y of every row, or of all
+        return (torch.autograd.grad(y.sum(), l64, retain_graph=True)[0] * tangent.double()).sum(1)
+
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
+    want = along(p.gather(1, idx))
+    assert torch.allclose(dscore.double().view(-1), want, atol=8 * eps)
+    assert torch.allclose(dloss.double(), along(4 * (share * p.sum(0) / 50).sum()).sum(), atol=8 * 2.0 ** -20)
+
+
 def test_balance_loss_second_derivative():
     r"""A gradient of the gradient goes through the PyTorch operations."""
     from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
