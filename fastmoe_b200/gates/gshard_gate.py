@@ -3,6 +3,7 @@ r"""GShard top-2 gate with local capacity and random second-expert routing.
 Parity: ``fmoe/gates/gshard_gate.py:12-49``.
 """
 import math
+from functools import partial
 
 import torch
 import torch.nn.functional as F
@@ -20,6 +21,10 @@ def gshard_balance_loss(logits, top1_idx, tot_expert, num_expert):
         0, top1_idx, torch.ones_like(top1_idx, dtype=torch.float32)) / n
     m_e = F.softmax(logits, dim=1).mean(dim=0)
     return torch.mean(c_e * m_e.float()) * (num_expert ** 2)
+
+
+def _loss_of_choices(logits, topk_idx, num_expert):
+    return gshard_balance_loss(logits, topk_idx[:, 0], logits.shape[1], num_expert)
 
 
 def drop_second_expert_randomly(topk_idx, topk_val):
@@ -46,9 +51,8 @@ class GShardGate(NaiveGate):
         cap = math.ceil(rate * x.shape[0]) * self.top_k // self.tot_expert
         # (under autocast the operations hold the probabilities in fp32: the kernels do not)
         if gating.balance_native(logits) and not torch.is_autocast_enabled():
-            self.set_loss(gating.gshard_loss(
-                logits, topk_idx, self.num_expert ** 2,
-                lambda l, ids: gshard_balance_loss(l, ids[:, 0], self.tot_expert, self.num_expert)))
+            self.set_loss(gating.gshard_loss(logits, topk_idx, self.num_expert ** 2,
+                                             partial(_loss_of_choices, num_expert=self.num_expert)))
         else:
             self.set_loss(gshard_balance_loss(logits, topk_idx[:, 0], self.tot_expert, self.num_expert))
         if topk_idx.is_cuda and topk_idx.numel() > 0:

@@ -19,6 +19,23 @@ from .utils import limit_by_capacity
 from ..ops import gating
 
 
+def switch_balance_loss(prob, winner, tot_expert):
+    r"""``tot_expert * sum_e fraction_e * mean_prob_e`` over the kept tokens, without boolean indexing
+    (no device-to-host read, so the gate can sit in a CUDA graph)."""
+    ids = winner.reshape(-1)
+    kept = (ids >= 0).to(prob.dtype)
+    n_kept = kept.sum().clamp(min=1.0)
+    share = torch.zeros(tot_expert, dtype=prob.dtype, device=prob.device)
+    share.scatter_add_(0, ids.clamp(min=0), kept)
+    return tot_expert * ((share / n_kept) * (prob.sum(dim=0) / n_kept)).sum()
+
+
+def switch_score_and_loss(logits, chosen, winner):
+    r"""The score of the experts ``chosen`` and the loss for the kept ones ``winner``."""
+    prob = torch.softmax(logits.float(), dim=-1)
+    return prob.gather(1, chosen).to(logits.dtype), switch_balance_loss(prob, winner, logits.shape[1])
+
+
 class SwitchGate(NaiveGate):
 
     def __init__(self, d_model, num_expert, world_size, topk=1, switch_eps=.1,
@@ -40,29 +57,18 @@ class SwitchGate(NaiveGate):
         return math.ceil(rate * n_tokens / self.num_expert)
 
     def _balance_loss(self, prob, winner):
-        r"""Without boolean indexing (no device-to-host read, so the gate can sit in a CUDA graph)."""
-        ids = winner.reshape(-1)
-        kept = (ids >= 0).to(prob.dtype)
-        n_kept = kept.sum().clamp(min=1.0)
-        share = torch.zeros(self.tot_expert, dtype=prob.dtype, device=prob.device)
-        share.scatter_add_(0, ids.clamp(min=0), kept)
-        return self.tot_expert * ((share / n_kept) * (prob.sum(dim=0) / n_kept)).sum()
+        return switch_balance_loss(prob, winner, self.tot_expert)
 
     def _usual_loss(self):
         r"""Whether the balance loss is this class's own, the one the kernels compute."""
         return type(self)._balance_loss is SwitchGate._balance_loss and "_balance_loss" not in vars(self)
-
-    def _score_and_loss(self, logits, chosen, winner):
-        r"""The score of the experts ``chosen`` and the loss for the kept ones ``winner``."""
-        prob = torch.softmax(logits.float(), dim=-1)
-        return prob.gather(1, chosen).to(logits.dtype), self._balance_loss(prob, winner)
 
     def forward(self, inp):
         logits = self._jitter(self.gate(inp))
         cap = self._slots_per_expert(inp.shape[0])
         if (self.world_size == 1 and logits.dtype == inp.dtype and gating.balance_native(logits)
                 and self._usual_loss() and forward_ad.unpack_dual(logits).tangent is None):
-            winner, score, loss = gating.switch_route(logits, cap, self._score_and_loss)
+            winner, score, loss = gating.switch_route(logits, cap, switch_score_and_loss)
             self.set_loss(loss)
             return winner, score
         prob = torch.softmax(logits.float(), dim=-1)

@@ -174,7 +174,8 @@ def prune_to_capacity(idx, cap, tot_expert):
 
 class _BalanceLoss(Function):
     r"""``reference(logits, ids)`` — GShard's loss — from two launches, its gradient from one.  Both
-    round to the type of the logits where the PyTorch operations do (without autocast)."""
+    round to the type of the logits where the PyTorch operations do (without autocast).
+    ``reference`` lives as long as the loss, so it must not hold the gate that holds the loss."""
 
     @staticmethod
     def forward(ctx, logits, ids, scale, reference):
@@ -200,8 +201,9 @@ def gshard_loss(logits, ids, scale, reference):
 
 class _SwitchRoute(Function):
     r"""Switch's choice, capacity limit and balance loss of one rank: ``(ids [n, 1], score [n, 1],
-    loss)``.  ``reference(logits, ids)`` gives ``(score, loss)`` in PyTorch operations for the
-    given pruned ids and winners."""
+    loss)``.  ``reference(logits, chosen, kept)`` gives ``(score, loss)`` in PyTorch operations for
+    the chosen experts and those of them that the capacity kept (-1 elsewhere).  It lives as long
+    as the loss, so it must not hold the gate that holds the loss."""
 
     @staticmethod
     def forward(ctx, logits, cap, reference):

@@ -716,6 +716,26 @@ def test_switch_gate_in_forward_mode(dtype):
     assert torch.allclose(dloss.double(), along(4 * (share * p.sum(0) / 50).sum()).sum(), atol=8 * 2.0 ** -20)
 
 
+@pytest.mark.parametrize("kind", ["GShardGate", "SwitchGate"])
+def test_gate_with_an_unread_loss_is_freed_at_once(kind):
+    r"""The loss a gate holds does not hold the gate: no cycle that waits for the collector with the
+    graph of the last pass."""
+    import gc
+    import weakref
+    from fastmoe_b200 import gates
+    gate = getattr(gates, kind)(64, 4, 1).to(DEV)
+    gate(torch.randn(8, 64, device=DEV))
+    assert gate.has_loss
+    gone = weakref.ref(gate)
+    gc.collect()
+    gc.disable()
+    try:
+        del gate
+        assert gone() is None
+    finally:
+        gc.enable()
+
+
 def test_balance_loss_second_derivative():
     r"""A gradient of the gradient goes through the PyTorch operations."""
     from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
