@@ -212,18 +212,20 @@ class _SwitchRoute(Function):
         win, score = nat.switch_top1(logits)
         kept = nat.prune_gate_scalar(win, cap, tot)
         loss, weight = nat.balance_loss(logits, kept, True, float(tot))
-        ctx.save_for_backward(logits, win, kept, weight)
-        ctx.reference = reference
+        # (`kept` is the caller's to change; a second derivative forms it again)
+        ctx.save_for_backward(logits, win, weight)
+        ctx.reference, ctx.cap = reference, cap
         ctx.mark_non_differentiable(kept)
         ctx.set_materialize_grads(False)
         return kept, score, loss
 
     @staticmethod
     def backward(ctx, _grad_kept, grad_score, grad_loss):
-        logits, win, kept, weight = ctx.saved_tensors
+        logits, win, weight = ctx.saved_tensors
         if grad_score is None and grad_loss is None:
             return None, None, None
         if torch.is_grad_enabled():   # a gradient of the gradient is wanted
+            kept = native.get().prune_gate_scalar(win, ctx.cap, logits.shape[1])
             with torch.enable_grad():
                 outs, grads = [], []
                 for out, grad in zip(ctx.reference(logits, win, kept), (grad_score, grad_loss)):

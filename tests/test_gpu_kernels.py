@@ -736,6 +736,27 @@ def test_gate_with_an_unread_loss_is_freed_at_once(kind):
         gc.enable()
 
 
+def test_switch_ids_belong_to_the_caller():
+    r"""Ids changed in place between forward and backward (by a gate hook, say) do not matter to the
+    gradients, of first or second order."""
+    from fastmoe_b200.gates import SwitchGate
+    torch.manual_seed(25)
+    gate = SwitchGate(64, 4, 1, switch_eps=0.0, capacity=(0.7, 0.7)).to(DEV)
+    x = torch.randn(30, 64, device=DEV)
+    grads = []
+    for change in (False, True):
+        idx, score = gate(x)
+        loss = gate.get_loss() + score.square().sum()
+        assert (idx < 0).any() and (idx >= 0).any()
+        if change:
+            idx.fill_(1)
+        first = torch.autograd.grad(loss, gate.gate.weight, retain_graph=True)[0]
+        again = torch.autograd.grad(loss, gate.gate.weight, create_graph=True)[0]
+        grads.append((first, torch.autograd.grad(again.square().sum(), gate.gate.weight)[0]))
+    for a, b in zip(*grads):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-6)   # scatter_add_ of the operations is unordered
+
+
 def test_balance_loss_second_derivative():
     r"""A gradient of the gradient goes through the PyTorch operations."""
     from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
