@@ -757,6 +757,29 @@ def test_switch_ids_belong_to_the_caller():
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-6)   # scatter_add_ of the operations is unordered
 
 
+@pytest.mark.parametrize("tot", [2, 8, 16, 33, 64])
+def test_fp32_switch_scores_and_gradients_are_no_further_off(tot):
+    r"""Distance of Switch's fp32 scores, loss and logit gradients from 64 bits, root of the mean square,
+    against that of the PyTorch operations: equal up to what 60000 draws leave to chance."""
+    from fastmoe_b200.gates.switch_gate import switch_score_and_loss
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(26)
+    n = 60000
+    logits = (torch.randn(n, tot, device=DEV) * 2).requires_grad_(True)
+    gs = torch.randn(n, 1, device=DEV)
+    ids, score, loss = gating.switch_route(logits, n, switch_score_and_loss)
+    outs = [(score, loss, torch.autograd.grad([score, loss], logits, [gs, None])[0])]
+    for dtype in (torch.float32, torch.float64):
+        x = logits.detach().to(dtype).requires_grad_(True)
+        prob = torch.softmax(x, 1)
+        share = torch.bincount(ids.view(-1), minlength=tot).to(dtype)
+        s, l = prob.gather(1, ids), tot * ((share / n) * (prob.sum(0) / n)).sum()
+        outs.append((s, l, torch.autograd.grad([s, l], x, [gs.to(dtype), None])[0]))
+    for name, native, ops, exact in zip(("score", "loss", "gradient"), *outs):
+        off = [float((t.detach().double() - exact.detach()).square().mean().sqrt()) for t in (native, ops)]
+        assert off[0] <= 1.05 * off[1] + (2.0 ** -23 * abs(float(exact)) if name == "loss" else 0.0), (name, off)
+
+
 def test_balance_loss_second_derivative():
     r"""A gradient of the gradient goes through the PyTorch operations."""
     from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
