@@ -220,8 +220,15 @@ __device__ __forceinline__ float tanh_approx(float x) {
   return y;
 }
 
+// max(x, 0) that lets NaN through, as torch.relu does
+__device__ __forceinline__ float relu(float x) {
+  float y;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 template <int ACT> __device__ __forceinline__ float act_fwd(float x) {
-  if (ACT == kActRelu) return fmaxf(x, 0.f);
+  if (ACT == kActRelu) return relu(x);
   if (ACT == kActGelu) return x * gelu_parts(x).cdf;
   if (ACT == kActGeluTanh) {
     const float u = 0.7978845608028654f * fmaf(0.044715f * x * x, x, x);
@@ -230,7 +237,6 @@ template <int ACT> __device__ __forceinline__ float act_fwd(float x) {
   return x;
 }
 template <int ACT> __device__ __forceinline__ float act_grad(float x) {
-  if (ACT == kActRelu) return x > 0.f ? 1.f : 0.f;
   if (ACT == kActGelu) {
     const GeluParts g = gelu_parts(x);
     return fmaf(x * 0.3989422804014327f, g.gauss, g.cdf);
@@ -243,6 +249,12 @@ template <int ACT> __device__ __forceinline__ float act_grad(float x) {
     return fmaf(0.5f * x * (1.0f - t * t), du, 0.5f * (1.0f + t));
   }
   return 1.f;
+}
+
+// g * act'(x); for ReLU the choice that torch makes: zero, whatever g, where x <= 0, and g elsewhere
+template <int ACT> __device__ __forceinline__ float act_bwd(float g, float x) {
+  if (ACT == kActRelu) return x <= 0.f ? 0.f : g;
+  return g * act_grad<ACT>(x);
 }
 
 template <typename T> struct Cvt;
@@ -347,8 +359,8 @@ __device__ __forceinline__ void rows_chunk(const RowTile& rt, int i, bool with_p
       for (int j = 0; j < 8; ++j) {
         float sa, sb;
         Cvt<T>::unpack(side_cur.w[q * 8 + j], sa, sb);
-        const float a = __uint_as_float(r[q * 16 + 2 * j]) * act_grad<ACT>(sa);
-        const float b = __uint_as_float(r[q * 16 + 2 * j + 1]) * act_grad<ACT>(sb);
+        const float a = act_bwd<ACT>(__uint_as_float(r[q * 16 + 2 * j]), sa);
+        const float b = act_bwd<ACT>(__uint_as_float(r[q * 16 + 2 * j + 1]), sb);
         wo[j] = Cvt<T>::pack(a, b);
       }
     } else {

@@ -166,8 +166,8 @@ template <int ACT> __device__ __forceinline__ void act_grad2(float x0, float x1,
                                    gelu_cdf2(x0, x1, h));
     ptx::unpack2(ptx::mul2(ptx::pack2(a, b), d), a, b);
   } else {
-    a *= gg::act_grad<ACT>(x0);
-    b *= gg::act_grad<ACT>(x1);
+    a = gg::act_bwd<ACT>(a, x0);
+    b = gg::act_bwd<ACT>(b, x1);
   }
 }
 

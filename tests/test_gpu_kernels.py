@@ -796,6 +796,48 @@ def test_balance_loss_second_derivative():
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-9)
 
 
+@pytest.mark.parametrize("counts,want_pre", [([200, 0, 130], True), ([200, 0, 130], False), ([3, 0, 5], True),
+                                             ([3, 0, 5], False)])
+def test_fused_relu_of_nan_and_infinities(counts, want_pre):
+    r"""The fused ReLU and its derivative treat NaN and infinities as torch.relu does, in the paired
+    kernel, the single-CTA kernel (few rows, pre-activation kept) and the narrow one: NaN is not
+    hidden, and a gradient, whatever it is, does not pass where the input is not positive."""
+    from fastmoe_b200.ops import grouped_gemm as gg
+    torch.manual_seed(27)
+    nan, inf = float("nan"), float("inf")
+    g, rows, k, n = len(counts), sum(counts), 64, 96
+    offs = _offs(counts)
+    x = torch.randn(rows, k, device=DEV).bfloat16()
+    x[1] = nan
+    w = torch.randn(g, n, k, device=DEV).bfloat16()
+    b = torch.randn(g, n, device=DEV).bfloat16()
+    b[:, 3], b[:, 40], b[:, 70] = nan, inf, -inf
+    y = gg.forward(x, w, offs, b, act="relu", want_pre=want_pre)
+    if want_pre:
+        y, blocked = y
+        plain = gg.forward(x, w, offs, b)
+        dy = torch.randn(rows, k, device=DEV).bfloat16()
+        dy[2] = inf
+        dx = gg.dgrad(dy, w.transpose(1, 2).contiguous(), offs, pre=blocked, act="relu")
+    for e, lo, hi in _segments(counts):
+        if hi == lo:
+            continue
+        pre = x[lo:hi].double() @ w[e].double().t() + b[e].double()
+        ref = torch.relu(pre)
+        assert torch.equal(y[lo:hi].isnan(), ref.isnan()) and torch.equal(y[lo:hi].isinf(), ref.isinf())
+        assert torch.allclose(y[lo:hi].double(), ref, rtol=2.0 ** -8, atol=1e-4, equal_nan=True)
+        if want_pre:
+            # (an infinite sum of the fp32 accumulators has no 64-bit counterpart: compare what is chosen)
+            ungated = dy[lo:hi].double() @ w[e].double().t()
+            off = plain[lo:hi].double() <= 0
+            assert (dx[lo:hi][off] == 0).all()
+            got, want = dx[lo:hi][~off].double(), ungated[~off]
+            assert torch.equal(got.isfinite(), want.isfinite())
+            keep = want.isfinite()
+            assert torch.allclose(got[keep], want[keep], rtol=2.0 ** -8, atol=1e-3)
+    assert _native().read_status(0) == 0
+
+
 def test_inert_dropout_is_fused_and_live_dropout_is_not():
     from fastmoe_b200.transformer import activation_kind
     seq = torch.nn.Sequential(torch.nn.ReLU(), torch.nn.Dropout(0.5))
