@@ -443,13 +443,15 @@ std::vector<torch::Tensor> moe_mlp_forward(torch::Tensor x_in, torch::Tensor idx
   return {out, xs, pre.has_value() ? *pre : torch::Tensor(), a, ys, rank, offs, score, idx};
 }
 
-// {dx, dscore, dw1, db1, dw2, db2}; what `need_*` leaves out is empty.
-std::vector<torch::Tensor> moe_mlp_backward(torch::Tensor dout_in, torch::Tensor xs, c10::optional<torch::Tensor> pre,
-                                            torch::Tensor a, torch::Tensor ys, torch::Tensor rank, torch::Tensor offs,
+// {dx, dscore, dw1, db1, dw2, db2}; what `need_*` leaves out is empty.  Saved tensors may have been
+// through hooks of the caller, which need not return them where they were.
+std::vector<torch::Tensor> moe_mlp_backward(torch::Tensor dout_in, torch::Tensor xs_in, c10::optional<torch::Tensor> pre,
+                                            torch::Tensor a_in, torch::Tensor ys_in, torch::Tensor rank, torch::Tensor offs,
                                             torch::Tensor score, torch::Tensor idx, torch::Tensor w1_in,
                                             torch::Tensor w2_in, int64_t act, bool need_dx, bool need_w1, bool need_w2) {
-  c10::cuda::CUDAGuard guard(xs.device());
-  const torch::Tensor dout = aligned(dout_in, 16);
+  c10::cuda::CUDAGuard guard(xs_in.device());
+  const torch::Tensor dout = aligned(dout_in, 16), xs = aligned32(xs_in), a = aligned32(a_in), ys = aligned(ys_in, 16);
+  if (pre.has_value()) pre = aligned32(*pre);
   const torch::Tensor w1 = aligned32(w1_in), w2 = aligned32(w2_in);
   const int64_t groups = w1.size(0), h = w1.size(1), d = w1.size(2), n_tok = dout.size(0), k = idx.numel() / n_tok;
   auto dys = torch::empty_like(ys);

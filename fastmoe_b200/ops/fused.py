@@ -89,7 +89,7 @@ class _Combine(Function):
         ys, score, idx, rank, offs = ctx.saved_tensors
         dys = torch.empty_like(ys)
         dscore = torch.empty_like(score)
-        native.get().combine_bwd(gg.aligned(dout, 16), ys, idx, rank, offs, score, ctx.k, dys, dscore)
+        native.get().combine_bwd(gg.aligned(dout, 16), gg.aligned(ys, 16), idx, rank, offs, score, ctx.k, dys, dscore)
         return dys, dscore, None, None, None, None
 
 

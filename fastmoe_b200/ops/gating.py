@@ -72,6 +72,8 @@ class _LinearTopkSoftmax(Function):
         x, weight, idx, prob = ctx.saved_tensors
         if grad_logits is None and grad_prob is None:
             return None, None, None, None
+        if (x.data_ptr() | weight.data_ptr()) % 16 != 0:   # moved by hooks on the saved tensors
+            x, weight = gg.aligned(x, 16), gg.aligned(weight, 16)
         dx, dw, db, _dl = native.get().gate_linear_topk_bwd(
             None if grad_prob is None else grad_prob.contiguous(), idx, prob,
             None if grad_logits is None else grad_logits.contiguous(), x, weight,

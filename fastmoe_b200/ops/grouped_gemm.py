@@ -115,7 +115,7 @@ def dgrad(dy, weight, offs, pre=None, act=None):
         return out
     if _tc_ok(dy, MODE_NN, 0, n, k, groups) and (not code or pre.dim() == 1):
         nat.grouped_gemm(MODE_NN, aligned(dy), aligned(weight), offs, out, None, None,
-                         pre if code else None, code, EPI_DACT if code else EPI_BIAS_ACT, False)
+                         aligned(pre) if code else None, code, EPI_DACT if code else EPI_BIAS_ACT, False)
     elif _tc_ok(dy, MODE_NN, 0, n, k, groups):
         # a row-major pre-activation: plain tensor-core product, derivative as a PyTorch op
         nat.grouped_gemm(MODE_NN, aligned(dy), aligned(weight), offs, out, None, None, None, 0,

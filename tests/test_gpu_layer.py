@@ -235,6 +235,31 @@ def test_rows_that_start_anywhere(dtype, act, experts, monkeypatch):
             assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("experts", [5, 12])
+@pytest.mark.parametrize("act", [nn.GELU(), nn.Tanh()])
+def test_saved_tensors_that_come_back_elsewhere(experts, act, monkeypatch):
+    r"""Hooks on saved tensors may return them at any address: the bits of a run without hooks."""
+    from fastmoe_b200 import FMoETransformerMLP
+    torch.manual_seed(28)
+    layer = FMoETransformerMLP(num_expert=experts, d_model=128, d_hidden=192, top_k=2, activation=act).to(DEV).bfloat16()
+    x = torch.randn(77, 128, device=DEV).bfloat16()
+    gy = torch.randn(77, 128, device=DEV).bfloat16()
+
+    def run(unpack):
+        layer.zero_grad(set_to_none=True)
+        xi = x.detach().requires_grad_(True)
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            y = layer(xi)
+        y.backward(gy)
+        return [y, xi.grad] + [p.grad for p in layer.parameters()]
+
+    for checks in ("0", "1"):
+        monkeypatch.setenv("FMOE_DEBUG_BOUNDS", checks)
+        want = run(lambda t: t)
+        for a, b in zip(run(lambda t: _shifted(t) if t.dtype == torch.bfloat16 else t), want):
+            assert torch.equal(a, b)
+
+
 def test_native_calls_refuse_unaligned_rows():
     r"""The kernels with 16-byte accesses are not launched on rows that start elsewhere."""
     from fastmoe_b200.ops import native
