@@ -7,9 +7,9 @@ registers, writes ids and probabilities, and a second small kernel applies the s
 Jacobian in backward and scatters the result into the dense logits gradient.
 
 ``linear_topk_softmax`` goes one step further for the plain linear gate
-(``fmoe/gates/naive_gate.py:24-38``: ``nn.Linear`` → ``topk`` → ``softmax``): with at most 64
-experts the logits of a token fit in registers, so one kernel reads the token once and writes
-logits, ids and probabilities, and the backward is three kernels (softmax Jacobian + ``dx``; partial
+(``fmoe/gates/naive_gate.py:24-38``: ``nn.Linear`` → ``topk`` → ``softmax``): with at most 8
+experts one kernel reads the token once, keeps its logits in registers and writes logits, ids
+and probabilities, and the backward is three kernels (softmax Jacobian + ``dx``; partial
 sums of ``dW`` and ``db``; their merge) instead of the six of the ATen sequence.
 """
 import torch

@@ -134,8 +134,11 @@ class FMoETransformerMLP(FMoE):
     r"""A complete MoE MLP block: ``[..., d_model] → [..., d_model]``.
 
     * ``activation``: module applied between the two expert linears.  GELU (erf or tanh),
-      ReLU and Identity are fused into the first GEMM's epilogue on the GPU; anything else
-      (e.g. ``Sequential(ReLU, Dropout)``) runs as a PyTorch op between two grouped GEMMs.
+      ReLU and Identity are fused into the first GEMM's epilogue on the GPU, and so is a
+      ``Sequential`` of one of them and members that do nothing in the call (``Dropout`` at
+      evaluation or with ``p = 0``, which nobody has hooks on); anything else (e.g.
+      ``Sequential(ReLU, Dropout(0.1))`` in training) runs as a PyTorch op between two grouped
+      GEMMs.  Under expert parallelism a ``Sequential`` always takes the unfused exchange.
     * ``d_hidden``: hidden size of each expert.
     * ``expert_dp_comm``: gradient-reduction group name of the expert parameters.
     * ``expert_rank``: accepted and ignored, as in the reference.
