@@ -944,39 +944,47 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
     pos += (other > key || (other == key && e < e_of)) ? 1 : 0;
     top = fmaxf(top, other);
   }
-  if (__any_sync(0xffffffffu, e_of < tot && mine != mine)) {
-    // With a NaN the choice is what k scans over the experts left give, in which only a greater
-    // logit replaces the first one: a NaN that comes first is chosen and shows in every score.
-    bool taken = false;
-    pos = TOT;
-#pragma unroll 1
-    for (int j = 0; j < k; ++j) {
-      float best = 0.f;
-      int best_e = -1;
-#pragma unroll 1
-      for (int e = 0; e < tot; ++e) {
-        const float other = __shfl_sync(0xffffffffu, mine, base + e * kStep);
-        const int gone = __shfl_sync(0xffffffffu, static_cast<int>(taken), base + e * kStep);
-        if (gone == 0 && (best_e < 0 || other > best)) {
-          best = other;
-          best_e = e;
-        }
-      }
-      if (best_e == e_of) {
-        taken = true;
-        pos = j;
-      }
-    }
-  }
   const bool chosen = e_of < tot && pos < k;
   const float ex = chosen ? __expf(mine - top) : 0.f;
   float den = ex;
 #pragma unroll
   for (int o = kStep; o < TOT * kStep; o <<= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-  if (row_ok && chosen && (lane & (kStep - 1)) == 0) {
-    const long o = static_cast<long>(row0 + r) * k + pos;
-    idx[o] = e_of;
-    prob[o] = V2<T>::from_f(ex / den);
+  const bool writes = row_ok && (lane & (kStep - 1)) == 0;
+  const long out = static_cast<long>(row0 + r) * k;
+  const bool nan = e_of < tot && mine != mine;
+  if (!__any_sync(0xffffffffu, nan)) {
+    if (writes && chosen) {
+      idx[out + pos] = e_of;
+      prob[out + pos] = V2<T>::from_f(ex / den);
+    }
+    return;
+  }
+  // With a NaN in the warp the choice is what k scans over the experts left give, in which only a
+  // greater logit replaces the first one: a NaN that comes first is chosen, and makes all scores of
+  // its token NaN.  (After the usual path, whose registers these loops would cost.)
+  pos = TOT;
+#pragma unroll 1
+  for (int j = 0; j < k; ++j) {
+    float best = 0.f;
+    int best_e = -1;
+#pragma unroll 1
+    for (int e = 0; e < tot; ++e) {
+      const float other = __shfl_sync(0xffffffffu, mine, base + e * kStep);
+      const int taken = __shfl_sync(0xffffffffu, pos, base + e * kStep) < TOT;
+      if (!taken && (best_e < 0 || other > best)) {
+        best = other;
+        best_e = e;
+      }
+    }
+    if (best_e == e_of) pos = j;
+  }
+  const float again = pos < k ? __expf(mine - top) : 0.f;
+  float sum = again;
+#pragma unroll
+  for (int o = kStep; o < TOT * kStep; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (writes && pos < k) {
+    idx[out + pos] = e_of;
+    prob[out + pos] = V2<T>::from_f(again / sum);
   }
 }
 
@@ -1609,6 +1617,8 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
     return chained;
   }
 #undef FMOE_GATE_ROWS
+  // The layer's gates come here with at most 8 experts (above, the tensor-core gate is faster):
+  // the wider instances, which spill from 16 experts on, serve direct calls of the gate's function.
 #define FMOE_GATE_WIDE(TOT)                                                                             \
   FMOE_DISPATCH_16(dtype, (gate_linear_topk_kernel<T, TOT><<<grid, 256, 0, stream>>>(                   \
       static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,  \
