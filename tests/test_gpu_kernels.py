@@ -569,9 +569,10 @@ def test_gate_with_nan_logits(rows, tot, k):
 @pytest.mark.parametrize("kind", ["gshard", "switch"])
 @pytest.mark.parametrize("n,tot", [(1, 2), (127, 3), (129, 64), (5000, 8), (40000, 2)])
 def test_balanced_gates_native_loss(dtype, kind, n, tot, monkeypatch):
-    r"""Ids, scores, loss and gradients of the capacity-limited gates with the balance-loss kernels
-    against the PyTorch operations, which run in 64 bits on the same logits: one rounding to the
-    layer's type, fp32 sums over the tokens and experts."""
+    r"""Whole gates: ids, scores, loss and parameter gradients of the capacity-limited gates with the
+    balance-loss kernels against the same gate as PyTorch operations in the layer's type, with a
+    gradient arriving through the scores and from the loss together.  (The scores' part is the
+    larger one: the tests that follow take the loss by itself.)"""
     from fastmoe_b200.gates import GShardGate, SwitchGate
     from fastmoe_b200.ops import gating
     torch.manual_seed(16)
@@ -780,8 +781,37 @@ def test_fp32_switch_scores_and_gradients_are_no_further_off(tot):
         assert off[0] <= 1.05 * off[1] + (2.0 ** -23 * abs(float(exact)) if name == "loss" else 0.0), (name, off)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n,tot,cap", [(1, 2, 9), (127, 3, 30), (1000, 2, 600), (5000, 8, 700), (9001, 64, 100)])
+def test_switch_loss_alone_in_64_bits(dtype, n, tot, cap):
+    r"""Switch's loss and the logit gradient that comes from it alone, some tokens beyond the capacity,
+    against 64 bits on the same logits.  The kernels hold everything in fp32: the loss is a sum of n
+    terms, the gradient the difference of two numbers that are each right to a few units of fp32
+    (softmax, weight, sum over 64 experts: below 2^-18), rounded once to the logits' type (relative
+    error 2^-8 with the 8 significant bits of bf16, 2^-11 with the 11 of fp16)."""
+    from fastmoe_b200.gates.switch_gate import switch_score_and_loss
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(29)
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -24}[dtype]
+    tiny = 2.0 ** -25 if dtype == torch.float16 else 0.0   # half a unit of fp16's smallest numbers
+    logits = torch.randn(n, tot, device=DEV).to(dtype).requires_grad_(True)
+    kept, _score, loss = gating.switch_route(logits, cap, switch_score_and_loss)
+    (got,) = torch.autograd.grad(loss, logits, torch.full_like(loss, 3.0))
+    x = logits.detach().double().requires_grad_(True)
+    prob = torch.softmax(x, 1)
+    ids = kept.view(-1)[kept.view(-1) >= 0]
+    share, n_kept = torch.bincount(ids, minlength=tot).double(), max(1, ids.numel())
+    want_loss = tot * ((share / n_kept) * (prob.sum(0) / n_kept)).sum()
+    (want,) = torch.autograd.grad(3.0 * want_loss, x)
+    assert torch.allclose(loss.double(), want_loss, rtol=1e-5)
+    term = prob.detach() * (3.0 * tot / n_kept ** 2 * share)
+    bound = eps * want.abs() + 2.0 ** -18 * (term + prob.detach() * term.sum(1, keepdim=True)) + tiny
+    assert ((got.double() - want).abs() <= bound).all()
+
+
 def test_balance_loss_second_derivative():
-    r"""A gradient of the gradient goes through the PyTorch operations."""
+    r"""A gradient of the gradient goes through the PyTorch operations; the first one, where no second
+    is wanted, comes from the kernel and is the same."""
     from fastmoe_b200.gates.gshard_gate import gshard_balance_loss
     from fastmoe_b200.ops import gating
     torch.manual_seed(17)
@@ -789,7 +819,10 @@ def test_balance_loss_second_derivative():
     ids = torch.randint(0, 4, (50, 2), device=DEV)
     ref = lambda l, i: gshard_balance_loss(l, i[:, 0], 4, 4)   # noqa: E731
     got = []
-    for loss in (gating.gshard_loss(logits, ids, 16, ref), ref(logits, ids)):
+    native = gating.gshard_loss(logits, ids, 16, ref)
+    (first,) = torch.autograd.grad(native, logits, retain_graph=True)
+    assert torch.allclose(first, torch.autograd.grad(ref(logits, ids), logits)[0], rtol=1e-4, atol=1e-9)
+    for loss in (native, ref(logits, ids)):
         (g,) = torch.autograd.grad(loss, logits, create_graph=True)
         got.append((g, torch.autograd.grad(g.pow(2).sum(), logits)[0]))
     for a, b in zip(*got):
