@@ -17,6 +17,8 @@
 #include "cpu/cpu_ops.h"
 #include "sm100/grouped_gemm.cuh"
 #include "sm100/routing.cuh"
+#include "sm100/split_gemm.cuh"
+#include "sm100/tile_walk.cuh"
 #include "sm100/p2p.cuh"
 
 namespace {
@@ -354,6 +356,159 @@ void simt_grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Te
                                                  cur_stream()));
 }
 
+// ------------------------------------------------------------------------------ fp32 on the tensor cores
+torch::Tensor plane_rows(long rows, int64_t groups, int64_t width, const torch::Tensor& like) {
+  return torch::empty({3, fmoe::split_rows_cap(rows, static_cast<int>(groups)), width}, like.options().dtype(torch::kBFloat16));
+}
+
+torch::Tensor split_weight(const torch::Tensor& w, const torch::Tensor& offs) {
+  auto planes = torch::empty({3, w.numel()}, w.options().dtype(torch::kBFloat16));
+  FMOE_CUDA_CHECK(fmoe::launch_split_weight(w.data_ptr<float>(), offs.data_ptr<int>(), static_cast<int>(w.size(0)),
+                                            w.numel() / w.size(0), planes.data_ptr(), cur_stream()));
+  return planes;
+}
+
+// Scratch of split GEMMs that follow one another in a stream; its flags are zeroed by the kernel
+// that splits the token rows before them.  `sums_of`: the widths whose column sums are wanted.
+struct SplitScratch {
+  torch::Tensor work, flags, sums;
+  int per_gemm, gemms, groups;
+  SplitScratch(const torch::Tensor& like, int n_gemms, int64_t rows, int64_t n_groups, std::initializer_list<int64_t> sums_of)
+      : gemms(n_gemms), groups(static_cast<int>(n_groups)) {
+    const int sms = num_sms(like.device().index());
+    per_gemm = fmoe::split_num_flags(sms);
+    int64_t n = static_cast<int64_t>(gemms) * per_gemm, widest = 0;
+    for (int64_t m : sums_of) {
+      n += fmoe::split_num_counts(groups, static_cast<int>(m));
+      widest = std::max(widest, m);
+    }
+    work = torch::empty({fmoe::split_work_floats(sms)}, like.options().dtype(torch::kFloat));
+    flags = torch::empty({n}, like.options().dtype(torch::kInt));
+    if (widest > 0) {
+      sums = torch::empty({fmoe::split_sum_floats(rows, groups, static_cast<int>(widest))}, like.options().dtype(torch::kFloat));
+    }
+    next_count = flags.data_ptr<int>() + static_cast<int64_t>(gemms) * per_gemm;
+  }
+  int* all() { return flags.data_ptr<int>(); }
+  int count() { return static_cast<int>(flags.numel()); }
+  void give(fmoe::SplitGemmArgs& g) {
+    g.work = work.data_ptr<float>();
+    g.flags = all() + (given++) * per_gemm;
+  }
+  void give_sums(fmoe::SplitGemmArgs& g, float* psum) {
+    g.psum = psum;
+    g.sums = sums.data_ptr<float>();
+    g.sum_counts = next_count;
+    next_count += fmoe::split_num_counts(groups, g.m);
+  }
+
+ private:
+  int given = 0;
+  int* next_count;
+};
+
+torch::Tensor split_token_rows(const torch::Tensor& x, const torch::Tensor& offs, SplitScratch* scratch) {
+  const int groups = static_cast<int>(offs.numel() - 1);
+  auto planes = plane_rows(x.size(0), groups, x.size(1), x);
+  FMOE_CUDA_CHECK(fmoe::launch_split_rows(x.data_ptr<float>(), offs.data_ptr<int>(), groups, x.size(0),
+                                          static_cast<int>(x.size(1)), planes.data_ptr(),
+                                          scratch != nullptr ? scratch->all() : nullptr,
+                                          scratch != nullptr ? scratch->count() : 0, cur_stream()));
+  return planes;
+}
+
+fmoe::SplitGemmArgs split_args(int64_t mode, int64_t rows, int64_t m, int64_t n, int64_t k, const torch::Tensor& a,
+                               const torch::Tensor& b, const torch::Tensor& offs) {
+  fmoe::SplitGemmArgs g;
+  g.mode = static_cast<int>(mode);
+  g.num_groups = static_cast<int>(offs.numel() - 1);
+  g.rows_cap = rows;
+  g.m = static_cast<int>(m);
+  g.n = static_cast<int>(n);
+  g.k = static_cast<int>(k);
+  g.a = a.data_ptr();
+  g.b = b.data_ptr();
+  g.offs = offs.data_ptr<int>();
+  g.status = status_tensor(a.device().index()).data_ptr<int>();
+  g.num_sms = num_sms(a.device().index());
+  g.stream = cur_stream();
+  return g;
+}
+
+struct GemmSizes {
+  int groups, m, n, k;
+};
+GemmSizes gemm_sizes(int64_t mode, const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& offs) {
+  const int groups = static_cast<int>(offs.numel() - 1), inner = static_cast<int>(a.size(1));
+  if (mode == fmoe::kWgrad) return {groups, inner, static_cast<int>(b.size(1)), 0};
+  return {groups, 0, static_cast<int>(mode == fmoe::kRowsNT ? b.size(1) : b.size(2)), inner};
+}
+
+// The three products of a grouped linear in fp32, each operand split by a launch of its own.
+void split_grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor offs, torch::Tensor out,
+                        c10::optional<torch::Tensor> bias, c10::optional<torch::Tensor> psum) {
+  const GemmSizes z = gemm_sizes(mode, a, b, offs);
+  for (const auto& t : {a, b, out}) {
+    check_rows(t, "operand");
+    TORCH_CHECK(t.scalar_type() == torch::kFloat, "split_grouped_gemm: fp32 operands");
+  }
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(out.data_ptr()) % 32 == 0, "split_grouped_gemm: out must be 32-byte aligned");
+  TORCH_CHECK(fmoe::split_gemm_supported(static_cast<int>(mode), z.m, z.n, z.k, z.groups, a.size(0)),
+              "split_grouped_gemm: shape not supported");
+  c10::cuda::CUDAGuard guard(a.device());
+  const bool sums = psum.has_value() && psum->defined();
+  SplitScratch scratch = sums ? SplitScratch(a, 1, a.size(0), z.groups, {z.m}) : SplitScratch(a, 1, a.size(0), z.groups, {});
+  const torch::Tensor pa = split_token_rows(a, offs, &scratch);
+  const torch::Tensor pb = mode == fmoe::kWgrad ? split_token_rows(b, offs, nullptr) : split_weight(b, offs);
+  auto g = split_args(mode, a.size(0), z.m, z.n, z.k, pa, pb, offs);
+  scratch.give(g);
+  g.out = out.data_ptr<float>();
+  if (bias.has_value() && bias->defined()) {
+    check_rows(*bias, "bias");
+    g.bias = bias->data_ptr<float>();
+  }
+  if (sums) {
+    check_rows(*psum, "psum");
+    scratch.give_sums(g, psum->data_ptr<float>());
+  }
+  FMOE_CUDA_CHECK(fmoe::launch_split_gemm(g));
+}
+
+// When one product by itself is faster split than on the FMA units.  Those take the larger of the
+// operations at 47 TFLOP/s and their serial chain (one sum over k, or over an expert's rows: 0.066 us
+// per element).  Split, the operands are read and written first (16 bytes an element in all), the
+// weight gradient is stored by few tiles, and the chain is short.  Taken where the estimate is 25 us
+// lower, which is what issuing the other launches costs an eager program (8 experts, 277 rows each,
+// 160 -> 320, eager, forward and backward: 203 us split, 183 not).  us measured, split against FMA, forward / input gradient / weight gradient: 8
+// experts, 512 rows each, 512 -> 2048: 94, 113, 108 against 203, 220, 177; 16 experts, 64 rows each:
+// 92, 110, 74 against 83, 152, 54; 8 experts, 128 rows each, 128 -> 512: 17, 26, 27 against 12, 37, 12;
+// 4 experts, 7500 rows each, 64 -> 64: 20, 17, 43 against 17, 15, 544.
+bool split_worth_it(int64_t mode, int64_t rows, const GemmSizes& z) {
+  const bool wgrad = mode == fmoe::kWgrad;
+  const double r = static_cast<double>(rows), n = z.n, k = wgrad ? z.m : z.k, weights = n * k * z.groups;
+  const double flops = 2 * r * n * k, chain = wgrad ? r / z.groups : k;
+  const double fma = 4 + std::max(0.066 * chain, flops / 47e6);
+  const double split = 14 + ((wgrad ? 8 : 16) * weights + 16 * r * (wgrad ? n + k : k)) / 6.5e6 + 6 * flops / 1.1e9;
+  return split + 25 < fma;
+}
+
+// fp32, fp64 and what the 16-bit tensor-core kernel does not take.
+void wide_grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Tensor offs, torch::Tensor out,
+                       c10::optional<torch::Tensor> bias, c10::optional<torch::Tensor> psum) {
+  const GemmSizes z = gemm_sizes(mode, a, b, offs);
+  auto usable = [](const torch::Tensor& t) {
+    return t.scalar_type() == torch::kFloat && t.is_cuda() && t.is_contiguous() &&
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 32 == 0;
+  };
+  auto usable_or_none = [&](const c10::optional<torch::Tensor>& t) { return !t.has_value() || !t->defined() || usable(*t); };
+  if (usable(a) && usable(b) && usable(out) && usable_or_none(bias) && usable_or_none(psum) &&
+      fmoe::split_gemm_supported(static_cast<int>(mode), z.m, z.n, z.k, z.groups, a.size(0)) &&
+      split_worth_it(mode, a.size(0), z)) {
+    return split_grouped_gemm(mode, a, b, offs, out, bias, psum);
+  }
+  simt_grouped_gemm(mode, a, b, offs, out, bias, psum);
+}
+
 // ------------------------------------------------------------------------------ row movement
 void scatter_rows(torch::Tensor src, torch::Tensor idx, torch::Tensor rank, torch::Tensor base,
                   c10::optional<torch::Tensor> scale, int64_t k, torch::Tensor dst,
@@ -415,6 +570,112 @@ bool moe_mlp_supported(int64_t experts, int64_t d, int64_t h) {
          fmoe::grouped_gemm_supported(fmoe::kRowsNT, 0, id, ih, g);
 }
 
+// Whether the fp32 layer runs on the tensor cores: `rows` are tokens times choices.  What it replaces,
+// the general path with its host read and three dozen launches, takes about 0.7 ms of host time, as
+// long as splitting 280 M weights, so only a layer of many weights needs rows to be worth it.
+bool moe_mlp_supported_f32(int64_t experts, int64_t d, int64_t h, int64_t rows) {
+  const int g = static_cast<int>(experts), id = static_cast<int>(d), ih = static_cast<int>(h);
+  return fmoe::split_gemm_supported(fmoe::kRowsNT, 0, ih, id, g, rows) &&
+         fmoe::split_gemm_supported(fmoe::kRowsNT, 0, id, ih, g, rows) &&
+         (rows >= 64 * experts || 2 * experts * d * h <= 80000000);
+}
+
+// As moe_mlp_forward for fp32: xs and a are planes.
+std::vector<torch::Tensor> moe_mlp_forward_f32(const torch::Tensor& x, const torch::Tensor& idx, const torch::Tensor& score,
+                                               const torch::Tensor& w1, const torch::Tensor& b1, const torch::Tensor& w2,
+                                               const torch::Tensor& b2, int64_t act, bool keep) {
+  const int64_t groups = w1.size(0), h = w1.size(1), d = w1.size(2), rows = idx.numel(), k = rows / x.size(0);
+  auto r = route(idx, groups, true);
+  const torch::Tensor rank = r[1], offs = r[2];
+  auto xs = plane_rows(rows, groups, d, x);
+  SplitScratch scratch(x, 2, rows, groups, {});
+  FMOE_CUDA_CHECK(fmoe::launch_split_scatter(x.data_ptr<float>(), idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
+                                             offs.data_ptr<int>(), static_cast<int>(groups), rows, static_cast<int>(k),
+                                             static_cast<int>(d), xs.data_ptr(), scratch.all(), scratch.count(), cur_stream()));
+  auto a = plane_rows(rows, groups, h, x);
+  torch::Tensor pre;
+  if (keep && act != fmoe::kActNone) pre = torch::empty({rows, h}, x.options());
+  {
+    const torch::Tensor planes = split_weight(w1, offs);
+    auto g = split_args(fmoe::kRowsNT, rows, 0, h, d, xs, planes, offs);
+    scratch.give(g);
+    g.kind = fmoe::kSplitAct;
+    g.act = static_cast<int>(act);
+    g.bias = b1.data_ptr<float>();
+    g.planes = a.data_ptr();
+    g.pre = pre.defined() ? pre.data_ptr<float>() : nullptr;
+    FMOE_CUDA_CHECK(fmoe::launch_split_gemm(g));
+  }
+  auto ys = torch::empty({rows, d}, x.options());
+  {
+    const torch::Tensor planes = split_weight(w2, offs);
+    auto g = split_args(fmoe::kRowsNT, rows, 0, d, h, a, planes, offs);
+    scratch.give(g);
+    g.bias = b2.data_ptr<float>();
+    g.out = ys.data_ptr<float>();
+    FMOE_CUDA_CHECK(fmoe::launch_split_gemm(g));
+  }
+  auto out = torch::empty_like(x);
+  FMOE_CUDA_CHECK(fmoe::launch_combine_f32(ys.data_ptr<float>(), idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
+                                           offs.data_ptr<int>(), score.data_ptr<float>(), static_cast<int>(groups), x.size(0),
+                                           static_cast<int>(k), static_cast<int>(d), out.data_ptr<float>(), cur_stream()));
+  return {out, xs, pre, a, ys, rank, offs, score, idx};
+}
+
+std::vector<torch::Tensor> moe_mlp_backward_f32(const torch::Tensor& dout, const torch::Tensor& xs,
+                                                const c10::optional<torch::Tensor>& pre, const torch::Tensor& a,
+                                                const torch::Tensor& ys, const torch::Tensor& rank, const torch::Tensor& offs,
+                                                const torch::Tensor& score, const torch::Tensor& idx, const torch::Tensor& w1,
+                                                const torch::Tensor& w2, int64_t act, bool need_dx, bool need_w1, bool need_w2) {
+  const int64_t groups = w1.size(0), h = w1.size(1), d = w1.size(2), n_tok = dout.size(0), rows = idx.numel(), k = rows / n_tok;
+  auto dys = plane_rows(rows, groups, d, dout);
+  auto dscore = torch::empty_like(score);
+  SplitScratch scratch(dout, 4, rows, groups, {d, h});
+  FMOE_CUDA_CHECK(fmoe::launch_split_combine_bwd(dout.data_ptr<float>(), ys.data_ptr<float>(), idx.data_ptr<int64_t>(),
+                                                 rank.data_ptr<int>(), offs.data_ptr<int>(), score.data_ptr<float>(),
+                                                 static_cast<int>(groups), rows, static_cast<int>(k), static_cast<int>(d),
+                                                 dys.data_ptr(), dscore.data_ptr<float>(), scratch.all(),
+                                                 scratch.count(), cur_stream()));
+  auto wgrad = [&](const torch::Tensor& p, const torch::Tensor& q, int64_t m, int64_t n, torch::Tensor& dw, torch::Tensor& db) {
+    dw = torch::empty({groups, m, n}, dout.options());
+    db = torch::empty({groups, m}, dout.options());
+    auto g = split_args(fmoe::kWgrad, rows, m, n, 0, p, q, offs);
+    scratch.give(g);
+    scratch.give_sums(g, db.data_ptr<float>());
+    g.out = dw.data_ptr<float>();
+    FMOE_CUDA_CHECK(fmoe::launch_split_gemm(g));
+  };
+  torch::Tensor dw1, db1, dw2, db2, dx;
+  if (need_w2) wgrad(dys, a, d, h, dw2, db2);
+  if (need_dx || need_w1) {
+    auto da = plane_rows(rows, groups, h, dout);
+    {
+      const torch::Tensor planes = split_weight(w2, offs);
+      auto g = split_args(fmoe::kRowsNN, rows, 0, h, d, dys, planes, offs);
+      scratch.give(g);
+      g.kind = fmoe::kSplitDAct;
+      g.act = pre.has_value() ? static_cast<int>(act) : fmoe::kActNone;
+      g.planes = da.data_ptr();
+      g.pre = pre.has_value() ? pre->data_ptr<float>() : nullptr;
+      FMOE_CUDA_CHECK(fmoe::launch_split_gemm(g));
+    }
+    if (need_w1) wgrad(da, xs, h, d, dw1, db1);
+    if (need_dx) {
+      auto dxs = torch::empty_like(ys);
+      const torch::Tensor planes = split_weight(w1, offs);
+      auto g = split_args(fmoe::kRowsNN, rows, 0, d, h, da, planes, offs);
+      scratch.give(g);
+      g.out = dxs.data_ptr<float>();
+      FMOE_CUDA_CHECK(fmoe::launch_split_gemm(g));
+      dx = torch::empty({n_tok, d}, dout.options());
+      FMOE_CUDA_CHECK(fmoe::launch_combine_f32(dxs.data_ptr<float>(), idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
+                                               offs.data_ptr<int>(), nullptr, static_cast<int>(groups), n_tok,
+                                               static_cast<int>(k), static_cast<int>(d), dx.data_ptr<float>(), cur_stream()));
+    }
+  }
+  return {dx, dscore, dw1, db1, dw2, db2};
+}
+
 // {out, xs, pre (empty when not kept), a, ys, rank, offs, score in the layer's type, idx}
 std::vector<torch::Tensor> moe_mlp_forward(torch::Tensor x_in, torch::Tensor idx_in, torch::Tensor score_in,
                                            torch::Tensor w1_in, torch::Tensor b1_in, torch::Tensor w2_in,
@@ -424,6 +685,7 @@ std::vector<torch::Tensor> moe_mlp_forward(torch::Tensor x_in, torch::Tensor idx
   const torch::Tensor idx = idx_in.contiguous().view({-1});
   const torch::Tensor score = score_in.reshape({-1}).to(x.scalar_type()).contiguous();
   const torch::Tensor w1 = aligned32(w1_in), b1 = aligned32(b1_in), w2 = aligned32(w2_in), b2 = aligned32(b2_in);
+  if (x.scalar_type() == torch::kFloat) return moe_mlp_forward_f32(aligned32(x), idx, score, w1, b1, w2, b2, act, keep);
   const int64_t groups = w1.size(0), h = w1.size(1), d = w1.size(2), rows = idx.numel(), k = rows / x.size(0);
   auto r = route(idx, groups, true);
   const torch::Tensor rank = r[1], offs = r[2];
@@ -453,6 +715,9 @@ std::vector<torch::Tensor> moe_mlp_backward(torch::Tensor dout_in, torch::Tensor
   const torch::Tensor dout = aligned(dout_in, 16), xs = aligned32(xs_in), a = aligned32(a_in), ys = aligned(ys_in, 16);
   if (pre.has_value()) pre = aligned32(*pre);
   const torch::Tensor w1 = aligned32(w1_in), w2 = aligned32(w2_in);
+  if (ys.scalar_type() == torch::kFloat) {
+    return moe_mlp_backward_f32(dout, xs, pre, a, ys, rank, offs, score, idx, w1, w2, act, need_dx, need_w1, need_w2);
+  }
   const int64_t groups = w1.size(0), h = w1.size(1), d = w1.size(2), n_tok = dout.size(0), k = idx.numel() / n_tok;
   auto dys = torch::empty_like(ys);
   auto dscore = torch::empty_like(score);
@@ -677,6 +942,18 @@ torch::Tensor status_word(int64_t device) { return status_tensor(static_cast<int
 
 }  // namespace
 
+namespace {
+// The parts {group, tile, kb0, kb1, num_kb, last_piece} that one pair of a persistent GEMM walks (host).
+std::vector<std::vector<int>> tile_walk(std::vector<int> tiles, std::vector<int> units, int pair, int pairs, int min_kb) {
+  TORCH_CHECK(tiles.size() >= 2 && tiles.size() == units.size() && pair >= 0 && pair < pairs, "tile_walk");
+  fmoe::TileWalk walk(tiles.data(), units.data(), static_cast<int>(tiles.size()) - 1, pair, pairs, min_kb);
+  std::vector<std::vector<int>> parts;
+  fmoe::WalkPart p;
+  while (walk.next(p)) parts.push_back({p.group, p.tile, p.kb0, p.kb1, p.num_kb, p.last_piece});
+  return parts;
+}
+}  // namespace
+
 void bind_p2p(pybind11::module& m);  // sm100/p2p_binding.cpp
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -701,6 +978,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("simt_grouped_gemm", &simt_grouped_gemm, py::arg("mode"), py::arg("a"), py::arg("b"),
         py::arg("offs"), py::arg("out"), py::arg("bias") = py::none(), py::arg("psum") = py::none());
   m.def("simt_column_sums", &simt_column_sums);
+  m.def("split_grouped_gemm", &split_grouped_gemm, py::arg("mode"), py::arg("a"), py::arg("b"),
+        py::arg("offs"), py::arg("out"), py::arg("bias") = py::none(), py::arg("psum") = py::none());
+  m.def("wide_grouped_gemm", &wide_grouped_gemm, py::arg("mode"), py::arg("a"), py::arg("b"),
+        py::arg("offs"), py::arg("out"), py::arg("bias") = py::none(), py::arg("psum") = py::none());
+  m.def("tile_walk", &tile_walk);
+  m.def("moe_mlp_supported_f32", &moe_mlp_supported_f32);
   m.def("scatter_rows", &scatter_rows, py::arg("src"), py::arg("idx"), py::arg("rank"),
         py::arg("base"), py::arg("scale"), py::arg("k"), py::arg("dst"),
         py::arg("row_slot") = py::none());

@@ -5,6 +5,7 @@
 #include "grouped_gemm_kernel.cuh"
 #include "narrow_gemm.cuh"
 #include "pair_gemm_kernel.cuh"
+#include "tensor_map.cuh"
 
 namespace fmoe {
 using namespace gg;
@@ -31,24 +32,36 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// 2-D row-major tensor [outer, inner] of 16-bit elements, 128-byte swizzle.
-bool make_map_2d(CUtensorMap* map, int dtype, const void* base, uint64_t inner, uint64_t outer,
-                 uint32_t box_inner, uint32_t box_outer) {
+bool encode(CUtensorMap* map, int dtype, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
+            const cuuint32_t* box) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return false;
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {inner * 2};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, dtype == kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                       : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                  2, const_cast<void*>(base), dims, strides, box, estr,
+                  rank, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
 }  // namespace
+
+bool make_map_2d(CUtensorMap* map, int dtype, const void* base, uint64_t inner, uint64_t outer, uint32_t box_inner,
+                 uint32_t box_outer) {
+  cuuint64_t dims[2] = {inner, outer};
+  cuuint64_t strides[1] = {inner * 2};
+  cuuint32_t box[2] = {box_inner, box_outer};
+  return encode(map, dtype, base, 2, dims, strides, box);
+}
+
+bool make_map_3d(CUtensorMap* map, int dtype, const void* base, uint64_t inner, uint64_t mid, uint64_t outer,
+                 uint32_t box_inner, uint32_t box_mid) {
+  cuuint64_t dims[3] = {inner, mid, outer};
+  cuuint64_t strides[2] = {inner * 2, mid * inner * 2};
+  cuuint32_t box[3] = {box_inner, box_mid, 1};
+  return encode(map, dtype, base, 3, dims, strides, box);
+}
 
 bool grouped_gemm_supported(int mode, int m, int n, int k, int num_groups) {
   if (num_groups < 1 || num_groups > MAX_GROUPS) return false;

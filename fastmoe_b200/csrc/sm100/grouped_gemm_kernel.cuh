@@ -91,6 +91,7 @@ constexpr int STATUS_TIMEOUT_PRODUCER = 101;
 constexpr int STATUS_TIMEOUT_MMA = 102;
 constexpr int STATUS_TIMEOUT_EPILOGUE = 103;
 constexpr int STATUS_TIMEOUT_SENDER = 104;
+constexpr int STATUS_TIMEOUT_COLLECT = 106;
 constexpr int STATUS_BAD_PUSH_META = 105;    // a row's (source, slot) word was out of range: row skipped
 
 struct SharedAux {

@@ -109,6 +109,33 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
+// ----------------------------------------------------------------------------- flags in global memory
+__device__ __forceinline__ void st_release(int* p, int v) {
+  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// All lanes of a warp wait until `*p` is not zero (bounded, as mbar_wait).
+__device__ __forceinline__ bool wait_flag(const int* p, const volatile int* abort_flag, unsigned long long limit_ns) {
+  unsigned long long t0 = 0;
+  uint32_t spins = 0;
+  bool ok = true;
+  while (ld_acquire(p) == 0) {
+    if ((++spins & 0xff) == 0) {
+      const unsigned long long now = globaltimer();
+      if (t0 == 0) t0 = now;
+      if (*abort_flag != 0 || now - t0 > limit_ns) {
+        ok = false;
+        break;
+      }
+    }
+  }
+  return __all_sync(0xffffffffu, ok);
+}
+
 // ----------------------------------------------------------------------------- proxies
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -276,6 +303,16 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tma
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr,
+                                                 int32_t x, int32_t y, int32_t z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr),
+      "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+
 // One warp of EACH CTA of the pair executes these.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
@@ -300,6 +337,26 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, 
       "}\n"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// The same with a hint about the operand collector: A is kept there (fill) for the MMAs that follow with
+// the same A (use; lastuse is the last of them), which then do not read it from shared memory.
+enum CollectorA : int { kCollectFill, kCollectUse, kCollectLast };
+template <int HINT>
+__device__ __forceinline__ void umma_f16_pair_collect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                                      uint32_t idesc, uint32_t accumulate) {
+#define FMOE_UMMA_COLLECT(OP)                                                             \
+  asm volatile(                                                                           \
+      "{\n"                                                                               \
+      ".reg .pred p;\n"                                                                   \
+      "setp.ne.b32 p, %4, 0;\n"                                                           \
+      "tcgen05.mma.cta_group::2.kind::f16.collector::a::" OP " [%0], %1, %2, %3, p;\n"    \
+      "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)          \
+      : "memory")
+  if (HINT == kCollectFill) FMOE_UMMA_COLLECT("fill");
+  if (HINT == kCollectUse) FMOE_UMMA_COLLECT("use");
+  if (HINT == kCollectLast) FMOE_UMMA_COLLECT("lastuse");
+#undef FMOE_UMMA_COLLECT
 }
 
 // The barrier at this shared-memory offset of BOTH CTAs gets one arrival when all MMAs issued so

@@ -22,7 +22,7 @@ from torch.autograd import Function
 from . import grouped_gemm as gg
 from . import native
 from .. import config
-from ..transformer import activation_kind
+from ..transformer import activation_kind, plain_experts
 from ..utils.profiling import check_routing, fused_range
 
 _TC = (torch.bfloat16, torch.float16)
@@ -30,7 +30,11 @@ _TC = (torch.bfloat16, torch.float16)
 
 def supports(layer, x, idx):
     r"""Whether the fused kernels can run this call (else the general path is used)."""
-    if not native.available() or x.dtype not in _TC or idx.dim() != 2:
+    if not native.available() or idx.dim() != 2:
+        return False
+    if x.dtype == torch.float32:
+        return _fp32_layer_ok(layer, x, idx)
+    if x.dtype not in _TC:
         return False
     e = layer.experts
     if e.htoh4.weight.dtype != x.dtype or e.htoh4.bias is None or e.h4toh.bias is None:
@@ -42,6 +46,21 @@ def supports(layer, x, idx):
         from ..parallel import symm
         return symm.fused_available(layer, x)
     return True
+
+
+def _fp32_layer_ok(layer, x, idx):
+    r"""Whether the fp32 layer on one GPU runs as :class:`_MoEMLP`.  The general path, which takes the
+    rest, calls the expert modules: a call that somebody watches stays there, and so does autocast,
+    under which the weighted sum is formed in 16 bits."""
+    e = layer.experts
+    if (layer.world_size > 1 or _forced_ep() or not config.fused_enabled() or config.faster_schedule_enabled()
+            or torch.is_autocast_enabled() or not plain_experts(e)):
+        return False
+    if any(t is None or t.dtype != torch.float32 or not t.is_cuda
+           for t in (e.htoh4.weight, e.htoh4.bias, e.h4toh.weight, e.h4toh.bias)):
+        return False
+    return (_native_call_ok(layer, x, idx) and native.get().moe_mlp_supported_f32(
+        layer.num_expert, layer.d_model, layer.d_hidden, idx.numel()))
 
 
 def _forced_ep():
@@ -176,7 +195,7 @@ class _MoEMLP(Function):
     r"""The whole single-GPU layer behind the gate as one node: :class:`_Dispatch`,
     :class:`_ExpertMLP` and :class:`_Combine` with their launches issued by one native call per
     direction.  With ``keep`` false (nothing will be differentiated) the pre-activation is not
-    written."""
+    written.  In fp32 ``xs`` and ``a`` are kept as the bf16 parts that the tensor cores multiply."""
 
     @staticmethod
     def forward(ctx, x, score, w1, b1, w2, b2, idx, act, keep):
@@ -199,14 +218,19 @@ class _MoEMLP(Function):
         return (dx, dscore.to(dtype).view(shape) if need[1] else None, dw1, db1, dw2, db2, None, None, None)
 
 
-def _native_layer_ok(layer, x, gate_idx):
-    r"""Whether :class:`_MoEMLP` takes the call: an activation the GEMM epilogue knows, shapes of the
-    tensor-core kernel, at least one row, and nobody who wants to look between the launches."""
+def _native_call_ok(layer, x, gate_idx):
+    r"""What :class:`_MoEMLP` asks of a call in any type: an activation the GEMM epilogue knows, at
+    least one row, and nobody who wants to look between the launches."""
     act = activation_kind(layer.experts.activation)
     return (act is not None and x.dim() == 2 and x.shape[0] > 0 and gate_idx.shape[1] > 0
             and gate_idx.shape[0] == x.shape[0] and gate_idx.dtype == torch.int64
-            and not config.nvtx_enabled() and not config.debug_bounds()
-            and native.get().moe_mlp_supported(layer.num_expert, layer.d_model, layer.d_hidden))
+            and not config.nvtx_enabled() and not config.debug_bounds())
+
+
+def _native_layer_ok(layer, x, gate_idx):
+    return (_native_call_ok(layer, x, gate_idx)
+            and (x.dtype == torch.float32   # `supports` has looked at the shapes
+                 or native.get().moe_mlp_supported(layer.num_expert, layer.d_model, layer.d_hidden)))
 
 
 def moe_mlp_forward(layer, x, gate_idx, gate_score):

@@ -4,8 +4,9 @@ Python front-end of the grouped GEMM kernels.
 The three products of a grouped linear — forward ``Y_e = X_e W_e^T (+b_e)``, input gradient
 ``dX_e = dY_e W_e`` and weight gradient ``dW_e = dY_e^T X_e`` (``cuda/parallel_linear.cuh:74-84,
 124-147`` in the reference, one cuBLAS call each per expert) — are single launches of the
-tcgen05 kernel for bf16/fp16 with tensor-core-friendly shapes, and of the reference-precision
-SIMT kernel for fp32/fp64 or odd shapes.  Row offsets are an int32 device tensor
+tcgen05 kernel for bf16/fp16 with tensor-core-friendly shapes.  fp32 runs on the tensor cores
+too where there is enough to compute, as six products of bf16 parts that together keep fp32's
+precision; small fp32 calls, fp64 and odd shapes take the reference-precision SIMT kernels.  Row offsets are an int32 device tensor
 ``offs[E+1]`` (``None`` for a single group of all rows, tensor-core shapes only); only the
 compatibility entry points below take host counts.
 """
@@ -96,7 +97,7 @@ def forward(x, weight, offs, bias=None, act=None, want_pre=False):
         if want_pre and pre is None:
             pre = out
     else:
-        nat.simt_grouped_gemm(MODE_NT, x, weight, offs, out, bias)
+        nat.wide_grouped_gemm(MODE_NT, x, weight, offs, out, bias)
         if want_pre:
             pre = out
         if code != 0:
@@ -123,7 +124,7 @@ def dgrad(dy, weight, offs, pre=None, act=None):
         _zero_tail(out, offs)
         out = out * _torch_act_grad(pre, act)
     else:
-        nat.simt_grouped_gemm(MODE_NN, dy, weight, offs, out, None)
+        nat.wide_grouped_gemm(MODE_NN, dy, weight, offs, out, None)
         if code:
             out = out * _torch_act_grad(pre, act)
     return out
@@ -153,7 +154,7 @@ def wgrad(dy, x, offs, groups, out=None, accumulate=False, with_bias_grad=False)
         tmp = out if fresh else torch.empty(groups, m, n, dtype=dy.dtype, device=dy.device)
         if with_bias_grad and nat.simt_column_sums(dy, x, tmp):
             db = torch.empty(groups, m, dtype=dy.dtype, device=dy.device)
-        nat.simt_grouped_gemm(MODE_WGRAD, dy, x, offs, tmp, None, db)
+        nat.wide_grouped_gemm(MODE_WGRAD, dy, x, offs, tmp, None, db)
         if accumulate:
             out += tmp
         elif not fresh:

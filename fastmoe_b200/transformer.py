@@ -70,6 +70,16 @@ def _does_nothing(module):
     return inert and not _hooked(module)
 
 
+def plain_experts(experts):
+    r"""Whether calling ``experts`` does no more than the arithmetic of its two linears and its
+    activation: no subclass, nobody who watches one of the modules."""
+    act = experts.activation
+    modules = [experts, experts.htoh4, experts.h4toh] + ([act] if isinstance(act, nn.Module) else [])
+    return (type(experts) is _Expert and type(experts.htoh4) is FMoELinear and type(experts.h4toh) is FMoELinear
+            and type(act) in (nn.GELU, nn.ReLU, nn.Identity, nn.Sequential)
+            and not any(_hooked(m) for m in modules) and not _hooked_globally())
+
+
 class _Expert(nn.Module):
     r"""``num_expert`` two-layer MLPs: ``htoh4`` → activation → ``h4toh``."""
 

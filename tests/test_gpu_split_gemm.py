@@ -1,0 +1,202 @@
+r"""GPU tier: the fp32 grouped GEMM on the tensor cores and the fp32 layer that is built on it."""
+import pytest
+import torch
+import torch.nn as nn
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def _native():
+    from fastmoe_b200.ops import native
+    return native.get()
+
+
+def _offs(counts):
+    from fastmoe_b200.ops import grouped_gemm as gg
+    return gg.offsets_from_counts(counts, DEV)
+
+
+def _bound(a_abs, terms):
+    r"""What the sum of ``terms`` products may be off by, given the sum of their magnitudes: the parts of a
+    product left out (2^-26); per K block of 64 four additions of the tensor cores that truncate
+    (2^-23 each), one of fp32 for every block, and the small products' truncated sum, 2^-8 of it with five
+    additions per 16 terms."""
+    blocks = (terms + 63) // 64
+    return a_abs * (2.0 ** -26 + 4 * 2.0 ** -23 + (blocks + 2) * 2.0 ** -24 + 5 * (terms / 16 + 1) * 2.0 ** -31)
+
+
+@pytest.mark.parametrize("counts,k,n", [
+    ([1, 0, 3], 16, 16),                      # the narrowest, a single row
+    ([64, 63, 65, 0], 64, 128),               # edges of the 64-row blocks
+    ([256, 255, 257, 128, 129], 72, 136),     # edges of the 256 x 128 tiles, ragged in every direction
+    ([700], 520, 264),
+    ([9, 0, 0, 1200, 31], 264, 1032),
+    ([40] * 40, 128, 64),                     # more experts than a warp has lanes
+    ([5000, 17], 64, 72),                     # one expert's rows shared among many pairs
+    ([300, 200], 4096, 128),                  # a long sum whose tiles are cut
+    ([2048] * 3 + [100], 256, 2048),          # several rounds and a cut rest
+])
+def test_split_gemm_against_64_bits(counts, k, n):
+    nat = _native()
+    torch.manual_seed(len(counts) * 1000 + k + n)
+    rows, groups, tail = sum(counts), len(counts), 5
+    offs = _offs(counts)
+    x = torch.randn(rows + tail, k, device=DEV)
+    dy = torch.randn(rows + tail, n, device=DEV)
+    w = torch.randn(groups, n, k, device=DEV)
+    b = torch.randn(groups, n, device=DEV)
+    y = torch.full((rows + tail, n), float("nan"), device=DEV)
+    dx = torch.full((rows + tail, k), float("nan"), device=DEV)
+    dw = torch.full((groups, n, k), float("nan"), device=DEV)
+    db = torch.full((groups, n), float("nan"), device=DEV)
+    for _ in range(2):   # equal calls add in equal order
+        nat.split_grouped_gemm(0, x, w, offs, y, b, None)
+        nat.split_grouped_gemm(1, dy, w, offs, dx, None, None)
+        nat.split_grouped_gemm(2, dy, x, offs, dw, None, db)
+        again = [t.clone() for t in (y, dx, dw, db)] if _ == 0 else again
+    assert all(torch.equal(p, q) for p, q in zip(again, (y, dx, dw, db)))
+    assert not y[rows:].any() and not dx[rows:].any()   # rows past the last expert
+    base = 0
+    for e, c in enumerate(counts):
+        s = slice(base, base + c)
+        base += c
+        X, D, W = x[s].double(), dy[s].double(), w[e].double()
+        for got, ref, size, terms in [
+                (y[s], X @ W.t() + b[e].double(), X.abs() @ W.abs().t() + b[e].abs().double(), k),
+                (dx[s], D @ W, D.abs() @ W.abs(), n),
+                (dw[e], D.t() @ X, D.abs().t() @ X.abs(), c)]:
+            assert bool(((got.double() - ref).abs() <= _bound(size, terms)).all())
+        # pieces of 256 rows, each a sum of 16 steps, 4 rows and 4 lanes; then the pieces
+        assert bool(((db[e].double() - D.sum(0)).abs() <= D.abs().sum(0) * (24 + c / 256) * 2.0 ** -24).all())
+    assert nat.read_status(0) == 0
+
+
+def test_split_gemm_keeps_infinities_large_and_small_values():
+    nat = _native()
+    torch.manual_seed(0)
+    counts, k, n = [70, 30], 128, 128
+    offs = _offs(counts)
+    x = torch.randn(100, k, device=DEV)
+    w = torch.randn(2, n, k, device=DEV)
+    x[3, 5] = float("inf")
+    x[4, 6] = float("-inf")
+    x[5, 7] = float("nan")
+    x[6] = 0
+    x[6, 0] = torch.finfo(torch.float32).max    # would round up to infinity in bf16
+    w[:, :, 0] = 0.5
+    x[7] *= 2.0 ** -100
+    x[8] *= 2.0 ** 100
+    y = torch.empty(100, n, device=DEV)
+    nat.split_grouped_gemm(0, x, w, offs, y, None, None)
+    ref = torch.cat([x[:70].double() @ w[0].double().t(), x[70:].double() @ w[1].double().t()])
+    assert torch.equal(torch.isnan(y), torch.isnan(ref))
+    inf = torch.isinf(ref)
+    assert torch.equal(y[inf].double(), ref[inf]) and inf[3].all() and inf[4].all()
+    ok = torch.isfinite(ref)
+    size = torch.cat([x[:70].double().abs() @ w[0].double().abs().t(), x[70:].double().abs() @ w[1].double().abs().t()])
+    assert bool(((y.double() - ref).abs()[ok] <= _bound(size, k)[ok]).all())
+
+
+@pytest.mark.parametrize("act", [nn.GELU(), nn.ReLU(), nn.GELU(approximate="tanh"), nn.Identity(),
+                                 nn.Sequential(nn.ReLU(), nn.Dropout(0.0))])
+@pytest.mark.parametrize("experts,k,d,h,tokens", [(4, 2, 64, 136, 300), (3, 1, 40, 72, 65), (8, 3, 128, 512, 1000)])
+def test_fp32_layer_as_the_general_path(monkeypatch, act, experts, k, d, h, tokens):
+    r"""Outputs and gradients of the one-call layer against 64 bits: no further off than the general
+    path, up to what the last bits of single sums make of it."""
+    from fastmoe_b200 import FMoETransformerMLP
+    from fastmoe_b200.ops import fused
+    torch.manual_seed(experts + tokens)
+    moe = FMoETransformerMLP(num_expert=experts, d_model=d, d_hidden=h, top_k=k, activation=act).to(DEV)
+    x = torch.randn(tokens, d, device=DEV)
+    gy = torch.randn(tokens, d, device=DEV)
+    ids, score = moe.gate(x)
+    ids = torch.where(torch.rand(ids.shape, device=DEV) < 0.1, -1, ids)   # dropped slots
+    score = score.detach()
+
+    def run(module, dtype):
+        leaves = {n: p.detach().to(dtype).requires_grad_(True) for n, p in module.experts.named_parameters()}
+        xs, sc = (t.detach().to(dtype, copy=True).requires_grad_(True) for t in (x, score))
+        if dtype == torch.float64:
+            rows = []
+            for e in range(experts):
+                hid = act(xs @ leaves["htoh4.weight"][e].t() + leaves["htoh4.bias"][e])
+                rows.append(hid @ leaves["h4toh.weight"][e].t() + leaves["h4toh.bias"][e])
+            picked = torch.stack(rows)[ids.clamp(min=0), torch.arange(tokens, device=DEV)[:, None]]
+            y = (picked * (sc * (ids >= 0))[..., None]).sum(1)
+            y.backward(gy.to(dtype))
+            grads = [leaves[n].grad for n in sorted(leaves)]
+        else:
+            module.zero_grad()
+            y = module._fused_forward(xs, ids, sc)
+            if y is None:
+                y = module._general_path(xs, ids, sc)
+            y.backward(gy)
+            grads = [p.grad for n, p in sorted(module.experts.named_parameters())]
+        return [y.detach(), xs.grad, sc.grad] + grads
+
+    assert fused.supports(moe, x, ids)
+    new = run(moe, torch.float32)
+    monkeypatch.setenv("FMOE_FUSED", "0")
+    assert not fused.supports(moe, x, ids)
+    old = run(moe, torch.float32)
+    ref = run(moe, torch.float64)
+    for a, b, r in zip(new, old, ref):
+        far = lambda t: float((t.double() - r).norm() / r.norm().clamp(min=1e-30))
+        assert far(a) <= 1.1 * far(b) + 2.0 ** -24, (far(a), far(b))
+
+
+def test_fp32_calls_that_keep_the_general_path(monkeypatch):
+    from fastmoe_b200 import FMoETransformerMLP
+    from fastmoe_b200.ops import fused
+    moe = FMoETransformerMLP(num_expert=2, d_model=64, d_hidden=64, top_k=2).to(DEV)
+    x = torch.randn(128, 64, device=DEV)
+    ids = torch.zeros(128, 2, dtype=torch.long, device=DEV)
+    assert fused.supports(moe, x, ids)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert not fused.supports(moe, x, ids)
+    for module in (moe.experts, moe.experts.htoh4, moe.experts.activation):
+        seen = []
+        handle = module.register_forward_hook(lambda *_: seen.append(1))
+        assert not fused.supports(moe, x, ids)
+        moe(x)
+        handle.remove()
+        assert seen
+    monkeypatch.setenv("FMOE_FASTER_SCHEDULE_ENABLE", "1")
+    assert not fused.supports(moe, x, ids)
+    monkeypatch.undo()
+    moe.experts.htoh4.register_parameter("bias", None)
+    assert not fused.supports(moe, x, ids)
+
+
+def test_fp32_layer_in_a_graph_and_on_two_streams():
+    from fastmoe_b200 import FMoETransformerMLP
+    from fastmoe_b200.utils.graph import GraphedStep
+    torch.manual_seed(1)
+    moe = FMoETransformerMLP(num_expert=4, d_model=128, d_hidden=512, top_k=2).to(DEV)
+    xs = [torch.randn(700, 128, device=DEV) for _ in range(2)]
+
+    def step(x):
+        moe.zero_grad(set_to_none=True)
+        y = moe(x)
+        y.square().sum().backward()
+        return y.detach(), [p.grad for p in moe.parameters()]
+
+    graphed = GraphedStep(step, xs[0])
+    for x in xs:
+        got = [t.clone() for t in [graphed(x)[0]] + graphed(x)[1]]
+        y, grads = step(x)
+        assert all(torch.equal(a, b) for a, b in zip(got, [y] + grads))
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    with torch.no_grad():
+        want = [moe(x) for x in xs]
+        torch.cuda.synchronize()
+        for _ in range(5):
+            outs = []
+            for s, x in zip(streams, xs):
+                with torch.cuda.stream(s):
+                    outs.append(moe(x))
+            torch.cuda.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(outs, want))
