@@ -122,8 +122,11 @@ cudaError_t launch_narrow_gemm(const GroupedGemmArgs& a) {
 }
 
 cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
-  CUtensorMap ta, tb;
-  bool ok = true;
+  CUtensorMap ta, tb, tc;
+  // (an fp32 or accumulated gradient is not stored through the map)
+  bool ok = a.mode == kWgrad ? make_map_3d(&tc, a.dtype, a.out, a.n, a.m, a.num_groups, 64, 32)
+                             : make_map_3d(&tc, a.dtype, a.out, a.n, a.rows_cap, 1, 64, 32);
+  if (!ok) return cudaErrorInvalidValue;
   if (a.mode == kRowsNT) {
     ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, pg::CTA_M) &&
          make_map_2d(&tb, a.dtype, a.b, a.k, static_cast<uint64_t>(a.num_groups) * a.n, BK, pg::CTA_N);
@@ -151,8 +154,8 @@ cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
   p.psrc = a.a;
   p.status = a.status;
   const int grid = (a.num_sms > 1 ? a.num_sms : 148) & ~1;
-  return a.dtype == kBF16 ? pg::launch_bf16(a.mode, a.act, ta, tb, p, grid, a.stream)
-                          : pg::launch_f16(a.mode, a.act, ta, tb, p, grid, a.stream);
+  return a.dtype == kBF16 ? pg::launch_bf16(a.mode, a.act, ta, tb, tc, p, grid, a.stream)
+                          : pg::launch_f16(a.mode, a.act, ta, tb, tc, p, grid, a.stream);
 }
 
 }  // namespace

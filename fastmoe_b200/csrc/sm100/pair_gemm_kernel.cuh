@@ -4,8 +4,8 @@
 // A pair of CTAs (one cluster, two neighbouring SMs) works on a 256 x 256 output tile: CTA r
 // holds rows [128 r, 128 r + 128) of A, columns [128 r, 128 r + 128) of B and the accumulators of
 // its rows.  Per 64-wide K block an SM loads 32 KB where a 128 x 256 tile on one SM loads 48 KB.
-// Measured, bf16, 8192 rows, 2 experts, 1024 <-> 4096: forward 69.0 (GELU, saved pre-activation)
-// and 52.5 us, input gradient 69.0 and 51.8 us, weight gradient 64.4 us (1068 to 1327 TFLOP/s
+// Measured, bf16, 8192 rows, 2 experts, 1024 <-> 4096: forward 68.0 (GELU, saved pre-activation)
+// and 52.5 us, input gradient 69.0 and 51.8 us, weight gradient 63.5 us (1080 to 1327 TFLOP/s
 // without activation), where the single-CTA kernel took 85.5, 56.0, 78.4, 54.5 and 70.1 us.  What
 // bounds it: the last of the waves (128 tiles on 74 pairs) and, with an activation, the epilogue.
 //
@@ -17,7 +17,8 @@
 //   warp 2      weight gradient: zeroes the rows past an expert's end in the expert's last K block
 //               (shared memory), off the producer's path, so that loads of the next tiles go on;
 //   warp 3      weight gradient: zeroes the gradients of experts without rows, beside the MMAs;
-//   warps 4-11  epilogue: as in the single-CTA kernel, 32 rows x 128 columns per warp.
+//   warps 4-11  epilogue: as in the single-CTA kernel, 32 rows x 128 columns per warp; whole rows of
+//               32 leave by TMA.
 // The last K block of an expert in the weight gradient issues only the 16-row MMA steps that
 // contain rows of the expert.  With the zeroing in the producer warp, which waited for the copies
 // first, 64 experts of 128 rows took 394 us; now 200 us, 537 MB of gradients written.
@@ -97,77 +98,112 @@ struct Tile {
   int rows;
 };
 
-__device__ __forceinline__ Tile decode(const Shared* sh, int num_groups, int n_tiles, int tile) {
-  int lo = 0, hi = num_groups;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (sh->tiles[mid] <= tile) lo = mid; else hi = mid;
-  }
+// `hint`: a group at or before the tile's (a role's tiles come in ascending order, and the next one
+// is mostly in the same group or in the one after: a binary search was a fifth of a tile's time in
+// the weight gradient of 64 experts).
+__device__ __forceinline__ Tile decode(const Shared* sh, int n_tiles, int tile, int& hint) {
+  int g = hint;
+  while (sh->tiles[g + 1] <= tile) ++g;
+  hint = g;
   Tile t;
-  const int local = tile - sh->tiles[lo];
-  t.group = lo;
+  const int local = tile - sh->tiles[g];
+  t.group = g;
   t.m_tile = local / n_tiles;
   t.n_tile = local - t.m_tile * n_tiles;
-  t.row_begin = sh->offs[lo];
-  t.rows = sh->offs[lo + 1] - t.row_begin;
+  t.row_begin = sh->offs[g];
+  t.rows = sh->offs[g + 1] - t.row_begin;
   return t;
 }
 
 // ------------------------------------------------------------------------------ activations
-// The formulas of gg::gelu_parts on two values at a time: 0.5 erfc(|x| / sqrt 2) and
-// exp(-x^2 / 2).  The packed instructions halve the work of the FMA pipe in the epilogue, which
-// bounds a GEMM with a short K.
-__device__ __forceinline__ void gelu_parts2(ptx::f32x2 x, float a, float b, ptx::f32x2& half_erfc, ptx::f32x2& gauss) {
+// The formulas of gg::gelu_parts on eight pairs at a time, one step of all pairs after the other, as
+// an epilogue has two warps per scheduler.  The packed instructions halve the issue slots of the FMAs.
+// Measured per tile and CTA (K = 512): 5 thousand cycles without activation, 10 with GELU, 9.2 with
+// its reciprocals and exponentials left out: the packed FMAs are most of it.
+constexpr int PAIRS = 8;
+struct GeluPairs {
+  ptx::f32x2 half_erfc[PAIRS];   // 0.5 erfc(|x| / sqrt 2)
+  ptx::f32x2 gauss[PAIRS];       // exp(-x^2 / 2)
+};
+__device__ __forceinline__ void gelu_pairs(const ptx::f32x2 (&x)[PAIRS], GeluPairs& g) {
   using namespace ptx;
-  const f32x2 ax = pack2(fabsf(a), fabsf(b));
-  float d0, d1, t0, t1, e0, e1, g0, g1;
-  unpack2(fma2(ax, pack2(0.3275911f * 0.70710678118654752f, 0.3275911f * 0.70710678118654752f), pack2(1.f, 1.f)), d0, d1);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(d0));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(d1));
-  const f32x2 t = pack2(t0, t1);
-  f32x2 poly = fma2(pack2(0.5f * 1.061405429f, 0.5f * 1.061405429f), t, pack2(0.5f * -1.453152027f, 0.5f * -1.453152027f));
-  poly = fma2(poly, t, pack2(0.5f * 1.421413741f, 0.5f * 1.421413741f));
-  poly = fma2(poly, t, pack2(0.5f * -0.284496736f, 0.5f * -0.284496736f));
-  poly = fma2(poly, t, pack2(0.5f * 0.254829592f, 0.5f * 0.254829592f));
-  poly = mul2(poly, t);
-  unpack2(mul2(x, mul2(x, pack2(-0.72134752044448170f, -0.72134752044448170f))), e0, e1);
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(g0) : "f"(e0));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(g1) : "f"(e1));
-  gauss = pack2(g0, g1);
-  half_erfc = mul2(poly, gauss);
+  auto both = [](float c) { return pack2(c, c); };
+  f32x2 t[PAIRS];
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) {
+    float a, b, d0, d1, t0, t1;
+    unpack2(x[i], a, b);
+    unpack2(fma2(pack2(fabsf(a), fabsf(b)), both(0.3275911f * 0.70710678118654752f), both(1.f)), d0, d1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(d0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(d1));
+    t[i] = pack2(t0, t1);
+  }
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) {
+    float e0, e1, g0, g1;
+    unpack2(mul2(x[i], mul2(x[i], both(-0.72134752044448170f))), e0, e1);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(g0) : "f"(e0));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(g1) : "f"(e1));
+    g.gauss[i] = pack2(g0, g1);
+  }
+  f32x2 poly[PAIRS];
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) poly[i] = fma2(both(0.5f * 1.061405429f), t[i], both(0.5f * -1.453152027f));
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) poly[i] = fma2(poly[i], t[i], both(0.5f * 1.421413741f));
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) poly[i] = fma2(poly[i], t[i], both(0.5f * -0.284496736f));
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) poly[i] = fma2(poly[i], t[i], both(0.5f * 0.254829592f));
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) poly[i] = mul2(poly[i], t[i]);
+#pragma unroll
+  for (int i = 0; i < PAIRS; ++i) g.half_erfc[i] = mul2(poly[i], g.gauss[i]);
 }
 
-__device__ __forceinline__ ptx::f32x2 gelu_cdf2(float a, float b, ptx::f32x2 half_erfc) {
-  float h0, h1, u0, u1;
+__device__ __forceinline__ ptx::f32x2 gelu_cdf2(ptx::f32x2 x, ptx::f32x2 half_erfc) {
+  float a, b, h0, h1, u0, u1;
+  ptx::unpack2(x, a, b);
   ptx::unpack2(half_erfc, h0, h1);
   ptx::unpack2(ptx::fma2(half_erfc, ptx::pack2(-1.f, -1.f), ptx::pack2(1.f, 1.f)), u0, u1);
   return ptx::pack2(a >= 0.f ? u0 : h0, b >= 0.f ? u1 : h1);
 }
 
-template <int ACT> __device__ __forceinline__ void act_fwd2(float& a, float& b) {
+template <int ACT> __device__ __forceinline__ void act_pairs(ptx::f32x2 (&v)[PAIRS]) {
   if (ACT == kActGelu) {
-    const ptx::f32x2 x = ptx::pack2(a, b);
-    ptx::f32x2 h, g;
-    gelu_parts2(x, a, b, h, g);
-    ptx::unpack2(ptx::mul2(x, gelu_cdf2(a, b, h)), a, b);
+    GeluPairs g;
+    gelu_pairs(v, g);
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) v[i] = ptx::mul2(v[i], gelu_cdf2(v[i], g.half_erfc[i]));
   } else {
-    a = gg::act_fwd<ACT>(a);
-    b = gg::act_fwd<ACT>(b);
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
+      float a, b;
+      ptx::unpack2(v[i], a, b);
+      v[i] = ptx::pack2(gg::act_fwd<ACT>(a), gg::act_fwd<ACT>(b));
+    }
   }
 }
 
-// (a, b) *= act'(x0), act'(x1)
-template <int ACT> __device__ __forceinline__ void act_grad2(float x0, float x1, float& a, float& b) {
+// v *= act'(x)
+template <int ACT> __device__ __forceinline__ void act_grad_pairs(const ptx::f32x2 (&x)[PAIRS], ptx::f32x2 (&v)[PAIRS]) {
   if (ACT == kActGelu) {
-    const ptx::f32x2 x = ptx::pack2(x0, x1);
-    ptx::f32x2 h, g;
-    gelu_parts2(x, x0, x1, h, g);
-    const ptx::f32x2 d = ptx::fma2(ptx::mul2(x, ptx::pack2(0.3989422804014327f, 0.3989422804014327f)), g,
-                                   gelu_cdf2(x0, x1, h));
-    ptx::unpack2(ptx::mul2(ptx::pack2(a, b), d), a, b);
+    GeluPairs g;
+    gelu_pairs(x, g);
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
+      const ptx::f32x2 d = ptx::fma2(ptx::mul2(x[i], ptx::pack2(0.3989422804014327f, 0.3989422804014327f)), g.gauss[i],
+                                     gelu_cdf2(x[i], g.half_erfc[i]));
+      v[i] = ptx::mul2(v[i], d);
+    }
   } else {
-    a = gg::act_bwd<ACT>(a, x0);
-    b = gg::act_bwd<ACT>(b, x1);
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
+      float x0, x1, a, b;
+      ptx::unpack2(x[i], x0, x1);
+      ptx::unpack2(v[i], a, b);
+      v[i] = ptx::pack2(gg::act_bwd<ACT>(a, x0), gg::act_bwd<ACT>(b, x1));
+    }
   }
 }
 
@@ -183,6 +219,8 @@ struct EpiTile {
   long out_pitch;
   uint8_t* pre_tile;        // this warp's 4 x 2 KB of the tile-blocked pre-activation, or null
   uint32_t empty_bar;       // CTA 0's accumulator-free barrier
+  const CUtensorMap* map;   // output, boxes of 32 rows x 64 columns; null: not all 32 rows may be written
+  int x, y, z;              // first column, row and matrix of the span there
 };
 
 // Bias / activation, or activation derivative (DACT), of one 32-column chunk into the patch.
@@ -190,56 +228,74 @@ template <typename T, int ACT, bool DACT>
 __device__ __forceinline__ void finish_chunk(const EpiTile& et, int i, const uint32_t (&r)[32], const Packed32& side) {
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
-    uint32_t wo[8];
-    if (DACT) {
+    ptx::f32x2 v[PAIRS];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float s0, s1;
-        Cvt<T>::unpack(side.w[q * 8 + j], s0, s1);
-        float a = __uint_as_float(r[q * 16 + 2 * j]);
-        float b = __uint_as_float(r[q * 16 + 2 * j + 1]);
-        act_grad2<ACT>(s0, s1, a, b);
-        wo[j] = Cvt<T>::pack(a, b);
+    for (int j = 0; j < PAIRS; ++j) v[j] = ptx::pack2(__uint_as_float(r[q * 16 + 2 * j]), __uint_as_float(r[q * 16 + 2 * j + 1]));
+    auto packed = [&](uint32_t (&w)[PAIRS]) {
+#pragma unroll
+      for (int j = 0; j < PAIRS; ++j) {
+        float a, b;
+        ptx::unpack2(v[j], a, b);
+        w[j] = Cvt<T>::pack(a, b);
       }
+    };
+    if (DACT) {
+      ptx::f32x2 x[PAIRS];
+#pragma unroll
+      for (int j = 0; j < PAIRS; ++j) {
+        float a, b;
+        Cvt<T>::unpack(side.w[q * 8 + j], a, b);
+        x[j] = ptx::pack2(a, b);
+      }
+      act_grad_pairs<ACT>(x, v);
     } else {
-      uint32_t bw[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
       if (et.bias != nullptr) {
         const uint4 b0 = *reinterpret_cast<const uint4*>(et.bias + i * 64 + q * 32);
         const uint4 b1 = *reinterpret_cast<const uint4*>(et.bias + i * 64 + q * 32 + 16);
-        bw[0] = b0.x; bw[1] = b0.y; bw[2] = b0.z; bw[3] = b0.w;
-        bw[4] = b1.x; bw[5] = b1.y; bw[6] = b1.z; bw[7] = b1.w;
-      }
-      uint32_t wp[8];
+        const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float a = __uint_as_float(r[q * 16 + 2 * j]);
-        float b = __uint_as_float(r[q * 16 + 2 * j + 1]);
-        if (et.bias != nullptr) {
-          float b0, b1;
-          Cvt<T>::unpack(bw[j], b0, b1);
-          ptx::unpack2(ptx::add2(ptx::pack2(a, b), ptx::pack2(b0, b1)), a, b);
+        for (int j = 0; j < PAIRS; ++j) {
+          float a, b;
+          Cvt<T>::unpack(bw[j], a, b);
+          v[j] = ptx::add2(v[j], ptx::pack2(a, b));
         }
-        if (ACT != kActNone) {
-          wp[j] = Cvt<T>::pack(a, b);
-          act_fwd2<ACT>(a, b);
-        }
-        wo[j] = Cvt<T>::pack(a, b);
       }
-      if (ACT != kActNone && et.pre_tile != nullptr) {
-        uint8_t* pd = et.pre_tile + i * gg::PRE_CHUNK_BYTES + et.lane * 16 + q * 1024;
-        *reinterpret_cast<uint4*>(pd) = make_uint4(wp[0], wp[1], wp[2], wp[3]);
-        *reinterpret_cast<uint4*>(pd + 512) = make_uint4(wp[4], wp[5], wp[6], wp[7]);
+      if (ACT != kActNone) {
+        if (et.pre_tile != nullptr) {
+          uint32_t wp[PAIRS];
+          packed(wp);
+          uint8_t* pd = et.pre_tile + i * gg::PRE_CHUNK_BYTES + et.lane * 16 + q * 1024;
+          *reinterpret_cast<uint4*>(pd) = make_uint4(wp[0], wp[1], wp[2], wp[3]);
+          *reinterpret_cast<uint4*>(pd + 512) = make_uint4(wp[4], wp[5], wp[6], wp[7]);
+        }
+        act_pairs<ACT>(v);
       }
     }
+    uint32_t wo[PAIRS];
+    packed(wo);
     const int c = (i & 1) * 4 + q * 2;
     *reinterpret_cast<uint4*>(gg::patch_piece(et.patch, et.lane, c)) = make_uint4(wo[0], wo[1], wo[2], wo[3]);
     *reinterpret_cast<uint4*>(gg::patch_piece(et.patch, et.lane, c + 1)) = make_uint4(wo[4], wo[5], wo[6], wo[7]);
   }
 }
 
-// After an odd chunk (or the last one): whole 128-byte lines, 8 lanes per row.
+// After an odd chunk (or the last one) the patch holds whole 128-byte lines.  Its swizzle is that of a
+// tensor map, so one copy takes all 32 rows (what lies outside the matrix is not written); rows of
+// which the last ones belong to the next expert are stored one by one, 8 lanes per row.  Loads from
+// the patch and stores were 2.5 of the 5 thousand cycles of a plain tile's epilogue: 22528 rows, 8
+// experts, 512 -> 2048, forward and input gradient, with GELU 72 and 72 us, now 67 and 66; with ReLU 59
+// and 62, now 55 and 52 (its instances no longer spill either).
 __device__ __forceinline__ void send_lines(const EpiTile& et, int i) {
   if (!(i + 1 == et.n_chunks || (i & 1))) return;
+  if (et.map != nullptr) {
+    ptx::fence_proxy_async_smem();
+    __syncwarp();
+    if (et.lane == 0) {
+      ptx::tma_store_3d(et.map, et.patch, et.x + (i & ~1) * 32, et.y, et.z);
+      ptx::bulk_commit();
+    }
+    return;
+  }
   const int bytes = ((i & 1) + 1) * 64;
   const int sub = et.lane & 7;
   uint8_t* dst = et.out + (i & ~1) * 64 + sub * 16 + (et.lane >> 3) * et.out_pitch;
@@ -252,6 +308,12 @@ __device__ __forceinline__ void send_lines(const EpiTile& et, int i) {
           *reinterpret_cast<const uint4*>(gg::patch_piece(et.patch, row, sub));
     }
   }
+  __syncwarp();
+}
+
+// Before the patch is written again: the copies out of it have read it.
+__device__ __forceinline__ void patch_free(const EpiTile& et) {
+  if (et.lane == 0) ptx::bulk_wait_read<0>();
   __syncwarp();
 }
 
@@ -281,6 +343,7 @@ __device__ __forceinline__ void epilogue_tile(const EpiTile& et, Packed32& side_
         release_accumulator(et);
         released = true;
       }
+      patch_free(et);
       finish_chunk<T, ACT, DACT>(et, i, ra, side_a);
       send_lines(et, i);
       if (!second) break;
@@ -399,7 +462,7 @@ __device__ __forceinline__ void column_sums(const Params& p, uint8_t* patches, c
 template <int MODE, typename T, int ACT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                 const __grid_constant__ Params p) {
+                 const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   Shared* sh = reinterpret_cast<Shared*>(smem + AUX_OFF);
@@ -427,6 +490,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     ptx::fence_barrier_init();
     ptx::prefetch_tmap(&tm_a);
     ptx::prefetch_tmap(&tm_b);
+    ptx::prefetch_tmap(&tm_c);
   }
   if (warp == 1) ptx::tmem_alloc_pair(&sh->tmem_base, TMEM_COLS);
   ptx::chain_begin();   // nothing an earlier kernel writes is read above
@@ -472,6 +536,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
   const uint32_t tmem_base = sh->tmem_base;
   const int total = sh->tiles[p.num_groups];
+  int group = 0;   // of the role's latest tile
 
   if (warp == 0) {
     // ============================================================== TMA producer
@@ -480,7 +545,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       uint32_t phase = 0;
       bool ok = true;
       for (int tile = pair; tile < total && ok; tile += num_pairs) {
-        const Tile c = decode(sh, p.num_groups, n_tiles, tile);
+        const Tile c = decode(sh, n_tiles, tile, group);
         const int num_kb = (MODE == kWgrad) ? (c.rows + BK - 1) / BK : p.k / BK;
         const int n0 = c.n_tile * TILE_N + rank * CTA_N;
         const int m0 = c.m_tile * TILE_M + rank * CTA_M;
@@ -536,7 +601,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       int iter = 0;
       bool ok = true;
       for (int tile = pair; tile < total && ok; tile += num_pairs, ++iter) {
-        const Tile c = decode(sh, p.num_groups, n_tiles, tile);
+        const Tile c = decode(sh, n_tiles, tile, group);
         const int num_kb = (MODE == kWgrad) ? (c.rows + BK - 1) / BK : p.k / BK;
         const int acc = iter & 1;
         if (!ptx::mbar_wait(&sh->tmem_empty[acc], ((iter >> 1) & 1) ^ 1, abort_flag)) {
@@ -584,7 +649,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       int stage = 0;
       uint32_t phases = 0;   // bit s: parity of the next use of tail[s]
       for (int tile = pair; tile < total; tile += num_pairs) {
-        const Tile c = decode(sh, p.num_groups, n_tiles, tile);
+        const Tile c = decode(sh, n_tiles, tile, group);
         const int num_kb = (c.rows + BK - 1) / BK;
         const int last = (stage + num_kb - 1) % STAGES;
         stage = (stage + num_kb) % STAGES;
@@ -645,7 +710,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     auto load_bias = [&](int tile) -> uint2 {
       uint2 v = make_uint2(0u, 0u);
       if (has_bias && tile < total) {
-        const Tile c = decode(sh, p.num_groups, n_tiles, tile);
+        int ahead = group;
+        const Tile c = decode(sh, n_tiles, tile, ahead);
         const int col = c.n_tile * TILE_N + half * EPI_COLS + lane * 4;
         if (col < p.n) v = __ldg(reinterpret_cast<const uint2*>(static_cast<const T*>(p.bias) + static_cast<long>(c.group) * p.n + col));
       }
@@ -655,7 +721,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     int iter = 0;
     bool dead = false;   // a wait ran out: walk the remaining tiles' barriers, touch nothing else
     for (int tile = pair; tile < total; tile += num_pairs, ++iter) {
-      const Tile c = decode(sh, p.num_groups, n_tiles, tile);
+      const Tile c = decode(sh, n_tiles, tile, group);
       const int acc = iter & 1;
       const int col_first = c.n_tile * TILE_N + half * EPI_COLS;
       const int m0 = c.m_tile * TILE_M + rank * CTA_M + part * 32;
@@ -671,9 +737,14 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       et.t_row = tmem_base + (static_cast<uint32_t>(part * 32) << 16) + acc * TILE_N + half * EPI_COLS;
       const long first_elem = ((MODE == kWgrad) ? static_cast<long>(c.group) * p.m + m0 : static_cast<long>(c.row_begin) + m0) * p.n + col_first;
       et.out = static_cast<uint8_t*>(p.out) + first_elem * 2;
+      et.map = MODE == kWgrad || et.warp_valid == 32 ? &tm_c : nullptr;
+      et.x = col_first;
+      et.y = MODE == kWgrad ? m0 : c.row_begin + m0;
+      et.z = MODE == kWgrad ? c.group : 0;
       Packed32 side;
       if constexpr (MODE == kWgrad) {
         if (p.psum != nullptr && c.n_tile == 0) {
+          patch_free(et);
           column_sums<T>(p, patches, c, c.m_tile * TILE_M + rank * CTA_M, warp, lane);
         }
       } else {
@@ -688,7 +759,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             // pull the next tile's chunks of this warp (8 KB, two lines per lane) into L2
             gg::load_pre_chunk(et.pre_tile, 0, lane, side);
             if (tile + num_pairs < total) {
-              const Tile cn = decode(sh, p.num_groups, n_tiles, tile + num_pairs);
+              int ahead = group;
+              const Tile cn = decode(sh, n_tiles, tile + num_pairs, ahead);
               if (cn.m_tile * TILE_M + rank * CTA_M < cn.rows) {
                 const long nb = (static_cast<long>(sh->blocks[cn.group]) + cn.m_tile * 2 + rank) * n_tiles + cn.n_tile;
                 const uint8_t* nx = static_cast<const uint8_t*>(pre) + nb * gg::PRE_TILE_BYTES +
@@ -725,6 +797,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   }
 
   // ---------------------------------------------------------------- tear-down
+  if (lane == 0) ptx::bulk_wait<0>();
   __syncwarp();
   if (*abort_flag != 0) {
     // give copies that were already issued time to land before the shared memory goes away
@@ -742,7 +815,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
 // ------------------------------------------------------------------------------ launch
 template <int MODE, typename T, int ACT>
-cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int grid, cudaStream_t stream) {
+cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, int grid, cudaStream_t stream) {
   static std::mutex mu;   // the shared-memory attribute is per device
   static uint64_t configured = 0;
   auto kernel = pair_gemm_kernel<MODE, T, ACT>;
@@ -756,33 +829,34 @@ cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const Param
       configured |= 1ull << (dev & 63);
     }
   }
-  return launch_chained(kernel, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, ta, tb, p);
+  return launch_chained(kernel, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, ta, tb, tc, p);
 }
 
 template <int MODE, typename T>
-cudaError_t launch_act(int act, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int grid, cudaStream_t stream) {
+cudaError_t launch_act(int act, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, int grid,
+                       cudaStream_t stream) {
   switch (act) {
-    case kActRelu: return launch_one<MODE, T, kActRelu>(ta, tb, p, grid, stream);
-    case kActGelu: return launch_one<MODE, T, kActGelu>(ta, tb, p, grid, stream);
-    case kActGeluTanh: return launch_one<MODE, T, kActGeluTanh>(ta, tb, p, grid, stream);
-    default: return launch_one<MODE, T, kActNone>(ta, tb, p, grid, stream);
+    case kActRelu: return launch_one<MODE, T, kActRelu>(ta, tb, tc, p, grid, stream);
+    case kActGelu: return launch_one<MODE, T, kActGelu>(ta, tb, tc, p, grid, stream);
+    case kActGeluTanh: return launch_one<MODE, T, kActGeluTanh>(ta, tb, tc, p, grid, stream);
+    default: return launch_one<MODE, T, kActNone>(ta, tb, tc, p, grid, stream);
   }
 }
 
 // One translation unit per element type instantiates this.
 template <typename T>
-cudaError_t launch_for_type(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int grid,
+cudaError_t launch_for_type(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, int grid,
                             cudaStream_t stream) {
   switch (mode) {
-    case kRowsNT: return launch_act<kRowsNT, T>(act, ta, tb, p, grid, stream);
-    case kRowsNN: return launch_act<kRowsNN, T>(act, ta, tb, p, grid, stream);
-    default: return launch_one<kWgrad, T, kActNone>(ta, tb, p, grid, stream);
+    case kRowsNT: return launch_act<kRowsNT, T>(act, ta, tb, tc, p, grid, stream);
+    case kRowsNN: return launch_act<kRowsNN, T>(act, ta, tb, tc, p, grid, stream);
+    default: return launch_one<kWgrad, T, kActNone>(ta, tb, tc, p, grid, stream);
   }
 }
 
-cudaError_t launch_bf16(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int grid,
+cudaError_t launch_bf16(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, int grid,
                         cudaStream_t stream);
-cudaError_t launch_f16(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int grid,
+cudaError_t launch_f16(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, int grid,
                        cudaStream_t stream);
 
 }  // namespace pg

@@ -110,7 +110,7 @@ struct Params {
 
 // A shared sum: one piece of 32 x 64 per epilogue warp.
 constexpr int WORK_FLOATS = 32 * EPI_COLS;
-constexpr int MIN_KB = 4;   // 3 us of MMAs; handing a sum over takes about 2
+constexpr int COST_KB = 3;   // of 0.8 us: handing a sum over and collecting one takes about 2 us
 constexpr unsigned long long COLLECT_LIMIT_NS = 30000000000ull;   // other streams may hold the SMs meanwhile
 
 // Pieces of the column sums: expert e's begin at slot sum_slot(offs[e], e).
@@ -283,7 +283,7 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   ptx::tc_fence_after_sync();
 
   const uint32_t tmem_base = sh->tmem_base;
-  TileWalk walk(sh->tiles, sh->units, p.num_groups, pair, num_pairs, p.work != nullptr ? MIN_KB : 0);
+  TileWalk walk(sh->tiles, sh->units, p.num_groups, pair, num_pairs, p.work != nullptr ? COST_KB : 0);
   WalkPart part_of;
 
   if (warp == 0) {

@@ -23,31 +23,31 @@ struct WalkPart {
   int last_piece;   // kb0 == 0: the pieces after this pair's up to this one hold the rest of the tile
 };
 
-// Tiles dealt out in turn.  All of them when the last round is nearly full (less than an eighth of
-// the pairs idle in it).
-__host__ __device__ inline int dealt_tiles(int tiles, int pairs) {
+// Tiles dealt out in turn.  All of them unless cutting saves more than the `cost_kb` K blocks of time
+// that a pair spends on handing its sum over and on collecting another.
+__host__ __device__ inline int dealt_tiles(int tiles, int units, int pairs, int cost_kb) {
   const int rest = tiles % pairs;
-  if (rest == 0 || rest * 8 > pairs * 7) return tiles;
-  const int rounds = tiles / pairs;
-  return rounds <= 1 ? 0 : (rounds - 1) * pairs;
+  if (cost_kb <= 0 || rest == 0) return tiles;
+  const long idle = static_cast<long>(pairs - rest) * units / tiles;   // K blocks that nobody works on
+  if (idle <= static_cast<long>(cost_kb) * pairs) return tiles;
+  return tiles - rest;
 }
 
 // `tiles` and `units` are exclusive prefixes over the groups ([num_groups + 1]) of the tiles and of
 // their K blocks.  Every role of a kernel walks the same parts.
 class TileWalk {
  public:
-  // min_kb: no piece is shorter than that on average (handing a sum over has a price); 0: no tile
-  // is cut.
-  __host__ __device__ TileWalk(const int* tiles, const int* units, int num_groups, int pair, int pairs, int min_kb)
+  // cost_kb: see dealt_tiles; 0: no tile is cut.
+  __host__ __device__ TileWalk(const int* tiles, const int* units, int num_groups, int pair, int pairs, int cost_kb)
       : tiles_(tiles), units_(units), groups_(num_groups), pairs_(pairs), next_(pair) {
     const int total = tiles[num_groups];
-    dealt_ = min_kb > 0 ? dealt_tiles(total, pairs) : total;
+    dealt_ = dealt_tiles(total, units[num_groups], pairs, cost_kb);
     if (dealt_ == total) return;
     const int g = find(tiles, dealt_);
     first_ = units[g] + (dealt_ - tiles[g]) * blocks(g);
     len_ = units[num_groups] - first_;
     const int left = total - dealt_;
-    pieces_ = len_ / min_kb;
+    pieces_ = len_ / cost_kb;   // no shorter than that on average
     if (pieces_ < left) pieces_ = left;
     if (pieces_ > pairs) pieces_ = pairs;
     if (pair < pieces_) {

@@ -12,14 +12,14 @@ def test_every_block_once_and_every_sum_collected(seed):
     walk = native.get().tile_walk
     rng = random.Random(seed)
     groups, pairs = rng.randint(1, 12), rng.choice([1, 3, 74, 74])
-    min_kb, equal = rng.choice([0, 1, 4, 16]), rng.randint(1, 40)
+    cost_kb, equal = rng.choice([0, 1, 4, 16]), rng.randint(1, 40)
     per_tile = [equal if seed % 2 else rng.randint(1, 40) for _ in range(groups)]
     count = [rng.choice([0, rng.randint(0, 40)]) for _ in range(groups)]
     tiles, units = [0], [0]
     for t, kb in zip(count, per_tile):
         tiles.append(tiles[-1] + t)
         units.append(units[-1] + t * kb)
-    parts = [walk(tiles, units, p, pairs, min_kb) for p in range(pairs)]
+    parts = [walk(tiles, units, p, pairs, cost_kb) for p in range(pairs)]
     blocks = sorted((g, t, kb) for mine in parts for g, t, kb0, kb1, _n, _l in mine for kb in range(kb0, kb1))
     assert blocks == [(g, t, kb) for g in range(groups) for t in range(count[g]) for kb in range(per_tile[g])]
     handed = 0
@@ -38,5 +38,5 @@ def test_every_block_once_and_every_sum_collected(seed):
                 handed -= 1
             assert end == num_kb
     assert handed == 0
-    if min_kb == 0:
+    if cost_kb == 0:
         assert all(part[2] == 0 and part[3] == part[4] for mine in parts for part in mine)
