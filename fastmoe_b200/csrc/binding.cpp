@@ -518,10 +518,13 @@ void scatter_rows(torch::Tensor src, torch::Tensor idx, torch::Tensor rank, torc
   c10::cuda::CUDAGuard guard(src.device());
   const void* sc = (scale.has_value() && scale->defined()) ? scale->data_ptr() : nullptr;
   int* rs = (row_slot.has_value() && row_slot->defined()) ? row_slot->data_ptr<int>() : nullptr;
-  FMOE_CUDA_CHECK(fmoe::launch_scatter_rows(dtype16(src), src.data_ptr(), idx.data_ptr<int64_t>(),
+  // unscaled fp32 rows are moved as 16-bit rows of twice the width
+  const bool wide = src.scalar_type() == torch::kFloat;
+  TORCH_CHECK(!wide || sc == nullptr, "scatter_rows: only 16-bit rows are scaled");
+  FMOE_CUDA_CHECK(fmoe::launch_scatter_rows(wide ? fmoe::kBF16 : dtype16(src), src.data_ptr(), idx.data_ptr<int64_t>(),
                                             rank.data_ptr<int>(), base.data_ptr<int>(), sc,
                                             static_cast<int>(idx.numel()), static_cast<int>(k),
-                                            static_cast<int>(src.size(1)), dst.data_ptr(), rs,
+                                            static_cast<int>(src.size(1)) * (wide ? 2 : 1), dst.data_ptr(), rs,
                                             cur_stream()));
 }
 
@@ -531,6 +534,14 @@ void gather_combine(torch::Tensor rows, torch::Tensor idx, torch::Tensor rank, t
   check_rows(out, "out");
   c10::cuda::CUDAGuard guard(rows.device());
   const void* w = (weight.has_value() && weight->defined()) ? weight->data_ptr() : nullptr;
+  if (rows.scalar_type() == torch::kFloat) {
+    TORCH_CHECK(rows.size(1) % 8 == 0, "fp32 rows of a multiple of 8 columns");
+    FMOE_CUDA_CHECK(fmoe::launch_combine_f32(rows.data_ptr<float>(), idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
+                                             base.data_ptr<int>(), static_cast<const float*>(w), out.size(0),
+                                             static_cast<int>(k), static_cast<int>(rows.size(1)), out.data_ptr<float>(),
+                                             cur_stream()));
+    return;
+  }
   FMOE_CUDA_CHECK(fmoe::launch_gather_combine(dtype16(rows), rows.data_ptr(),
                                               idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
                                               base.data_ptr<int>(), w,
@@ -546,6 +557,14 @@ void combine_bwd(torch::Tensor dout, torch::Tensor rows, torch::Tensor idx, torc
   check_rows(rows, "rows");
   check_rows(drows, "drows");
   c10::cuda::CUDAGuard guard(dout.device());
+  if (dout.scalar_type() == torch::kFloat) {
+    TORCH_CHECK(dout.size(1) % 8 == 0, "fp32 rows of a multiple of 8 columns");
+    FMOE_CUDA_CHECK(fmoe::launch_combine_bwd_f32(dout.data_ptr<float>(), rows.data_ptr<float>(), idx.data_ptr<int64_t>(),
+                                                 rank.data_ptr<int>(), base.data_ptr<int>(), weight.data_ptr<float>(),
+                                                 idx.numel(), static_cast<int>(k), static_cast<int>(dout.size(1)),
+                                                 drows.data_ptr<float>(), dscore.data_ptr<float>(), cur_stream()));
+    return;
+  }
   FMOE_CUDA_CHECK(fmoe::launch_combine_bwd(dtype16(dout), dout.data_ptr(), rows.data_ptr(),
                                            idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
                                            base.data_ptr<int>(), weight.data_ptr(),
@@ -617,7 +636,7 @@ std::vector<torch::Tensor> moe_mlp_forward_f32(const torch::Tensor& x, const tor
   }
   auto out = torch::empty_like(x);
   FMOE_CUDA_CHECK(fmoe::launch_combine_f32(ys.data_ptr<float>(), idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
-                                           offs.data_ptr<int>(), score.data_ptr<float>(), static_cast<int>(groups), x.size(0),
+                                           offs.data_ptr<int>(), score.data_ptr<float>(), x.size(0),
                                            static_cast<int>(k), static_cast<int>(d), out.data_ptr<float>(), cur_stream()));
   return {out, xs, pre, a, ys, rank, offs, score, idx};
 }
@@ -669,7 +688,7 @@ std::vector<torch::Tensor> moe_mlp_backward_f32(const torch::Tensor& dout, const
       FMOE_CUDA_CHECK(fmoe::launch_split_gemm(g));
       dx = torch::empty({n_tok, d}, dout.options());
       FMOE_CUDA_CHECK(fmoe::launch_combine_f32(dxs.data_ptr<float>(), idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
-                                               offs.data_ptr<int>(), nullptr, static_cast<int>(groups), n_tok,
+                                               offs.data_ptr<int>(), nullptr, n_tok,
                                                static_cast<int>(k), static_cast<int>(d), dx.data_ptr<float>(), cur_stream()));
     }
   }

@@ -279,9 +279,9 @@ __global__ void scatter_rows_kernel(const T* __restrict__ src, const int64_t* __
   const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (s >= n_slots) return;
-  const long e = idx[s];
-  if (e < 0) return;
-  const long row = static_cast<long>(base[e]) + rank[s];
+  const int rk = rank[s];   // negative for dropped slots and for ids that name no expert
+  if (rk < 0) return;
+  const long row = static_cast<long>(base[idx[s]]) + rk;
   const uint4* in = reinterpret_cast<const uint4*>(src + static_cast<long>(s / k) * d);
   uint4* out = reinterpret_cast<uint4*>(dst + row * d);
   const int nv = d >> 3;
@@ -334,9 +334,9 @@ __global__ void __launch_bounds__(256, 4) gather_combine_kernel(const T* __restr
     w_of[j] = 0.f;
     if (j < kk) {
       const int s = t * k + j;
-      const long e = idx[s];
-      if (e >= 0) {
-        rows_of[j] = static_cast<long>(base[e]) + rank[s];
+      const int rk = rank[s];
+      if (rk >= 0) {
+        rows_of[j] = static_cast<long>(base[idx[s]]) + rk;
         w_of[j] = weight != nullptr ? V2<T>::to_f(weight[s]) : 1.f;
       }
     }
@@ -369,9 +369,9 @@ __global__ void __launch_bounds__(256, 4) gather_combine_kernel(const T* __restr
     }
     for (int j = kk; j < k; ++j) {  // more than kMaxInline slots per token: plain path
       const int s = t * k + j;
-      const long e = idx[s];
-      if (e < 0) continue;
-      const long row = static_cast<long>(base[e]) + rank[s];
+      const int rk = rank[s];
+      if (rk < 0) continue;
+      const long row = static_cast<long>(base[idx[s]]) + rk;
       const float w = weight != nullptr ? V2<T>::to_f(weight[s]) : 1.f;
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
@@ -401,12 +401,12 @@ __global__ void combine_bwd_kernel(const T* __restrict__ dout, const T* __restri
   const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (s >= n_slots) return;
-  const long e = idx[s];
-  if (e < 0) {
+  const int rk = rank[s];
+  if (rk < 0) {
     if (lane == 0 && dscore != nullptr) dscore[s] = V2<T>::from_f(0.f);
     return;
   }
-  const long row = static_cast<long>(base[e]) + rank[s];
+  const long row = static_cast<long>(base[idx[s]]) + rk;
   const uint4* g = reinterpret_cast<const uint4*>(dout + static_cast<long>(s / k) * d);
   const uint4* y = reinterpret_cast<const uint4*>(rows + row * d);
   uint4* dy = reinterpret_cast<uint4*>(drows + row * d);

@@ -715,6 +715,39 @@ split_rows_kernel(const float* __restrict__ src, const int* __restrict__ offs, i
   }
 }
 
+// Backward of the weighted combine into fp32 rows.  One warp per slot.
+__global__ void __launch_bounds__(kSplitThreads)
+combine_bwd_f32_kernel(const float* __restrict__ dout, const float* __restrict__ rows, const int64_t* __restrict__ idx,
+                       const int* __restrict__ rank, const int* __restrict__ offs, const float* __restrict__ score,
+                       long n_slots, int k, int width, float* __restrict__ drows, float* __restrict__ dscore) {
+  ptx::chain_begin();
+  const int lane = threadIdx.x & 31;
+  const long s = static_cast<long>(blockIdx.x) * (kSplitThreads / 32) + (threadIdx.x >> 5);
+  if (s >= n_slots) return;
+  const int rk = rank[s];
+  if (rk < 0) {
+    if (lane == 0) dscore[s] = 0.f;
+    return;
+  }
+  const long row = static_cast<long>(offs[idx[s]]) + rk;
+  const float w = score[s];
+  float dot = 0.f;
+  for (int i = lane; i < (width >> 3); i += 32) {
+    float g[8], y[8];
+    load8(dout + s / k * width + i * 8, g);
+    load8(rows + row * width + i * 8, y);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      dot += g[q] * y[q];
+      g[q] *= w;
+    }
+    store8(drows + row * width + i * 8, g);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  if (lane == 0) dscore[s] = dot;
+}
+
 // One warp per slot; the blocks behind those of the slots write the zero rows of one expert each.
 // BWD: the rows are scaled by their slot's score, whose gradient is formed on the way.
 template <bool BWD>
@@ -741,12 +774,13 @@ split_scatter_kernel(const float* __restrict__ src, const float* __restrict__ ro
   }
   const long s = static_cast<long>(blockIdx.x) * (kSplitThreads / 32) + (threadIdx.x >> 5);
   if (s >= n_slots) return;
-  const long e = idx[s];
-  if (e < 0 || e >= num_groups) {
+  const int rk = rank[s];   // negative for dropped slots and for ids that name no expert
+  if (rk < 0) {
     if (BWD && lane == 0) dscore[s] = 0.f;
     return;
   }
-  const int lo = offs[e], rk = rank[s];
+  const long e = idx[s];
+  const int lo = offs[e];
   const float* in = src + s / k * width;
   bf16* out = planes + (split_row(lo, e) + rk) * width;
   if (!BWD) {
@@ -779,7 +813,7 @@ split_scatter_kernel(const float* __restrict__ src, const float* __restrict__ ro
 // One warp per token.
 __global__ void __launch_bounds__(kSplitThreads)
 combine_f32_kernel(const float* __restrict__ rows, const int64_t* __restrict__ idx, const int* __restrict__ rank,
-                   const int* __restrict__ offs, const float* __restrict__ weight, int num_groups, long n_tokens, int k,
+                   const int* __restrict__ offs, const float* __restrict__ weight, long n_tokens, int k,
                    int width, float* __restrict__ out) {
   ptx::chain_begin();
   const int lane = threadIdx.x & 31;
@@ -789,11 +823,11 @@ combine_f32_kernel(const float* __restrict__ rows, const int64_t* __restrict__ i
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int j = 0; j < k; ++j) {
       const long s = t * k + j;
-      const long e = idx[s];
-      if (e < 0 || e >= num_groups) continue;
+      const int rk = rank[s];
+      if (rk < 0) continue;
       const float w = weight != nullptr ? weight[s] : 1.f;
       float v[8];
-      load8(rows + (static_cast<long>(offs[e]) + rank[s]) * width + i * 8, v);
+      load8(rows + (static_cast<long>(offs[idx[s]]) + rk) * width + i * 8, v);
 #pragma unroll
       for (int q = 0; q < 8; ++q) acc[q] += w * v[q];
     }
@@ -923,10 +957,18 @@ cudaError_t launch_split_combine_bwd(const float* dout, const float* rows, const
 }
 
 cudaError_t launch_combine_f32(const float* rows, const int64_t* idx, const int* rank, const int* offs,
-                               const float* weight, int num_groups, long n_tokens, int k, int width, float* out,
-                               cudaStream_t stream) {
+                               const float* weight, long n_tokens, int k, int width, float* out, cudaStream_t stream) {
+  if (n_tokens == 0) return cudaSuccess;
   return launch_chained(combine_f32_kernel, dim3(blocks_of(n_tokens, kSplitThreads / 32)), dim3(kSplitThreads), 0, stream, rows,
-                        idx, rank, offs, weight, num_groups, n_tokens, k, width, out);
+                        idx, rank, offs, weight, n_tokens, k, width, out);
+}
+
+cudaError_t launch_combine_bwd_f32(const float* dout, const float* rows, const int64_t* idx, const int* rank,
+                                   const int* offs, const float* score, long n_slots, int k, int width, float* drows,
+                                   float* dscore, cudaStream_t stream) {
+  if (n_slots == 0) return cudaSuccess;
+  return launch_chained(combine_bwd_f32_kernel, dim3(blocks_of(n_slots, kSplitThreads / 32)), dim3(kSplitThreads), 0, stream,
+                        dout, rows, idx, rank, offs, score, n_slots, k, width, drows, dscore);
 }
 
 }  // namespace fmoe

@@ -68,9 +68,12 @@ cudaError_t launch_split_scatter(const float* src, const int64_t* idx, const int
 cudaError_t launch_split_combine_bwd(const float* dout, const float* rows, const int64_t* idx, const int* rank,
                                      const int* offs, const float* score, int num_groups, long n_slots, int k, int width,
                                      void* planes, float* dscore, int* flags, int num_flags, cudaStream_t stream);
-// out[t] = sum over the slots of token t of weight[s] * rows[offs[e] + rank[s]] (weights null: 1).
+// out[t] = sum over the slots of token t of weight[s] * rows[offs[e] + rank[s]] (weights null: 1), and
+// its backward: drows[offs[e] + rank[s]] = score[s] * dout[s / k], dscore as above.
 cudaError_t launch_combine_f32(const float* rows, const int64_t* idx, const int* rank, const int* offs,
-                               const float* weight, int num_groups, long n_tokens, int k, int width, float* out,
-                               cudaStream_t stream);
+                               const float* weight, long n_tokens, int k, int width, float* out, cudaStream_t stream);
+cudaError_t launch_combine_bwd_f32(const float* dout, const float* rows, const int64_t* idx, const int* rank,
+                                   const int* offs, const float* score, long n_slots, int k, int width, float* drows,
+                                   float* dscore, cudaStream_t stream);
 
 }  // namespace fmoe

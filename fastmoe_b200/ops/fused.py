@@ -70,13 +70,20 @@ def _forced_ep():
     return dist.is_available() and dist.is_initialized()
 
 
+def _rows_of_slots(idx, rank, offs):
+    r"""``(row, kept)`` of every slot as PyTorch operations: for a gradient of the gradient."""
+    kept = rank >= 0
+    return torch.where(kept, offs[idx.clamp(0, offs.numel() - 2)] + rank, 0).long(), kept
+
+
 class _Dispatch(Function):
-    r"""``xs[offs[e] + rank[s]] = x[s // k]`` for every kept slot ``s`` routed to expert ``e``."""
+    r"""``xs[offs[e] + rank[s]] = x[s // k]`` for every kept slot ``s`` routed to expert ``e``;
+    ``n_rows``: rows of ``xs`` where the caller knows how many slots are kept."""
 
     @staticmethod
-    def forward(ctx, x, idx, rank, offs, k):
+    def forward(ctx, x, idx, rank, offs, k, n_rows=None):
         nat = native.get()
-        xs = torch.empty(idx.numel(), x.shape[1], dtype=x.dtype, device=x.device)
+        xs = torch.empty(idx.numel() if n_rows is None else n_rows, x.shape[1], dtype=x.dtype, device=x.device)
         nat.scatter_rows(gg.aligned(x, 16), idx, rank, offs, None, k, xs, None)
         ctx.save_for_backward(idx, rank, offs)
         ctx.k = k
@@ -86,9 +93,15 @@ class _Dispatch(Function):
     @staticmethod
     def backward(ctx, dxs):
         idx, rank, offs = ctx.saved_tensors
+        if torch.is_grad_enabled():   # a gradient of the gradient is wanted
+            if dxs.shape[0] == 0:
+                return dxs.new_zeros(ctx.n_tok, dxs.shape[1]) + dxs.sum(), None, None, None, None, None
+            row, kept = _rows_of_slots(idx, rank, offs)
+            dx = torch.where(kept[:, None], dxs[row], 0).view(ctx.n_tok, ctx.k, -1).sum(1)
+            return dx, None, None, None, None, None
         dx = torch.empty(ctx.n_tok, dxs.shape[1], dtype=dxs.dtype, device=dxs.device)
         native.get().gather_combine(gg.aligned(dxs, 16), idx, rank, offs, None, ctx.k, dx)
-        return dx, None, None, None, None
+        return dx, None, None, None, None, None
 
 
 class _Combine(Function):
@@ -98,7 +111,7 @@ class _Combine(Function):
     def forward(ctx, ys, score, idx, rank, offs, k):
         n_tok = idx.numel() // k
         out = torch.empty(n_tok, ys.shape[1], dtype=ys.dtype, device=ys.device)
-        native.get().gather_combine(ys, idx, rank, offs, score, k, out)
+        native.get().gather_combine(gg.aligned(ys, 16), idx, rank, offs, score, k, out)
         ctx.save_for_backward(ys, score, idx, rank, offs)
         ctx.k = k
         return out
@@ -106,10 +119,51 @@ class _Combine(Function):
     @staticmethod
     def backward(ctx, dout):
         ys, score, idx, rank, offs = ctx.saved_tensors
-        dys = torch.empty_like(ys)
+        if torch.is_grad_enabled():   # a gradient of the gradient is wanted
+            row, kept = _rows_of_slots(idx, rank, offs)
+            with torch.enable_grad():
+                picked = torch.where(kept[:, None], ys[row], 0) if ys.shape[0] else ys.sum() + ys.new_zeros(
+                    idx.numel(), ys.shape[1])
+                out = (picked * score[:, None]).view(-1, ctx.k, ys.shape[1]).sum(1)
+                dys, dscore = torch.autograd.grad(out, (ys, score), dout, create_graph=True, allow_unused=True)
+            return dys, dscore, None, None, None, None
+        dys = torch.empty_like(ys, memory_format=torch.contiguous_format)
         dscore = torch.empty_like(score)
         native.get().combine_bwd(gg.aligned(dout, 16), gg.aligned(ys, 16), idx, rank, offs, score, ctx.k, dys, dscore)
         return dys, dscore, None, None, None, None
+
+
+def rows_supported(x, ids, scores):
+    r"""Whether the kernels that move and combine rows take a call of the general path."""
+    return (torch.is_tensor(x) and x.is_cuda and x.dim() == 2 and x.dtype in _TC + (torch.float32,)
+            and x.shape[1] % 8 == 0 and x.shape[1] > 0 and ids.is_cuda and ids.dtype == torch.int64 and ids.dim() in (1, 2)
+            and ids.device == x.device and scores.device == x.device
+            and ids.shape[0] == x.shape[0] and ids.numel() > 0 and ids.numel() < 2 ** 31
+            and scores.numel() == ids.numel() and scores.is_floating_point()
+            and not torch.is_autocast_enabled())
+
+
+def general_path(x, ids, scores, expert_fn, num_expert):
+    r"""The general path of one GPU around ``expert_fn(rows, counts)``: rows to their experts, the
+    weighted sum of what comes back.  One read of the counts on the host, as the experts are called
+    with Python slices.  ``(out, rows, routing)``: ``out`` is ``None``, and ``routing`` what
+    ``MOEGather`` needs, where ``expert_fn`` did not return rows that the kernels combine.
+
+    8 experts of two ``nn.Linear`` with 2048 tokens, top-2, d 512: the zeroed tensors, copies and additions
+    behind slices, and index operations and ``bmm`` around the experts, were 33 of 123 launches."""
+    nat = native.get()
+    k = ids.shape[1] if ids.dim() == 2 else 1
+    idx = ids.contiguous().view(-1)
+    counts, rank, offs, pos = nat.route_pos(idx, num_expert)
+    counts = counts.cpu().long()
+    n_rows = int(counts.sum())
+    xs = _Dispatch.apply(x.contiguous(), idx, rank, offs, k, n_rows)
+    xs.fmoe_own_rows = True   # a buffer that nobody else holds (see FMoE.expert_fn)
+    ys = expert_fn(xs, counts)
+    if (torch.is_tensor(ys) and ys.is_cuda and ys.dim() == 2 and ys.dtype in _TC + (torch.float32,)
+            and ys.shape[0] == n_rows and ys.shape[1] % 8 == 0 and ys.shape[1] > 0 and ys.device == x.device):
+        return _Combine.apply(ys.contiguous(), scores.reshape(-1).to(ys.dtype), idx, rank, offs, k), ys, None
+    return None, ys, (pos[:n_rows].long(), counts)
 
 
 class _ExpertMLP(Function):
