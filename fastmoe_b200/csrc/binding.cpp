@@ -889,7 +889,7 @@ bool gate_fused_supported(int64_t tot, int64_t d, int64_t k) {
 
 // logits [B, tot], idx [B, k] and prob [B, k] of a linear gate in one pass over x.
 std::vector<torch::Tensor> gate_linear_topk(torch::Tensor x, torch::Tensor w,
-                                            c10::optional<torch::Tensor> bias, int64_t k) {
+                                            c10::optional<torch::Tensor> bias, int64_t k, bool few) {
   check_rows(x, "x");
   check_rows(w, "w");
   TORCH_CHECK(x.scalar_type() == w.scalar_type(), "gate input and weight dtypes differ");
@@ -900,7 +900,7 @@ std::vector<torch::Tensor> gate_linear_topk(torch::Tensor x, torch::Tensor w,
   auto logits = torch::empty({rows, tot}, x.options());
   auto idx = torch::empty({rows, k}, torch::dtype(torch::kLong).device(x.device()));
   auto prob = torch::empty({rows, k}, x.options());
-  FMOE_CUDA_CHECK(fmoe::launch_gate_linear_topk(
+  FMOE_CUDA_CHECK((few ? fmoe::launch_gate_linear_topk_few : fmoe::launch_gate_linear_topk)(
       dtype16(x), x.data_ptr(), w.data_ptr(), bias.has_value() ? bias->data_ptr() : nullptr, rows, d,
       tot, static_cast<int>(k), logits.data_ptr(), idx.data_ptr<int64_t>(), prob.data_ptr(),
       cur_stream()));
@@ -1020,7 +1020,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("balance_bwd", &balance_bwd);
   m.def("switch_top1", &switch_top1);
   m.def("gate_fused_supported", &gate_fused_supported);
-  m.def("gate_linear_topk", &gate_linear_topk);
+  m.def("gate_linear_topk", &gate_linear_topk, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("k"),
+        py::arg("few") = false);
   m.def("gate_linear_topk_bwd", &gate_linear_topk_bwd);
   m.def("launch_count", []() { return g_launches.load(); });
   m.def("read_status", &read_status);

@@ -492,15 +492,42 @@ template <> struct Ld<__half> {
 
 constexpr int kMaxK = 8;
 
-// One warp per row.  k rounds of warp arg-max; ties go to the lower expert id.
+// Top-k with softmax of one row of at most 64 logits without a NaN, two per lane (-inf where there is
+// none): k rounds of a warp-wide maximum of keys that order as the logits do; ties go to the lower id.
+// 4096 rows of 64, k = 2: 5.1 us with rounds of shuffles and the choices in local arrays, now 2.0.
+__device__ __forceinline__ unsigned order_key(float v) {
+  const unsigned u = __float_as_uint(v + 0.f);   // (-0 and +0 are a tie)
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
 template <typename T>
-__global__ void gate_topk_softmax_kernel(const T* __restrict__ logits, int n_rows, int n_experts,
-                                         int k, int64_t* __restrict__ idx, T* __restrict__ prob) {
-  ptx::chain_begin();
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= n_rows) return;
-  const T* in = logits + static_cast<long>(row) * n_experts;
+__device__ __forceinline__ void topk_row64(float v0, float v1, bool on0, bool on1, int lane, int k, int64_t* idx, T* prob) {
+  unsigned k0 = on0 ? order_key(v0) : 0u, k1 = on1 ? order_key(v1) : 0u;   // 0: taken, or none
+  float top = 0.f, den = 0.f, my_ex = 0.f;
+  int my_e = 0;
+  for (int j = 0; j < k; ++j) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, k0 > k1 ? k0 : k1);
+    const unsigned low = __ballot_sync(0xffffffffu, k0 == m), high = __ballot_sync(0xffffffffu, k1 == m);
+    const int e = low != 0 ? __ffs(low) - 1 : 31 + __ffs(high);
+    const float v = __uint_as_float(m & 0x80000000u ? m & 0x7fffffffu : ~m);
+    if (j == 0) top = v;
+    const float ex = __expf(v - top);
+    den += ex;
+    if (lane == j) {
+      my_e = e;
+      my_ex = ex;
+    }
+    if (e == lane) k0 = 0u;
+    if (e == lane + 32) k1 = 0u;
+  }
+  if (lane < k) {
+    idx[lane] = my_e;
+    Ld<T>::put(prob, lane, my_ex / den);
+  }
+}
+
+// The same for any number of experts, and with NaN: k rounds of warp arg-max.
+template <typename T>
+__device__ __noinline__ void topk_row(const T* in, int n_experts, int lane, int k, int64_t* idx, T* prob) {
   float sel_v[kMaxK];
   int sel_i[kMaxK];
   for (int j = 0; j < k; ++j) {
@@ -525,8 +552,9 @@ __global__ void gate_topk_softmax_kernel(const T* __restrict__ logits, int n_row
         best_i = oi;
       }
     }
-    sel_v[j] = best;
-    sel_i[j] = best_i;
+    // (with NaN the lanes may disagree: all go by lane 0, so that k different experts are chosen)
+    sel_v[j] = __shfl_sync(0xffffffffu, best, 0);
+    sel_i[j] = __shfl_sync(0xffffffffu, best_i, 0);
   }
   if (lane == 0) {
     const float mx = sel_v[0];
@@ -537,10 +565,32 @@ __global__ void gate_topk_softmax_kernel(const T* __restrict__ logits, int n_row
       den += ex[j];
     }
     for (int j = 0; j < k; ++j) {
-      idx[static_cast<long>(row) * k + j] = sel_i[j];
-      Ld<T>::put(prob, static_cast<long>(row) * k + j, ex[j] / den);
+      idx[j] = sel_i[j];
+      Ld<T>::put(prob, j, ex[j] / den);
     }
   }
+}
+
+// One warp per row.
+template <typename T>
+__global__ void gate_topk_softmax_kernel(const T* __restrict__ logits, int n_rows, int n_experts,
+                                         int k, int64_t* __restrict__ idx, T* __restrict__ prob) {
+  ptx::chain_begin();
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= n_rows) return;
+  const T* in = logits + static_cast<long>(row) * n_experts;
+  idx += static_cast<long>(row) * k;
+  prob += static_cast<long>(row) * k;
+  if (n_experts <= 64) {
+    const bool on0 = lane < n_experts, on1 = lane + 32 < n_experts;
+    const float v0 = on0 ? Ld<T>::get(in, lane) : 0.f, v1 = on1 ? Ld<T>::get(in, lane + 32) : 0.f;
+    if (!__any_sync(0xffffffffu, v0 != v0 || v1 != v1)) {
+      topk_row64<T>(v0, v1, on0, on1, lane, k, idx, prob);
+      return;
+    }
+  }
+  topk_row<T>(in, n_experts, lane, k, idx, prob);
 }
 
 // dlogits[row, idx_j] = p_j * (g_j - sum_i g_i p_i), zero elsewhere.  One warp per row.
@@ -853,6 +903,68 @@ gate_linear_topk_kernel(const T* __restrict__ x, const T* __restrict__ w, const 
   }
 }
 
+// The same for a few tokens and 9 to 64 experts: one block per token, a warp for every eighth expert.
+// All of W comes out of the L2 once per token, which at 64 experts, d = 1024 is 128 KB: 64 tokens 6.0
+// us, where padding W and the bias, the tensor-core product and the top-k were five launches, 16.5 us.
+template <typename T>
+__global__ void __launch_bounds__(256)
+gate_linear_topk_few_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, int d, int tot,
+                            int k, T* __restrict__ logits, int64_t* __restrict__ idx, T* __restrict__ prob) {
+  ptx::chain_begin();
+  __shared__ T row_logits[kGateMaxExperts];
+  constexpr int PER = kGateMaxExperts / 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long row = blockIdx.x;
+  float acc[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) acc[u] = 0.f;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + row * d);
+  const int nv = d >> 3;
+  const int mine = (tot - warp + 7) / 8;   // experts warp, warp + 8, ...
+  for (int i = lane; i < nv; i += 32) {
+    uint4 wv[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      if (u < mine) wv[u] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(warp + 8 * u) * d) + i);
+    }
+    float xf[8];
+    unpack8<T>(__ldg(xr + i), xf);
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      if (u < mine) {
+        float wf[8];
+        unpack8<T>(wv[u], wf);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[u] = fmaf(xf[q], wf[q], acc[u]);
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    if (u < mine) {
+      float v = acc[u];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      const int e = warp + 8 * u;
+      if (bias != nullptr) v += V2<T>::to_f(bias[e]);
+      if (lane == 0) {
+        row_logits[e] = V2<T>::from_f(v);
+        logits[row * tot + e] = V2<T>::from_f(v);
+      }
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  // the choice and the probabilities follow the rounded logits
+  const bool on0 = lane < tot, on1 = lane + 32 < tot;
+  const float v0 = on0 ? V2<T>::to_f(row_logits[lane]) : 0.f, v1 = on1 ? V2<T>::to_f(row_logits[lane + 32]) : 0.f;
+  if (!__any_sync(0xffffffffu, v0 != v0 || v1 != v1)) {
+    topk_row64<T>(v0, v1, on0, on1, lane, k, idx + row * k, prob + row * k);
+  } else {
+    topk_row<T>(row_logits, tot, lane, k, idx + row * k, prob + row * k);
+  }
+}
+
 // The same result for R tokens per warp, TOT <= 8 and R * TOT <= 32: a slice of W is loaded and
 // unpacked once for R tokens, and the R * TOT sums over the lanes are formed together (each
 // exchange step halves the number of values a lane still holds; the additions are those of the
@@ -991,8 +1103,7 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
 // dl[t, e] = softmax backward of the selected logits scattered to their experts, plus the
 // gradient that reached the logits directly (may be null).  dx[t, :] = sum_e dl[t, e] W[e, :].
 // dl is written out (fp32) for the weight-gradient kernel.  One warp per token; every lane forms
-// the dl of one expert and the warp shares them: with all lanes walking the k choices of the
-// token 8192 tokens (d = 2048, 8 experts) took 37 us, now 21.
+// the dl of one expert and the warp shares them.  9 and more experts (fewer: below).
 template <typename T, int TOT>
 __global__ void __launch_bounds__(256)
 gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
@@ -1046,6 +1157,78 @@ gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
   }
 }
 
+// The same for R tokens per warp, TOT <= 8: a slice of W is loaded and unpacked once for R tokens, and
+// its loads carry no predicates.  The sums are those of the one-token kernel.  All of the gate's
+// backward, 8192 tokens, d = 2048, 8 experts: 35 us, 41 with gradients at all logits; with this kernel
+// and dl in shared memory in the next one 30 and 33.
+template <typename T, int TOT, int R>
+__global__ void __launch_bounds__(256)
+gate_bwd_dx_rows_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx, const T* __restrict__ prob,
+                        const T* __restrict__ dlogits_in, const T* __restrict__ w, int n_rows, int d, int tot, int k,
+                        float* __restrict__ dl_out, T* __restrict__ dx) {
+  ptx::chain_begin();
+  const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
+  const int lane = threadIdx.x & 31;
+  if (row0 >= n_rows) return;
+  float mine = 0.f;
+  {
+    const int row = row0 + lane / TOT, e = lane % TOT;
+    if (lane < R * TOT && row < n_rows && e < tot) {
+      if (dlogits_in != nullptr) mine = V2<T>::to_f(dlogits_in[static_cast<long>(row) * tot + e]);
+      if (dprob != nullptr) {
+        const T* g = dprob + static_cast<long>(row) * k;
+        const T* p = prob + static_cast<long>(row) * k;
+        const int64_t* id = idx + static_cast<long>(row) * k;
+        float dotp = 0.f;
+        for (int j = 0; j < k; ++j) dotp += V2<T>::to_f(g[j]) * V2<T>::to_f(p[j]);
+        for (int j = 0; j < k; ++j) {
+          if (id[j] == e) mine += V2<T>::to_f(p[j]) * (V2<T>::to_f(g[j]) - dotp);
+        }
+      }
+      dl_out[static_cast<long>(row) * tot + e] = mine;
+    }
+  }
+  if (dx == nullptr) return;
+  float dl[R][TOT];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+#pragma unroll
+    for (int e = 0; e < TOT; ++e) dl[r][e] = __shfl_sync(0xffffffffu, mine, r * TOT + e);
+  }
+  const int nv = d >> 3;
+#pragma unroll 2
+  for (int i = lane; i < nv; i += 32) {
+    uint4 wv[TOT];
+#pragma unroll
+    for (int e = 0; e < TOT; ++e) {
+      // (past the last expert the last one again, for nothing)
+      wv[e] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(min(e, tot - 1)) * d) + i);
+    }
+    float acc[R][8];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[r][q] = 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < TOT; ++e) {
+      float wf[8];
+      unpack8<T>(wv[e], wf);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (dl[r][e] != 0.f) {   // the same for the whole warp; an expert without gradient adds nothing
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[r][q] = fmaf(dl[r][e], wf[q], acc[r][q]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (row0 + r < n_rows) reinterpret_cast<uint4*>(dx + static_cast<long>(row0 + r) * d)[i] = pack8<T>(acc[r]);
+    }
+  }
+}
+
 // Partial sums of dW[e, c] = sum_t dl[t, e] x[t, c] and db[e] = sum_t dl[t, e] over one of
 // `gridDim.y` token ranges: part[range][tot * d + tot] in fp32.  A block takes a 256-column strip;
 // a lane owns eight columns, so that a token is one 16-byte load per lane (two columns per lane,
@@ -1058,7 +1241,9 @@ __global__ void __launch_bounds__(256, TOT <= 8 ? 2 : 1)
 gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_rows, int d, int tot,
                    float* __restrict__ part) {
   ptx::chain_begin();
+  constexpr int CHUNK = 128;   // tokens whose dl are held at a time: a multiple of the warps' step of 32
   __shared__ float red[8][256 + 8];
+  __shared__ __align__(16) float dls[CHUNK][TOT];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 256 + lane * 8;
   const int per = (n_rows + gridDim.y - 1) / gridDim.y;
@@ -1073,25 +1258,37 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
     for (int q = 0; q < 8; ++q) acc[e][q] = 0.f;
   }
   constexpr int U = 4;
-  for (int t = t0 + warp; t < t1; t += 8 * U) {
-    uint4 xv[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      xv[u] = (t + 8 * u < t1 && col < d) ? __ldg(reinterpret_cast<const uint4*>(x + static_cast<long>(t + 8 * u) * d + col))
-                                          : make_uint4(0u, 0u, 0u, 0u);
+  for (int c0 = t0; c0 < t1; c0 += CHUNK) {
+    const int c1 = min(t1, c0 + CHUNK);
+    __syncthreads();
+    for (int i = threadIdx.x; i < CHUNK * TOT; i += 256) {
+      const int t = c0 + i / TOT, e = i % TOT;
+      dls[i / TOT][e] = t < c1 && e < tot ? __ldg(dl + static_cast<long>(t) * tot + e) : 0.f;
     }
+    __syncthreads();
+    for (int t = c0 + warp; t < c1; t += 8 * U) {
+      uint4 xv[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (t + 8 * u >= t1) break;
-      float xf[8];
-      unpack8<T>(xv[u], xf);
+      for (int u = 0; u < U; ++u) {
+        xv[u] = (t + 8 * u < c1 && col < d) ? __ldg(reinterpret_cast<const uint4*>(x + static_cast<long>(t + 8 * u) * d + col))
+                                            : make_uint4(0u, 0u, 0u, 0u);
+      }
 #pragma unroll
-      for (int e = 0; e < TOT; ++e) {
-        if (e < tot) {
-          const float g = __ldg(dl + static_cast<long>(t + 8 * u) * tot + e);
+      for (int u = 0; u < U; ++u) {
+        if (t + 8 * u >= c1) break;
+        float xf[8], g[TOT];
+        unpack8<T>(xv[u], xf);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) acc[e][q] = fmaf(g, xf[q], acc[e][q]);
-          if (sums) bsum[e] += g;
+        for (int e = 0; e < TOT; e += 2) {
+          const float2 two = *reinterpret_cast<const float2*>(&dls[t + 8 * u - c0][e]);
+          g[e] = two.x;
+          g[e + 1] = two.y;
+        }
+#pragma unroll
+        for (int e = 0; e < TOT; ++e) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[e][q] = fmaf(g[e], xf[q], acc[e][q]);
+          if (sums) bsum[e] += g[e];
         }
       }
     }
@@ -1575,14 +1772,6 @@ cudaError_t launch_prune_scalar(const int64_t* idx, const int* rank, int cap, in
   return cudaGetLastError();
 }
 
-#define FMOE_GATE_TOT(tot, ...)                          \
-  if ((tot) <= 2) { constexpr int TOT = 2; __VA_ARGS__; }       \
-  else if ((tot) <= 4) { constexpr int TOT = 4; __VA_ARGS__; }  \
-  else if ((tot) <= 8) { constexpr int TOT = 8; __VA_ARGS__; }  \
-  else if ((tot) <= 16) { constexpr int TOT = 16; __VA_ARGS__; } \
-  else if ((tot) <= 32) { constexpr int TOT = 32; __VA_ARGS__; } \
-  else { constexpr int TOT = 64; __VA_ARGS__; }
-
 bool gate_fused_supported(int tot, int d, int k) {
   return tot >= 1 && tot <= kGateMaxExperts && d % 8 == 0 && k >= 1 && k <= kMaxK && k <= tot;
 }
@@ -1634,6 +1823,17 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
   return cudaGetLastError();
 }
 
+cudaError_t launch_gate_linear_topk_few(int dtype, const void* x, const void* w, const void* bias, int n_rows, int d,
+                                        int tot, int k, void* logits, int64_t* idx, void* prob, cudaStream_t stream) {
+  cudaError_t chained = cudaSuccess;
+  if (n_rows == 0) return cudaSuccess;
+  if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_linear_topk_few_kernel<T>, dim3(n_rows), dim3(256), 0, stream,
+      static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), d, tot, k,
+      static_cast<T*>(logits), idx, static_cast<T*>(prob))));
+  return chained;
+}
+
 int gate_bwd_ranges(int n_rows, int d) {
   // two blocks per SM over the strips and token ranges, a warp at least four tokens
   const int strips = (d + 255) / 256;
@@ -1649,10 +1849,27 @@ cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, co
   cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
   if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
-  const int grid = (n_rows + 7) / 8;
-  FMOE_DISPATCH_16(dtype, FMOE_GATE_TOT(tot, (chained = launch_chained(gate_bwd_dx_kernel<T, TOT>, dim3(grid), dim3(256), 0, stream,
-      static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in),
-      static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx)))));
+  const int per = gate_rows_per_warp(n_rows, tot);
+  const int grid = (n_rows + 8 * per - 1) / (8 * per);
+#define FMOE_GATE_DX(TOT, R)                                                                            \
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dx_rows_kernel<T, TOT, R>, dim3(grid), dim3(256), 0, stream,    \
+      static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in),                  \
+      static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx))))
+  if (tot <= 2) {
+    if (per == 1) { FMOE_GATE_DX(2, 1); } else if (per == 2) { FMOE_GATE_DX(2, 2); } else { FMOE_GATE_DX(2, 4); }
+  } else if (tot <= 4) {
+    if (per == 1) { FMOE_GATE_DX(4, 1); } else if (per == 2) { FMOE_GATE_DX(4, 2); } else { FMOE_GATE_DX(4, 4); }
+  } else if (tot <= 8) {
+    if (per == 1) { FMOE_GATE_DX(8, 1); } else if (per == 2) { FMOE_GATE_DX(8, 2); } else { FMOE_GATE_DX(8, 4); }
+  } else {
+#define FMOE_GATE_DX_WIDE(TOT)                                                                          \
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dx_kernel<T, TOT>, dim3(grid), dim3(256), 0, stream,          \
+      static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in),                  \
+      static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx))))
+    if (tot <= 16) { FMOE_GATE_DX_WIDE(16); } else if (tot <= 32) { FMOE_GATE_DX_WIDE(32); } else { FMOE_GATE_DX_WIDE(64); }
+#undef FMOE_GATE_DX_WIDE
+  }
+#undef FMOE_GATE_DX
   if (chained != cudaSuccess) return chained;
   if (part == nullptr) return cudaSuccess;
   if (tot > 16) return cudaErrorInvalidValue;

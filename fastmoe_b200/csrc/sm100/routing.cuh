@@ -94,6 +94,9 @@ bool gate_fused_supported(int tot, int d, int k);
 cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, const void* bias,
                                     int n_rows, int d, int tot, int k, void* logits, int64_t* idx,
                                     void* prob, cudaStream_t stream);
+// The same result for a few tokens (one block each).
+cudaError_t launch_gate_linear_topk_few(int dtype, const void* x, const void* w, const void* bias, int n_rows, int d,
+                                        int tot, int k, void* logits, int64_t* idx, void* prob, cudaStream_t stream);
 // Backward of the fused gate.  dl_scratch: fp32 [n_rows, tot]; dx (optional) [n_rows, d].
 // part (optional, tot <= 16): fp32 scratch of gate_bwd_ranges() * (tot * d + tot) entries; with it
 // dw_db receives dW [tot, d] followed by db [tot] in the layer's type.  Above 16 experts pass

@@ -21,6 +21,11 @@ from . import native
 MAX_FUSED_K = 8
 MAX_FUSED_EXPERTS = 4096
 MAX_SINGLE_PASS_EXPERTS = 8
+# Up to here the one-block-per-token kernel is faster than the tensor-core product and the top-k after
+# it, which take 11 us or more (64 experts, d 1024: 6.0 us for 64 tokens, 10.0 for 512, 15.8 for 1024; d
+# 2048: 17.0 for 512, against 15.6).
+MAX_FEW_TOKENS = 512
+MAX_FEW_PRODUCTS = 1 << 25
 
 
 def _topk_softmax_torch(logits, k):
@@ -88,20 +93,24 @@ _PAD_BIAS = -30000.0   # bias of the padding columns: representable in bf16 and 
 class _GateGemm(Function):
     r"""``logits = x W^T + b`` on the tcgen05 grouped-GEMM kernel (one group, whose row count goes
     with the launch: no offsets on the device), for any number of experts.  The expert dimension is padded to a multiple of 64 — the padding columns get a
-    large negative bias, so a top-k over the padded logits never selects them — and the
-    backward products ``dx = dl W`` and ``dW = dl^T x`` (with ``db`` from the same launch) run on
+    large negative bias, so a top-k over the padded logits never selects them; 64, 128 ... experts need no
+    copies — and the backward products ``dx = dl W`` and ``dW = dl^T x`` (with ``db`` from the same launch) run on
     the same kernel's input-gradient and weight-gradient modes."""
 
     @staticmethod
     def forward(ctx, x, weight, bias):
         tot, d = weight.shape
         pad = (-tot) % 64
-        wp = torch.nn.functional.pad(weight, (0, 0, 0, pad)).unsqueeze(0).contiguous()
-        bp = torch.full((1, tot + pad), _PAD_BIAS, dtype=x.dtype, device=x.device)
-        if bias is not None:
-            bp[0, :tot] = bias
+        if pad == 0:   # nothing to pad: the parameters as they are
+            wp = weight.contiguous().unsqueeze(0)
+            bp = None if bias is None else bias.contiguous().unsqueeze(0)
         else:
-            bp[0, :tot] = 0
+            wp = torch.nn.functional.pad(weight, (0, 0, 0, pad)).unsqueeze(0).contiguous()
+            bp = torch.full((1, tot + pad), _PAD_BIAS, dtype=x.dtype, device=x.device)
+            if bias is not None:
+                bp[0, :tot] = bias
+            else:
+                bp[0, :tot] = 0
         logits = gg.forward(x, wp, None, bp)
         ctx.save_for_backward(x, wp)
         ctx.tot = tot
@@ -130,6 +139,17 @@ def _gate_gemm_ok(x, weight, bias):
                                                     x.shape[1], 1))
 
 
+def _few_tokens_ok(x, weight, bias, k):
+    r"""A decoding step over 9 to 64 experts without gradients, which the kernel for few tokens takes in one
+    launch instead of five."""
+    return (x.is_cuda and x.dim() == 2 and 0 < x.shape[0] <= MAX_FEW_TOKENS
+            and x.shape[0] * x.shape[1] * weight.shape[0] <= MAX_FEW_PRODUCTS
+            and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype
+            and (bias is None or bias.dtype == x.dtype)
+            and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, weight, bias)))
+            and not torch.is_autocast_enabled() and native.get().gate_fused_supported(weight.shape[0], x.shape[1], k))
+
+
 def linear_topk_softmax(x, weight, bias, k):
     r"""``(logits [B,E], idx int64 [B,k], prob [B,k])`` of a linear gate over 2-D ``x``.
 
@@ -138,7 +158,7 @@ def linear_topk_softmax(x, weight, bias, k):
     (with one token per warp, 4096 tokens, ``d_model`` 1024: 30.6 vs 35.5 µs forward + backward at 2
     experts, 52 vs 37 µs at 16; up to 8 experts warps take several tokens, 17.5 µs at 2).  Above that the
     product runs on the tcgen05 grouped-GEMM kernel with a single group (:class:`_GateGemm`),
-    followed by :func:`topk_softmax`; only 32-/64-bit inputs, CPU tensors and odd ``d_model``
+    followed by :func:`topk_softmax`, but for a few tokens without gradients (one launch); only 32-/64-bit inputs, CPU tensors and odd ``d_model``
     take the ``linear`` → :func:`topk_softmax` sequence of PyTorch ops.
     """
     if (x.is_cuda and x.dim() == 2 and x.dtype in (torch.bfloat16, torch.float16)
@@ -148,6 +168,10 @@ def linear_topk_softmax(x, weight, bias, k):
             and native.get().gate_fused_supported(weight.shape[0], x.shape[1], k)):
         xc = x if x.is_contiguous() else x.contiguous()
         return _LinearTopkSoftmax.apply(xc, weight.contiguous(), bias, k)
+    if _few_tokens_ok(x, weight, bias, k):
+        x, weight = gg.aligned(x, 16), gg.aligned(weight, 16)
+        logits, idx, prob = native.get().gate_linear_topk(x, weight, None if bias is None else bias.contiguous(), int(k), True)
+        return logits, idx, prob
     if _gate_gemm_ok(x, weight, bias) and k <= MAX_FUSED_K:
         # more experts: tensor-core product on this library's own kernel, then the top-k /
         # softmax kernel over the (padded) logits

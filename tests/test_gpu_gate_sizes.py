@@ -1,0 +1,81 @@
+r"""GPU tier: the gate's kernels at the sizes their launch rules choose by."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def _native():
+    from fastmoe_b200.ops import native
+    return native.get()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,d,experts,k", [(1, 8, 9, 1), (3, 264, 17, 8), (129, 256, 33, 4), (512, 1024, 64, 2), (5, 2048, 63, 3)])
+def test_few_tokens_many_experts(dtype, tokens, d, experts, k):
+    r"""Logits within one rounding and an fp32 sum of d terms of 64 bits; ids and probabilities those of
+    the top-k kernel on the same logits, also with ties, infinities and NaN."""
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(tokens + experts)
+    x = torch.randn(tokens, d, device=DEV, dtype=dtype)
+    w = (torch.randn(experts, d, device=DEV) / d ** 0.5).to(dtype)
+    w[experts // 2] = w[0]            # a tie in every token
+    b = torch.randn(experts, device=DEV).to(dtype) * 0
+    if tokens > 2:
+        x[0, 0], x[1, 0], x[2, 0] = float("nan"), float("inf"), 0
+    with torch.no_grad():
+        assert gating._few_tokens_ok(x, w, b, k)
+        logits, idx, prob = gating.linear_topk_softmax(x, w, b, k)
+    ref = x.double() @ w.double().t() + b.double()
+    size = x.double().abs() @ w.double().abs().t()
+    ok = torch.isfinite(ref)
+    eps = torch.finfo(dtype).eps
+    assert bool(((logits.double() - ref).abs() <= eps * ref.abs() + d * 2.0 ** -24 * size + 1e-7)[ok].all())
+    i2, p2 = _native().gate_topk_softmax(logits, k)
+    assert torch.equal(idx, i2) and torch.equal(prob.nan_to_num(7.0), p2.nan_to_num(7.0))
+    chosen = idx.cpu()
+    assert int(chosen.min()) >= 0 and int(chosen.max()) < experts
+    assert all(len(set(row)) == k for row in chosen.tolist())   # NaN or not
+    finite = ok.all(1)
+    top = torch.topk(logits.float(), k, dim=1).values
+    assert torch.equal(logits.float().cpu().gather(1, chosen)[finite.cpu()], top[finite].cpu())
+
+
+def test_few_tokens_rule():
+    from fastmoe_b200.ops import gating
+    x = torch.randn(16, 64, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(16, 64, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    assert not gating._few_tokens_ok(x, w, None, 2)            # gradients are wanted
+    with torch.no_grad():
+        assert gating._few_tokens_ok(x, w, None, 2)
+        assert not gating._few_tokens_ok(x.repeat(33, 1), w, None, 2)
+        assert not gating._few_tokens_ok(x.float(), w.float(), None, 2)
+        assert not gating._few_tokens_ok(x, w.repeat(5, 1), None, 2)   # more than 64 experts
+
+
+@pytest.mark.parametrize("experts", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("tokens,d", [(2367, 264), (2369, 256), (4737, 64)])   # 1, 2 and 4 tokens per warp, odd ends
+def test_gate_backward_of_several_tokens_per_warp(experts, tokens, d):
+    r"""Against 64 bits: dl is exact to a few fp32 roundings; dx a sum of as many terms as experts and one
+    rounding to bf16; dW and db fp32 sums over the tokens and one rounding."""
+    nat = _native()
+    torch.manual_seed(tokens + experts)
+    k = min(2, experts)
+    x = torch.randn(tokens, d, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(experts, d, device=DEV, dtype=torch.bfloat16)
+    logits, idx, prob = nat.gate_linear_topk(x, w, None, k)
+    dp, dlog = torch.randn_like(prob), torch.randn_like(logits)
+    dlog[::3] = 0
+    dx, dw, db, dl = nat.gate_linear_topk_bwd(dp, idx, prob, dlog, x, w, True, True)
+    p, g = prob.double(), dp.double()
+    sel = p * (g - (p * g).sum(1, keepdim=True))
+    ref = dlog.double().scatter_add(1, idx, sel)
+    assert bool(((dl.double() - ref).abs() <= 8 * 2.0 ** -24 * (dlog.double().abs() + 4 * g.abs().sum(1, keepdim=True))).all())
+    dl = dl.double()
+    eps = 2.0 ** -8
+    for got, want, size, terms in [(dx, dl @ w.double(), dl.abs() @ w.double().abs(), experts),
+                                   (dw, dl.t() @ x.double(), dl.abs().t() @ x.double().abs(), tokens),
+                                   (db, dl.sum(0), dl.abs().sum(0), tokens)]:
+        assert bool(((got.double() - want).abs() <= eps * want.abs() + terms * 2.0 ** -24 * size + 1e-30).all())
