@@ -786,7 +786,15 @@ int logit_code(const torch::Tensor& t) {
   return 2;
 }
 
-std::vector<torch::Tensor> gate_topk_softmax(torch::Tensor logits, int64_t k) {
+// A one-element fp32 tensor of the caller that the kernel is to zero, or null.
+float* zero_of(const c10::optional<torch::Tensor>& zero) {
+  if (!zero.has_value() || !zero->defined()) return nullptr;
+  TORCH_CHECK(zero->is_cuda() && zero->scalar_type() == torch::kFloat && zero->numel() == 1, "zero: one fp32 element");
+  return zero->data_ptr<float>();
+}
+
+std::vector<torch::Tensor> gate_topk_softmax(torch::Tensor logits, int64_t k,
+                                             c10::optional<torch::Tensor> zero = c10::nullopt) {
   check_cuda_contig(logits, "logits");
   c10::cuda::CUDAGuard guard(logits.device());
   const int rows = static_cast<int>(logits.size(0));
@@ -795,7 +803,7 @@ std::vector<torch::Tensor> gate_topk_softmax(torch::Tensor logits, int64_t k) {
   auto prob = torch::empty({rows, k}, logits.options());
   FMOE_CUDA_CHECK(fmoe::launch_gate_topk_softmax(logit_code(logits), logits.data_ptr(), rows, ne,
                                                  static_cast<int>(k), idx.data_ptr<int64_t>(),
-                                                 prob.data_ptr(), cur_stream()));
+                                                 prob.data_ptr(), zero_of(zero), cur_stream()));
   return {idx, prob};
 }
 
@@ -888,8 +896,8 @@ bool gate_fused_supported(int64_t tot, int64_t d, int64_t k) {
 }
 
 // logits [B, tot], idx [B, k] and prob [B, k] of a linear gate in one pass over x.
-std::vector<torch::Tensor> gate_linear_topk(torch::Tensor x, torch::Tensor w,
-                                            c10::optional<torch::Tensor> bias, int64_t k, bool few) {
+std::vector<torch::Tensor> gate_forward(const torch::Tensor& x, const torch::Tensor& w,
+                                        const c10::optional<torch::Tensor>& bias, int64_t k, bool few, float* zero) {
   check_rows(x, "x");
   check_rows(w, "w");
   TORCH_CHECK(x.scalar_type() == w.scalar_type(), "gate input and weight dtypes differ");
@@ -903,8 +911,13 @@ std::vector<torch::Tensor> gate_linear_topk(torch::Tensor x, torch::Tensor w,
   FMOE_CUDA_CHECK((few ? fmoe::launch_gate_linear_topk_few : fmoe::launch_gate_linear_topk)(
       dtype16(x), x.data_ptr(), w.data_ptr(), bias.has_value() ? bias->data_ptr() : nullptr, rows, d,
       tot, static_cast<int>(k), logits.data_ptr(), idx.data_ptr<int64_t>(), prob.data_ptr(),
-      cur_stream()));
+      zero, cur_stream()));
   return {logits, idx, prob};
+}
+
+std::vector<torch::Tensor> gate_linear_topk(torch::Tensor x, torch::Tensor w, c10::optional<torch::Tensor> bias, int64_t k,
+                                            bool few, c10::optional<torch::Tensor> zero) {
+  return gate_forward(x, w, bias, k, few, zero_of(zero));
 }
 
 // Returns {dx or empty, dw (layer dtype), db or empty, dl fp32 [B, tot]}.
@@ -947,6 +960,84 @@ std::vector<torch::Tensor> gate_linear_topk_bwd(c10::optional<torch::Tensor> dpr
     if (need_db) db = dl.sum(0).to(x.scalar_type());
   }
   return {dx, dw, db, dl};
+}
+
+// ------------------------------------------------------------------------------ autograd nodes
+// The layer behind the gate and the linear gate as nodes of the native engine: their backward runs
+// without the interpreter, and a forward costs one call from Python.
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+class MoEMLP : public torch::autograd::Function<MoEMLP> {
+ public:
+  static torch::Tensor forward(AutogradContext* ctx, const torch::Tensor& x, const torch::Tensor& score,
+                               const torch::Tensor& w1, const torch::Tensor& b1, const torch::Tensor& w2,
+                               const torch::Tensor& b2, const torch::Tensor& idx, int64_t act, bool keep) {
+    auto r = moe_mlp_forward(x, idx, score, w1, b1, w2, b2, act, keep);
+    if (keep) ctx->save_for_backward({r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], w1, w2});
+    ctx->saved_data["act"] = act;
+    ctx->saved_data["shape"] = score.sizes().vec();
+    ctx->saved_data["dtype"] = static_cast<int64_t>(score.scalar_type());
+    return r[0];
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();   // xs, pre, a, ys, rank, offs, score, slots, w1, w2
+    const bool need_dx = ctx->needs_input_grad(0), need_score = ctx->needs_input_grad(1);
+    const bool need_w1 = ctx->needs_input_grad(2) || ctx->needs_input_grad(3);
+    const bool need_w2 = ctx->needs_input_grad(4) || ctx->needs_input_grad(5);
+    c10::optional<torch::Tensor> pre;
+    if (s[1].defined()) pre = s[1];
+    auto r = moe_mlp_backward(grads[0], s[0], pre, s[2], s[3], s[4], s[5], s[6], s[7], s[8], s[9],
+                              ctx->saved_data["act"].toInt(), need_dx, need_w1, need_w2);
+    torch::Tensor dscore;
+    if (need_score) {
+      dscore = r[1].to(static_cast<torch::ScalarType>(ctx->saved_data["dtype"].toInt()))
+                   .view(ctx->saved_data["shape"].toIntVector());
+    }
+    return {r[0], dscore, r[2], r[3], r[4], r[5], torch::Tensor(), torch::Tensor(), torch::Tensor()};
+  }
+};
+
+class GateLinearTopk : public torch::autograd::Function<GateLinearTopk> {
+ public:
+  static variable_list forward(AutogradContext* ctx, const torch::Tensor& x_in, const torch::Tensor& w_in,
+                               const c10::optional<torch::Tensor>& bias, int64_t k, int64_t zero) {
+    // `zero`: address of the caller's one-element tensor, which is not an input of the node
+    const torch::Tensor x = aligned(x_in, 16), w = aligned(w_in, 16);   // the kernels load 16 bytes at a time
+    auto r = gate_forward(x, w, bias, k, false, reinterpret_cast<float*>(zero));
+    ctx->save_for_backward({x, w, r[1], r[2]});
+    ctx->saved_data["bias"] = bias.has_value() && bias->defined();
+    ctx->mark_non_differentiable({r[1]});
+    ctx->set_materialize_grads(false);
+    return {r[0], r[1], r[2]};
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    if (!grads[0].defined() && !grads[2].defined()) return variable_list(5);
+    const variable_list s = ctx->get_saved_variables();
+    const bool has_bias = ctx->saved_data["bias"].toBool();
+    const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
+    const bool need_db = has_bias && ctx->needs_input_grad(2);
+    auto given = [](const torch::Tensor& g) {
+      return g.defined() ? c10::optional<torch::Tensor>(g.contiguous()) : c10::nullopt;
+    };
+    // (saved tensors may have been moved by hooks)
+    auto r = gate_linear_topk_bwd(given(grads[2]), s[2], s[3], given(grads[0]), aligned(s[0], 16), aligned(s[1], 16),
+                                  need_dx, need_db);
+    return {need_dx ? r[0] : torch::Tensor(), need_dw ? r[1] : torch::Tensor(), need_db ? r[2] : torch::Tensor(),
+            torch::Tensor(), torch::Tensor()};
+  }
+};
+
+torch::Tensor moe_mlp(torch::Tensor x, torch::Tensor score, torch::Tensor w1, torch::Tensor b1, torch::Tensor w2,
+                      torch::Tensor b2, torch::Tensor idx, int64_t act, bool keep) {
+  return MoEMLP::apply(x, score, w1, b1, w2, b2, idx, act, keep);
+}
+
+variable_list gate_linear_topk_node(torch::Tensor x, torch::Tensor w, c10::optional<torch::Tensor> bias, int64_t k,
+                                    c10::optional<torch::Tensor> zero) {
+  return GateLinearTopk::apply(x, w, bias, k, reinterpret_cast<int64_t>(zero_of(zero)));
 }
 
 // ------------------------------------------------------------------------------ status
@@ -1012,7 +1103,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_mlp_supported", &moe_mlp_supported);
   m.def("moe_mlp_forward", &moe_mlp_forward);
   m.def("moe_mlp_backward", &moe_mlp_backward);
-  m.def("gate_topk_softmax", &gate_topk_softmax);
+  m.def("gate_topk_softmax", &gate_topk_softmax, py::arg("logits"), py::arg("k"), py::arg("zero") = py::none());
+  m.def("moe_mlp", &moe_mlp);
+  m.def("gate_linear_topk_node", &gate_linear_topk_node, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("k"),
+        py::arg("zero") = py::none());
   m.def("gate_topk_softmax_bwd", &gate_topk_softmax_bwd);
   m.def("balance_supported", &balance_supported);
   m.def("prune_gate_scalar", &prune_gate_scalar);
@@ -1021,7 +1115,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("switch_top1", &switch_top1);
   m.def("gate_fused_supported", &gate_fused_supported);
   m.def("gate_linear_topk", &gate_linear_topk, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("k"),
-        py::arg("few") = false);
+        py::arg("few") = false, py::arg("zero") = py::none());
   m.def("gate_linear_topk_bwd", &gate_linear_topk_bwd);
   m.def("launch_count", []() { return g_launches.load(); });
   m.def("read_status", &read_status);

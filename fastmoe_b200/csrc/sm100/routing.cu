@@ -574,8 +574,9 @@ __device__ __noinline__ void topk_row(const T* in, int n_experts, int lane, int 
 // One warp per row.
 template <typename T>
 __global__ void gate_topk_softmax_kernel(const T* __restrict__ logits, int n_rows, int n_experts,
-                                         int k, int64_t* __restrict__ idx, T* __restrict__ prob) {
+                                         int k, int64_t* __restrict__ idx, T* __restrict__ prob, float* zero) {
   ptx::chain_begin();
+  if (zero != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0.f;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= n_rows) return;
@@ -825,7 +826,8 @@ template <typename T, int TOT>
 __global__ void __launch_bounds__(256)
 gate_linear_topk_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias,
                         int n_rows, int d, int tot, int k, T* __restrict__ logits,
-                        int64_t* __restrict__ idx, T* __restrict__ prob) {
+                        int64_t* __restrict__ idx, T* __restrict__ prob, float* zero) {
+  if (zero != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0.f;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= n_rows) return;
@@ -909,8 +911,9 @@ gate_linear_topk_kernel(const T* __restrict__ x, const T* __restrict__ w, const 
 template <typename T>
 __global__ void __launch_bounds__(256)
 gate_linear_topk_few_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, int d, int tot,
-                            int k, T* __restrict__ logits, int64_t* __restrict__ idx, T* __restrict__ prob) {
+                            int k, T* __restrict__ logits, int64_t* __restrict__ idx, T* __restrict__ prob, float* zero) {
   ptx::chain_begin();
+  if (zero != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0.f;
   __shared__ T row_logits[kGateMaxExperts];
   constexpr int PER = kGateMaxExperts / 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -976,8 +979,9 @@ template <typename T, int TOT, int R>
 __global__ void __launch_bounds__(256)
 gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias,
                              int n_rows, int d, int tot, int k, T* __restrict__ logits,
-                             int64_t* __restrict__ idx, T* __restrict__ prob) {
+                             int64_t* __restrict__ idx, T* __restrict__ prob, float* zero) {
   ptx::chain_begin();
+  if (zero != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0.f;
   constexpr int V = R * TOT;
   const int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R;
   const int lane = threadIdx.x & 31;
@@ -1671,7 +1675,7 @@ cudaError_t launch_colsum(int dtype, const void* x, const int* offs, int num_gro
 }
 
 cudaError_t launch_gate_topk_softmax(int logit_dtype, const void* logits, int n_rows, int n_experts,
-                                     int k, int64_t* idx, void* prob, cudaStream_t stream) {
+                                     int k, int64_t* idx, void* prob, float* zero, cudaStream_t stream) {
   cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
   if (k < 1 || k > kMaxK || k > n_experts) return cudaErrorInvalidValue;
@@ -1680,13 +1684,13 @@ cudaError_t launch_gate_topk_softmax(int logit_dtype, const void* logits, int n_
   if (logit_dtype == 0) {
     chained = launch_chained(gate_topk_softmax_kernel<__nv_bfloat16>, dim3(grid), dim3(wpb * 32), 0, stream,
         static_cast<const __nv_bfloat16*>(logits), n_rows, n_experts, k, idx,
-        static_cast<__nv_bfloat16*>(prob));
+        static_cast<__nv_bfloat16*>(prob), zero);
   } else if (logit_dtype == 1) {
     chained = launch_chained(gate_topk_softmax_kernel<__half>, dim3(grid), dim3(wpb * 32), 0, stream,
-        static_cast<const __half*>(logits), n_rows, n_experts, k, idx, static_cast<__half*>(prob));
+        static_cast<const __half*>(logits), n_rows, n_experts, k, idx, static_cast<__half*>(prob), zero);
   } else {
     chained = launch_chained(gate_topk_softmax_kernel<float>, dim3(grid), dim3(wpb * 32), 0, stream,
-        static_cast<const float*>(logits), n_rows, n_experts, k, idx, static_cast<float*>(prob));
+        static_cast<const float*>(logits), n_rows, n_experts, k, idx, static_cast<float*>(prob), zero);
   }
   return chained;
 }
@@ -1785,7 +1789,7 @@ int gate_rows_per_warp(int n_rows, int tot) {
 
 cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, const void* bias,
                                     int n_rows, int d, int tot, int k, void* logits, int64_t* idx,
-                                    void* prob, cudaStream_t stream) {
+                                    void* prob, float* zero, cudaStream_t stream) {
   cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
   if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
@@ -1794,7 +1798,7 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
 #define FMOE_GATE_ROWS(TOT, R)                                                                          \
   FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_linear_topk_rows_kernel<T, TOT, R>, dim3(grid), dim3(256), 0, stream,  \
       static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,  \
-      k, static_cast<T*>(logits), idx, static_cast<T*>(prob))))
+      k, static_cast<T*>(logits), idx, static_cast<T*>(prob), zero)))
   if (tot <= 8) {
     if (tot <= 2) {
       if (per == 1) { FMOE_GATE_ROWS(2, 1); } else if (per == 2) { FMOE_GATE_ROWS(2, 2); } else { FMOE_GATE_ROWS(2, 4); }
@@ -1811,7 +1815,7 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
 #define FMOE_GATE_WIDE(TOT)                                                                             \
   FMOE_DISPATCH_16(dtype, (gate_linear_topk_kernel<T, TOT><<<grid, 256, 0, stream>>>(                   \
       static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,  \
-      k, static_cast<T*>(logits), idx, static_cast<T*>(prob))))
+      k, static_cast<T*>(logits), idx, static_cast<T*>(prob), zero)))
   if (tot <= 16) {
     FMOE_GATE_WIDE(16);
   } else if (tot <= 32) {
@@ -1824,13 +1828,13 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
 }
 
 cudaError_t launch_gate_linear_topk_few(int dtype, const void* x, const void* w, const void* bias, int n_rows, int d,
-                                        int tot, int k, void* logits, int64_t* idx, void* prob, cudaStream_t stream) {
+                                        int tot, int k, void* logits, int64_t* idx, void* prob, float* zero, cudaStream_t stream) {
   cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
   if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
   FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_linear_topk_few_kernel<T>, dim3(n_rows), dim3(256), 0, stream,
       static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), d, tot, k,
-      static_cast<T*>(logits), idx, static_cast<T*>(prob))));
+      static_cast<T*>(logits), idx, static_cast<T*>(prob), zero)));
   return chained;
 }
 

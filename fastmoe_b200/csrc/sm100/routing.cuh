@@ -60,9 +60,10 @@ cudaError_t launch_colsum(int dtype, const void* x, const int* offs, int num_gro
                           int n, float* out, cudaStream_t stream);
 
 // Top-k of each logits row (descending) with softmax over the selected values.
-// logit_dtype: 0 bf16, 1 f16, 2 f32; prob has the dtype of the logits.
+// logit_dtype: 0 bf16, 1 f16, 2 f32; prob has the dtype of the logits.  `zero` (here and below,
+// optional) is set to 0 unless there are no rows.
 cudaError_t launch_gate_topk_softmax(int logit_dtype, const void* logits, int n_rows, int n_experts,
-                                     int k, int64_t* idx, void* prob, cudaStream_t stream);
+                                     int k, int64_t* idx, void* prob, float* zero, cudaStream_t stream);
 cudaError_t launch_gate_topk_softmax_bwd(int logit_dtype, const void* dprob, const int64_t* idx,
                                          const void* prob, int n_rows, int n_experts, int k,
                                          void* dlogits, cudaStream_t stream);
@@ -93,10 +94,11 @@ cudaError_t launch_prune_scalar(const int64_t* idx, const int* rank, int cap, in
 bool gate_fused_supported(int tot, int d, int k);
 cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, const void* bias,
                                     int n_rows, int d, int tot, int k, void* logits, int64_t* idx,
-                                    void* prob, cudaStream_t stream);
+                                    void* prob, float* zero, cudaStream_t stream);
 // The same result for a few tokens (one block each).
 cudaError_t launch_gate_linear_topk_few(int dtype, const void* x, const void* w, const void* bias, int n_rows, int d,
-                                        int tot, int k, void* logits, int64_t* idx, void* prob, cudaStream_t stream);
+                                        int tot, int k, void* logits, int64_t* idx, void* prob, float* zero,
+                                        cudaStream_t stream);
 // Backward of the fused gate.  dl_scratch: fp32 [n_rows, tot]; dx (optional) [n_rows, d].
 // part (optional, tot <= 16): fp32 scratch of gate_bwd_ranges() * (tot * d + tot) entries; with it
 // dw_db receives dW [tot, d] followed by db [tot] in the layer's type.  Above 16 experts pass

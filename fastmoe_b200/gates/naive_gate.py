@@ -19,15 +19,20 @@ class NaiveGate(BaseGate):
         self.gate = nn.Linear(d_model, self.tot_expert, bias=gate_bias)
         self.top_k = top_k
 
-    def _choose(self, inp):
+    def _choose(self, inp, zero=None):
+        linear = self.gate
         return gating.linear_topk_softmax(
-            inp.reshape(-1, inp.shape[-1]), self.gate.weight, self.gate.bias, self.top_k)
+            inp if inp.dim() == 2 else inp.reshape(-1, inp.shape[-1]), linear.weight, linear.bias, self.top_k, zero)
 
     def forward(self, inp, return_all_scores=False):
-        logits, idx, score = self._choose(inp)
-        logits = logits.view(*inp.shape[:-1], self.tot_expert)
         # The reference installs a zero "dummy" loss so that callers can always add it.
-        self.set_loss(torch.zeros(1, device=inp.device, requires_grad=True))
+        loss = torch.empty(1, device=inp.device)
+        if loss.dtype == torch.float32 and not loss.requires_grad:
+            logits, idx, score = self._choose(inp, loss)
+        else:
+            logits, idx, score = self._choose(inp)
+            loss.zero_()
+        self.set_loss(loss.requires_grad_(True))
         if return_all_scores:
-            return idx, score, logits
+            return idx, score, logits.view(*inp.shape[:-1], self.tot_expert)
         return idx, score

@@ -21,6 +21,7 @@ from torch.autograd import Function
 
 from . import grouped_gemm as gg
 from . import native
+from .gating import traced
 from .. import config
 from ..transformer import activation_kind, plain_experts
 from ..utils.profiling import check_routing, fused_range
@@ -249,7 +250,11 @@ class _MoEMLP(Function):
     r"""The whole single-GPU layer behind the gate as one node: :class:`_Dispatch`,
     :class:`_ExpertMLP` and :class:`_Combine` with their launches issued by one native call per
     direction.  With ``keep`` false (nothing will be differentiated) the pre-activation is not
-    written.  In fp32 ``xs`` and ``a`` are kept as the bf16 parts that the tensor cores multiply."""
+    written.  In fp32 ``xs`` and ``a`` are kept as the bf16 parts that the tensor cores multiply.
+
+    The native node of the same (``binding.cpp::MoEMLP``) takes all calls but traced ones: its backward
+    runs without the interpreter (a small layer's step, 512 tokens, d 256, 4 experts: 429 us of host time
+    with this class and the gate's, 262 with theirs)."""
 
     @staticmethod
     def forward(ctx, x, score, w1, b1, w2, b2, idx, act, keep):
@@ -297,7 +302,8 @@ def moe_mlp_forward(layer, x, gate_idx, gate_score):
         e = layer.experts
         args = (x, gate_score, e.htoh4.weight, e.htoh4.bias, e.h4toh.weight, e.h4toh.bias)
         keep = torch.is_grad_enabled() and any(t.requires_grad for t in args)
-        return _MoEMLP.apply(*args, gate_idx, gg.ACT_CODES[activation_kind(e.activation)], keep)
+        run = _MoEMLP.apply if traced() else nat.moe_mlp
+        return run(*args, gate_idx, gg.ACT_CODES[activation_kind(e.activation)], keep)
     k = gate_idx.shape[1]
     idx = gate_idx.contiguous().view(-1)
     score = gate_score.reshape(-1).to(x.dtype)

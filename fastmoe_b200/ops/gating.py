@@ -35,8 +35,8 @@ def _topk_softmax_torch(logits, k):
 
 class _TopkSoftmax(Function):
     @staticmethod
-    def forward(ctx, logits, k):
-        idx, score = native.get().gate_topk_softmax(logits.contiguous(), int(k))
+    def forward(ctx, logits, k, zero=None):
+        idx, score = native.get().gate_topk_softmax(logits.contiguous(), int(k), zero)
         ctx.save_for_backward(idx, score)
         ctx.shape = logits.shape
         ctx.mark_non_differentiable(idx)
@@ -47,7 +47,7 @@ class _TopkSoftmax(Function):
         idx, score = ctx.saved_tensors
         grad_logits = native.get().gate_topk_softmax_bwd(
             grad_score.contiguous(), idx, score, int(ctx.shape[-1]))
-        return grad_logits, None
+        return grad_logits, None, None
 
 
 def topk_softmax(logits, k):
@@ -59,7 +59,9 @@ def topk_softmax(logits, k):
 
 
 class _LinearTopkSoftmax(Function):
-    r"""``logits = x W^T + b``, top-k ids and softmax of the selected logits as one op."""
+    r"""``logits = x W^T + b``, top-k ids and softmax of the selected logits as one op.  The native node of
+    the same (``binding.cpp::GateLinearTopk``) takes all calls but those that are traced: a trace records
+    a Python function, and nothing of a native one."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, k):
@@ -85,6 +87,11 @@ class _LinearTopkSoftmax(Function):
             ctx.needs_input_grad[0], ctx.has_bias and ctx.needs_input_grad[2])
         return (dx if ctx.needs_input_grad[0] else None, dw if ctx.needs_input_grad[1] else None,
                 db if ctx.has_bias and ctx.needs_input_grad[2] else None, None)
+
+
+def traced():
+    r"""Whether ``torch.jit.trace`` watches."""
+    return torch._C._get_tracing_state() is not None   # pylint: disable=protected-access
 
 
 _PAD_BIAS = -30000.0   # bias of the padding columns: representable in bf16 and fp16, never selected
@@ -147,10 +154,11 @@ def _few_tokens_ok(x, weight, bias, k):
             and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype
             and (bias is None or bias.dtype == x.dtype)
             and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, weight, bias)))
-            and not torch.is_autocast_enabled() and native.get().gate_fused_supported(weight.shape[0], x.shape[1], k))
+            and not torch.is_autocast_enabled() and not traced()
+            and native.get().gate_fused_supported(weight.shape[0], x.shape[1], k))
 
 
-def linear_topk_softmax(x, weight, bias, k):
+def linear_topk_softmax(x, weight, bias, k, zero=None):
     r"""``(logits [B,E], idx int64 [B,k], prob [B,k])`` of a linear gate over 2-D ``x``.
 
     Uses the single-pass kernel when the shape allows it (16-bit types on a GPU, ``d_model`` a
@@ -160,25 +168,41 @@ def linear_topk_softmax(x, weight, bias, k):
     product runs on the tcgen05 grouped-GEMM kernel with a single group (:class:`_GateGemm`),
     followed by :func:`topk_softmax`, but for a few tokens without gradients (one launch); only 32-/64-bit inputs, CPU tensors and odd ``d_model``
     take the ``linear`` → :func:`topk_softmax` sequence of PyTorch ops.
+
+    ``zero``: a one-element fp32 tensor on ``x``'s device that is set to 0 on the way, by the gate's
+    kernel where there is one (a launch of its own took a fiftieth of a small decoding step).
     """
+    if zero is not None and (not x.is_cuda or x.shape[0] == 0):
+        zero.zero_()
+        zero = None
     if (x.is_cuda and x.dim() == 2 and x.dtype in (torch.bfloat16, torch.float16)
             and weight.shape[0] <= MAX_SINGLE_PASS_EXPERTS
             and weight.dtype == x.dtype and (bias is None or bias.dtype == x.dtype)
             and not torch.is_autocast_enabled()
             and native.get().gate_fused_supported(weight.shape[0], x.shape[1], k)):
         xc = x if x.is_contiguous() else x.contiguous()
-        return _LinearTopkSoftmax.apply(xc, weight.contiguous(), bias, k)
+        if traced():
+            if zero is not None:
+                zero.zero_()
+            return _LinearTopkSoftmax.apply(xc, weight.contiguous(), bias, k)
+        return tuple(native.get().gate_linear_topk_node(xc, weight.contiguous(), bias, int(k), zero))
     if _few_tokens_ok(x, weight, bias, k):
         x, weight = gg.aligned(x, 16), gg.aligned(weight, 16)
-        logits, idx, prob = native.get().gate_linear_topk(x, weight, None if bias is None else bias.contiguous(), int(k), True)
+        logits, idx, prob = native.get().gate_linear_topk(x, weight, None if bias is None else bias.contiguous(), int(k), True,
+                                                            zero)
         return logits, idx, prob
     if _gate_gemm_ok(x, weight, bias) and k <= MAX_FUSED_K:
         # more experts: tensor-core product on this library's own kernel, then the top-k /
         # softmax kernel over the (padded) logits
         tot = weight.shape[0]
         padded = _GateGemm.apply(x if x.is_contiguous() else x.contiguous(), weight, bias)
-        idx, prob = topk_softmax(padded, k)
+        if zero is not None and traced():
+            zero.zero_()
+            zero = None
+        idx, prob = _TopkSoftmax.apply(padded, k, zero)
         return padded[:, :tot], idx, prob
+    if zero is not None:
+        zero.zero_()
     logits = torch.nn.functional.linear(x, weight, bias)
     idx, prob = topk_softmax(logits, k)
     return logits, idx, prob

@@ -177,6 +177,8 @@ class FMoETransformerMLP(FMoE):
         return fused.moe_mlp_forward(self, moe_inp, gate_top_k_idx, gate_score)
 
     def forward(self, inp: torch.Tensor):
+        if inp.dim() == 2 and inp.shape[1] == self.d_model:
+            return super().forward(inp)
         original_shape = inp.shape
         out = super().forward(inp.reshape(-1, self.d_model))
         return out.reshape(original_shape)

@@ -327,3 +327,60 @@ def test_no_rows_leave_an_accumulated_gradient_alone():
     empty = [torch.empty(0, n, device=DEV, dtype=torch.bfloat16) for n in (64, 32)]
     assert (gg.wgrad(*empty, offs, 2, out=out, accumulate=True) == 1).all()
     assert not gg.wgrad(*empty, offs, 2, out=out).any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_native_nodes_as_the_python_ones(monkeypatch, dtype):
+    r"""The layer's and the gate's nodes of the native engine and those a trace records give the same bits:
+    all gradients, single ones, and with a gradient at the gate's scores and logits."""
+    from fastmoe_b200 import FMoETransformerMLP
+    from fastmoe_b200.ops import fused, gating
+    torch.manual_seed(0)
+    moe = FMoETransformerMLP(num_expert=4, d_model=64, d_hidden=128, top_k=2).to(DEV).to(dtype)
+    x0 = torch.randn(300, 64, device=DEV, dtype=dtype)
+    gy = torch.randn_like(x0)
+
+    def grads(wanted):
+        x = x0.clone().requires_grad_(True)
+        leaves = dict(moe.named_parameters(), x=x)
+        ids, score, logits = moe.gate(x, return_all_scores=True)
+        y = fused.moe_mlp_forward(moe, x, ids, score)
+        loss = (y * gy).float().sum() + score.float().square().sum() + logits.float().square().sum() + moe.gate.get_loss().sum()
+        return [y.detach()] + list(torch.autograd.grad(loss, [leaves[n] for n in wanted]))
+
+    names = [n for n, _ in moe.named_parameters()] + ["x"]
+    for wanted in [names] + [[n] for n in names]:
+        native_ones = grads(wanted)
+        with monkeypatch.context() as m:
+            m.setattr(fused, "traced", lambda: True)
+            m.setattr(gating, "traced", lambda: True)
+            python_ones = grads(wanted)
+        assert all(torch.equal(a, b) for a, b in zip(native_ones, python_ones))
+
+
+def test_traced_layer_follows_its_input():
+    from fastmoe_b200 import FMoETransformerMLP
+    torch.manual_seed(0)
+    for experts in (4, 16):
+        moe = FMoETransformerMLP(num_expert=experts, d_model=64, d_hidden=64, top_k=2).to(DEV).bfloat16().eval()
+        xs = [torch.randn(40, 64, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+        with torch.no_grad():
+            traced = torch.jit.trace(moe, xs[0], check_trace=False)
+            want = moe(xs[1])
+            if experts <= 8:
+                assert torch.equal(traced(xs[1]), want)
+            else:   # (traced, many experts keep the tensor-core gate: sums in another order)
+                assert torch.allclose(traced(xs[1]).float(), want.float(), atol=2e-2, rtol=2e-2)
+
+
+def test_native_nodes_refuse_what_the_python_ones_refuse():
+    from torch.autograd import forward_ad
+    from fastmoe_b200 import FMoETransformerMLP
+    moe = FMoETransformerMLP(num_expert=4, d_model=64, d_hidden=64, top_k=2).to(DEV).bfloat16()
+    x = torch.randn(16, 64, device=DEV, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError), forward_ad.dual_level():
+        moe(forward_ad.make_dual(x, torch.ones_like(x)))
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: moe(t).float().sum())(x)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(moe)(x.view(2, 8, 64))
