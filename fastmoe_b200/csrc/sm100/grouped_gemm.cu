@@ -1,10 +1,12 @@
 // Host side of the tcgen05 grouped GEMM: tensor-map construction and dispatch.  The kernels live
-// in pair_gemm_kernel.cuh (CTA pairs: most launches), grouped_gemm_kernel.cuh (row modes with rows
-// arriving from or leaving for other GPUs) — instantiated per element type in pair_gemm_*.cu /
-// grouped_gemm_*.cu — and narrow_gemm.cu (decoding).
+// in slim_gemm_kernel.cuh (CTA pairs, most row modes), pair_gemm_kernel.cuh (CTA pairs, weight
+// gradients), grouped_gemm_kernel.cuh (row modes with rows arriving from or leaving for other GPUs) —
+// instantiated per element type in slim_gemm_*.cu / pair_gemm_*.cu / grouped_gemm_*.cu — and
+// narrow_gemm.cu (decoding).
 #include "grouped_gemm_kernel.cuh"
 #include "narrow_gemm.cuh"
 #include "pair_gemm_kernel.cuh"
+#include "slim_gemm_kernel.cuh"
 #include "tensor_map.cuh"
 
 namespace fmoe {
@@ -34,13 +36,14 @@ EncodeTiledFn get_encode_fn() {
 
 bool encode(CUtensorMap* map, int dtype, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
             const cuuint32_t* box) {
+  const bool half_line = box[0] * 2 == 64;   // 32 columns: 64-byte swizzle
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return false;
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, dtype == kBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                       : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                   rank, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, half_line ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
@@ -63,6 +66,14 @@ bool make_map_3d(CUtensorMap* map, int dtype, const void* base, uint64_t inner, 
   return encode(map, dtype, base, 3, dims, strides, box);
 }
 
+bool make_map_columns(CUtensorMap* map, int dtype, const void* base, uint64_t inner, uint64_t outer, uint32_t box_outer,
+                      uint32_t box_blocks) {
+  cuuint64_t dims[3] = {64, outer, inner / 64};
+  cuuint64_t strides[2] = {inner * 2, 128};
+  cuuint32_t box[3] = {64, box_outer, box_blocks};
+  return encode(map, dtype, base, 3, dims, strides, box);
+}
+
 bool grouped_gemm_supported(int mode, int m, int n, int k, int num_groups) {
   if (num_groups < 1 || num_groups > MAX_GROUPS) return false;
   if (n % 32 != 0 || n < 32) return false;
@@ -72,20 +83,8 @@ bool grouped_gemm_supported(int mode, int m, int n, int k, int num_groups) {
 
 namespace {
 
-// The CTA-pair kernel takes the launches in which no rows arrive from or leave for other GPUs
-// (8192 rows, 2 experts, 1024 -> 4096 with GELU: 69.0 against 85.5 us; 22528 rows, 8 experts,
-// 512 -> 2048: 79.6 against 101.2 us; weight gradient of 64 experts with 128 rows: 200 against
-// 394 us).  The single-CTA kernel keeps the exchange, whose flags and send units count 128-row
-// blocks, and the launches with at most 16 rows per expert that narrow_applies leaves, where the
-// weights' bytes are most of the work and the finer tiles share them more evenly (a layer of 64
-// experts on 64 tokens: 227 against 238 us).
-bool pair_applies(const GroupedGemmArgs& a) {
-  if (a.mode == kWgrad) return true;
-  if (a.send.enabled || a.gate.flags != nullptr || a.push_meta != nullptr || a.trace != nullptr) return false;
-  if (a.rows_cap <= 16L * a.num_groups) return false;
-  if (a.mode == kRowsNT) return a.epi == kEpiBiasAct;
-  return a.bias == nullptr && a.pre_out == nullptr &&
-         (a.act == kActNone || (a.epi == kEpiDAct && a.aux != nullptr));
+bool exchanges(const GroupedGemmArgs& a) {
+  return a.send.enabled || a.gate.flags != nullptr || a.push_meta != nullptr || a.trace != nullptr;
 }
 
 // A handful of rows per expert and nothing saved for a backward: the weights' bytes are the work
@@ -94,8 +93,38 @@ bool pair_applies(const GroupedGemmArgs& a) {
 // two of 64 experts every 32-row tile reads the weights again, 43 against 19 us.
 bool narrow_applies(const GroupedGemmArgs& a) {
   return a.mode == kRowsNT && a.epi == kEpiBiasAct && a.pre_out == nullptr && a.rows_cap <= 256 &&
-         a.rows_cap <= 16L * a.num_groups &&
-         !a.send.enabled && a.gate.flags == nullptr && a.push_meta == nullptr && a.trace == nullptr;
+         a.rows_cap <= 16L * a.num_groups && !exchanges(a);
+}
+
+// The kernel with the token rows on the N side takes nearly all row modes without an exchange.  us, it
+// against the kernel of 256-row tiles, forward with GELU and saved pre-activation / forward without /
+// input gradient with the derivative / without: 1024 <-> 4096, 64 experts, 128 rows each: 122, 114, 117,
+// 110 against 133, 124, 133, 120; 8 experts, 64 rows each: 17.5, 24.6, 18.3, 24.5 against 22.6, 26.1,
+// 22.1, 25.7; 8 experts, 750 rows each: 54, 50, 56, 49 against 56, 53, 56, 52; 512 <-> 2048, 64 experts,
+// 64 rows each: 36, 32, 36, 32 against 55, 35, 54, 34.  With up to 16 rows per expert against the
+// single-CTA kernel: 512 <-> 2048, 8 experts: 7.7, -, 7.7, 13.7 against 15.6, -, 13.6, 16.0.
+// The others stay where they are better: with few rows per expert, no activation and more tiles than
+// pairs the single-CTA kernel shares the weights' bytes more evenly (64 experts, 4 rows each, 4096 ->
+// 1024: 94 against 82), and with many rows the derivative's chunks need not be transposed (2 experts,
+// 4096 rows each: 69.0 against 67.3; 4915 rows each: 81 against 78).
+bool slim_applies(const GroupedGemmArgs& a) {
+  if (a.mode == kWgrad || exchanges(a)) return false;
+  const bool plain = a.act == kActNone;
+  if (a.mode == kRowsNT ? a.epi != kEpiBiasAct
+                        : a.bias != nullptr || a.pre_out != nullptr || !(plain || (a.epi == kEpiDAct && a.aux != nullptr))) {
+    return false;
+  }
+  if (plain && a.rows_cap <= 16L * a.num_groups) {
+    return static_cast<long>(a.num_groups) * ((a.n + slim::TILE_N - 1) / slim::TILE_N) <= a.num_sms / 2;
+  }
+  return a.mode == kRowsNT || plain || a.rows_cap <= 512L * a.num_groups;
+}
+
+// The paired kernel of 256-row tiles: weight gradients, and the derivative of many rows.
+bool pair_applies(const GroupedGemmArgs& a) {
+  if (a.mode == kWgrad) return true;
+  return a.mode == kRowsNN && !exchanges(a) && a.rows_cap > 512L * a.num_groups && a.bias == nullptr &&
+         a.pre_out == nullptr && a.act != kActNone && a.epi == kEpiDAct && a.aux != nullptr;
 }
 
 template <typename P> void set_offsets(P& p, const GroupedGemmArgs& a) {
@@ -121,16 +150,45 @@ cudaError_t launch_narrow_gemm(const GroupedGemmArgs& a) {
   return ng::launch(a.dtype, a.act, tw, tx, p, a.num_sms > 0 ? a.num_sms : 148, a.stream);
 }
 
+cudaError_t launch_slim_gemm(const GroupedGemmArgs& a) {
+  slim::Maps m;
+  const uint64_t groups = a.num_groups;
+  const bool blocks = a.mode == kRowsNN && a.n % 64 == 0;
+  bool ok = make_map_3d(&m.c, a.dtype, a.out, a.n, a.rows_cap, 1, 32, 32);
+  if (a.mode == kRowsNT) {
+    ok = ok && make_map_2d(&m.w, a.dtype, a.b, a.k, groups * a.n, BK, slim::CTA_N);
+  } else if (blocks) {
+    ok = ok && make_map_columns(&m.w, a.dtype, a.b, a.n, groups * a.k, BK, 2);
+  } else {
+    ok = ok && make_map_2d(&m.w, a.dtype, a.b, a.n, groups * a.k, 64, BK);
+  }
+  for (int i = 0; i < slim::HALF_SIZES; ++i) {
+    ok = ok && make_map_2d(&m.x[i], a.dtype, a.a, a.k, a.rows_cap, BK, (i + 1) * slim::HALF_STEP);
+  }
+  if (!ok) return cudaErrorInvalidValue;
+  slim::Params p;
+  p.num_groups = a.num_groups;
+  p.n = a.n;
+  p.k = a.k;
+  p.w_blocks = blocks ? 1 : 0;
+  set_offsets(p, a);
+  p.out = a.out;
+  p.pre_out = a.pre_out;
+  p.bias = a.bias;
+  p.aux = a.aux;
+  p.status = a.status;
+  const int grid = (a.num_sms > 1 ? a.num_sms : 148) & ~1;
+  return a.dtype == kBF16 ? slim::launch_bf16(a.mode, a.act, m, p, grid, a.stream)
+                          : slim::launch_f16(a.mode, a.act, m, p, grid, a.stream);
+}
+
 cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
   CUtensorMap ta, tb, tc;
   // (an fp32 or accumulated gradient is not stored through the map)
   bool ok = a.mode == kWgrad ? make_map_3d(&tc, a.dtype, a.out, a.n, a.m, a.num_groups, 64, 32)
                              : make_map_3d(&tc, a.dtype, a.out, a.n, a.rows_cap, 1, 64, 32);
   if (!ok) return cudaErrorInvalidValue;
-  if (a.mode == kRowsNT) {
-    ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, pg::CTA_M) &&
-         make_map_2d(&tb, a.dtype, a.b, a.k, static_cast<uint64_t>(a.num_groups) * a.n, BK, pg::CTA_N);
-  } else if (a.mode == kRowsNN) {
+  if (a.mode == kRowsNN) {
     ok = make_map_2d(&ta, a.dtype, a.a, a.k, a.rows_cap, BK, pg::CTA_M) &&
          make_map_2d(&tb, a.dtype, a.b, a.n, static_cast<uint64_t>(a.num_groups) * a.k, 64, BK);
   } else {
@@ -145,8 +203,6 @@ cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
   p.k = a.k;
   set_offsets(p, a);
   p.out = a.out;
-  p.pre_out = a.pre_out;
-  p.bias = a.bias;
   p.aux = a.aux;
   p.accumulate = a.accumulate;
   p.out_fp32 = a.out_fp32;
@@ -172,6 +228,7 @@ cudaError_t launch_grouped_gemm(const GroupedGemmArgs& a) {
     return cudaMemsetAsync(a.psum, 0, width * 2, a.stream);
   }
   if (narrow_applies(a)) return launch_narrow_gemm(a);
+  if (slim_applies(a)) return launch_slim_gemm(a);
   if (pair_applies(a)) return launch_pair_gemm(a);
   CUtensorMap ta, tb;
   bool ok = true;

@@ -1,7 +1,7 @@
 // Grouped GEMM on the 5th-generation tensor cores (tcgen05) for the expert linears: the row modes
 // (forward and input gradient) whose rows arrive from or leave for other GPUs inside the launch.
-// The weight gradient and nearly all launches without an exchange run in pair_gemm_kernel.cuh and
-// narrow_gemm.cu (grouped_gemm.cu has the rule).
+// Nearly all launches without an exchange run in slim_gemm_kernel.cuh, pair_gemm_kernel.cuh (weight
+// gradients) and narrow_gemm.cu (grouped_gemm.cu has the rule).
 //
 // Replaces the reference's host loop of one cuBLAS call per expert with stream
 // synchronisations around it (cuda/parallel_linear.cuh:56-163): one persistent kernel covers

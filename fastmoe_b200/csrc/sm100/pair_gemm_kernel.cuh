@@ -1,12 +1,12 @@
-// Grouped GEMM on CTA pairs (tcgen05 cta_group::2): the launches in which no rows arrive from or
-// leave for other GPUs.
+// Grouped GEMM on CTA pairs (tcgen05 cta_group::2) with 256 x 256 tiles: weight gradients, and input
+// gradients of many rows that apply an activation's derivative (the other row modes without an
+// exchange: slim_gemm_kernel.cuh).
 //
 // A pair of CTAs (one cluster, two neighbouring SMs) works on a 256 x 256 output tile: CTA r
 // holds rows [128 r, 128 r + 128) of A, columns [128 r, 128 r + 128) of B and the accumulators of
 // its rows.  Per 64-wide K block an SM loads 32 KB where a 128 x 256 tile on one SM loads 48 KB.
-// Measured, bf16, 8192 rows, 2 experts, 1024 <-> 4096: forward 68.0 (GELU, saved pre-activation)
-// and 52.5 us, input gradient 69.0 and 51.8 us, weight gradient 63.5 us (1080 to 1327 TFLOP/s
-// without activation), where the single-CTA kernel took 85.5, 56.0, 78.4, 54.5 and 70.1 us.  What
+// Measured, bf16, 8192 rows, 2 experts, 1024 <-> 4096: input gradient with GELU's derivative 67.3 us,
+// weight gradient 63.5 us (1080 TFLOP/s), where the single-CTA kernel took 78.4 and 70.1 us.  What
 // bounds it: the last of the waves (128 tiles on 74 pairs) and, with an activation, the epilogue.
 //
 // Roles of a CTA (384 threads), persistent over the tiles of its pair:
@@ -61,14 +61,12 @@ struct Shared {
   int abort;
   int offs[MAX_GROUPS + 1];
   int tiles[MAX_GROUPS + 1];    // exclusive prefix of the 256 x 256 tiles
-  int blocks[MAX_GROUPS + 1];   // row modes: exclusive prefix of the 128-row blocks
+  int blocks[MAX_GROUPS + 1];   // input gradient: exclusive prefix of the 128-row blocks
 };
 
 constexpr int PATCH_BYTES = gg::PATCH_BYTES;
-constexpr int BIAS_BYTES = EPI_COLS * 2;
 constexpr int PATCH_OFF = STAGES * STAGE_BYTES;
-constexpr int BIAS_OFF = PATCH_OFF + NUM_EPI_WARPS * PATCH_BYTES;
-constexpr int AUX_OFF = BIAS_OFF + NUM_EPI_WARPS * BIAS_BYTES;
+constexpr int AUX_OFF = PATCH_OFF + NUM_EPI_WARPS * PATCH_BYTES;
 constexpr int SMEM_BYTES = AUX_OFF + static_cast<int>(sizeof(Shared)) + 1024;
 static_assert(SMEM_BYTES <= 232448, "shared memory");
 
@@ -76,12 +74,10 @@ struct Params {
   int num_groups;
   int m;   // weight gradient only
   int n;
-  int k;   // row modes only
+  int k;   // input gradient only
   const int* offs;       // null: `one_group` instead
   int one_group[2];
   void* out;
-  void* pre_out;
-  const void* bias;
   const void* aux;
   int accumulate;
   int out_fp32;
@@ -214,16 +210,15 @@ struct EpiTile {
   int n_chunks;             // valid 32-column chunks of the span (0..4)
   int warp_valid;           // valid rows of the warp's 32
   uint8_t* patch;
-  const uint8_t* bias;      // shared memory: the span's bias values, or null
   uint8_t* out;             // first row, first column of the span
   long out_pitch;
-  uint8_t* pre_tile;        // this warp's 4 x 2 KB of the tile-blocked pre-activation, or null
+  const uint8_t* pre_tile;  // DACT: this warp's 4 x 2 KB of the tile-blocked pre-activation
   uint32_t empty_bar;       // CTA 0's accumulator-free barrier
   const CUtensorMap* map;   // output, boxes of 32 rows x 64 columns; null: not all 32 rows may be written
   int x, y, z;              // first column, row and matrix of the span there
 };
 
-// Bias / activation, or activation derivative (DACT), of one 32-column chunk into the patch.
+// One 32-column chunk, multiplied by the activation's derivative (DACT), into the patch.
 template <typename T, int ACT, bool DACT>
 __device__ __forceinline__ void finish_chunk(const EpiTile& et, int i, const uint32_t (&r)[32], const Packed32& side) {
 #pragma unroll
@@ -231,14 +226,6 @@ __device__ __forceinline__ void finish_chunk(const EpiTile& et, int i, const uin
     ptx::f32x2 v[PAIRS];
 #pragma unroll
     for (int j = 0; j < PAIRS; ++j) v[j] = ptx::pack2(__uint_as_float(r[q * 16 + 2 * j]), __uint_as_float(r[q * 16 + 2 * j + 1]));
-    auto packed = [&](uint32_t (&w)[PAIRS]) {
-#pragma unroll
-      for (int j = 0; j < PAIRS; ++j) {
-        float a, b;
-        ptx::unpack2(v[j], a, b);
-        w[j] = Cvt<T>::pack(a, b);
-      }
-    };
     if (DACT) {
       ptx::f32x2 x[PAIRS];
 #pragma unroll
@@ -248,31 +235,14 @@ __device__ __forceinline__ void finish_chunk(const EpiTile& et, int i, const uin
         x[j] = ptx::pack2(a, b);
       }
       act_grad_pairs<ACT>(x, v);
-    } else {
-      if (et.bias != nullptr) {
-        const uint4 b0 = *reinterpret_cast<const uint4*>(et.bias + i * 64 + q * 32);
-        const uint4 b1 = *reinterpret_cast<const uint4*>(et.bias + i * 64 + q * 32 + 16);
-        const uint32_t bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-        for (int j = 0; j < PAIRS; ++j) {
-          float a, b;
-          Cvt<T>::unpack(bw[j], a, b);
-          v[j] = ptx::add2(v[j], ptx::pack2(a, b));
-        }
-      }
-      if (ACT != kActNone) {
-        if (et.pre_tile != nullptr) {
-          uint32_t wp[PAIRS];
-          packed(wp);
-          uint8_t* pd = et.pre_tile + i * gg::PRE_CHUNK_BYTES + et.lane * 16 + q * 1024;
-          *reinterpret_cast<uint4*>(pd) = make_uint4(wp[0], wp[1], wp[2], wp[3]);
-          *reinterpret_cast<uint4*>(pd + 512) = make_uint4(wp[4], wp[5], wp[6], wp[7]);
-        }
-        act_pairs<ACT>(v);
-      }
     }
     uint32_t wo[PAIRS];
-    packed(wo);
+#pragma unroll
+    for (int j = 0; j < PAIRS; ++j) {
+      float a, b;
+      ptx::unpack2(v[j], a, b);
+      wo[j] = Cvt<T>::pack(a, b);
+    }
     const int c = (i & 1) * 4 + q * 2;
     *reinterpret_cast<uint4*>(gg::patch_piece(et.patch, et.lane, c)) = make_uint4(wo[0], wo[1], wo[2], wo[3]);
     *reinterpret_cast<uint4*>(gg::patch_piece(et.patch, et.lane, c + 1)) = make_uint4(wo[4], wo[5], wo[6], wo[7]);
@@ -570,10 +540,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           } else {
             const uint32_t bar = ptx::mapa(&sh->full[stage], 0);
             ptx::mbar_arrive_expect_tx_cluster(bar, STAGE_BYTES);
-            if (MODE == kRowsNT) {
-              ptx::tma_load_2d_pair(sa, &tm_a, bar, kb * BK, c.row_begin + m0);
-              ptx::tma_load_2d_pair(sb, &tm_b, bar, kb * BK, c.group * p.n + n0);
-            } else if (MODE == kRowsNN) {
+            if (MODE == kRowsNN) {
               ptx::tma_load_2d_pair(sa, &tm_a, bar, kb * BK, c.row_begin + m0);
 #pragma unroll
               for (int ch = 0; ch < CTA_N / 64; ++ch) {
@@ -595,7 +562,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // ============================================================== MMA issuer (CTA 0)
     if (rank == 0 && lane == 0) {
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
-      constexpr uint32_t idesc = ptx::make_idesc(kBf16, MODE == kWgrad, MODE != kRowsNT, TILE_M, TILE_N);
+      constexpr uint32_t idesc = ptx::make_idesc(kBf16, MODE == kWgrad, true, TILE_M, TILE_N);
       int stage = 0;
       uint32_t phase = 0;
       int iter = 0;
@@ -631,9 +598,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const uint64_t a_desc = (MODE == kWgrad)
                 ? ptx::make_smem_desc_sw128(sa + k16 * (UMMA_K * 128), BOX_BYTES, 1024)
                 : ptx::make_smem_desc_sw128(sa + k16 * (UMMA_K * 2), 16, 1024);
-            const uint64_t b_desc = (MODE == kRowsNT)
-                ? ptx::make_smem_desc_sw128(sb + k16 * (UMMA_K * 2), 16, 1024)
-                : ptx::make_smem_desc_sw128(sb + k16 * (UMMA_K * 128), BOX_BYTES, 1024);
+            const uint64_t b_desc = ptx::make_smem_desc_sw128(sb + k16 * (UMMA_K * 128), BOX_BYTES, 1024);
             ptx::umma_f16_pair(d_tmem, a_desc, b_desc, idesc, (kb | k16) != 0 ? 1u : 0u);
           }
           ptx::umma_commit_pair(&sh->empty[stage]);
@@ -704,20 +669,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     const int half = (warp - FIRST_EPI_WARP) >> 2;   // which half of the accumulator columns
     const int ew = warp - FIRST_EPI_WARP;
     uint8_t* patches = smem + PATCH_OFF;
-    uint8_t* bias_sm = smem + BIAS_OFF + ew * BIAS_BYTES;
-    const bool has_bias = MODE == kRowsNT && p.bias != nullptr;
-    // this lane's four bias values of a tile, loaded one tile ahead
-    auto load_bias = [&](int tile) -> uint2 {
-      uint2 v = make_uint2(0u, 0u);
-      if (has_bias && tile < total) {
-        int ahead = group;
-        const Tile c = decode(sh, n_tiles, tile, ahead);
-        const int col = c.n_tile * TILE_N + half * EPI_COLS + lane * 4;
-        if (col < p.n) v = __ldg(reinterpret_cast<const uint2*>(static_cast<const T*>(p.bias) + static_cast<long>(c.group) * p.n + col));
-      }
-      return v;
-    };
-    uint2 bias_next = load_bias(pair);
     int iter = 0;
     bool dead = false;   // a wait ran out: walk the remaining tiles' barriers, touch nothing else
     for (int tile = pair; tile < total; tile += num_pairs, ++iter) {
@@ -730,7 +681,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       et.n_chunks = max(0, min(EPI_CHUNKS, (p.n - col_first) / 32));
       et.warp_valid = max(0, min(32, ((MODE == kWgrad) ? p.m : c.rows) - m0));
       et.patch = patches + ew * PATCH_BYTES;
-      et.bias = has_bias ? bias_sm : nullptr;
       et.out_pitch = static_cast<long>(p.n) * 2;
       et.pre_tile = nullptr;
       et.empty_bar = ptx::mapa(&sh->tmem_empty[acc], 0);
@@ -748,33 +698,24 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           column_sums<T>(p, patches, c, c.m_tile * TILE_M + rank * CTA_M, warp, lane);
         }
       } else {
-        const void* pre = (MODE == kRowsNN) ? p.aux : p.pre_out;
-        if (ACT != kActNone && pre != nullptr) {
-          // the tile-blocked layout counts 128 x 256 blocks, groups in order
-          const long blk = (static_cast<long>(sh->blocks[c.group]) + c.m_tile * 2 + rank) * n_tiles + c.n_tile;
-          et.pre_tile = const_cast<uint8_t*>(static_cast<const uint8_t*>(pre)) + blk * gg::PRE_TILE_BYTES +
-                        ew * (gg::CHUNKS_PER_WARP * gg::PRE_CHUNK_BYTES);
-          if (MODE == kRowsNN && et.n_chunks > 0 && et.warp_valid > 0) {
-            // it does not depend on the accumulator: fetch the first chunk before the wait, and
-            // pull the next tile's chunks of this warp (8 KB, two lines per lane) into L2
-            gg::load_pre_chunk(et.pre_tile, 0, lane, side);
-            if (tile + num_pairs < total) {
-              int ahead = group;
-              const Tile cn = decode(sh, n_tiles, tile + num_pairs, ahead);
-              if (cn.m_tile * TILE_M + rank * CTA_M < cn.rows) {
-                const long nb = (static_cast<long>(sh->blocks[cn.group]) + cn.m_tile * 2 + rank) * n_tiles + cn.n_tile;
-                const uint8_t* nx = static_cast<const uint8_t*>(pre) + nb * gg::PRE_TILE_BYTES +
-                                    ew * (gg::CHUNKS_PER_WARP * gg::PRE_CHUNK_BYTES) + lane * 256;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + 128));
-              }
+        // the tile-blocked layout counts 128 x 256 blocks, groups in order
+        const long blk = (static_cast<long>(sh->blocks[c.group]) + c.m_tile * 2 + rank) * n_tiles + c.n_tile;
+        et.pre_tile = static_cast<const uint8_t*>(p.aux) + blk * gg::PRE_TILE_BYTES + ew * (gg::CHUNKS_PER_WARP * gg::PRE_CHUNK_BYTES);
+        if (et.n_chunks > 0 && et.warp_valid > 0) {
+          // it does not depend on the accumulator: fetch the first chunk before the wait, and
+          // pull the next tile's chunks of this warp (8 KB, two lines per lane) into L2
+          gg::load_pre_chunk(et.pre_tile, 0, lane, side);
+          if (tile + num_pairs < total) {
+            int ahead = group;
+            const Tile cn = decode(sh, n_tiles, tile + num_pairs, ahead);
+            if (cn.m_tile * TILE_M + rank * CTA_M < cn.rows) {
+              const long nb = (static_cast<long>(sh->blocks[cn.group]) + cn.m_tile * 2 + rank) * n_tiles + cn.n_tile;
+              const uint8_t* nx = static_cast<const uint8_t*>(p.aux) + nb * gg::PRE_TILE_BYTES +
+                                  ew * (gg::CHUNKS_PER_WARP * gg::PRE_CHUNK_BYTES) + lane * 256;
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(nx));
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + 128));
             }
           }
-        }
-        if (has_bias) {
-          *reinterpret_cast<uint2*>(bias_sm + lane * 8) = bias_next;
-          __syncwarp();
-          bias_next = load_bias(tile + num_pairs);
         }
       }
       if (dead) continue;
@@ -790,7 +731,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if (MODE == kWgrad && (p.out_fp32 || p.accumulate)) {
         epilogue_tile_update<T>(p, et, first_elem);
       } else {
-        epilogue_tile<T, ACT, MODE == kRowsNN && ACT != kActNone>(et, side);
+        epilogue_tile<T, ACT, MODE == kRowsNN>(et, side);
       }
       __syncwarp();
     }
@@ -832,25 +773,16 @@ cudaError_t launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   return launch_chained(kernel, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, ta, tb, tc, p);
 }
 
-template <int MODE, typename T>
-cudaError_t launch_act(int act, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, int grid,
-                       cudaStream_t stream) {
-  switch (act) {
-    case kActRelu: return launch_one<MODE, T, kActRelu>(ta, tb, tc, p, grid, stream);
-    case kActGelu: return launch_one<MODE, T, kActGelu>(ta, tb, tc, p, grid, stream);
-    case kActGeluTanh: return launch_one<MODE, T, kActGeluTanh>(ta, tb, tc, p, grid, stream);
-    default: return launch_one<MODE, T, kActNone>(ta, tb, tc, p, grid, stream);
-  }
-}
-
 // One translation unit per element type instantiates this.
 template <typename T>
-cudaError_t launch_for_type(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, int grid,
-                            cudaStream_t stream) {
-  switch (mode) {
-    case kRowsNT: return launch_act<kRowsNT, T>(act, ta, tb, tc, p, grid, stream);
-    case kRowsNN: return launch_act<kRowsNN, T>(act, ta, tb, tc, p, grid, stream);
-    default: return launch_one<kWgrad, T, kActNone>(ta, tb, tc, p, grid, stream);
+cudaError_t launch_for_type(int mode, int act, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p,
+                            int grid, cudaStream_t stream) {
+  if (mode == kWgrad) return launch_one<kWgrad, T, kActNone>(ta, tb, tc, p, grid, stream);
+  switch (act) {
+    case kActRelu: return launch_one<kRowsNN, T, kActRelu>(ta, tb, tc, p, grid, stream);
+    case kActGelu: return launch_one<kRowsNN, T, kActGelu>(ta, tb, tc, p, grid, stream);
+    case kActGeluTanh: return launch_one<kRowsNN, T, kActGeluTanh>(ta, tb, tc, p, grid, stream);
+    default: return cudaErrorInvalidValue;
   }
 }
 
