@@ -1019,6 +1019,11 @@ class GateLinearTopk : public torch::autograd::Function<GateLinearTopk> {
     const bool has_bias = ctx->saved_data["bias"].toBool();
     const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
     const bool need_db = has_bias && ctx->needs_input_grad(2);
+    if (at::GradMode::is_enabled() && !grads[2].defined()) {
+      // a gradient of the gradient is wanted: the linear's, in operations that have one
+      return {need_dx ? grads[0].matmul(s[1]) : torch::Tensor(), need_dw ? grads[0].t().matmul(s[0]) : torch::Tensor(),
+              need_db ? grads[0].sum(0) : torch::Tensor(), torch::Tensor(), torch::Tensor()};
+    }
     auto given = [](const torch::Tensor& g) {
       return g.defined() ? c10::optional<torch::Tensor>(g.contiguous()) : c10::nullopt;
     };

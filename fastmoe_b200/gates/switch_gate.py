@@ -64,7 +64,8 @@ class SwitchGate(NaiveGate):
         return type(self)._balance_loss is SwitchGate._balance_loss and "_balance_loss" not in vars(self)
 
     def forward(self, inp):
-        logits = self._jitter(self.gate(inp))
+        logits = gating.linear_logits(inp, self.gate)
+        logits = self._jitter(self.gate(inp) if logits is None else logits)
         cap = self._slots_per_expert(inp.shape[0])
         if (self.world_size == 1 and logits.dtype == inp.dtype and gating.balance_native(logits)
                 and self._usual_loss() and forward_ad.unpack_dual(logits).tangent is None):

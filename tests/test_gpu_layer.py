@@ -384,3 +384,31 @@ def test_native_nodes_refuse_what_the_python_ones_refuse():
         torch.func.grad(lambda t: moe(t).float().sum())(x)
     with pytest.raises(RuntimeError):
         torch.func.vmap(moe)(x.view(2, 8, 64))
+
+
+def test_switch_gate_linear_is_the_kernel_only_when_nobody_looks():
+    from fastmoe_b200.gates import SwitchGate
+    from fastmoe_b200.ops import gating
+    gate = SwitchGate(64, 4, 1, switch_eps=0.0).to(DEV).bfloat16()
+    x = torch.randn(32, 64, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    logits = gating.linear_logits(x, gate.gate)
+    assert torch.allclose(logits.float(), gate.gate(x).float(), atol=2e-2)
+    seen = []
+    handle = gate.gate.register_forward_hook(lambda *_: seen.append(1))
+    assert gating.linear_logits(x, gate.gate) is None
+    gate(x)
+    assert seen
+    handle.remove()
+    # a gradient of the gradient, as of the linear
+    results = []
+    for fused in (True, False):
+        p = [t.detach().clone().requires_grad_(True) for t in (x, gate.gate.weight, gate.gate.bias)]
+        linear = torch.nn.Linear(64, 4).to(DEV).bfloat16()
+        linear.weight, linear.bias = torch.nn.Parameter(p[1]), torch.nn.Parameter(p[2])
+        leaves = [p[0], linear.weight, linear.bias]
+        out = gating.linear_logits(p[0], linear) if fused else linear(p[0])
+        first = torch.autograd.grad(out.float().square().sum(), leaves, create_graph=True)
+        second = torch.autograd.grad(sum(g.float().square().sum() for g in first), leaves)
+        results.append([t.detach().float() for t in first + second])
+    for a, b in zip(*results):
+        assert float((a - b).norm()) <= 2e-2 * float(b.norm())
