@@ -901,6 +901,11 @@ std::vector<torch::Tensor> gate_forward(const torch::Tensor& x, const torch::Ten
   check_rows(x, "x");
   check_rows(w, "w");
   TORCH_CHECK(x.scalar_type() == w.scalar_type(), "gate input and weight dtypes differ");
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && x.device() == w.device(),
+              "gate input and weight do not fit");
+  const torch::Tensor b = bias.has_value() && bias->defined() ? bias->contiguous() : torch::Tensor();
+  TORCH_CHECK(!b.defined() || (b.device() == x.device() && b.scalar_type() == x.scalar_type() && b.numel() == w.size(0)),
+              "gate bias does not fit");
   c10::cuda::CUDAGuard guard(x.device());
   const int rows = static_cast<int>(x.size(0));
   const int d = static_cast<int>(x.size(1));
@@ -909,7 +914,7 @@ std::vector<torch::Tensor> gate_forward(const torch::Tensor& x, const torch::Ten
   auto idx = torch::empty({rows, k}, torch::dtype(torch::kLong).device(x.device()));
   auto prob = torch::empty({rows, k}, x.options());
   FMOE_CUDA_CHECK((few ? fmoe::launch_gate_linear_topk_few : fmoe::launch_gate_linear_topk)(
-      dtype16(x), x.data_ptr(), w.data_ptr(), bias.has_value() ? bias->data_ptr() : nullptr, rows, d,
+      logit_code(x), x.data_ptr(), w.data_ptr(), b.defined() ? b.data_ptr() : nullptr, rows, d,
       tot, static_cast<int>(k), logits.data_ptr(), idx.data_ptr<int64_t>(), prob.data_ptr(),
       zero, cur_stream()));
   return {logits, idx, prob};
@@ -942,10 +947,10 @@ std::vector<torch::Tensor> gate_linear_topk_bwd(c10::optional<torch::Tensor> dpr
     const long elems = static_cast<long>(tot) * d + tot;
     // without rows nothing is launched: the sums over no tokens are zero
     dw_db = rows > 0 ? torch::empty({elems}, x.options()) : torch::zeros({elems}, x.options());
-    part = torch::empty({fmoe::gate_bwd_ranges(rows, d) * elems}, f32);
+    part = torch::empty({fmoe::gate_bwd_ranges(logit_code(x), rows, d) * elems}, f32);
   }
   FMOE_CUDA_CHECK(fmoe::launch_gate_bwd(
-      dtype16(x), dprob.has_value() ? dprob->data_ptr() : nullptr, idx.data_ptr<int64_t>(),
+      logit_code(x), dprob.has_value() ? dprob->data_ptr() : nullptr, idx.data_ptr<int64_t>(),
       prob.data_ptr(), dlogits.has_value() ? dlogits->data_ptr() : nullptr, x.data_ptr(),
       w.data_ptr(), rows, d, tot, k, dl.data_ptr<float>(), need_dx ? dx.data_ptr() : nullptr,
       fused_dw ? part.data_ptr<float>() : nullptr, fused_dw ? dw_db.data_ptr() : nullptr, cur_stream()));
@@ -1019,10 +1024,16 @@ class GateLinearTopk : public torch::autograd::Function<GateLinearTopk> {
     const bool has_bias = ctx->saved_data["bias"].toBool();
     const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
     const bool need_db = has_bias && ctx->needs_input_grad(2);
-    if (at::GradMode::is_enabled() && !grads[2].defined()) {
-      // a gradient of the gradient is wanted: the linear's, in operations that have one
-      return {need_dx ? grads[0].matmul(s[1]) : torch::Tensor(), need_dw ? grads[0].t().matmul(s[0]) : torch::Tensor(),
-              need_db ? grads[0].sum(0) : torch::Tensor(), torch::Tensor(), torch::Tensor()};
+    if (at::GradMode::is_enabled() && (!grads[2].defined() || s[0].scalar_type() == torch::kFloat)) {
+      // a gradient of the gradient is wanted: the linear's, in operations that have one (the scores'
+      // counts as a constant)
+      torch::Tensor dl = grads[0];
+      if (grads[2].defined()) {
+        auto through = gate_topk_softmax_bwd(grads[2].contiguous(), s[2], s[3], s[1].size(0));
+        dl = dl.defined() ? dl + through : through;
+      }
+      return {need_dx ? dl.matmul(s[1]) : torch::Tensor(), need_dw ? dl.t().matmul(s[0]) : torch::Tensor(),
+              need_db ? dl.sum(0) : torch::Tensor(), torch::Tensor(), torch::Tensor()};
     }
     auto given = [](const torch::Tensor& g) {
       return g.defined() ? c10::optional<torch::Tensor>(g.contiguous()) : c10::nullopt;

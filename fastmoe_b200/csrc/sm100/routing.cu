@@ -247,6 +247,10 @@ template <> struct V2<__half> {
   static __device__ __forceinline__ float to_f(__half v) { return __half2float(v); }
   static __device__ __forceinline__ __half from_f(float v) { return __float2half(v); }
 };
+template <> struct V2<float> {
+  static __device__ __forceinline__ float to_f(float v) { return v; }
+  static __device__ __forceinline__ float from_f(float v) { return v; }
+};
 
 template <typename T>
 __device__ __forceinline__ void unpack8(const uint4& w, float (&f)[8]) {
@@ -267,6 +271,28 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) p[i] = V2<T>::from_f2(f[2 * i], f[2 * i + 1]);
   return w;
+}
+
+// The values of one 16-byte load: eight of 16 bits, four of 32.
+template <typename T> constexpr int kPer16 = 16 / static_cast<int>(sizeof(T));
+template <typename T>
+__device__ __forceinline__ void unpack16(const uint4& w, float (&f)[kPer16<T>]) {
+  if constexpr (sizeof(T) == 4) {
+    f[0] = __uint_as_float(w.x);
+    f[1] = __uint_as_float(w.y);
+    f[2] = __uint_as_float(w.z);
+    f[3] = __uint_as_float(w.w);
+  } else {
+    unpack8<T>(w, f);
+  }
+}
+template <typename T>
+__device__ __forceinline__ uint4 pack16(const float (&f)[kPer16<T>]) {
+  if constexpr (sizeof(T) == 4) {
+    return make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+  } else {
+    return pack8<T>(f);
+  }
 }
 
 // One warp per slot; d % 8 == 0.
@@ -989,7 +1015,8 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
   float acc[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) acc[v] = 0.f;
-  const int nv = d >> 3;
+  constexpr int W = kPer16<T>;
+  const int nv = d / W;
   const uint4* xr[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) xr[r] = reinterpret_cast<const uint4*>(x + static_cast<long>(min(row0 + r, n_rows - 1)) * d);
@@ -1004,17 +1031,17 @@ gate_linear_topk_rows_kernel(const T* __restrict__ x, const T* __restrict__ w, c
       // (past the last expert the last one again, for nothing: the loads need no predicate)
       wv[e] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(min(e, tot - 1)) * d) + i);
     }
-    float xf[R][8];
+    float xf[R][W];
 #pragma unroll
-    for (int r = 0; r < R; ++r) unpack8<T>(xv[r], xf[r]);
+    for (int r = 0; r < R; ++r) unpack16<T>(xv[r], xf[r]);
 #pragma unroll
     for (int e = 0; e < TOT; ++e) {
-      float wf[8];
-      unpack8<T>(wv[e], wf);
+      float wf[W];
+      unpack16<T>(wv[e], wf);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc[r * TOT + e] = fmaf(xf[r][q], wf[q], acc[r * TOT + e]);
+        for (int q = 0; q < W; ++q) acc[r * TOT + e] = fmaf(xf[r][q], wf[q], acc[r * TOT + e]);
       }
     }
   }
@@ -1164,7 +1191,8 @@ gate_bwd_dx_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx,
 // The same for R tokens per warp, TOT <= 8: a slice of W is loaded and unpacked once for R tokens, and
 // its loads carry no predicates.  The sums are those of the one-token kernel.  All of the gate's
 // backward, 8192 tokens, d = 2048, 8 experts: 35 us, 41 with gradients at all logits; with this kernel
-// and dl in shared memory in the next one 30 and 33.
+// and dl in shared memory in the next one 30 and 33, with that one's sums of dl shared out and four
+// chains in the merge 28 and 31 (16384 tokens, d = 256: 18.9 -> 17.1).
 template <typename T, int TOT, int R>
 __global__ void __launch_bounds__(256)
 gate_bwd_dx_rows_kernel(const T* __restrict__ dprob, const int64_t* __restrict__ idx, const T* __restrict__ prob,
@@ -1199,7 +1227,8 @@ gate_bwd_dx_rows_kernel(const T* __restrict__ dprob, const int64_t* __restrict__
 #pragma unroll
     for (int e = 0; e < TOT; ++e) dl[r][e] = __shfl_sync(0xffffffffu, mine, r * TOT + e);
   }
-  const int nv = d >> 3;
+  constexpr int W = kPer16<T>;
+  const int nv = d / W;
 #pragma unroll 2
   for (int i = lane; i < nv; i += 32) {
     uint4 wv[TOT];
@@ -1208,34 +1237,36 @@ gate_bwd_dx_rows_kernel(const T* __restrict__ dprob, const int64_t* __restrict__
       // (past the last expert the last one again, for nothing)
       wv[e] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<long>(min(e, tot - 1)) * d) + i);
     }
-    float acc[R][8];
+    float acc[R][W];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[r][q] = 0.f;
+      for (int q = 0; q < W; ++q) acc[r][q] = 0.f;
     }
 #pragma unroll
     for (int e = 0; e < TOT; ++e) {
-      float wf[8];
-      unpack8<T>(wv[e], wf);
+      float wf[W];
+      unpack16<T>(wv[e], wf);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        if (dl[r][e] != 0.f) {   // the same for the whole warp; an expert without gradient adds nothing
+        // (the same for the whole warp; an expert without gradient adds nothing, but in 32 bits, where
+        // 0 times an infinite weight is NaN, as a product makes it)
+        if (sizeof(T) == 4 ? e < tot : dl[r][e] != 0.f) {
 #pragma unroll
-          for (int q = 0; q < 8; ++q) acc[r][q] = fmaf(dl[r][e], wf[q], acc[r][q]);
+          for (int q = 0; q < W; ++q) acc[r][q] = fmaf(dl[r][e], wf[q], acc[r][q]);
         }
       }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      if (row0 + r < n_rows) reinterpret_cast<uint4*>(dx + static_cast<long>(row0 + r) * d)[i] = pack8<T>(acc[r]);
+      if (row0 + r < n_rows) reinterpret_cast<uint4*>(dx + static_cast<long>(row0 + r) * d)[i] = pack16<T>(acc[r]);
     }
   }
 }
 
 // Partial sums of dW[e, c] = sum_t dl[t, e] x[t, c] and db[e] = sum_t dl[t, e] over one of
-// `gridDim.y` token ranges: part[range][tot * d + tot] in fp32.  A block takes a 256-column strip;
-// a lane owns eight columns, so that a token is one 16-byte load per lane (two columns per lane,
+// `gridDim.y` token ranges: part[range][tot * d + tot] in fp32.  A block takes a strip of 256 columns
+// (fp32: 128); a lane owns eight (four) of them, so that a token is one 16-byte load per lane (two columns per lane,
 // as before, kept too few bytes in flight).  The ranges used to be merged with atomics on a
 // zeroed buffer: 296 additions per address took most of the 20 us of 16384 tokens with d = 256,
 // which take 6 us now and 5 in the merge; 8192 tokens, d = 2048, 8 experts 40 -> 18 us, 11264 tokens,
@@ -1246,20 +1277,21 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
                    float* __restrict__ part) {
   ptx::chain_begin();
   constexpr int CHUNK = 128;   // tokens whose dl are held at a time: a multiple of the warps' step of 32
-  __shared__ float red[8][256 + 8];
+  constexpr int W = kPer16<T>, STRIP = 32 * W;
+  __shared__ float red[8][STRIP];
   __shared__ __align__(16) float dls[CHUNK][TOT];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = blockIdx.x * 256 + lane * 8;
+  const int col = blockIdx.x * STRIP + lane * W;
   const int per = (n_rows + gridDim.y - 1) / gridDim.y;
   const int t0 = blockIdx.y * per, t1 = min(n_rows, t0 + per);
   const bool sums = blockIdx.x == 0;
   float* mine = part + static_cast<long>(blockIdx.y) * (static_cast<long>(tot) * d + tot);
-  float acc[TOT][8], bsum[TOT];
+  __shared__ float bred[8][TOT];
+  float acc[TOT][W], bsum = 0.f;   // bsum: of expert threadIdx.x % TOT
 #pragma unroll
   for (int e = 0; e < TOT; ++e) {
-    bsum[e] = 0.f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) acc[e][q] = 0.f;
+    for (int q = 0; q < W; ++q) acc[e][q] = 0.f;
   }
   constexpr int U = 4;
   for (int c0 = t0; c0 < t1; c0 += CHUNK) {
@@ -1267,7 +1299,9 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
     __syncthreads();
     for (int i = threadIdx.x; i < CHUNK * TOT; i += 256) {
       const int t = c0 + i / TOT, e = i % TOT;
-      dls[i / TOT][e] = t < c1 && e < tot ? __ldg(dl + static_cast<long>(t) * tot + e) : 0.f;
+      const float v = t < c1 && e < tot ? __ldg(dl + static_cast<long>(t) * tot + e) : 0.f;
+      dls[i / TOT][e] = v;
+      if (sums) bsum += v;
     }
     __syncthreads();
     for (int t = c0 + warp; t < c1; t += 8 * U) {
@@ -1280,8 +1314,8 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (t + 8 * u >= c1) break;
-        float xf[8], g[TOT];
-        unpack8<T>(xv[u], xf);
+        float xf[W], g[TOT];
+        unpack16<T>(xv[u], xf);
 #pragma unroll
         for (int e = 0; e < TOT; e += 2) {
           const float2 two = *reinterpret_cast<const float2*>(&dls[t + 8 * u - c0][e]);
@@ -1291,38 +1325,41 @@ gate_bwd_dw_kernel(const float* __restrict__ dl, const T* __restrict__ x, int n_
 #pragma unroll
         for (int e = 0; e < TOT; ++e) {
 #pragma unroll
-          for (int q = 0; q < 8; ++q) acc[e][q] = fmaf(g[e], xf[q], acc[e][q]);
-          if (sums) bsum[e] += g[e];
+          for (int q = 0; q < W; ++q) acc[e][q] = fmaf(g[e], xf[q], acc[e][q]);
         }
       }
     }
+  }
+  if (sums) {   // short chains: the sum of a softmax's gradients over the tokens cancels
+#pragma unroll
+    for (int o = 16; o >= TOT; o >>= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
+    if (lane < TOT) bred[warp][lane] = bsum;
   }
 #pragma unroll
   for (int e = 0; e < TOT; ++e) {
     if (e >= tot) break;
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 8; ++q) red[warp][lane * 8 + q] = acc[e][q];
-    if (sums && lane == 0) red[warp][256] = bsum[e];
+    for (int q = 0; q < W; ++q) red[warp][lane * W + q] = acc[e][q];
     __syncthreads();
-    const int c = blockIdx.x * 256 + threadIdx.x;
-    if (c < d) {
+    const int c = blockIdx.x * STRIP + threadIdx.x;
+    if (threadIdx.x < STRIP && c < d) {
       float s = 0.f;
 #pragma unroll
       for (int wv = 0; wv < 8; ++wv) s += red[wv][threadIdx.x];
       mine[static_cast<long>(e) * d + c] = s;
     }
     if (sums && threadIdx.x == 0) {
-      float s = 0.f;
+      float s[8];
 #pragma unroll
-      for (int wv = 0; wv < 8; ++wv) s += red[wv][256];
-      mine[static_cast<long>(tot) * d + e] = s;
+      for (int wv = 0; wv < 8; ++wv) s[wv] = bred[wv][e];
+      mine[static_cast<long>(tot) * d + e] = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
     }
   }
 }
 
 // out[i] = sum over the ranges of part[range][i], in a fixed order, in the layer's type: eight
-// lanes of ranges per 32 elements.
+// lanes of ranges per 32 elements, in short chains (a gradient of the bias cancels).
 template <typename T>
 __global__ void __launch_bounds__(256)
 gate_bwd_merge_kernel(const float* __restrict__ part, int ranges, long elems, T* __restrict__ out) {
@@ -1330,18 +1367,26 @@ gate_bwd_merge_kernel(const float* __restrict__ part, int ranges, long elems, T*
   __shared__ float red[8][33];
   const int sub = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long i = static_cast<long>(blockIdx.x) * 32 + lane;
-  float s = 0.f;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
   if (i < elems) {
-#pragma unroll 4
-    for (int r = sub; r < ranges; r += 8) s += __ldg(part + static_cast<long>(r) * elems + i);
+    int r = sub;
+#pragma unroll 2
+    for (; r + 24 < ranges; r += 32) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[u] += __ldg(part + static_cast<long>(r + 8 * u) * elems + i);
+    }
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      if (r + 8 * u < ranges) s[u] += __ldg(part + static_cast<long>(r + 8 * u) * elems + i);
+    }
   }
-  red[sub][lane] = s;
+  red[sub][lane] = (s[0] + s[1]) + (s[2] + s[3]);
   __syncthreads();
   if (sub == 0 && i < elems) {
-    float total = 0.f;
+    float t[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) total += red[u][lane];
-    out[i] = V2<T>::from_f(total);
+    for (int u = 0; u < 8; ++u) t[u] = red[u][lane];
+    out[i] = V2<T>::from_f(((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7])));
   }
 }
 
@@ -1619,6 +1664,9 @@ cudaError_t launch_fill_pos(const int64_t* idx, const int* rank, const int* cum_
 #define FMOE_DISPATCH_16(dtype, ...)                                  \
   if ((dtype) == 0) { using T = __nv_bfloat16; __VA_ARGS__; }         \
   else { using T = __half; __VA_ARGS__; }
+#define FMOE_DISPATCH_ANY(dtype, ...)                                 \
+  if ((dtype) == 2) { using T = float; __VA_ARGS__; }                 \
+  else FMOE_DISPATCH_16(dtype, __VA_ARGS__)
 
 cudaError_t launch_scatter_rows(int dtype, const void* src, const int64_t* idx, const int* rank,
                                 const int* base, const void* scale, int n_slots, int k, int d,
@@ -1792,11 +1840,11 @@ cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, con
                                     void* prob, float* zero, cudaStream_t stream) {
   cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
-  if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
+  if (!gate_fused_supported(tot, d, k) || (dtype == 2 && tot > 8)) return cudaErrorInvalidValue;
   const int per = gate_rows_per_warp(n_rows, tot);
   const int grid = (n_rows + 8 * per - 1) / (8 * per);
 #define FMOE_GATE_ROWS(TOT, R)                                                                          \
-  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_linear_topk_rows_kernel<T, TOT, R>, dim3(grid), dim3(256), 0, stream,  \
+  FMOE_DISPATCH_ANY(dtype, (chained = launch_chained(gate_linear_topk_rows_kernel<T, TOT, R>, dim3(grid), dim3(256), 0, stream,  \
       static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), n_rows, d, tot,  \
       k, static_cast<T*>(logits), idx, static_cast<T*>(prob), zero)))
   if (tot <= 8) {
@@ -1831,16 +1879,16 @@ cudaError_t launch_gate_linear_topk_few(int dtype, const void* x, const void* w,
                                         int tot, int k, void* logits, int64_t* idx, void* prob, float* zero, cudaStream_t stream) {
   cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
-  if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
+  if (!gate_fused_supported(tot, d, k) || dtype == 2) return cudaErrorInvalidValue;
   FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_linear_topk_few_kernel<T>, dim3(n_rows), dim3(256), 0, stream,
       static_cast<const T*>(x), static_cast<const T*>(w), static_cast<const T*>(bias), d, tot, k,
       static_cast<T*>(logits), idx, static_cast<T*>(prob), zero)));
   return chained;
 }
 
-int gate_bwd_ranges(int n_rows, int d) {
+int gate_bwd_ranges(int dtype, int n_rows, int d) {
   // two blocks per SM over the strips and token ranges, a warp at least four tokens
-  const int strips = (d + 255) / 256;
+  const int strip = dtype == 2 ? 128 : 256, strips = (d + strip - 1) / strip;
   int ranges = (2 * 148 + strips - 1) / strips;
   if (ranges > (n_rows + 31) / 32) ranges = (n_rows + 31) / 32;
   return ranges > 0 ? ranges : 1;
@@ -1852,11 +1900,11 @@ cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, co
                             cudaStream_t stream) {
   cudaError_t chained = cudaSuccess;
   if (n_rows == 0) return cudaSuccess;
-  if (!gate_fused_supported(tot, d, k)) return cudaErrorInvalidValue;
+  if (!gate_fused_supported(tot, d, k) || (dtype == 2 && tot > 8)) return cudaErrorInvalidValue;
   const int per = gate_rows_per_warp(n_rows, tot);
   const int grid = (n_rows + 8 * per - 1) / (8 * per);
 #define FMOE_GATE_DX(TOT, R)                                                                            \
-  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dx_rows_kernel<T, TOT, R>, dim3(grid), dim3(256), 0, stream,    \
+  FMOE_DISPATCH_ANY(dtype, (chained = launch_chained(gate_bwd_dx_rows_kernel<T, TOT, R>, dim3(grid), dim3(256), 0, stream,    \
       static_cast<const T*>(dprob), idx, static_cast<const T*>(prob), static_cast<const T*>(dlogits_in),                  \
       static_cast<const T*>(w), n_rows, d, tot, k, dl_scratch, static_cast<T*>(dx))))
   if (tot <= 2) {
@@ -1877,16 +1925,16 @@ cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, co
   if (chained != cudaSuccess) return chained;
   if (part == nullptr) return cudaSuccess;
   if (tot > 16) return cudaErrorInvalidValue;
-  const int ranges = gate_bwd_ranges(n_rows, d);
-  dim3 g2((d + 255) / 256, ranges);
+  const int ranges = gate_bwd_ranges(dtype, n_rows, d), strip = dtype == 2 ? 128 : 256;
+  dim3 g2((d + strip - 1) / strip, ranges);
   if (tot <= 2) {
-    FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 2>, g2, dim3(256), 0, stream,
+    FMOE_DISPATCH_ANY(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 2>, g2, dim3(256), 0, stream,
         dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   } else if (tot <= 4) {
-    FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 4>, g2, dim3(256), 0, stream,
+    FMOE_DISPATCH_ANY(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 4>, g2, dim3(256), 0, stream,
         dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   } else if (tot <= 8) {
-    FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 8>, g2, dim3(256), 0, stream,
+    FMOE_DISPATCH_ANY(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 8>, g2, dim3(256), 0, stream,
         dl_scratch, static_cast<const T*>(x), n_rows, d, tot, part)));
   } else {
     FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_dw_kernel<T, 16>, g2, dim3(256), 0, stream,
@@ -1894,7 +1942,7 @@ cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, co
   }
   if (chained != cudaSuccess) return chained;
   const long elems = static_cast<long>(tot) * d + tot;
-  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_bwd_merge_kernel<T>, dim3(static_cast<unsigned>((elems + 31) / 32)), dim3(256), 0, stream,
+  FMOE_DISPATCH_ANY(dtype, (chained = launch_chained(gate_bwd_merge_kernel<T>, dim3(static_cast<unsigned>((elems + 31) / 32)), dim3(256), 0, stream,
       part, ranges, elems, static_cast<T*>(dw_db))));
   return chained;
 }

@@ -89,13 +89,13 @@ cudaError_t launch_switch_top1(int logit_dtype, const void* logits, int n, int t
 cudaError_t launch_prune_scalar(const int64_t* idx, const int* rank, int cap, int n_slots, int tot, int64_t* new_idx,
                                 cudaStream_t stream);
 
-// Fused gate: logits = x W^T + b (tot <= 64 experts, 16-bit types), top-k ids (descending) and
+// Fused gate (dtype: 0 bf16, 1 f16, 2 f32): logits = x W^T + b (tot <= 64 experts; f32: 8), top-k ids (descending) and
 // softmax over the selected logits; one pass over x.
 bool gate_fused_supported(int tot, int d, int k);
 cudaError_t launch_gate_linear_topk(int dtype, const void* x, const void* w, const void* bias,
                                     int n_rows, int d, int tot, int k, void* logits, int64_t* idx,
                                     void* prob, float* zero, cudaStream_t stream);
-// The same result for a few tokens (one block each).
+// The same result for a few tokens (one block each), 16 bits.
 cudaError_t launch_gate_linear_topk_few(int dtype, const void* x, const void* w, const void* bias, int n_rows, int d,
                                         int tot, int k, void* logits, int64_t* idx, void* prob, float* zero,
                                         cudaStream_t stream);
@@ -103,7 +103,7 @@ cudaError_t launch_gate_linear_topk_few(int dtype, const void* x, const void* w,
 // part (optional, tot <= 16): fp32 scratch of gate_bwd_ranges() * (tot * d + tot) entries; with it
 // dw_db receives dW [tot, d] followed by db [tot] in the layer's type.  Above 16 experts pass
 // part = nullptr and form dW = dl^T x from dl_scratch with a library GEMM.
-int gate_bwd_ranges(int n_rows, int d);
+int gate_bwd_ranges(int dtype, int n_rows, int d);
 cudaError_t launch_gate_bwd(int dtype, const void* dprob, const int64_t* idx, const void* prob,
                             const void* dlogits_in, const void* x, const void* w, int n_rows, int d,
                             int tot, int k, float* dl_scratch, void* dx, float* part, void* dw_db,

@@ -10,7 +10,7 @@ class NaiveGate(BaseGate):
     r"""``Linear(d_model → tot_expert)``, top-k of the logits, softmax over the k selected logits.
 
     State-dict keys: ``gate.weight [tot_expert, d_model]``, ``gate.bias [tot_expert]``.
-    On a GPU with 16-bit parameters and at most 8 experts the linear layer, the top-k and the
+    On a GPU with 16- or 32-bit parameters and at most 8 experts the linear layer, the top-k and the
     softmax are one kernel (three in backward); otherwise the top-k + softmax are.
     """
 

@@ -79,6 +79,12 @@ class _LinearTopkSoftmax(Function):
         x, weight, idx, prob = ctx.saved_tensors
         if grad_logits is None and grad_prob is None:
             return None, None, None, None
+        if torch.is_grad_enabled() and x.dtype == torch.float32:   # a gradient of the gradient, as in the native node
+            dl = grad_logits
+            if grad_prob is not None:
+                through = native.get().gate_topk_softmax_bwd(grad_prob.contiguous(), idx, prob, weight.shape[0])
+                dl = through if dl is None else dl + through
+            return dl.matmul(weight), dl.t().matmul(x), dl.sum(0) if ctx.has_bias else None, None
         if (x.data_ptr() | weight.data_ptr()) % 16 != 0:   # moved by hooks on the saved tensors
             x, weight = gg.aligned(x, 16), gg.aligned(weight, 16)
         dx, dw, db, _dl = native.get().gate_linear_topk_bwd(
@@ -89,6 +95,18 @@ class _LinearTopkSoftmax(Function):
                 db if ctx.has_bias and ctx.needs_input_grad[2] else None, None)
 
 
+def _single_pass_type(x, weight, bias):
+    r"""Whether the single-pass kernel takes these types: all 16 bits, or all 32 as plain tensors (a linear, top-k,
+    softmax and their backward as operations, 8192 tokens, d 1024, 8 experts: 163 us, 87 in the kernels, whose
+    logits are within 1.2 units of 2^-24 of 64 bits, weight gradients 2.3, against 5.5 and 4.9)."""
+    if weight.dtype != x.dtype or (bias is not None and bias.dtype != x.dtype):
+        return False
+    if x.dtype in (torch.bfloat16, torch.float16):
+        return True
+    return (x.dtype == torch.float32
+            and all(t is None or type(t) in (torch.Tensor, torch.nn.Parameter) for t in (x, weight, bias)))
+
+
 def linear_logits(x, linear):
     r"""``linear(x)`` of a gate's ``nn.Linear`` in the single-pass kernel, or ``None`` where that does not
     take the call or somebody watches the module.  It stands for three library products and a column sum
@@ -97,8 +115,7 @@ def linear_logits(x, linear):
     w, b = linear.weight, linear.bias
     if (w.shape[0] <= MAX_SINGLE_PASS_EXPERTS and type(linear) is torch.nn.Linear
             and x.is_cuda and x.dim() == 2 and x.is_contiguous()
-            and x.dtype in (torch.bfloat16, torch.float16) and w.dtype == x.dtype and x.shape[0] > 0
-            and (b is None or b.dtype == x.dtype) and not torch.is_autocast_enabled() and not traced()
+            and x.shape[0] > 0 and _single_pass_type(x, w, b) and not torch.is_autocast_enabled() and not traced()
             and native.get().gate_fused_supported(w.shape[0], x.shape[1], 1)
             and all(t is None or forward_ad.unpack_dual(t).tangent is None for t in (x, w, b))
             and not _hooked(linear) and not _hooked_globally()):
@@ -178,13 +195,14 @@ def _few_tokens_ok(x, weight, bias, k):
 def linear_topk_softmax(x, weight, bias, k, zero=None):
     r"""``(logits [B,E], idx int64 [B,k], prob [B,k])`` of a linear gate over 2-D ``x``.
 
-    Uses the single-pass kernel when the shape allows it (16-bit types on a GPU, ``d_model`` a
+    Uses the single-pass kernel when the shape allows it (16 or 32 bits on a GPU, ``d_model`` a
     multiple of 8) and the expert count is small enough for its SIMT dot products to beat a GEMM
     (with one token per warp, 4096 tokens, ``d_model`` 1024: 30.6 vs 35.5 µs forward + backward at 2
     experts, 52 vs 37 µs at 16; up to 8 experts warps take several tokens, 17.5 µs at 2).  Above that the
     product runs on the tcgen05 grouped-GEMM kernel with a single group (:class:`_GateGemm`),
-    followed by :func:`topk_softmax`, but for a few tokens without gradients (one launch); only 32-/64-bit inputs, CPU tensors and odd ``d_model``
-    take the ``linear`` → :func:`topk_softmax` sequence of PyTorch ops.
+    followed by :func:`topk_softmax`, but for a few tokens without gradients (one launch); 64-bit inputs,
+    32-bit ones with more than 8 experts, CPU tensors and odd ``d_model`` take the ``linear`` →
+    :func:`topk_softmax` sequence of PyTorch ops.
 
     ``zero``: a one-element fp32 tensor on ``x``'s device that is set to 0 on the way, by the gate's
     kernel where there is one (a launch of its own took a fiftieth of a small decoding step).
@@ -192,10 +210,8 @@ def linear_topk_softmax(x, weight, bias, k, zero=None):
     if zero is not None and (not x.is_cuda or x.shape[0] == 0):
         zero.zero_()
         zero = None
-    if (x.is_cuda and x.dim() == 2 and x.dtype in (torch.bfloat16, torch.float16)
-            and weight.shape[0] <= MAX_SINGLE_PASS_EXPERTS
-            and weight.dtype == x.dtype and (bias is None or bias.dtype == x.dtype)
-            and not torch.is_autocast_enabled()
+    if (x.is_cuda and x.dim() == 2 and weight.shape[0] <= MAX_SINGLE_PASS_EXPERTS
+            and _single_pass_type(x, weight, bias) and not torch.is_autocast_enabled()
             and native.get().gate_fused_supported(weight.shape[0], x.shape[1], k)):
         xc = x if x.is_contiguous() else x.contiguous()
         if traced():

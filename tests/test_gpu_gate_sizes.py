@@ -79,3 +79,68 @@ def test_gate_backward_of_several_tokens_per_warp(experts, tokens, d):
                                    (dw, dl.t() @ x.double(), dl.abs().t() @ x.double().abs(), tokens),
                                    (db, dl.sum(0), dl.abs().sum(0), tokens)]:
         assert bool(((got.double() - want).abs() <= eps * want.abs() + terms * 2.0 ** -24 * size + 1e-30).all())
+
+
+# 1, 2 and 4 tokens per warp, strips of 128 columns with a rest, fewer tokens than a block has warps
+@pytest.mark.parametrize("experts,k,bias", [(1, 1, True), (2, 2, False), (3, 1, True), (4, 2, True), (5, 3, True), (8, 2, True)])
+@pytest.mark.parametrize("tokens,d", [(3, 8), (257, 136), (2369, 264), (4737, 64), (4800, 1024)])
+def test_fp32_gate(tokens, d, experts, k, bias):
+    r"""The fp32 linear gate against 64 bits.  Every sum of n products is formed in fp32: its error is at most
+    n 2^-24 times the sum of the magnitudes; the softmax's exponential has 2 units in the last place and an
+    argument of at most 2^-24 |v| error, taken as 32 units of 2^-24."""
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(tokens + experts)
+    x = torch.randn(tokens, d, device=DEV, requires_grad=True)
+    w = (torch.randn(experts, d, device=DEV) / d ** 0.5).requires_grad_(True)
+    b = torch.randn(experts, device=DEV, requires_grad=True) if bias else None
+    assert gating._single_pass_type(x, w, b)
+    logits, idx, prob = gating.linear_topk_softmax(x, w, b, k)
+    u = 2.0 ** -24
+    x64, w64 = x.detach().double(), w.detach().double()
+    b64 = b.detach().double() if bias else 0.0
+    ref, size = x64 @ w64.t() + b64, x64.abs() @ w64.abs().t() + (b64.abs() if bias else 0.0)
+    assert bool(((logits.double() - ref).abs() <= (d + 2) * u * size).all())
+    val, chosen = torch.topk(logits.detach(), k, dim=1)
+    assert torch.equal(idx, chosen)
+    assert bool(((prob.double() - torch.softmax(val.double(), 1)).abs() <= 32 * u).all())
+    gl, gp = torch.randn_like(logits), torch.randn_like(prob)
+    torch.autograd.backward([logits, prob], [gl, gp])
+    p, g = prob.detach().double(), gp.double()
+    through = p * (g - (p * g).sum(1, keepdim=True))
+    dl = gl.double().scatter_add(1, idx, through)
+    dl_err = (8 + 2 * k) * u * gl.double().abs().scatter_add(1, idx, p * (g.abs() + (p * g).abs().sum(1, keepdim=True)))
+    for got, want, bound in [
+            (x.grad, dl @ w64, (experts + 1) * u * (dl.abs() @ w64.abs()) + dl_err @ w64.abs()),
+            (w.grad, dl.t() @ x64, (tokens + 1) * u * (dl.abs().t() @ x64.abs()) + dl_err.t() @ x64.abs())] + (
+            [(b.grad, dl.sum(0), (tokens + 1) * u * dl.abs().sum(0) + dl_err.sum(0))] if bias else []):
+        assert bool(((got.double() - want).abs() <= bound).all())
+
+
+def test_fp32_gate_gradient_of_the_gradient():
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(0)
+    x = torch.randn(40, 32, device=DEV, requires_grad=True)
+    w = torch.randn(4, 32, device=DEV, requires_grad=True)
+    second = []
+    for logits in (gating.linear_topk_softmax(x, w, None, 2)[0], gating._LinearTopkSoftmax.apply(x, w, None, 2)[0],
+                   torch.nn.functional.linear(x, w)):
+        dx, = torch.autograd.grad(logits.square().sum(), x, create_graph=True)
+        second.append(torch.autograd.grad(dx.square().sum(), w)[0])
+    # sums of at most 40 * 32 terms in fp32
+    for got in second[:2]:
+        assert torch.allclose(got, second[2], rtol=1e-3, atol=1e-3 * float(second[2].abs().max()))
+
+
+def test_fp32_gate_keeps_subclasses_and_autocast_on_the_operations():
+    from fastmoe_b200.ops import gating
+
+    class Mine(torch.Tensor):
+        pass
+    x, w = torch.randn(16, 64, device=DEV), torch.randn(4, 64, device=DEV)
+    assert gating._single_pass_type(x, w, None)
+    assert not gating._single_pass_type(x, w.as_subclass(Mine), None)
+    assert not gating._single_pass_type(x.bfloat16(), w, None)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert gating.linear_topk_softmax(x, w, None, 2)[0].dtype == torch.bfloat16
+    with pytest.raises(RuntimeError):
+        gating.linear_topk_softmax(x, w[:, :56], None, 2)   # widths that differ
