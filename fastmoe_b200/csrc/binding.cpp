@@ -837,6 +837,24 @@ torch::Tensor prune_gate_scalar(torch::Tensor idx, int64_t cap, int64_t tot) {
   return out;
 }
 
+// int32 [groups + 1] exclusive prefix of host counts, on `device` (-1: the current one).
+torch::Tensor host_offsets(torch::Tensor counts_in, int64_t device) {
+  TORCH_CHECK(counts_in.device().is_cpu() && counts_in.scalar_type() == torch::kLong && counts_in.dim() == 1 &&
+              counts_in.numel() < fmoe::kMaxHostOffsets, "host counts");
+  const torch::Tensor counts = counts_in.contiguous();
+  c10::cuda::OptionalCUDAGuard guard;
+  if (device >= 0) guard.set_index(static_cast<c10::DeviceIndex>(device));
+  const int n = static_cast<int>(counts.numel());
+  int values[fmoe::kMaxHostOffsets];
+  const int64_t* c = counts.data_ptr<int64_t>();
+  int64_t sum = 0;
+  values[0] = 0;
+  for (int i = 0; i < n; ++i) values[i + 1] = static_cast<int>(sum += c[i]);
+  auto offs = torch::empty({n + 1}, torch::dtype(torch::kInt32).device(torch::kCUDA, c10::cuda::current_device()));
+  FMOE_CUDA_CHECK(fmoe::launch_host_offsets(values, n + 1, offs.data_ptr<int>(), cur_stream()));
+  return offs;
+}
+
 void check_logits(const torch::Tensor& logits) {
   TORCH_CHECK(logits.is_cuda() && logits.dim() == 2 && logits.stride(1) == 1 && logits.size(0) > 0,
               "logits must be a non-empty CUDA matrix with contiguous rows");
@@ -1126,6 +1144,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gate_topk_softmax_bwd", &gate_topk_softmax_bwd);
   m.def("balance_supported", &balance_supported);
   m.def("prune_gate_scalar", &prune_gate_scalar);
+  m.def("host_offsets", &host_offsets);
   m.def("balance_loss", &balance_loss);
   m.def("balance_bwd", &balance_bwd);
   m.def("switch_top1", &switch_top1);

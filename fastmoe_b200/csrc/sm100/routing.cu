@@ -834,6 +834,17 @@ switch_top1_kernel(const T* __restrict__ logits, int n, int tot, int64_t* __rest
 }
 
 // new_idx[s] = idx[s] when fewer than `cap` slots of its expert come before it, else -1
+// Host values that travel with the launch, in place of the operations that formed the prefix on the host and a
+// copy from pageable memory: a grouped linear's forward and backward, 16 experts, 142 rows, d 320, 197 -> 162 us.
+template <int N> struct HostValues {
+  int v[N];
+};
+template <int N>
+__global__ void host_offsets_kernel(const __grid_constant__ HostValues<N> values, int n, int* __restrict__ dst) {
+  ptx::chain_begin();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = values.v[i];
+}
+
 __global__ void prune_scalar_kernel(const int64_t* __restrict__ idx, const int* __restrict__ rank, int cap, int n_slots,
                                     int tot, int64_t* __restrict__ out) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1815,6 +1826,19 @@ cudaError_t launch_switch_top1(int code, const void* logits, int n, int tot, int
       (switch_top1_kernel<T, TOT><<<balance_blocks(n), kBalanceThreads, 0, stream>>>(
            static_cast<const T*>(logits), n, tot, win, static_cast<T*>(score)))));
   return cudaGetLastError();
+}
+
+template <int N>
+static cudaError_t host_offsets(const int* values, int n, int* dst, cudaStream_t stream) {
+  HostValues<N> v;
+  for (int i = 0; i < n; ++i) v.v[i] = values[i];
+  return launch_chained(host_offsets_kernel<N>, dim3(1), dim3(128), 0, stream, v, n, dst);
+}
+
+cudaError_t launch_host_offsets(const int* values, int n, int* dst, cudaStream_t stream) {
+  if (n < 1 || n > kMaxHostOffsets) return cudaErrorInvalidValue;
+  // (launches copy all of their parameters)
+  return n <= 80 ? host_offsets<80>(values, n, dst, stream) : host_offsets<kMaxHostOffsets>(values, n, dst, stream);
 }
 
 cudaError_t launch_prune_scalar(const int64_t* idx, const int* rank, int cap, int n_slots, int tot, int64_t* new_idx,

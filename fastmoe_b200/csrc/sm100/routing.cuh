@@ -85,6 +85,10 @@ cudaError_t launch_balance_bwd(int logit_dtype, const void* logits, long pitch, 
 cudaError_t launch_switch_top1(int logit_dtype, const void* logits, int n, int tot, int64_t* win, void* score,
                                cudaStream_t stream);
 
+// dst[i] = values[i] for host values, i < n <= kMaxHostOffsets.
+constexpr int kMaxHostOffsets = 960;
+cudaError_t launch_host_offsets(const int* values, int n, int* dst, cudaStream_t stream);
+
 // new_idx[s] = (idx[s] in range && rank[s] < cap) ? idx[s] : -1
 cudaError_t launch_prune_scalar(const int64_t* idx, const int* rank, int cap, int n_slots, int tot, int64_t* new_idx,
                                 cudaStream_t stream);

@@ -19,11 +19,17 @@ ACT_CODES = {None: 0, "identity": 0, "relu": 1, "gelu": 2, "gelu_tanh": 3}
 EPI_BIAS_ACT, EPI_DACT = 0, 1
 
 _TC = (torch.bfloat16, torch.float16)
+MAX_HOST_COUNTS = 960   # with the leading 0, what a launch carries in its parameters
 
 
 def offsets_from_counts(counts, device):
-    r"""int32 ``[E+1]`` exclusive prefix of host-resident ``counts``, placed on ``device``."""
+    r"""int32 ``[E+1]`` exclusive prefix of host-resident ``counts``, placed on ``device``.  On a GPU one launch,
+    which carries the values, writes it; counts for a graph's capture are copied as before."""
     c = torch.as_tensor(counts).reshape(-1).to(torch.int64)
+    device = torch.device(device)
+    if (device.type == "cuda" and not c.is_cuda and c.numel() < MAX_HOST_COUNTS
+            and not torch.cuda.is_current_stream_capturing()):
+        return native.get().host_offsets(c, -1 if device.index is None else device.index)
     offs = torch.zeros(c.numel() + 1, dtype=torch.int32)
     offs[1:] = torch.cumsum(c, 0).to(torch.int32)
     return offs.to(device, non_blocking=True)

@@ -113,3 +113,17 @@ def test_gradient_of_the_gradient(monkeypatch):
         results.append([x.grad, s.grad] + [p.grad.clone() for p in layer.experts.parameters()])
     for a, b in zip(*results):
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("groups", [1, 79, 80, 255, 959, 960, 3000])   # parameters of 80 and 960 values, the copy
+def test_offsets_of_host_counts(groups):
+    from fastmoe_b200.ops import grouped_gemm as gg
+    counts = torch.randint(0, 50, (groups,), generator=torch.Generator().manual_seed(groups))
+    want = torch.cat([torch.zeros(1, dtype=torch.int64), counts.cumsum(0)]).int()
+    for given in (counts, counts.int(), counts.tolist(), torch.stack([counts, counts], 1)[:, 0]):
+        offs = gg.offsets_from_counts(given, "cuda")
+        assert offs.is_cuda and offs.dtype == torch.int32 and torch.equal(offs.cpu(), want)
+    kept = counts.clone()
+    offs = gg.offsets_from_counts(kept, torch.device("cuda", 0))
+    kept.zero_()   # the call has taken what it needs
+    assert torch.equal(offs.cpu(), want)
