@@ -208,6 +208,7 @@ cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
   p.out_fp32 = a.out_fp32;
   p.psum = a.mode == kWgrad ? a.psum : nullptr;
   p.psrc = a.a;
+  p.qsrc = a.b;
   p.status = a.status;
   const int grid = (a.num_sms > 1 ? a.num_sms : 148) & ~1;
   return a.dtype == kBF16 ? pg::launch_bf16(a.mode, a.act, ta, tb, tc, p, grid, a.stream)

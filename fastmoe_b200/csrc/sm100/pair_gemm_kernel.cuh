@@ -14,14 +14,15 @@
 //               bytes of both CTAs are counted on CTA 0's barrier of the stage;
 //   warp 1      CTA 0: one lane issues the pair's MMAs and commits to both CTAs' barriers; in
 //               both CTAs the warp owns the TMEM allocation;
-//   warp 2      weight gradient: zeroes the rows past an expert's end in the expert's last K block
-//               (shared memory), off the producer's path, so that loads of the next tiles go on;
+//   warp 2      weight gradient: an expert's last rows, where they do not fill an MMA step of 16, by plain
+//               loads into a buffer of their own, filled up with zeros, a tile or two ahead;
 //   warp 3      weight gradient: zeroes the gradients of experts without rows, beside the MMAs;
 //   warps 4-11  epilogue: as in the single-CTA kernel, 32 rows x 128 columns per warp; whole rows of
 //               32 leave by TMA.
-// The last K block of an expert in the weight gradient issues only the 16-row MMA steps that
-// contain rows of the expert.  With the zeroing in the producer warp, which waited for the copies
-// first, 64 experts of 128 rows took 394 us; now 200 us, 537 MB of gradients written.
+// The ring brings whole K blocks, of which the MMA steps that are full of the expert's rows are issued.
+// The step that is not has its operands beside the ring: zeroed in the ring after they had landed, the rows
+// past the end held every tile of a ragged expert up by 1.3 us (16 experts, 1024 <-> 4096: 375 rows each
+// 70.2 us against 51.9 with 384; now 52.8).
 #pragma once
 #include "grouped_gemm_kernel.cuh"
 #include "launch.cuh"
@@ -51,10 +52,16 @@ constexpr int EPI_COLS = TILE_N / 2;        // columns per epilogue warp
 constexpr int EPI_CHUNKS = EPI_COLS / 32;
 constexpr int TMEM_COLS = 512;
 
+// Operands of the MMA step of an expert's last rows: as the ring's, 64-wide boxes of 16 rows.
+constexpr int SIDE_BOX_BYTES = 64 * UMMA_K * 2;
+constexpr int SIDE_A_BYTES = CTA_M / 64 * SIDE_BOX_BYTES;
+constexpr int SIDE_BYTES = SIDE_A_BYTES + CTA_N / 64 * SIDE_BOX_BYTES;
+
 struct Shared {
   uint64_t full[STAGES];        // CTA 0's counts: one arrival and the bytes of each CTA
   uint64_t empty[STAGES];
-  uint64_t tail[STAGES];        // this CTA's copies of a ragged K block have landed
+  uint64_t side_full[2];        // CTA 0's counts: one arrival of each CTA
+  uint64_t side_empty[2];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];       // CTA 0's counts: every epilogue warp of both CTAs
   uint32_t tmem_base;
@@ -65,7 +72,8 @@ struct Shared {
 };
 
 constexpr int PATCH_BYTES = gg::PATCH_BYTES;
-constexpr int PATCH_OFF = STAGES * STAGE_BYTES;
+constexpr int SIDE_OFF = STAGES * STAGE_BYTES;
+constexpr int PATCH_OFF = SIDE_OFF + 2 * SIDE_BYTES;
 constexpr int AUX_OFF = PATCH_OFF + NUM_EPI_WARPS * PATCH_BYTES;
 constexpr int SMEM_BYTES = AUX_OFF + static_cast<int>(sizeof(Shared)) + 1024;
 static_assert(SMEM_BYTES <= 232448, "shared memory");
@@ -82,7 +90,8 @@ struct Params {
   int accumulate;
   int out_fp32;
   void* psum;
-  const void* psrc;
+  const void* psrc;      // weight gradient: the operands again
+  const void* qsrc;
   int* status;
 };
 
@@ -378,7 +387,7 @@ __device__ __forceinline__ void epilogue_tile_update(const Params& p, const EpiT
 }
 
 // The bias gradient of a grouped linear is the column sum, per expert, of the matrix its weight
-// gradient takes as P.  On the tiles of the first N column block the epilogue warps, which wait
+// gradient takes as P.  Of an expert with many rows (few have): on the tiles of the first N column block the epilogue warps, which wait
 // for the main loop then, add up this CTA's 128 columns of P with plain 16-byte loads (the rows
 // pass through the L2 for the TMA loads at the same time).
 template <typename T>
@@ -407,7 +416,18 @@ __device__ __forceinline__ void column_sums(const Params& p, uint8_t* patches, c
 #pragma unroll
       for (int i = 0; i < kUnroll; ++i) add(v[i]);
     }
-    for (; r < row_end; r += 16) add(__ldg(reinterpret_cast<const uint4*>(src + static_cast<long>(r) * p.m)));
+    // (one load after the other, the last 255 rows took 16 times the latency of a load)
+    constexpr int kRest = 8;
+    for (; r < row_end; r += 16 * kRest) {
+      uint4 v[kRest];
+#pragma unroll
+      for (int i = 0; i < kRest; ++i) {
+        v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (r + 16 * i < row_end) v[i] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<long>(r + 16 * i) * p.m));
+      }
+#pragma unroll
+      for (int i = 0; i < kRest; ++i) add(v[i]);
+    }
   }
   float* mine = reinterpret_cast<float*>(patches + ew * PATCH_BYTES);
 #pragma unroll
@@ -426,6 +446,63 @@ __device__ __forceinline__ void column_sums(const Params& p, uint8_t* patches, c
     *dst = Cvt<T>::from_f(total);
   }
   asm volatile("bar.sync 2, %0;" ::"n"(NUM_EPI_WARPS * 32) : "memory");
+}
+
+// Of the others: 32 columns at a time by the warps that have little else to do, beside the main loops.  The
+// epilogue warps wait for the loads' latency on every tile of the first column block: what the sums add,
+// 1024 <-> 4096, 16 experts of 64 rows 9.6 us, here 1 to 3, of 128 rows 8.7, here 0.5; 8 of 2048 rows 10.1, here 3.
+// (64 columns at a time and 32 loads in flight took two to three times as long.)
+constexpr int SUM_COLS = 32;
+constexpr int MAX_SIDE_ROWS = 2048;
+template <typename T>
+__device__ __forceinline__ void side_sums(const Params& p, const Shared* sh, int worker, int workers, int lane) {
+  const int blocks = (p.m + SUM_COLS - 1) / SUM_COLS;
+  auto add = [](float (&cs)[8], const uint4& v) {
+    float a, b;
+    Cvt<T>::unpack(v.x, a, b); cs[0] += a; cs[1] += b;
+    Cvt<T>::unpack(v.y, a, b); cs[2] += a; cs[3] += b;
+    Cvt<T>::unpack(v.z, a, b); cs[4] += a; cs[5] += b;
+    Cvt<T>::unpack(v.w, a, b); cs[6] += a; cs[7] += b;
+  };
+  long item = worker;
+  for (int g = 0; g < p.num_groups; ++g) {
+    const int begin = sh->offs[g], end = sh->offs[g + 1];
+    if (end == begin || end - begin > MAX_SIDE_ROWS) continue;
+    for (; item < blocks; item += workers) {
+      const int col = static_cast<int>(item) * SUM_COLS + (lane & 3) * 8;
+      float cs[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) cs[q] = 0.f;
+      if (col < p.m) {
+        const T* src = static_cast<const T*>(p.psrc) + col;
+        constexpr int kUnroll = 16;
+        for (int r = begin + (lane >> 2); r < end; r += 8 * kUnroll) {
+          uint4 v[kUnroll];
+#pragma unroll
+          for (int i = 0; i < kUnroll; ++i) {
+            v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (r + 8 * i < end) v[i] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<long>(r + 8 * i) * p.m));
+          }
+#pragma unroll
+          for (int i = 0; i < kUnroll; ++i) add(cs, v[i]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) cs[q] += __shfl_xor_sync(0xffffffffu, cs[q], o);
+      }
+      if (lane < 4 && col < p.m) {
+        T* dst = static_cast<T*>(p.psum) + static_cast<long>(g) * p.m + col;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          if (p.accumulate) cs[q] += Cvt<T>::to_f(dst[q]);
+          dst[q] = Cvt<T>::from_f(cs[q]);
+        }
+      }
+    }
+    item -= blocks;
+  }
 }
 
 // ------------------------------------------------------------------------------ kernel
@@ -450,7 +527,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     for (int s = 0; s < STAGES; ++s) {
       ptx::mbar_init(&sh->full[s], 2);
       ptx::mbar_init(&sh->empty[s], 1);
-      ptx::mbar_init(&sh->tail[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      ptx::mbar_init(&sh->side_full[b], 2);
+      ptx::mbar_init(&sh->side_empty[b], 1);
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(&sh->tmem_full[a], 1);
@@ -516,7 +596,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       bool ok = true;
       for (int tile = pair; tile < total && ok; tile += num_pairs) {
         const Tile c = decode(sh, n_tiles, tile, group);
-        const int num_kb = (MODE == kWgrad) ? (c.rows + BK - 1) / BK : p.k / BK;
+        const int num_kb = (MODE == kWgrad) ? (c.rows / UMMA_K * UMMA_K + BK - 1) / BK : p.k / BK;
         const int n0 = c.n_tile * TILE_N + rank * CTA_N;
         const int m0 = c.m_tile * TILE_M + rank * CTA_M;
         for (int kb = 0; kb < num_kb; ++kb) {
@@ -528,31 +608,20 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
-          if (MODE == kWgrad && c.rows - kb * BK < BK) {
-            // the expert's ragged end: counted on this CTA's own barrier, handed on by warp 2
-            uint64_t* bar = &sh->tail[stage];
-            const int row0 = c.row_begin + kb * BK;
-            ptx::mbar_arrive_expect_tx(bar, STAGE_BYTES);
+          const uint32_t bar = ptx::mapa(&sh->full[stage], 0);
+          ptx::mbar_arrive_expect_tx_cluster(bar, STAGE_BYTES);
+          if (MODE == kRowsNN) {
+            ptx::tma_load_2d_pair(sa, &tm_a, bar, kb * BK, c.row_begin + m0);
 #pragma unroll
-            for (int ch = 0; ch < CTA_M / 64; ++ch) ptx::tma_load_2d(sa + ch * BOX_BYTES, &tm_a, bar, m0 + ch * 64, row0);
-#pragma unroll
-            for (int ch = 0; ch < CTA_N / 64; ++ch) ptx::tma_load_2d(sb + ch * BOX_BYTES, &tm_b, bar, n0 + ch * 64, row0);
-          } else {
-            const uint32_t bar = ptx::mapa(&sh->full[stage], 0);
-            ptx::mbar_arrive_expect_tx_cluster(bar, STAGE_BYTES);
-            if (MODE == kRowsNN) {
-              ptx::tma_load_2d_pair(sa, &tm_a, bar, kb * BK, c.row_begin + m0);
-#pragma unroll
-              for (int ch = 0; ch < CTA_N / 64; ++ch) {
-                ptx::tma_load_2d_pair(sb + ch * BOX_BYTES, &tm_b, bar, n0 + ch * 64, c.group * p.k + kb * BK);
-              }
-            } else {
-              const int row0 = c.row_begin + kb * BK;
-#pragma unroll
-              for (int ch = 0; ch < CTA_M / 64; ++ch) ptx::tma_load_2d_pair(sa + ch * BOX_BYTES, &tm_a, bar, m0 + ch * 64, row0);
-#pragma unroll
-              for (int ch = 0; ch < CTA_N / 64; ++ch) ptx::tma_load_2d_pair(sb + ch * BOX_BYTES, &tm_b, bar, n0 + ch * 64, row0);
+            for (int ch = 0; ch < CTA_N / 64; ++ch) {
+              ptx::tma_load_2d_pair(sb + ch * BOX_BYTES, &tm_b, bar, n0 + ch * 64, c.group * p.k + kb * BK);
             }
+          } else {
+            const int row0 = c.row_begin + kb * BK;
+#pragma unroll
+            for (int ch = 0; ch < CTA_M / 64; ++ch) ptx::tma_load_2d_pair(sa + ch * BOX_BYTES, &tm_a, bar, m0 + ch * 64, row0);
+#pragma unroll
+            for (int ch = 0; ch < CTA_N / 64; ++ch) ptx::tma_load_2d_pair(sb + ch * BOX_BYTES, &tm_b, bar, n0 + ch * 64, row0);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -565,11 +634,12 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       constexpr uint32_t idesc = ptx::make_idesc(kBf16, MODE == kWgrad, true, TILE_M, TILE_N);
       int stage = 0;
       uint32_t phase = 0;
-      int iter = 0;
+      int iter = 0, side = 0;
       bool ok = true;
       for (int tile = pair; tile < total && ok; tile += num_pairs, ++iter) {
         const Tile c = decode(sh, n_tiles, tile, group);
-        const int num_kb = (MODE == kWgrad) ? (c.rows + BK - 1) / BK : p.k / BK;
+        const int whole = c.rows / UMMA_K * UMMA_K;   // rows in full MMA steps (weight gradient)
+        const int num_kb = (MODE == kWgrad) ? (whole + BK - 1) / BK : p.k / BK;
         const int acc = iter & 1;
         if (!ptx::mbar_wait(&sh->tmem_empty[acc], ((iter >> 1) & 1) ^ 1, abort_flag)) {
           sh->abort = 1;
@@ -578,6 +648,21 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * TILE_N;
+        const bool ragged = MODE == kWgrad && whole != c.rows;
+        if (ragged) {   // first: its operands have been there for long, and the ring goes on filling
+          if (!ptx::mbar_wait<true>(&sh->side_full[side & 1], (side >> 1) & 1, abort_flag)) {
+            sh->abort = 1;
+            if (p.status != nullptr) record_failure(p.status, gg::STATUS_TIMEOUT_MMA);
+            break;
+          }
+          ptx::tc_fence_after_sync();
+          const uint32_t sa = ptx::smem_u32(smem + SIDE_OFF + (side & 1) * SIDE_BYTES);
+          const uint64_t a_desc = ptx::make_smem_desc_sw128(sa, SIDE_BOX_BYTES, 1024);
+          const uint64_t b_desc = ptx::make_smem_desc_sw128(sa + SIDE_A_BYTES, SIDE_BOX_BYTES, 1024);
+          ptx::umma_f16_pair(d_tmem, a_desc, b_desc, idesc, 0u);
+          ptx::umma_commit_pair(&sh->side_empty[side & 1]);
+          ++side;
+        }
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!ptx::mbar_wait(&sh->full[stage], phase, abort_flag)) {
             sh->abort = 1;
@@ -585,11 +670,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             ok = false;
             break;
           }
-          if (MODE == kWgrad && c.rows - kb * BK < BK) ptx::fence_cluster();   // zeroed rows of CTA 1
           ptx::tc_fence_after_sync();
           const uint32_t sa = ptx::smem_u32(smem + stage * STAGE_BYTES);
           const uint32_t sb = sa + A_BYTES;
-          const int steps = (MODE == kWgrad) ? min(BK / UMMA_K, (c.rows - kb * BK + UMMA_K - 1) / UMMA_K) : BK / UMMA_K;
+          const int steps = (MODE == kWgrad) ? min(BK / UMMA_K, (whole - kb * BK) / UMMA_K) : BK / UMMA_K;
 #pragma unroll
           for (int k16 = 0; k16 < BK / UMMA_K; ++k16) {
             if (MODE == kWgrad && k16 >= steps) break;
@@ -599,7 +683,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 ? ptx::make_smem_desc_sw128(sa + k16 * (UMMA_K * 128), BOX_BYTES, 1024)
                 : ptx::make_smem_desc_sw128(sa + k16 * (UMMA_K * 2), 16, 1024);
             const uint64_t b_desc = ptx::make_smem_desc_sw128(sb + k16 * (UMMA_K * 128), BOX_BYTES, 1024);
-            ptx::umma_f16_pair(d_tmem, a_desc, b_desc, idesc, (kb | k16) != 0 ? 1u : 0u);
+            ptx::umma_f16_pair(d_tmem, a_desc, b_desc, idesc, (kb | k16) != 0 || ragged ? 1u : 0u);
           }
           ptx::umma_commit_pair(&sh->empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -611,37 +695,41 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   } else if (warp == 2) {
     // ============================================================== ragged ends
     if constexpr (MODE == kWgrad) {
-      int stage = 0;
-      uint32_t phases = 0;   // bit s: parity of the next use of tail[s]
+      static_assert((CTA_M + CTA_N) / 64 * 8 == 32, "16 bytes of a row per lane");
+      const int box = lane >> 3, chunk = lane & 7;
+      const bool of_a = box < CTA_M / 64;
+      const long pitch = of_a ? p.m : p.n;
+      int side = 0;
       for (int tile = pair; tile < total; tile += num_pairs) {
         const Tile c = decode(sh, n_tiles, tile, group);
-        const int num_kb = (c.rows + BK - 1) / BK;
-        const int last = (stage + num_kb - 1) % STAGES;
-        stage = (stage + num_kb) % STAGES;
-        const int valid = c.rows - (num_kb - 1) * BK;
-        if (valid == BK) continue;
-        if (!ptx::mbar_wait(&sh->tail[last], (phases >> last) & 1, abort_flag)) {
+        const int rest = c.rows % UMMA_K;
+        if (rest == 0) continue;
+        const int col = (of_a ? c.m_tile * TILE_M + rank * CTA_M + box * 64
+                              : c.n_tile * TILE_N + rank * CTA_N + (box - CTA_M / 64) * 64) + chunk * 8;
+        const T* src = static_cast<const T*>(of_a ? p.psrc : p.qsrc) + (static_cast<long>(c.row_begin) + c.rows - rest) * pitch + col;
+        uint4 v[UMMA_K - 1];
+#pragma unroll
+        for (int r = 0; r < UMMA_K - 1; ++r) {
+          v[r] = make_uint4(0u, 0u, 0u, 0u);
+          if (r < rest && col < pitch) v[r] = __ldg(reinterpret_cast<const uint4*>(src + r * pitch));
+        }
+        if (!ptx::mbar_wait(&sh->side_empty[side & 1], ((side >> 1) & 1) ^ 1, abort_flag)) {
           if (lane == 0) {
             sh->abort = 1;
             if (p.status != nullptr) record_failure(p.status, gg::STATUS_TIMEOUT_PRODUCER);
           }
           break;
         }
-        phases ^= 1u << last;
-        // Rows [valid, the next multiple of 16) take part in an MMA step but belong to the next
-        // expert (or lie past the matrix): zero them in all boxes, 128 bytes per row and box.
-        uint8_t* sa = smem + last * STAGE_BYTES;
-        const int zero_rows = ((valid + UMMA_K - 1) / UMMA_K) * UMMA_K - valid;
-        const int items = (CTA_M / 64 + CTA_N / 64) * zero_rows * 8;
-        for (int it = lane; it < items; it += 32) {
-          const int box = it / (zero_rows * 8);
-          const int rem = it - box * (zero_rows * 8);
-          *reinterpret_cast<uint4*>(sa + box * BOX_BYTES + (valid + rem / 8) * 128 + (rem & 7) * 16) = make_uint4(0, 0, 0, 0);
+        // 128-byte swizzle: the 16-byte chunks of row r change places by r % 8
+        uint8_t* at = smem + SIDE_OFF + (side & 1) * SIDE_BYTES + box * SIDE_BOX_BYTES;
+#pragma unroll
+        for (int r = 0; r < UMMA_K; ++r) {
+          *reinterpret_cast<uint4*>(at + r * 128 + ((chunk ^ (r & 7)) << 4)) = r < UMMA_K - 1 ? v[r < UMMA_K - 1 ? r : 0] : make_uint4(0u, 0u, 0u, 0u);
         }
         ptx::fence_proxy_async_smem();
-        ptx::fence_cluster();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa(&sh->full[last], 0));
+        if (lane == 0) ptx::mbar_arrive_release_cluster(ptx::mapa(&sh->side_full[side & 1], 0));
+        ++side;
       }
     }
   } else if (warp == 3) {
@@ -662,6 +750,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           }
         }
       }
+      if (p.psum != nullptr) side_sums<T>(p, sh, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), lane);
     }
   } else {
     // ============================================================== epilogue (warps 4..11)
@@ -693,7 +782,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       et.z = MODE == kWgrad ? c.group : 0;
       Packed32 side;
       if constexpr (MODE == kWgrad) {
-        if (p.psum != nullptr && c.n_tile == 0) {
+        if (p.psum != nullptr && c.n_tile == 0 && c.rows > MAX_SIDE_ROWS) {
           patch_free(et);
           column_sums<T>(p, patches, c, c.m_tile * TILE_M + rank * CTA_M, warp, lane);
         }

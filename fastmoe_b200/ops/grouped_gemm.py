@@ -141,8 +141,8 @@ def wgrad(dy, x, offs, groups, out=None, accumulate=False, with_bias_grad=False)
 
     With ``with_bias_grad`` the per-expert column sums of ``dy`` (the bias gradient of the same
     grouped linear, ``[E, dy.shape[1]]``) are returned as well: ``(dW, db)``.  The tensor-core
-    kernel adds them up in its epilogue warps, which wait for the main loop then, on the tiles of the
-    first column block: no extra launch, and one more read of ``dy``, mostly out of the L2.
+    kernel adds them up in warps that have little else to do beside its main loops: no extra launch, and one
+    more read of ``dy``, mostly out of the L2.
     """
     nat = native.get()
     m, n = dy.shape[1], x.shape[1]

@@ -70,3 +70,36 @@ def test_single_group_without_offsets():
     assert (gg.forward(x, w, None).double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max()
     ref = x[:, :64].double() @ w[0].double()
     assert (gg.dgrad(x[:, :64].contiguous(), w, None).double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max()
+
+
+# the last MMA step of 16 rows full, all but full, of one row, alone; sums by the side warps and, past 2048 rows, by the
+# epilogue; widths that end inside a tile, a 64-wide box and a block of 32 columns
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("counts", [[1], [15, 0, 16, 17, 31], [63, 64, 65, 2, 81], [375] * 6, [2047, 2048, 2049, 5], [0, 0, 7]])
+@pytest.mark.parametrize("m,n", [(8, 32), (264, 96), (520, 288), (1024, 256)])
+def test_weight_gradient_of_ragged_experts(dtype, counts, m, n):
+    r"""Against 64 bits: one rounding to the type and fp32 sums of `rows` products; the neighbours' rows, infinite
+    here, take no part."""
+    from fastmoe_b200.ops import grouped_gemm as gg
+    torch.manual_seed(len(counts) + m)
+    rows = sum(counts)
+    dy = torch.randn(rows + 20, m, device=DEV, dtype=dtype)
+    x = torch.randn(rows + 20, n, device=DEV, dtype=dtype)
+    dy[rows:], x[rows:] = float("inf"), float("nan")   # past the last expert
+    offs = gg.offsets_from_counts(counts, DEV)
+    starts = [sum(counts[:e]) for e in range(len(counts))]
+    poisoned = max(range(len(counts)), key=lambda e: (counts[e] > 0, e))
+    dy[starts[poisoned], 0] = float("inf")
+    dw, db = gg.wgrad(dy, x, offs, len(counts), with_bias_grad=True)
+    grown = torch.ones_like(dw)
+    gg.wgrad(dy, x, offs, len(counts), out=grown, accumulate=True)
+    eps, u = torch.finfo(dtype).eps, 2.0 ** -24
+    for e, c in enumerate(counts):
+        p, q = dy[starts[e]:starts[e] + c].double(), x[starts[e]:starts[e] + c].double()
+        if e == poisoned:
+            p = p[:, 1:]
+        ref, size = p.t() @ q, p.abs().t() @ q.abs()
+        got, more, sums = (t[e].double()[1:] if e == poisoned else t[e].double() for t in (dw, grown, db))
+        assert bool(((got - ref).abs() <= eps * ref.abs() + (c + 1) * u * size + 1e-7).all()), e
+        assert bool(((more - 1 - ref).abs() <= eps * (ref.abs() + 1) + (c + 2) * u * (size + 1)).all()), e
+        assert bool(((sums - p.sum(0)).abs() <= eps * p.sum(0).abs() + (c + 1) * u * p.abs().sum(0) + 1e-7).all()), e
