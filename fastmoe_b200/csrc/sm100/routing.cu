@@ -1424,8 +1424,8 @@ template <> __device__ __forceinline__ void stv<__half>(__half* p, long i, float
   p[i] = __float2half(v);
 }
 
-// Shared-memory tiled SIMT GEMM for fp64, for fp32 with rows that are not 16-byte aligned (sgemm.cu
-// takes the others) and for 16-bit shapes the tensor-core kernel does not take.  One CTA of 256 threads computes a 64 x 64 tile
+// Shared-memory tiled SIMT GEMM for fp64, for fp32 with rows that are not 16-byte aligned (split_gemm.cu
+// and sgemm.cu take the others) and for 16-bit shapes the tensor-core kernel does not take.  One CTA of 256 threads computes a 64 x 64 tile
 // of C = A B with a K step of 16; every thread owns a 4 x 4 block of the tile and accumulates in
 // fp32 (fp64 for doubles).  The three products of a grouped linear differ only in where A(i, kk)
 // and B(kk, j) live:

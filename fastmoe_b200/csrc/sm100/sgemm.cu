@@ -1,5 +1,6 @@
 // fp32 grouped GEMM on the FMA units: the three products of a grouped linear at the full precision
-// of fp32 (the tensor cores' tf32 would drop 13 bits of the inputs).
+// of fp32 (the tensor cores' tf32 would drop 13 bits of the inputs), for calls too small to be worth
+// splitting for the tensor cores (split_gemm.cu).
 //
 // One CTA of 128 threads computes a 64 x 128 tile with a K step of 16; a thread owns 8 x 8 outputs
 // and adds its products in ascending k, one fused multiply-add each (packed two to an instruction:

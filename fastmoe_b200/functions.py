@@ -10,7 +10,8 @@ This path needs the per-expert row counts on the host because user experts are c
 with Python slices; it therefore keeps exactly one device→host read per layer (the
 reference has two plus three ``.cpu()`` copies).  ``FMoETransformerMLP``-shaped experts
 never come here on a GPU: they take the fused path in :mod:`fastmoe_b200.ops.fused`,
-which has no host read at all.
+which has no host read at all.  Other experts of plain tensors on one GPU have their rows moved and
+combined by kernels (``ops/fused.py::general_path``), with one host read for the counts.
 """
 import torch
 import torch.distributed as dist
