@@ -837,6 +837,21 @@ torch::Tensor prune_gate_scalar(torch::Tensor idx, int64_t cap, int64_t tot) {
   return out;
 }
 
+// {[1, padded, d], [1, padded]}: see routing.cuh.
+std::vector<torch::Tensor> gate_pad(torch::Tensor w, c10::optional<torch::Tensor> bias, int64_t padded) {
+  check_rows(w, "w");
+  TORCH_CHECK(w.dim() == 2 && padded >= w.size(0), "gate weight");
+  TORCH_CHECK(!bias.has_value() || (bias->device() == w.device() && bias->scalar_type() == w.scalar_type() &&
+                                    bias->is_contiguous() && bias->numel() == w.size(0)), "gate bias does not fit");
+  c10::cuda::CUDAGuard guard(w.device());
+  auto wp = torch::empty({1, padded, w.size(1)}, w.options());
+  auto bp = torch::empty({1, padded}, w.options());
+  FMOE_CUDA_CHECK(fmoe::launch_gate_pad(dtype16(w), w.data_ptr(), bias.has_value() ? bias->data_ptr() : nullptr,
+                                        static_cast<int>(w.size(0)), static_cast<int>(padded), static_cast<int>(w.size(1)),
+                                        wp.data_ptr(), bp.data_ptr(), cur_stream()));
+  return {wp, bp};
+}
+
 // int32 [groups + 1] exclusive prefix of host counts, on `device` (-1: the current one).
 torch::Tensor host_offsets(torch::Tensor counts_in, int64_t device) {
   TORCH_CHECK(counts_in.device().is_cpu() && counts_in.scalar_type() == torch::kLong && counts_in.dim() == 1 &&
@@ -1145,6 +1160,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("balance_supported", &balance_supported);
   m.def("prune_gate_scalar", &prune_gate_scalar);
   m.def("host_offsets", &host_offsets);
+  m.def("gate_pad", &gate_pad);
   m.def("balance_loss", &balance_loss);
   m.def("balance_bwd", &balance_bwd);
   m.def("switch_top1", &switch_top1);

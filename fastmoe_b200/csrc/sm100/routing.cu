@@ -834,6 +834,25 @@ switch_top1_kernel(const T* __restrict__ logits, int n, int tot, int64_t* __rest
 }
 
 // new_idx[s] = idx[s] when fewer than `cap` slots of its expert come before it, else -1
+// What the tensor-core gate multiplies with when its experts are no multiple of 64: one launch where padding,
+// filling and copying were four (a layer's step, eager, 16 experts, 1237 tokens, d 256: 472 -> 430 us).
+template <typename T>
+__global__ void __launch_bounds__(256)
+gate_pad_kernel(const T* __restrict__ w, const T* __restrict__ bias, int tot, int padded, int d, T* __restrict__ w_out,
+                T* __restrict__ bias_out) {
+  ptx::chain_begin();
+  const long held = static_cast<long>(tot) * d / 8, all = static_cast<long>(padded) * d / 8;
+  for (long i = static_cast<long>(blockIdx.x) * 256 + threadIdx.x; i < all; i += static_cast<long>(gridDim.x) * 256) {
+    reinterpret_cast<uint4*>(w_out)[i] = i < held ? reinterpret_cast<const uint4*>(w)[i] : make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (blockIdx.x == 0) {
+    for (int e = threadIdx.x; e < padded; e += 256) {
+      // (-30000: representable in both types)
+      bias_out[e] = e >= tot ? V2<T>::from_f(-30000.f) : bias != nullptr ? bias[e] : V2<T>::from_f(0.f);
+    }
+  }
+}
+
 // Host values that travel with the launch, in place of the operations that formed the prefix on the host and a
 // copy from pageable memory: a grouped linear's forward and backward, 16 experts, 142 rows, d 320, 197 -> 162 us.
 template <int N> struct HostValues {
@@ -1826,6 +1845,17 @@ cudaError_t launch_switch_top1(int code, const void* logits, int n, int tot, int
       (switch_top1_kernel<T, TOT><<<balance_blocks(n), kBalanceThreads, 0, stream>>>(
            static_cast<const T*>(logits), n, tot, win, static_cast<T*>(score)))));
   return cudaGetLastError();
+}
+
+cudaError_t launch_gate_pad(int dtype, const void* w, const void* bias, int tot, int padded, int d, void* w_out, void* bias_out,
+                            cudaStream_t stream) {
+  cudaError_t chained = cudaSuccess;
+  if (tot < 1 || padded < tot || d < 8 || d % 8 != 0) return cudaErrorInvalidValue;
+  const long chunks = static_cast<long>(padded) * d / 8;
+  const unsigned grid = static_cast<unsigned>(chunks < 148L * 4 * 256 ? (chunks + 255) / 256 : 148 * 4);
+  FMOE_DISPATCH_16(dtype, (chained = launch_chained(gate_pad_kernel<T>, dim3(grid), dim3(256), 0, stream, static_cast<const T*>(w),
+      static_cast<const T*>(bias), tot, padded, d, static_cast<T*>(w_out), static_cast<T*>(bias_out))));
+  return chained;
 }
 
 template <int N>

@@ -85,6 +85,11 @@ cudaError_t launch_balance_bwd(int logit_dtype, const void* logits, long pitch, 
 cudaError_t launch_switch_top1(int logit_dtype, const void* logits, int n, int tot, int64_t* win, void* score,
                                cudaStream_t stream);
 
+// Weight [tot, d] and bias [tot] (or null) of a 16-bit gate followed by rows of zeros and a bias that no top-k
+// selects, up to `padded` experts.  d % 8 == 0, 16-byte aligned.
+cudaError_t launch_gate_pad(int dtype, const void* w, const void* bias, int tot, int padded, int d, void* w_out, void* bias_out,
+                            cudaStream_t stream);
+
 // dst[i] = values[i] for host values, i < n <= kMaxHostOffsets.
 constexpr int kMaxHostOffsets = 960;
 cudaError_t launch_host_offsets(const int* values, int n, int* dst, cudaStream_t stream);

@@ -128,14 +128,11 @@ def traced():
     return torch._C._get_tracing_state() is not None   # pylint: disable=protected-access
 
 
-_PAD_BIAS = -30000.0   # bias of the padding columns: representable in bf16 and fp16, never selected
-
-
 class _GateGemm(Function):
     r"""``logits = x W^T + b`` on the tcgen05 grouped-GEMM kernel (one group, whose row count goes
     with the launch: no offsets on the device), for any number of experts.  The expert dimension is padded to a multiple of 64 — the padding columns get a
     large negative bias, so a top-k over the padded logits never selects them; 64, 128 ... experts need no
-    copies — and the backward products ``dx = dl W`` and ``dW = dl^T x`` (with ``db`` from the same launch) run on
+    copies, others one launch — and the backward products ``dx = dl W`` and ``dW = dl^T x`` (with ``db`` from the same launch) run on
     the same kernel's input-gradient and weight-gradient modes."""
 
     @staticmethod
@@ -146,12 +143,7 @@ class _GateGemm(Function):
             wp = weight.contiguous().unsqueeze(0)
             bp = None if bias is None else bias.contiguous().unsqueeze(0)
         else:
-            wp = torch.nn.functional.pad(weight, (0, 0, 0, pad)).unsqueeze(0).contiguous()
-            bp = torch.full((1, tot + pad), _PAD_BIAS, dtype=x.dtype, device=x.device)
-            if bias is not None:
-                bp[0, :tot] = bias
-            else:
-                bp[0, :tot] = 0
+            wp, bp = native.get().gate_pad(gg.aligned(weight, 16), None if bias is None else bias.contiguous(), tot + pad)
         logits = gg.forward(x, wp, None, bp)
         ctx.save_for_backward(x, wp)
         ctx.tot = tot

@@ -144,3 +144,30 @@ def test_fp32_gate_keeps_subclasses_and_autocast_on_the_operations():
         assert gating.linear_topk_softmax(x, w, None, 2)[0].dtype == torch.bfloat16
     with pytest.raises(RuntimeError):
         gating.linear_topk_softmax(x, w[:, :56], None, 2)   # widths that differ
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tot,d,bias", [(9, 64, True), (16, 1024, True), (63, 192, False), (65, 16384, True), (200, 4096, False)])
+def test_padded_gate(dtype, tot, d, bias):
+    torch.manual_seed(tot)
+    w = torch.randn(tot, d, device=DEV, dtype=dtype)
+    b = torch.randn(tot, device=DEV, dtype=dtype) if bias else None
+    pad = -tot % 64
+    wp, bp = _native().gate_pad(w, b, tot + pad)
+    assert torch.equal(wp, torch.nn.functional.pad(w, (0, 0, 0, pad)).unsqueeze(0))
+    want = torch.full((1, tot + pad), -30000.0, device=DEV, dtype=dtype)
+    want[0, :tot] = b if bias else 0
+    assert torch.equal(bp, want)
+
+
+def test_padded_gate_of_views():
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(0)
+    flat = torch.randn(16 * 128 + 1, device=DEV).bfloat16()
+    w = flat[1:].view(16, 128)                                       # an odd address
+    b = torch.randn(32, device=DEV).bfloat16()[::2]
+    x = torch.randn(600, 128, device=DEV).bfloat16()
+    odd = gating._GateGemm.apply(x, w, b)
+    strided = gating._GateGemm.apply(x, w.t().contiguous().t(), b.clone())
+    plain = gating._GateGemm.apply(x, w.clone(), b.clone())
+    assert torch.equal(odd, plain) and torch.equal(strided, plain)
