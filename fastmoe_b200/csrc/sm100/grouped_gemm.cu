@@ -3,6 +3,8 @@
 // gradients), grouped_gemm_kernel.cuh (row modes with rows arriving from or leaving for other GPUs) —
 // instantiated per element type in slim_gemm_*.cu / pair_gemm_*.cu / grouped_gemm_*.cu — and
 // narrow_gemm.cu (decoding).
+#include <algorithm>
+
 #include "grouped_gemm_kernel.cuh"
 #include "narrow_gemm.cuh"
 #include "pair_gemm_kernel.cuh"
@@ -127,6 +129,21 @@ bool pair_applies(const GroupedGemmArgs& a) {
          a.pre_out == nullptr && a.act != kActNone && a.epi == kEpiDAct && a.aux != nullptr;
 }
 
+// Whether the column sums of a weight gradient end before its main loops when one warp per CTA forms them.  In
+// us: an item of 32 columns takes 1.7 and 0.9 more per 128 rows, a tile 0.6 per 64 rows and not less than 2.1.  The
+// epilogue warps' sums against that warp's (launch with the sums, us): 8 experts, 2048 rows, 2048 x 256: 21
+// against 73, x 512: 36, 72, x 1024: 64, 61; 8 of 1000, 4096 x 256: 24, 68, x 512: 39, 69, x 1024: 63, 60; 16 of 512,
+// 1024 x 256: 10, 16, x 1024: 21, 20; 16 of 64, 1024 x 1024: 13.0, 10.8; 2 of 4096, 4096 x 1024: 60, 57; 1 of 8192,
+// 64 x 1024: 59, 50.  The margin of 1.3 is for rows that are in the L2.
+bool sums_beside(const GroupedGemmArgs& a, int grid) {
+  const long rows = (a.rows_cap + a.num_groups - 1) / a.num_groups;
+  const long items = static_cast<long>(a.num_groups) * ((a.m + pg::SUM_COLS - 1) / pg::SUM_COLS);
+  const long tiles = static_cast<long>(a.num_groups) * ((a.m + pg::TILE_M - 1) / pg::TILE_M) * ((a.n + pg::TILE_N - 1) / pg::TILE_N);
+  const double item = 1.7 + 0.9 * static_cast<double>((rows + 127) / 128);
+  const double tile = std::max(2.1, 0.6 * static_cast<double>((rows + BK - 1) / BK));
+  return static_cast<double>((items + grid - 1) / grid) * item <= 1.3 * static_cast<double>((tiles + grid / 2 - 1) / (grid / 2)) * tile;
+}
+
 template <typename P> void set_offsets(P& p, const GroupedGemmArgs& a) {
   p.offs = a.offs;
   p.one_group[0] = 0;
@@ -211,6 +228,7 @@ cudaError_t launch_pair_gemm(const GroupedGemmArgs& a) {
   p.qsrc = a.b;
   p.status = a.status;
   const int grid = (a.num_sms > 1 ? a.num_sms : 148) & ~1;
+  p.side_sums = p.psum != nullptr && sums_beside(a, grid) ? 1 : 0;
   return a.dtype == kBF16 ? pg::launch_bf16(a.mode, a.act, ta, tb, tc, p, grid, a.stream)
                           : pg::launch_f16(a.mode, a.act, ta, tb, tc, p, grid, a.stream);
 }

@@ -90,6 +90,7 @@ struct Params {
   int accumulate;
   int out_fp32;
   void* psum;
+  int side_sums;
   const void* psrc;      // weight gradient: the operands again
   const void* qsrc;
   int* status;
@@ -387,7 +388,7 @@ __device__ __forceinline__ void epilogue_tile_update(const Params& p, const EpiT
 }
 
 // The bias gradient of a grouped linear is the column sum, per expert, of the matrix its weight
-// gradient takes as P.  Of an expert with many rows (few have): on the tiles of the first N column block the epilogue warps, which wait
+// gradient takes as P.  Either (`side_sums` = 0) on the tiles of the first N column block the epilogue warps, which wait
 // for the main loop then, add up this CTA's 128 columns of P with plain 16-byte loads (the rows
 // pass through the L2 for the TMA loads at the same time).
 template <typename T>
@@ -448,12 +449,12 @@ __device__ __forceinline__ void column_sums(const Params& p, uint8_t* patches, c
   asm volatile("bar.sync 2, %0;" ::"n"(NUM_EPI_WARPS * 32) : "memory");
 }
 
-// Of the others: 32 columns at a time by the warps that have little else to do, beside the main loops.  The
+// Or 32 columns at a time by the warps that have little else to do, beside the main loops.  The
 // epilogue warps wait for the loads' latency on every tile of the first column block: what the sums add,
 // 1024 <-> 4096, 16 experts of 64 rows 9.6 us, here 1 to 3, of 128 rows 8.7, here 0.5; 8 of 2048 rows 10.1, here 3.
-// (64 columns at a time and 32 loads in flight took two to three times as long.)
+// (64 columns at a time and 32 loads in flight took two to three times as long.)  The rule between the two
+// is sums_beside() in grouped_gemm.cu.
 constexpr int SUM_COLS = 32;
-constexpr int MAX_SIDE_ROWS = 2048;
 template <typename T>
 __device__ __forceinline__ void side_sums(const Params& p, const Shared* sh, int worker, int workers, int lane) {
   const int blocks = (p.m + SUM_COLS - 1) / SUM_COLS;
@@ -467,7 +468,7 @@ __device__ __forceinline__ void side_sums(const Params& p, const Shared* sh, int
   long item = worker;
   for (int g = 0; g < p.num_groups; ++g) {
     const int begin = sh->offs[g], end = sh->offs[g + 1];
-    if (end == begin || end - begin > MAX_SIDE_ROWS) continue;
+    if (end == begin) continue;
     for (; item < blocks; item += workers) {
       const int col = static_cast<int>(item) * SUM_COLS + (lane & 3) * 8;
       float cs[8];
@@ -750,7 +751,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           }
         }
       }
-      if (p.psum != nullptr) side_sums<T>(p, sh, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), lane);
+      if (p.psum != nullptr && p.side_sums) side_sums<T>(p, sh, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), lane);
     }
   } else {
     // ============================================================== epilogue (warps 4..11)
@@ -782,7 +783,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       et.z = MODE == kWgrad ? c.group : 0;
       Packed32 side;
       if constexpr (MODE == kWgrad) {
-        if (p.psum != nullptr && c.n_tile == 0 && c.rows > MAX_SIDE_ROWS) {
+        if (p.psum != nullptr && !p.side_sums && c.n_tile == 0) {
           patch_free(et);
           column_sums<T>(p, patches, c, c.m_tile * TILE_M + rank * CTA_M, warp, lane);
         }

@@ -72,10 +72,10 @@ def test_single_group_without_offsets():
     assert (gg.dgrad(x[:, :64].contiguous(), w, None).double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max()
 
 
-# the last MMA step of 16 rows full, all but full, of one row, alone; sums by the side warps and, past 2048 rows, by the
-# epilogue; widths that end inside a tile, a 64-wide box and a block of 32 columns
+# the last MMA step of 16 rows full, all but full, of one row, alone; sums by the side warps and, where those
+# would take longer than the tiles (12 experts), by the epilogue; widths that end inside a tile, a 64-wide box and a block of 32 columns
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("counts", [[1], [15, 0, 16, 17, 31], [63, 64, 65, 2, 81], [375] * 6, [2047, 2048, 2049, 5], [0, 0, 7]])
+@pytest.mark.parametrize("counts", [[1], [15, 0, 16, 17, 31], [63, 64, 65, 2, 81], [375] * 6, [300] * 12, [2047, 2048, 2049, 5], [0, 0, 7]])
 @pytest.mark.parametrize("m,n", [(8, 32), (264, 96), (520, 288), (1024, 256)])
 def test_weight_gradient_of_ragged_experts(dtype, counts, m, n):
     r"""Against 64 bits: one rounding to the type and fp32 sums of `rows` products; the neighbours' rows, infinite
