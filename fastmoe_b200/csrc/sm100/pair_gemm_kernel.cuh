@@ -6,8 +6,9 @@
 // holds rows [128 r, 128 r + 128) of A, columns [128 r, 128 r + 128) of B and the accumulators of
 // its rows.  Per 64-wide K block an SM loads 32 KB where a 128 x 256 tile on one SM loads 48 KB.
 // Measured, bf16, 8192 rows, 2 experts, 1024 <-> 4096: input gradient with GELU's derivative 67.3 us,
-// weight gradient 63.5 us (1080 TFLOP/s), where the single-CTA kernel took 78.4 and 70.1 us.  What
-// bounds it: the last of the waves (128 tiles on 74 pairs) and, with an activation, the epilogue.
+// weight gradient with the bias gradient 57.1 us (1200 TFLOP/s), where the single-CTA kernel took 78.4 and 70.1
+// us.  What bounds it: the last of the waves (128 tiles on 74 pairs), the L2 (8 TB/s to the SMs at 0.6 us per K
+// block) and, with an activation, the epilogue.
 //
 // Roles of a CTA (384 threads), persistent over the tiles of its pair:
 //   warp 0      TMA producer, one lane: this CTA's halves of A and B into a 5-stage ring; the
