@@ -510,13 +510,34 @@ void wide_grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::Te
 }
 
 // ------------------------------------------------------------------------------ row movement
+// The kernels read the tables of the slots, and a weight per slot in the type of the rows, through plain pointers.
+void check_slots(const torch::Tensor& rows, int64_t tokens, int64_t k, const torch::Tensor& idx, const torch::Tensor& rank,
+                 const torch::Tensor& base) {
+  for (const auto& t : {idx, rank, base}) {
+    check_cuda_contig(t, "slot table");
+    TORCH_CHECK(t.device() == rows.device(), "slot table on another device than the rows");
+  }
+  TORCH_CHECK(rows.dim() == 2 && k > 0 && idx.numel() == tokens * k && rank.numel() == idx.numel(), "slot tables do not fit the rows");
+}
+void check_weight(const torch::Tensor& rows, const torch::Tensor& idx, const torch::Tensor& weight) {
+  check_cuda_contig(weight, "slot weights");
+  TORCH_CHECK(weight.device() == rows.device() && weight.scalar_type() == rows.scalar_type() && weight.numel() == idx.numel(),
+              "slot weights: one per slot, in the type of the rows");
+}
+const void* weight_ptr(const torch::Tensor& rows, const torch::Tensor& idx, const c10::optional<torch::Tensor>& weight) {
+  if (!weight.has_value() || !weight->defined()) return nullptr;
+  check_weight(rows, idx, *weight);
+  return weight->data_ptr();
+}
+
 void scatter_rows(torch::Tensor src, torch::Tensor idx, torch::Tensor rank, torch::Tensor base,
                   c10::optional<torch::Tensor> scale, int64_t k, torch::Tensor dst,
                   c10::optional<torch::Tensor> row_slot) {
   check_rows(src, "src");
   check_rows(dst, "dst");
   c10::cuda::CUDAGuard guard(src.device());
-  const void* sc = (scale.has_value() && scale->defined()) ? scale->data_ptr() : nullptr;
+  check_slots(src, src.size(0), k, idx, rank, base);
+  const void* sc = weight_ptr(src, idx, scale);
   int* rs = (row_slot.has_value() && row_slot->defined()) ? row_slot->data_ptr<int>() : nullptr;
   // unscaled fp32 rows are moved as 16-bit rows of twice the width
   const bool wide = src.scalar_type() == torch::kFloat;
@@ -533,7 +554,8 @@ void gather_combine(torch::Tensor rows, torch::Tensor idx, torch::Tensor rank, t
   check_rows(rows, "rows");
   check_rows(out, "out");
   c10::cuda::CUDAGuard guard(rows.device());
-  const void* w = (weight.has_value() && weight->defined()) ? weight->data_ptr() : nullptr;
+  check_slots(rows, out.size(0), k, idx, rank, base);
+  const void* w = weight_ptr(rows, idx, weight);
   if (rows.scalar_type() == torch::kFloat) {
     TORCH_CHECK(rows.size(1) % 8 == 0, "fp32 rows of a multiple of 8 columns");
     FMOE_CUDA_CHECK(fmoe::launch_combine_f32(rows.data_ptr<float>(), idx.data_ptr<int64_t>(), rank.data_ptr<int>(),
@@ -557,6 +579,9 @@ void combine_bwd(torch::Tensor dout, torch::Tensor rows, torch::Tensor idx, torc
   check_rows(rows, "rows");
   check_rows(drows, "drows");
   c10::cuda::CUDAGuard guard(dout.device());
+  check_slots(rows, dout.size(0), k, idx, rank, base);
+  check_weight(rows, idx, weight);
+  check_weight(rows, idx, dscore);
   if (dout.scalar_type() == torch::kFloat) {
     TORCH_CHECK(dout.size(1) % 8 == 0, "fp32 rows of a multiple of 8 columns");
     FMOE_CUDA_CHECK(fmoe::launch_combine_bwd_f32(dout.data_ptr<float>(), rows.data_ptr<float>(), idx.data_ptr<int64_t>(),

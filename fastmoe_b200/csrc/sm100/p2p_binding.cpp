@@ -165,6 +165,9 @@ class ExchangeContext {
                     int64_t capacity_rows) {
     c10::cuda::CUDAGuard guard(out.device());
     const void* w = (weight.has_value() && weight->defined()) ? weight->data_ptr() : nullptr;
+    TORCH_CHECK(w == nullptr || (weight->is_cuda() && weight->is_contiguous() && weight->scalar_type() == out.scalar_type() &&
+                                 weight->numel() == idx.numel()),
+                "wait_combine: one weight per slot, in the type of the rows");
     void* kp = (keep.has_value() && keep->defined()) ? keep->data_ptr() : nullptr;
     const int* rk = nullptr;
     const int* db = nullptr;

@@ -77,6 +77,12 @@ def _rows_of_slots(idx, rank, offs):
     return torch.where(kept, offs[idx.clamp(0, offs.numel() - 2)] + rank, 0).long(), kept
 
 
+def slot_scores(scores, dtype):
+    r"""One score per slot for the kernels, which read them next to each other: ``reshape`` returns a strided
+    view where it can (a column of a table, an expanded constant)."""
+    return scores.reshape(-1).to(dtype).contiguous()
+
+
 class _Dispatch(Function):
     r"""``xs[offs[e] + rank[s]] = x[s // k]`` for every kept slot ``s`` routed to expert ``e``;
     ``n_rows``: rows of ``xs`` where the caller knows how many slots are kept."""
@@ -163,7 +169,7 @@ def general_path(x, ids, scores, expert_fn, num_expert):
     ys = expert_fn(xs, counts)
     if (torch.is_tensor(ys) and ys.is_cuda and ys.dim() == 2 and ys.dtype in _TC + (torch.float32,)
             and ys.shape[0] == n_rows and ys.shape[1] % 8 == 0 and ys.shape[1] > 0 and ys.device == x.device):
-        return _Combine.apply(ys.contiguous(), scores.reshape(-1).to(ys.dtype), idx, rank, offs, k), ys, None
+        return _Combine.apply(ys.contiguous(), slot_scores(scores, ys.dtype), idx, rank, offs, k), ys, None
     return None, ys, (pos[:n_rows].long(), counts)
 
 
@@ -238,7 +244,7 @@ def moe_mlp_local(x, gate_idx, gate_score, w1, b1, w2, b2, activation):
     nat = native.get()
     k = gate_idx.shape[1]
     idx = gate_idx.contiguous().view(-1)
-    score = gate_score.reshape(-1).to(x.dtype)
+    score = slot_scores(gate_score, x.dtype)
     _counts, rank, offs = nat.route_offs(idx, w1.shape[0])
     xs = _Dispatch.apply(x.contiguous(), idx, rank, offs, k)
     ys = expert_mlp_weights(xs, offs, w1.contiguous(), b1.contiguous(), w2.contiguous(), b2.contiguous(),
@@ -306,7 +312,7 @@ def moe_mlp_forward(layer, x, gate_idx, gate_score):
         return run(*args, gate_idx, gg.ACT_CODES[activation_kind(e.activation)], keep)
     k = gate_idx.shape[1]
     idx = gate_idx.contiguous().view(-1)
-    score = gate_score.reshape(-1).to(x.dtype)
+    score = slot_scores(gate_score, x.dtype)
     with fused_range("route"):
         counts, rank, offs = nat.route_offs(idx, layer.num_expert)
     if config.debug_bounds():

@@ -546,7 +546,7 @@ def moe_mlp_forward(layer, x, gate_idx, gate_score):
     n_expert = layer.num_expert
     budget = ws.token_budget(x.shape[0])
     idx = gate_idx.contiguous().view(-1)
-    score = gate_score.reshape(-1).to(x.dtype)
+    score = fused.slot_scores(gate_score, x.dtype)
     lec, rank, my_offs, pos = nat.route_pos(idx, n_expert * ws.world)
     if config.debug_bounds():
         from ..utils.profiling import check_routing

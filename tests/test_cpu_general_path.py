@@ -1,0 +1,96 @@
+r"""The glue around the general path's row kernels, with a stand-in for the kernels that runs on the CPU
+and, as they do, reads its operands through their pointers."""
+import pytest
+import torch
+import torch.nn as nn
+
+from fastmoe_b200 import FMoE
+from fastmoe_b200.ops import fused, native, torch_impl
+
+
+def _flat(t, n):
+    r"""What a kernel sees at ``t.data_ptr()``: ``n`` values in a row (an error where the storage is shorter)."""
+    return torch.as_strided(t, (n,), (1,))
+
+
+class _Kernels:
+    @staticmethod
+    def route_pos(idx, tot):
+        counts = torch_impl.expert_count(idx, tot).to(torch.int32)
+        rank = torch_impl.slot_rank(idx, tot).reshape(-1).to(torch.int32)
+        offs = torch.zeros(tot + 1, dtype=torch.int32)
+        offs[1:] = counts.cumsum(0)
+        pos = torch_impl.assign_pos(idx, tot).to(torch.int32)
+        return counts, rank, offs, pos
+
+    @staticmethod
+    def _rows(idx, rank, offs):
+        kept = rank >= 0
+        return kept, (offs[idx.clamp(min=0)] + rank)[kept].long()
+
+    def scatter_rows(self, src, idx, rank, offs, _scale, k, dst, _row_slot):
+        kept, row = self._rows(idx, rank, offs)
+        dst[row] = src.repeat_interleave(k, 0)[kept]
+
+    def gather_combine(self, rows, idx, rank, offs, weight, k, out):
+        kept, row = self._rows(idx, rank, offs)
+        slots = torch.zeros(idx.numel(), rows.shape[1], dtype=rows.dtype)
+        slots[kept] = rows[row]
+        if weight is not None:
+            slots = slots * _flat(weight, idx.numel())[:, None]
+        out.copy_(slots.view(out.shape[0], k, -1).sum(1))
+
+    def combine_bwd(self, dout, rows, idx, rank, offs, weight, k, drows, dscore):
+        kept, row = self._rows(idx, rank, offs)
+        g = dout.repeat_interleave(k, 0)
+        drows[row] = (g * _flat(weight, idx.numel())[:, None])[kept]
+        ds = _flat(dscore, idx.numel())
+        ds.zero_()
+        ds[kept] = (g[kept] * rows[row]).sum(1)
+
+
+@pytest.fixture(autouse=True)
+def kernels(monkeypatch):
+    monkeypatch.setattr(native, "get", _Kernels)
+
+
+class _Expert(nn.Module):
+    def __init__(self, d):
+        super().__init__()
+        self.fc = nn.Linear(d, d)
+
+    def forward(self, x, _count):
+        return torch.tanh(self.fc(x))
+
+
+def _layer(experts=3, d=16, k=2, cls=FMoE, expert=_Expert):
+    torch.manual_seed(0)
+    return cls(num_expert=experts, d_model=d, top_k=k, expert=expert).double()
+
+
+def _general(layer, x, ids, scores):
+    return fused.general_path(x, ids, scores, layer.expert_fn, layer.num_expert)[0]
+
+
+@pytest.fixture(autouse=True)
+def any_type(monkeypatch):
+    monkeypatch.setattr(fused, "_TC", (torch.float64,))
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True, raising=False)
+
+
+@pytest.mark.parametrize("kind", ["column", "one value"])
+def test_scores_need_not_lie_next_to_each_other(kind):
+    layer = _layer(k=1)
+    torch.manual_seed(1)
+    x, ids = torch.randn(10, 16, dtype=torch.float64), torch.randint(0, 3, (10, 1))
+    table = torch.rand(10, 5, dtype=torch.float64) if kind == "column" else torch.rand(1, 1, dtype=torch.float64)
+    results = []
+    for apart in (True, False):
+        leaf = table.clone().requires_grad_(True)
+        scores = leaf[:, :1] if kind == "column" else leaf.expand(10, 1)
+        assert scores.reshape(-1).is_contiguous() is False
+        out = _general(layer, x, ids, scores if apart else scores.contiguous())
+        out.square().sum().backward()
+        results.append((out.detach(), leaf.grad))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)

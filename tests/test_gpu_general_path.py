@@ -127,3 +127,44 @@ def test_offsets_of_host_counts(groups):
     offs = gg.offsets_from_counts(kept, torch.device("cuda", 0))
     kept.zero_()   # the call has taken what it needs
     assert torch.equal(offs.cpu(), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["column", "one value"])
+def test_scores_need_not_lie_next_to_each_other(dtype, kind):
+    from fastmoe_b200 import FMoETransformerMLP
+    general = _layer(3, 64, 64, 1, "plain", dtype)
+    between = FMoETransformerMLP(3, 64, 64, nn.Tanh(), top_k=1).to(DEV).to(dtype)   # no fused activation
+    torch.manual_seed(3)
+    x = torch.randn(50, 64, device=DEV, dtype=dtype)
+    ids = torch.randint(-1, 3, (50, 1), device=DEV)
+    table = torch.rand(50, 5, device=DEV, dtype=dtype) if kind == "column" else torch.rand(1, 1, device=DEV, dtype=dtype)
+    for run in (general._general_path, lambda *a: between._fused_forward(*a) if dtype != torch.float32 else general._general_path(*a)):
+        results = []
+        for apart in (True, False):
+            leaf = table.clone().requires_grad_(True)
+            scores = leaf[:, :1] if kind == "column" else leaf.expand(50, 1)
+            out = run(x, ids, scores if apart else scores.contiguous())
+            out.sum().backward()
+            results.append((out.detach(), leaf.grad))
+        for a, b in zip(*results):
+            assert torch.equal(a, b)
+
+
+def test_row_kernels_refuse_slot_tables_that_do_not_fit():
+    from fastmoe_b200.ops import native
+    nat = native.get()
+    rows, out = torch.zeros(8, 64, device=DEV), torch.zeros(4, 64, device=DEV)
+    idx = torch.zeros(8, device=DEV, dtype=torch.int64)
+    _counts, rank, offs = nat.route_offs(idx, 1)
+    score = torch.ones(8, 2, device=DEV)
+    for bad in (score[:, 0], score[:4, 0].contiguous(), score[:, 0].contiguous().double(), torch.ones(8)):
+        with pytest.raises(RuntimeError):
+            nat.gather_combine(rows, idx, rank, offs, bad, 2, out)
+        with pytest.raises(RuntimeError):
+            nat.combine_bwd(out, rows, idx, rank, offs, bad, 2, rows.clone(), torch.ones(8, device=DEV))
+    for k, table in ((1, idx), (2, idx[:4]), (2, idx.cpu())):
+        with pytest.raises(RuntimeError):
+            nat.gather_combine(rows, table, rank, offs, None, k, out)
+        with pytest.raises(RuntimeError):
+            nat.scatter_rows(out, table, rank, offs, None, k, rows, None)
