@@ -725,6 +725,9 @@ std::vector<torch::Tensor> moe_mlp_forward(torch::Tensor x_in, torch::Tensor idx
                                            torch::Tensor w1_in, torch::Tensor b1_in, torch::Tensor w2_in,
                                            torch::Tensor b2_in, int64_t act, bool keep) {
   c10::cuda::CUDAGuard guard(x_in.device());
+  TORCH_CHECK(x_in.dim() == 2 && idx_in.device() == x_in.device() && score_in.device() == x_in.device() &&
+              x_in.size(0) > 0 && idx_in.numel() % x_in.size(0) == 0 && idx_in.numel() > 0 && score_in.numel() == idx_in.numel(),
+              "moe_mlp: ids and scores do not fit the rows");
   const torch::Tensor x = aligned(x_in, 16);
   const torch::Tensor idx = idx_in.contiguous().view({-1});
   const torch::Tensor score = score_in.reshape({-1}).to(x.scalar_type()).contiguous();

@@ -29,12 +29,13 @@ from ..utils.profiling import check_routing, fused_range
 _TC = (torch.bfloat16, torch.float16)
 
 
-def supports(layer, x, idx):
-    r"""Whether the fused kernels can run this call (else the general path is used)."""
+def supports(layer, x, idx, score=None):
+    r"""Whether the fused kernels can run this call (else the general path is used).  Without ``score`` the
+    question is whether they can with scores that fit the ids."""
     if not native.available() or idx.dim() != 2:
         return False
     if x.dtype == torch.float32:
-        return _fp32_layer_ok(layer, x, idx)
+        return _fp32_layer_ok(layer, x, idx, score)
     if x.dtype not in _TC:
         return False
     e = layer.experts
@@ -49,7 +50,7 @@ def supports(layer, x, idx):
     return True
 
 
-def _fp32_layer_ok(layer, x, idx):
+def _fp32_layer_ok(layer, x, idx, score):
     r"""Whether the fp32 layer on one GPU runs as :class:`_MoEMLP`.  The general path, which takes the
     rest, calls the expert modules: a call that somebody watches stays there, and so does autocast,
     under which the weighted sum is formed in 16 bits."""
@@ -60,8 +61,9 @@ def _fp32_layer_ok(layer, x, idx):
     if any(t is None or t.dtype != torch.float32 or not t.is_cuda
            for t in (e.htoh4.weight, e.htoh4.bias, e.h4toh.weight, e.h4toh.bias)):
         return False
-    return (_native_call_ok(layer, x, idx) and native.get().moe_mlp_supported_f32(
-        layer.num_expert, layer.d_model, layer.d_hidden, idx.numel()))
+    # (as many choices as the layer was made for: the general path refuses others)
+    return (idx.shape[1] == layer.top_k and _native_call_ok(layer, x, idx, score)
+            and native.get().moe_mlp_supported_f32(layer.num_expert, layer.d_model, layer.d_hidden, idx.numel()))
 
 
 def _forced_ep():
@@ -283,17 +285,20 @@ class _MoEMLP(Function):
         return (dx, dscore.to(dtype).view(shape) if need[1] else None, dw1, db1, dw2, db2, None, None, None)
 
 
-def _native_call_ok(layer, x, gate_idx):
+def _native_call_ok(layer, x, gate_idx, gate_score):
     r"""What :class:`_MoEMLP` asks of a call in any type: an activation the GEMM epilogue knows, at
-    least one row, and nobody who wants to look between the launches."""
+    least one row, an id and a score per slot beside it, and nobody who wants to look between the launches."""
     act = activation_kind(layer.experts.activation)
     return (act is not None and x.dim() == 2 and x.shape[0] > 0 and gate_idx.shape[1] > 0
             and gate_idx.shape[0] == x.shape[0] and gate_idx.dtype == torch.int64
+            and gate_idx.device == x.device
+            and (gate_score is None or (gate_score.numel() == gate_idx.numel() and gate_score.device == x.device
+                                        and gate_score.is_floating_point()))
             and not config.nvtx_enabled() and not config.debug_bounds())
 
 
-def _native_layer_ok(layer, x, gate_idx):
-    return (_native_call_ok(layer, x, gate_idx)
+def _native_layer_ok(layer, x, gate_idx, gate_score):
+    return (_native_call_ok(layer, x, gate_idx, gate_score)
             and (x.dtype == torch.float32   # `supports` has looked at the shapes
                  or native.get().moe_mlp_supported(layer.num_expert, layer.d_model, layer.d_hidden)))
 
@@ -304,7 +309,7 @@ def moe_mlp_forward(layer, x, gate_idx, gate_score):
         from ..parallel import symm
         return symm.moe_mlp_forward(layer, x, gate_idx, gate_score)
     nat = native.get()
-    if _native_layer_ok(layer, x, gate_idx):
+    if _native_layer_ok(layer, x, gate_idx, gate_score):
         e = layer.experts
         args = (x, gate_score, e.htoh4.weight, e.htoh4.bias, e.h4toh.weight, e.h4toh.bias)
         keep = torch.is_grad_enabled() and any(t.requires_grad for t in args)

@@ -166,7 +166,7 @@ class FMoETransformerMLP(FMoE):
             return None
         from . import config
         from .ops import fused
-        if not fused.supports(self, moe_inp, gate_top_k_idx):
+        if not fused.supports(self, moe_inp, gate_top_k_idx, gate_score):
             return None
         if (config.faster_schedule_enabled() and config.faster_shadow_enabled()
                 and self.world_size > 1):

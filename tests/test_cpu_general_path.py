@@ -48,10 +48,19 @@ class _Kernels:
         ds.zero_()
         ds[kept] = (g[kept] * rows[row]).sum(1)
 
+    @staticmethod
+    def moe_mlp_supported_f32(*_sizes):
+        return True
+
+    @staticmethod
+    def moe_mlp(*_args):
+        raise AssertionError("the layer's kernels were launched")
+
 
 @pytest.fixture(autouse=True)
 def kernels(monkeypatch):
     monkeypatch.setattr(native, "get", _Kernels)
+    monkeypatch.setattr(native, "available", lambda: True)
 
 
 class _Expert(nn.Module):
@@ -94,3 +103,24 @@ def test_scores_need_not_lie_next_to_each_other(kind):
         results.append((out.detach(), leaf.grad))
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("what", ["fits", "one score per token", "more choices than the layer's", "scores elsewhere",
+                                  "ids elsewhere"])
+def test_fp32_layer_looks_at_what_the_gate_returned(what):
+    from fastmoe_b200 import FMoETransformerMLP
+    layer = FMoETransformerMLP(num_expert=3, d_model=16, d_hidden=16, top_k=2)
+    x, ids, scores = torch.randn(10, 16), torch.randint(0, 3, (10, 2)), torch.rand(10, 2)
+    if what == "one score per token":
+        scores = scores[:, :1]
+    elif what == "more choices than the layer's":
+        ids, scores = ids.repeat(1, 2), scores.repeat(1, 2)
+    elif what == "scores elsewhere":
+        scores = scores.to("meta")
+    elif what == "ids elsewhere":
+        ids = ids.to("meta")
+    if what == "fits":
+        with pytest.raises(AssertionError, match="kernels were launched"):
+            layer._fused_forward(x, ids, scores)
+    else:
+        assert layer._fused_forward(x, ids, scores) is None

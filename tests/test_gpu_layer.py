@@ -412,3 +412,26 @@ def test_switch_gate_linear_is_the_kernel_only_when_nobody_looks():
         results.append([t.detach().float() for t in first + second])
     for a, b in zip(*results):
         assert float((a - b).norm()) <= 2e-2 * float(b.norm())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("what", ["one score per token", "scores on the host", "ids on the host"])
+def test_layer_refuses_what_a_gate_should_not_return(dtype, what):
+    from fastmoe_b200 import FMoETransformerMLP
+    from fastmoe_b200.ops import native
+    layer = FMoETransformerMLP(num_expert=4, d_model=64, d_hidden=64, top_k=2).to(DEV).to(dtype)
+    x = torch.randn(64, 64, device=DEV, dtype=dtype)
+    ids = torch.randint(0, 4, (64, 2), device=DEV)
+    scores = torch.rand(64, 2, device=DEV, dtype=dtype)
+    if what == "one score per token":
+        scores = scores[:, :1]
+    elif what == "scores on the host":
+        scores = scores.cpu()
+    else:
+        ids = ids.cpu()
+    layer.gate.forward = lambda _x: (ids, scores)
+    with pytest.raises(RuntimeError):
+        layer(x)
+    e = layer.experts
+    with pytest.raises(RuntimeError, match="do not fit"):
+        native.get().moe_mlp(x, scores, e.htoh4.weight, e.htoh4.bias, e.h4toh.weight, e.h4toh.bias, ids, 2, False)
