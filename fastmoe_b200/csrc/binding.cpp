@@ -1067,11 +1067,12 @@ class MoEMLP : public torch::autograd::Function<MoEMLP> {
 
 class GateLinearTopk : public torch::autograd::Function<GateLinearTopk> {
  public:
-  static variable_list forward(AutogradContext* ctx, const torch::Tensor& x_in, const torch::Tensor& w_in,
+  static variable_list forward(AutogradContext* ctx, const torch::Tensor& x, const torch::Tensor& w,
                                const c10::optional<torch::Tensor>& bias, int64_t k, int64_t zero) {
     // `zero`: address of the caller's one-element tensor, which is not an input of the node
-    const torch::Tensor x = aligned(x_in, 16), w = aligned(w_in, 16);   // the kernels load 16 bytes at a time
-    auto r = gate_forward(x, w, bias, k, false, reinterpret_cast<float*>(zero));
+    // The kernels load 16 bytes at a time.  Saved are the inputs, which a gradient of the gradient goes
+    // on to: the graph does not know of copies made here.
+    auto r = gate_forward(aligned(x, 16), aligned(w, 16), bias, k, false, reinterpret_cast<float*>(zero));
     ctx->save_for_backward({x, w, r[1], r[2]});
     ctx->saved_data["bias"] = bias.has_value() && bias->defined();
     ctx->mark_non_differentiable({r[1]});
@@ -1099,7 +1100,7 @@ class GateLinearTopk : public torch::autograd::Function<GateLinearTopk> {
     auto given = [](const torch::Tensor& g) {
       return g.defined() ? c10::optional<torch::Tensor>(g.contiguous()) : c10::nullopt;
     };
-    // (saved tensors may have been moved by hooks)
+    // (at any address: the caller's, or where hooks on saved tensors put them)
     auto r = gate_linear_topk_bwd(given(grads[2]), s[2], s[3], given(grads[0]), aligned(s[0], 16), aligned(s[1], 16),
                                   need_dx, need_db);
     return {need_dx ? r[0] : torch::Tensor(), need_dw ? r[1] : torch::Tensor(), need_db ? r[2] : torch::Tensor(),

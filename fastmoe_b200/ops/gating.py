@@ -65,9 +65,9 @@ class _LinearTopkSoftmax(Function):
 
     @staticmethod
     def forward(ctx, x, weight, bias, k):
-        if (x.data_ptr() | weight.data_ptr()) % 16 != 0:   # the kernels load 16 bytes at a time
-            x, weight = gg.aligned(x, 16), gg.aligned(weight, 16)
-        logits, idx, prob = native.get().gate_linear_topk(x, weight, bias, int(k))
+        # (the kernels load 16 bytes at a time; saved are the inputs, which a gradient of the gradient goes
+        # on to, and not copies made here)
+        logits, idx, prob = native.get().gate_linear_topk(gg.aligned(x, 16), gg.aligned(weight, 16), bias, int(k))
         ctx.save_for_backward(x, weight, idx, prob)
         ctx.has_bias = bias is not None
         ctx.mark_non_differentiable(idx)
@@ -85,11 +85,9 @@ class _LinearTopkSoftmax(Function):
                 through = native.get().gate_topk_softmax_bwd(grad_prob.contiguous(), idx, prob, weight.shape[0])
                 dl = through if dl is None else dl + through
             return dl.matmul(weight), dl.t().matmul(x), dl.sum(0) if ctx.has_bias else None, None
-        if (x.data_ptr() | weight.data_ptr()) % 16 != 0:   # moved by hooks on the saved tensors
-            x, weight = gg.aligned(x, 16), gg.aligned(weight, 16)
         dx, dw, db, _dl = native.get().gate_linear_topk_bwd(
             None if grad_prob is None else grad_prob.contiguous(), idx, prob,
-            None if grad_logits is None else grad_logits.contiguous(), x, weight,
+            None if grad_logits is None else grad_logits.contiguous(), gg.aligned(x, 16), gg.aligned(weight, 16),
             ctx.needs_input_grad[0], ctx.has_bias and ctx.needs_input_grad[2])
         return (dx if ctx.needs_input_grad[0] else None, dw if ctx.needs_input_grad[1] else None,
                 db if ctx.has_bias and ctx.needs_input_grad[2] else None, None)

@@ -131,6 +131,23 @@ def test_fp32_gate_gradient_of_the_gradient():
         assert torch.allclose(got, second[2], rtol=1e-3, atol=1e-3 * float(second[2].abs().max()))
 
 
+def test_gate_gradient_of_the_gradient_at_odd_addresses():
+    r"""fp32 sums of at most 40 * 32 terms."""
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(0)
+    flat_x, flat_w = (torch.randn(n + 1, device=DEV, requires_grad=True) for n in (40 * 32, 4 * 32))
+    second = []
+    for gate in (lambda x, w: gating.linear_topk_softmax(x, w, None, 2)[0],
+                 lambda x, w: gating._LinearTopkSoftmax.apply(x, w, None, 2)[0], torch.nn.functional.linear):
+        x, w = flat_x[1:].view(40, 32), flat_w[1:].view(4, 32)
+        assert x.data_ptr() % 16 == 4 and w.data_ptr() % 16 == 4
+        dx, dw = torch.autograd.grad(gate(x, w).square().sum(), (x, w), create_graph=True)
+        second.append(torch.autograd.grad(dx.square().sum() + dw.square().sum(), (flat_x, flat_w)))
+    for got in second[:2]:
+        for a, b in zip(got, second[2]):
+            assert torch.allclose(a, b, rtol=1e-3, atol=1e-3 * float(b.abs().max()))
+
+
 def test_fp32_gate_keeps_subclasses_and_autocast_on_the_operations():
     from fastmoe_b200.ops import gating
 
