@@ -128,14 +128,14 @@ class _Combine(Function):
     @staticmethod
     def backward(ctx, dout):
         ys, score, idx, rank, offs = ctx.saved_tensors
-        if torch.is_grad_enabled():   # a gradient of the gradient is wanted
+        if torch.is_grad_enabled():   # a gradient of the gradient is wanted (rows or scores may be constants)
+            if ys.shape[0] == 0:
+                return dout[:0] * score[:1, None], torch.zeros_like(score) + ys.sum(), None, None, None, None
             row, kept = _rows_of_slots(idx, rank, offs)
-            with torch.enable_grad():
-                picked = torch.where(kept[:, None], ys[row], 0) if ys.shape[0] else ys.sum() + ys.new_zeros(
-                    idx.numel(), ys.shape[1])
-                out = (picked * score[:, None]).view(-1, ctx.k, ys.shape[1]).sum(1)
-                dys, dscore = torch.autograd.grad(out, (ys, score), dout, create_graph=True, allow_unused=True)
-            return dys, dscore, None, None, None, None
+            g = dout.repeat_interleave(ctx.k, 0)
+            dys = torch.zeros_like(ys, memory_format=torch.contiguous_format).index_add(
+                0, row, torch.where(kept[:, None], g * score[:, None], 0))
+            return dys, torch.where(kept, (g * ys[row]).sum(1), 0), None, None, None, None
         dys = torch.empty_like(ys, memory_format=torch.contiguous_format)
         dscore = torch.empty_like(score)
         native.get().combine_bwd(gg.aligned(dout, 16), gg.aligned(ys, 16), idx, rank, offs, score, ctx.k, dys, dscore)

@@ -124,3 +124,31 @@ def test_fp32_layer_looks_at_what_the_gate_returned(what):
             layer._fused_forward(x, ids, scores)
     else:
         assert layer._fused_forward(x, ids, scores) is None
+
+
+@pytest.mark.parametrize("constant", ["neither", "scores", "rows"])
+@pytest.mark.parametrize("dropped", ["some", "all"])
+def test_gradient_of_the_gradient(constant, dropped, monkeypatch):
+    r"""In 64 bits against the path of PyTorch operations."""
+    layer = _layer()
+    torch.manual_seed(2)
+    x0, s0 = torch.randn(10, 16, dtype=torch.float64), torch.rand(10, 2, dtype=torch.float64)
+    ids = torch.randint(-1, 3, (10, 2)) if dropped == "some" else torch.full((10, 2), -1)
+    if constant == "rows":
+        layer.experts.requires_grad_(False)
+
+    def operations(*args):
+        with monkeypatch.context() as m:
+            m.setenv("FMOE_FUSED", "0")
+            return layer._general_path(*args)
+    results = []
+    for run in (lambda *args: _general(layer, *args), operations):
+        x, s = x0.clone().requires_grad_(constant != "rows"), s0.clone().requires_grad_(constant != "scores")
+        wanted = [t for t in (x, s) if t.requires_grad]
+        params = [p for p in layer.parameters() if p.requires_grad and p.dim() == 2]
+        first = torch.autograd.grad(run(x, ids, s).square().sum(), wanted, create_graph=True, allow_unused=True)
+        total = sum(g.square().sum() for g in first if g is not None)
+        second = torch.autograd.grad(total, wanted + params, allow_unused=True)
+        results.append([torch.zeros(()).double() if g is None else g.detach() for g in list(first) + list(second)])
+    for a, b in zip(*results):
+        assert float((a - b).abs().max()) <= 1e-9 * (1 + float(b.abs().max()))

@@ -115,6 +115,24 @@ def test_gradient_of_the_gradient(monkeypatch):
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("constant", ["scores", "rows"])
+def test_gradient_of_the_gradient_beside_constants(monkeypatch, constant):
+    layer = _layer(3, 16, 16, 2, "plain", torch.float32)
+    torch.manual_seed(2)
+    x0, s0 = torch.randn(40, 16, device=DEV), torch.rand(40, 2, device=DEV)
+    ids = torch.randint(-1, 3, (40, 2), device=DEV)
+    layer.experts.requires_grad_(constant != "rows")
+    results = []
+    for fused in ("1", "0"):
+        monkeypatch.setenv("FMOE_FUSED", fused)
+        x, s = x0.clone().requires_grad_(constant != "rows"), s0.clone().requires_grad_(constant != "scores")
+        leaf = s if constant == "rows" else x
+        first, = torch.autograd.grad(layer._general_path(x, ids, s).square().sum(), leaf, create_graph=True)
+        results.append((first.detach(),) + torch.autograd.grad(first.square().sum(), leaf))
+    for a, b in zip(*results):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-4)
+
+
 @pytest.mark.parametrize("groups", [1, 79, 80, 255, 959, 960, 3000])   # parameters of 80 and 960 values, the copy
 def test_offsets_of_host_counts(groups):
     from fastmoe_b200.ops import grouped_gemm as gg
