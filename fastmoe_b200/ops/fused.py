@@ -130,7 +130,8 @@ class _Combine(Function):
         ys, score, idx, rank, offs = ctx.saved_tensors
         if torch.is_grad_enabled():   # a gradient of the gradient is wanted (rows or scores may be constants)
             if ys.shape[0] == 0:
-                return dout[:0] * score[:1, None], torch.zeros_like(score) + ys.sum(), None, None, None, None
+                return (dout[:0] * score[:1, None], torch.zeros_like(score) + ys.sum() + dout[:0].sum(),
+                        None, None, None, None)
             row, kept = _rows_of_slots(idx, rank, offs)
             g = dout.repeat_interleave(ctx.k, 0)
             dys = torch.zeros_like(ys, memory_format=torch.contiguous_format).index_add(
