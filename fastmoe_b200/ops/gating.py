@@ -105,6 +105,11 @@ def _single_pass_type(x, weight, bias):
             and all(t is None or type(t) in (torch.Tensor, torch.nn.Parameter) for t in (x, weight, bias)))
 
 
+def _no_tangent(*tensors):
+    r"""Whether no forward-mode derivative passes through: the native calls would drop it."""
+    return all(t is None or forward_ad.unpack_dual(t).tangent is None for t in tensors)
+
+
 def linear_logits(x, linear):
     r"""``linear(x)`` of a gate's ``nn.Linear`` in the single-pass kernel, or ``None`` where that does not
     take the call or somebody watches the module.  It stands for three library products and a column sum
@@ -115,7 +120,7 @@ def linear_logits(x, linear):
             and x.is_cuda and x.dim() == 2 and x.is_contiguous()
             and x.shape[0] > 0 and _single_pass_type(x, w, b) and not torch.is_autocast_enabled() and not traced()
             and native.get().gate_fused_supported(w.shape[0], x.shape[1], 1)
-            and all(t is None or forward_ad.unpack_dual(t).tangent is None for t in (x, w, b))
+            and _no_tangent(x, w, b)
             and not _hooked(linear) and not _hooked_globally()):
         return native.get().gate_linear_topk_node(x, w.contiguous(), b, 1, None)[0]
     return None
@@ -178,7 +183,7 @@ def _few_tokens_ok(x, weight, bias, k):
             and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype
             and (bias is None or bias.dtype == x.dtype)
             and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, weight, bias)))
-            and not torch.is_autocast_enabled() and not traced()
+            and not torch.is_autocast_enabled() and not traced() and _no_tangent(x, weight, bias)
             and native.get().gate_fused_supported(weight.shape[0], x.shape[1], k))
 
 

@@ -1,0 +1,29 @@
+r"""Which calls of the gates go to which kernels, on the CPU with stand-ins."""
+import pytest
+import torch
+from torch.autograd import forward_ad
+
+from fastmoe_b200.ops import gating, native
+
+
+class _Kernels:
+    @staticmethod
+    def gate_fused_supported(_tot, _d, _k):
+        return True
+
+
+@pytest.fixture
+def kernels(monkeypatch):
+    monkeypatch.setattr(native, "get", _Kernels)
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True, raising=False)
+
+
+def test_few_tokens_with_a_tangent_are_left_to_the_others(kernels):
+    r"""The native call is no autograd function: it would return scores without the tangent."""
+    x, w, b = torch.randn(4, 64).bfloat16(), torch.randn(16, 64).bfloat16(), torch.randn(16).bfloat16()
+    with torch.no_grad(), forward_ad.dual_level():
+        assert gating._few_tokens_ok(x, w, b, 2)
+        dual = lambda t: forward_ad.make_dual(t, torch.ones_like(t))
+        assert not gating._few_tokens_ok(dual(x), w, b, 2)
+        assert not gating._few_tokens_ok(x, dual(w), b, 2)
+        assert not gating._few_tokens_ok(x, w, dual(b), 2)

@@ -386,6 +386,15 @@ def test_native_nodes_refuse_what_the_python_ones_refuse():
         torch.func.vmap(moe)(x.view(2, 8, 64))
 
 
+def test_gate_for_few_tokens_refuses_forward_mode():
+    from torch.autograd import forward_ad
+    from fastmoe_b200.gates import NaiveGate
+    gate = NaiveGate(64, 16, 1, 2).to(DEV).bfloat16()
+    x = torch.randn(16, 64, device=DEV, dtype=torch.bfloat16)
+    with torch.no_grad(), forward_ad.dual_level(), pytest.raises(NotImplementedError):
+        gate(forward_ad.make_dual(x, torch.ones_like(x)))
+
+
 def test_switch_gate_linear_is_the_kernel_only_when_nobody_looks():
     from fastmoe_b200.gates import SwitchGate
     from fastmoe_b200.ops import gating
