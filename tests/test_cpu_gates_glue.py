@@ -27,3 +27,24 @@ def test_few_tokens_with_a_tangent_are_left_to_the_others(kernels):
         assert not gating._few_tokens_ok(dual(x), w, b, 2)
         assert not gating._few_tokens_ok(x, dual(w), b, 2)
         assert not gating._few_tokens_ok(x, w, dual(b), 2)
+
+
+def test_switch_gate_calls_whatever_module_is_its_linear():
+    from fastmoe_b200.gates import SwitchGate
+
+    class Quantised(torch.nn.Module):   # as PyTorch's dynamically quantised linear, whose weight is a method
+        def __init__(self, linear):
+            super().__init__()
+            self.held = linear
+
+        def weight(self):
+            return self.held.weight
+
+        def forward(self, x):
+            return self.held(x)
+    torch.manual_seed(0)
+    gate, x = SwitchGate(16, 4, 1).eval(), torch.randn(6, 16)
+    want = gate(x)
+    for module in (torch.nn.Sequential(gate.gate), Quantised(gate.gate)):
+        gate.gate = module
+        assert all(torch.equal(a, b) for a, b in zip(gate(x), want))
