@@ -93,6 +93,11 @@ class _LinearTopkSoftmax(Function):
                 db if ctx.has_bias and ctx.needs_input_grad[2] else None, None)
 
 
+def _plain(*tensors):
+    r"""Whether these are plain tensors: a subclass may want to see the operations."""
+    return all(t is None or type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors)
+
+
 def _single_pass_type(x, weight, bias):
     r"""Whether the single-pass kernel takes these types: all 16 bits, or all 32 as plain tensors (a linear, top-k,
     softmax and their backward as operations, 8192 tokens, d 1024, 8 experts: 163 us, 87 in the kernels, whose
@@ -101,8 +106,7 @@ def _single_pass_type(x, weight, bias):
         return False
     if x.dtype in (torch.bfloat16, torch.float16):
         return True
-    return (x.dtype == torch.float32
-            and all(t is None or type(t) in (torch.Tensor, torch.nn.Parameter) for t in (x, weight, bias)))
+    return x.dtype == torch.float32 and _plain(x, weight, bias)
 
 
 def _no_tangent(*tensors):
@@ -121,7 +125,7 @@ def linear_logits(x, linear):
     if (w.shape[0] <= MAX_SINGLE_PASS_EXPERTS and x.is_cuda and x.dim() == 2 and x.is_contiguous()
             and x.shape[0] > 0 and _single_pass_type(x, w, b) and not torch.is_autocast_enabled() and not traced()
             and native.get().gate_fused_supported(w.shape[0], x.shape[1], 1)
-            and _no_tangent(x, w, b)
+            and _plain(x, w, b) and _no_tangent(x, w, b)
             and not _hooked(linear) and not _hooked_globally()):
         return native.get().gate_linear_topk_node(x, w.contiguous(), b, 1, None)[0]
     return None

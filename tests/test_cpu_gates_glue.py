@@ -11,6 +11,10 @@ class _Kernels:
     def gate_fused_supported(_tot, _d, _k):
         return True
 
+    @staticmethod
+    def gate_linear_topk_node(*_args):
+        return ["kernel"]
+
 
 @pytest.fixture
 def kernels(monkeypatch):
@@ -48,3 +52,17 @@ def test_switch_gate_calls_whatever_module_is_its_linear():
     for module in (torch.nn.Sequential(gate.gate), Quantised(gate.gate)):
         gate.gate = module
         assert all(torch.equal(a, b) for a, b in zip(gate(x), want))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("what", ["input", "weight", "neither"])
+def test_switch_gate_leaves_tensor_subclasses_to_the_linear(kernels, dtype, what):
+    class Mine(torch.Tensor):
+        pass
+    linear, x = torch.nn.Linear(64, 4).to(dtype), torch.randn(6, 64).to(dtype)
+    if what == "input":
+        x = x.as_subclass(Mine)
+    elif what == "weight":
+        linear.weight = torch.nn.Parameter(linear.weight.detach().as_subclass(Mine))
+        assert type(linear.weight) is not torch.nn.Parameter
+    assert gating.linear_logits(x, linear) == (None if what != "neither" else "kernel")
