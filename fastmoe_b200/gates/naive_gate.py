@@ -26,13 +26,15 @@ class NaiveGate(BaseGate):
 
     def forward(self, inp, return_all_scores=False):
         # The reference installs a zero "dummy" loss so that callers can always add it.
-        loss = torch.empty(1, device=inp.device)
-        if loss.dtype == torch.float32 and not loss.requires_grad:
-            logits, idx, score = self._choose(inp, loss)
+        # (made a leaf at once: transforms of torch.func do not let it become one later)
+        loss = torch.empty(1, device=inp.device, requires_grad=True)
+        zero = loss.detach()
+        if zero.dtype == torch.float32:
+            logits, idx, score = self._choose(inp, zero)
         else:
             logits, idx, score = self._choose(inp)
-            loss.zero_()
-        self.set_loss(loss.requires_grad_(True))
+            zero.zero_()
+        self.set_loss(loss)
         if return_all_scores:
             return idx, score, logits.view(*inp.shape[:-1], self.tot_expert)
         return idx, score

@@ -66,3 +66,29 @@ def test_switch_gate_leaves_tensor_subclasses_to_the_linear(kernels, dtype, what
         linear.weight = torch.nn.Parameter(linear.weight.detach().as_subclass(Mine))
         assert type(linear.weight) is not torch.nn.Parameter
     assert gating.linear_logits(x, linear) == (None if what != "neither" else "kernel")
+
+
+@pytest.mark.parametrize("default", [torch.float32, torch.float64])
+def test_naive_gate_under_function_transforms(default):
+    from fastmoe_b200.gates import NaiveGate
+    torch.manual_seed(0)
+    gate, x = NaiveGate(16, 4, 1, 2).to(default), torch.randn(6, 16, dtype=default)
+    params = {n: p.detach() for n, p in gate.named_parameters()}
+
+    def loss(params, x):
+        return torch.func.functional_call(gate, params, (x,))[1].square().sum()
+    before = torch.get_default_dtype()
+    torch.set_default_dtype(default)
+    try:
+        grad = torch.func.grad(loss)(params, x)
+        each = torch.func.vmap(torch.func.grad(loss), (None, 0))(params, x[:, None])
+        torch.func.jvp(lambda t: loss(params, t), (x,), (torch.ones_like(x),))
+        gate(x)[1].square().sum().backward()
+    finally:
+        torch.set_default_dtype(before)
+    for n, p in gate.named_parameters():
+        assert torch.allclose(grad[n], p.grad, atol=1e-6) and torch.allclose(each[n].sum(0), p.grad, atol=1e-6)
+    held = gate.get_loss()
+    assert held.dtype == default and held.requires_grad and held.is_leaf and float(held.detach()) == 0
+    with torch.inference_mode():
+        gate(x)
