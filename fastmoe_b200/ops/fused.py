@@ -52,11 +52,11 @@ def supports(layer, x, idx, score=None):
 
 def _fp32_layer_ok(layer, x, idx, score):
     r"""Whether the fp32 layer on one GPU runs as :class:`_MoEMLP`.  The general path, which takes the
-    rest, calls the expert modules: a call that somebody watches stays there, and so does autocast,
-    under which the weighted sum is formed in 16 bits."""
+    rest, calls ``expert_fn`` and the expert modules: a call that somebody watches or does in another way
+    stays there, and so does autocast, under which the weighted sum is formed in 16 bits."""
     e = layer.experts
     if (layer.world_size > 1 or _forced_ep() or not config.fused_enabled() or config.faster_schedule_enabled()
-            or torch.is_autocast_enabled() or not plain_experts(e)):
+            or torch.is_autocast_enabled() or not layer._usual_expert_fn() or not plain_experts(e)):
         return False
     if any(t is None or t.dtype != torch.float32 or not t.is_cuda
            for t in (e.htoh4.weight, e.htoh4.bias, e.h4toh.weight, e.h4toh.bias)):

@@ -152,3 +152,16 @@ def test_gradient_of_the_gradient(constant, dropped, monkeypatch):
         results.append([torch.zeros(()).double() if g is None else g.detach() for g in list(first) + list(second)])
     for a, b in zip(*results):
         assert float((a - b).abs().max()) <= 1e-9 * (1 + float(b.abs().max()))
+
+
+@pytest.mark.parametrize("how", ["subclass", "instance"])
+def test_fp32_layer_calls_another_expert_fn(how):
+    from fastmoe_b200 import FMoETransformerMLP
+
+    class Doubled(FMoETransformerMLP):
+        def expert_fn(self, inp, fwd_expert_count):
+            return super().expert_fn(inp, fwd_expert_count) * 2
+    layer = (Doubled if how == "subclass" else FMoETransformerMLP)(num_expert=3, d_model=16, d_hidden=16, top_k=2)
+    if how == "instance":
+        layer.expert_fn = lambda inp, count: layer.experts(inp, count) * 2
+    assert layer._fused_forward(torch.randn(10, 16), torch.randint(0, 3, (10, 2)), torch.rand(10, 2)) is None
