@@ -153,10 +153,11 @@ def rows_supported(x, ids, scores):
             and not torch.is_autocast_enabled())
 
 
-def general_path(x, ids, scores, expert_fn, num_expert):
+def general_path(x, ids, scores, expert_fn, num_expert, own_rows=False):
     r"""The general path of one GPU around ``expert_fn(rows, counts)``: rows to their experts, the
     weighted sum of what comes back.  One read of the counts on the host, as the experts are called
-    with Python slices.  ``(out, rows, routing)``: ``out`` is ``None``, and ``routing`` what
+    with Python slices.  With ``own_rows`` ``expert_fn`` is known to hold the rows by their segments
+    only.  ``(out, rows, routing)``: ``out`` is ``None``, and ``routing`` what
     ``MOEGather`` needs, where ``expert_fn`` did not return rows that the kernels combine.
 
     8 experts of two ``nn.Linear`` with 2048 tokens, top-2, d 512: the zeroed tensors, copies and additions
@@ -168,7 +169,8 @@ def general_path(x, ids, scores, expert_fn, num_expert):
     counts = counts.cpu().long()
     n_rows = int(counts.sum())
     xs = _Dispatch.apply(x.contiguous(), idx, rank, offs, k, n_rows)
-    xs.fmoe_own_rows = True   # a buffer that nobody else holds (see FMoE.expert_fn)
+    if own_rows:
+        xs.fmoe_own_rows = True   # a buffer that nobody else holds (see FMoE.expert_fn)
     ys = expert_fn(xs, counts)
     if (torch.is_tensor(ys) and ys.is_cuda and ys.dim() == 2 and ys.dtype in _TC + (torch.float32,)
             and ys.shape[0] == n_rows and ys.shape[1] % 8 == 0 and ys.shape[1] > 0 and ys.device == x.device):

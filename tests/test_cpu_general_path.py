@@ -165,3 +165,32 @@ def test_fp32_layer_calls_another_expert_fn(how):
     if how == "instance":
         layer.expert_fn = lambda inp, count: layer.experts(inp, count) * 2
     assert layer._fused_forward(torch.randn(10, 16), torch.randint(0, 3, (10, 2)), torch.rand(10, 2)) is None
+
+
+class _InPlace(_Expert):
+    def forward(self, x, _count):
+        return torch.tanh(self.fc(x.mul_(2.0)))
+
+
+def test_rows_that_another_expert_fn_saves_are_watched():
+    r"""Experts that write to their rows, and an ``expert_fn`` that has used the rows before: autograd
+    has to notice, as it does with slices."""
+    class Shared(FMoE):
+        def expert_fn(self, inp, fwd_expert_count):
+            return self.shared(inp) + super().expert_fn(inp, fwd_expert_count)
+    layer = _layer(cls=Shared, expert=_InPlace)
+    layer.shared = nn.Linear(16, 16).double()
+    torch.manual_seed(4)
+    x, ids, scores = torch.randn(10, 16).double(), torch.randint(0, 3, (10, 2)), torch.rand(10, 2).double()
+    out = layer._general_path(x.requires_grad_(True), ids, scores)
+    with pytest.raises(RuntimeError, match="inplace operation"):
+        out.sum().backward()
+    # nobody else holds the rows of the usual one: its experts may write to them
+    plain = _layer(expert=_InPlace)
+    results = []
+    for module, rows in ((plain, x), (_layer(), x * 2.0)):
+        module.load_state_dict(plain.state_dict())
+        module.zero_grad()
+        module._general_path(rows, ids, scores).sum().backward()
+        results.append([p.grad for p in module.experts.parameters()])
+    assert all(torch.allclose(a, b) for a, b in zip(*results))
