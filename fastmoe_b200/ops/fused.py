@@ -21,7 +21,7 @@ from torch.autograd import Function
 
 from . import grouped_gemm as gg
 from . import native
-from .gating import traced
+from .gating import _no_tangent, _plain, traced
 from .. import config
 from ..transformer import activation_kind, plain_experts
 from ..utils.profiling import check_routing, fused_range
@@ -60,6 +60,8 @@ def _fp32_layer_ok(layer, x, idx, score):
         return False
     if any(t is None or t.dtype != torch.float32 or not t.is_cuda
            for t in (e.htoh4.weight, e.htoh4.bias, e.h4toh.weight, e.h4toh.bias)):
+        return False
+    if not _plain(x, score) or not _no_tangent(score):   # as in `rows_supported`
         return False
     # (as many choices as the layer was made for: the general path refuses others)
     return (idx.shape[1] == layer.top_k and _native_call_ok(layer, x, idx, score)
@@ -150,6 +152,8 @@ def rows_supported(x, ids, scores):
             and ids.device == x.device and scores.device == x.device
             and ids.shape[0] == x.shape[0] and ids.numel() > 0 and ids.numel() < 2 ** 31
             and scores.numel() == ids.numel() and scores.is_floating_point()
+            # (the operations keep a subclass for the experts, and a forward-mode derivative of the scores)
+            and _plain(x, ids, scores) and _no_tangent(scores)
             and not torch.is_autocast_enabled())
 
 

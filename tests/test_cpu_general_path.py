@@ -3,6 +3,7 @@ and, as they do, reads its operands through their pointers."""
 import pytest
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad
 
 from fastmoe_b200 import FMoE
 from fastmoe_b200.ops import fused, native, torch_impl
@@ -194,3 +195,30 @@ def test_rows_that_another_expert_fn_saves_are_watched():
         module._general_path(rows, ids, scores).sum().backward()
         results.append([p.grad for p in module.experts.parameters()])
     assert all(torch.allclose(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("path", ["custom experts", "fp32 layer"])
+def test_subclasses_and_tangents_of_scores_keep_the_operations(path, monkeypatch):
+    from fastmoe_b200 import FMoETransformerMLP
+
+    class Mine(torch.Tensor):
+        pass
+    dtype = torch.float64 if path == "custom experts" else torch.float32
+    torch.manual_seed(5)
+    x, ids, scores = torch.randn(10, 16, dtype=dtype), torch.randint(0, 3, (10, 2)), torch.rand(10, 2, dtype=dtype)
+    if path == "custom experts":
+        layer = _layer()
+        taken = lambda x, scores: fused.rows_supported(x, ids, scores)
+    else:
+        layer = FMoETransformerMLP(num_expert=3, d_model=16, d_hidden=16, top_k=2)
+        taken = lambda x, scores: fused.supports(layer, x, ids, scores)
+    assert taken(x, scores)
+    assert not taken(x.as_subclass(Mine), scores)
+    assert not taken(x, scores.as_subclass(Mine))
+    monkeypatch.delattr(torch.Tensor, "is_cuda")
+    with torch.no_grad(), forward_ad.dual_level():   # the derivative is that of a sum linear in the scores
+        out = layer._general_path(x, ids, forward_ad.make_dual(scores, scores))
+        assert torch.allclose(*forward_ad.unpack_dual(out))
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True, raising=False)
+    with torch.no_grad(), forward_ad.dual_level():
+        assert not taken(x, forward_ad.make_dual(scores, scores))
