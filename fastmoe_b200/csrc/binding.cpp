@@ -986,44 +986,49 @@ std::vector<torch::Tensor> gate_linear_topk(torch::Tensor x, torch::Tensor w, c1
   return gate_forward(x, w, bias, k, few, zero_of(zero));
 }
 
-// Returns {dx or empty, dw (layer dtype), db or empty, dl fp32 [B, tot]}.
+// Returns {dx or empty, dw (layer dtype) or empty, db or empty, dl fp32 [B, tot]}.  Without `x` no dw and db are
+// formed, without `w` (of which `tot` is the rows then) no dx.
 std::vector<torch::Tensor> gate_linear_topk_bwd(c10::optional<torch::Tensor> dprob, torch::Tensor idx,
                                                 torch::Tensor prob,
                                                 c10::optional<torch::Tensor> dlogits,
-                                                torch::Tensor x, torch::Tensor w, bool need_dx,
-                                                bool need_db) {
-  check_rows(x, "x");
-  check_rows(w, "w");
-  c10::cuda::CUDAGuard guard(x.device());
-  const int rows = static_cast<int>(x.size(0));
-  const int d = static_cast<int>(x.size(1));
-  const int tot = static_cast<int>(w.size(0));
+                                                c10::optional<torch::Tensor> x, c10::optional<torch::Tensor> w,
+                                                bool need_dx, bool need_db, int64_t tot_without_w) {
+  const bool need_dw = x.has_value() && x->defined(), has_w = w.has_value() && w->defined();
+  if (need_dw) check_rows(*x, "x");
+  if (has_w) check_rows(*w, "w");
+  TORCH_CHECK((need_dw || has_w) && (has_w || (!need_dx && tot_without_w > 0)) && (need_dw || !need_db), "gate gradient: operands missing");
+  const torch::Tensor& like = need_dw ? *x : *w;
+  c10::cuda::CUDAGuard guard(like.device());
+  const int rows = static_cast<int>(idx.size(0));
+  const int d = static_cast<int>(like.size(1));
+  const int tot = static_cast<int>(has_w ? w->size(0) : tot_without_w);
   const int k = static_cast<int>(idx.size(1));
-  auto f32 = torch::dtype(torch::kFloat).device(x.device());
+  TORCH_CHECK(!need_dw || (x->size(0) == rows && (!has_w || x->size(1) == w->size(1))), "gate gradient: operands do not fit");
+  auto f32 = torch::dtype(torch::kFloat).device(like.device());
   auto dl = torch::empty({rows, tot}, f32);
-  torch::Tensor dx = need_dx ? torch::empty_like(x) : torch::Tensor();
-  const bool fused_dw = tot <= 16;
+  torch::Tensor dx = need_dx ? torch::empty({rows, d}, like.options()) : torch::Tensor();
+  const bool fused_dw = need_dw && tot <= 16;
   torch::Tensor part, dw_db;
   if (fused_dw) {
     const long elems = static_cast<long>(tot) * d + tot;
     // without rows nothing is launched: the sums over no tokens are zero
-    dw_db = rows > 0 ? torch::empty({elems}, x.options()) : torch::zeros({elems}, x.options());
-    part = torch::empty({fmoe::gate_bwd_ranges(logit_code(x), rows, d) * elems}, f32);
+    dw_db = rows > 0 ? torch::empty({elems}, like.options()) : torch::zeros({elems}, like.options());
+    part = torch::empty({fmoe::gate_bwd_ranges(logit_code(like), rows, d) * elems}, f32);
   }
   FMOE_CUDA_CHECK(fmoe::launch_gate_bwd(
-      logit_code(x), dprob.has_value() ? dprob->data_ptr() : nullptr, idx.data_ptr<int64_t>(),
-      prob.data_ptr(), dlogits.has_value() ? dlogits->data_ptr() : nullptr, x.data_ptr(),
-      w.data_ptr(), rows, d, tot, k, dl.data_ptr<float>(), need_dx ? dx.data_ptr() : nullptr,
+      logit_code(like), dprob.has_value() ? dprob->data_ptr() : nullptr, idx.data_ptr<int64_t>(),
+      prob.data_ptr(), dlogits.has_value() ? dlogits->data_ptr() : nullptr, need_dw ? x->data_ptr() : nullptr,
+      has_w ? w->data_ptr() : nullptr, rows, d, tot, k, dl.data_ptr<float>(), need_dx ? dx.data_ptr() : nullptr,
       fused_dw ? part.data_ptr<float>() : nullptr, fused_dw ? dw_db.data_ptr() : nullptr, cur_stream()));
   torch::Tensor dw, db;
   if (fused_dw) {
     g_launches.fetch_add(2, std::memory_order_relaxed);  // the weight-gradient and merge kernels
     dw = dw_db.narrow(0, 0, static_cast<long>(tot) * d).view({tot, d});
     if (need_db) db = dw_db.narrow(0, static_cast<long>(tot) * d, tot);
-  } else {
-    auto dl16 = dl.to(x.scalar_type());
-    dw = dl16.t().matmul(x);
-    if (need_db) db = dl.sum(0).to(x.scalar_type());
+  } else if (need_dw) {
+    auto dl16 = dl.to(like.scalar_type());
+    dw = dl16.t().matmul(*x);
+    if (need_db) db = dl.sum(0).to(like.scalar_type());
   }
   return {dx, dw, db, dl};
 }
@@ -1073,8 +1078,12 @@ class GateLinearTopk : public torch::autograd::Function<GateLinearTopk> {
     // The kernels load 16 bytes at a time.  Saved are the inputs, which a gradient of the gradient goes
     // on to: the graph does not know of copies made here.
     auto r = gate_forward(aligned(x, 16), aligned(w, 16), bias, k, false, reinterpret_cast<float*>(zero));
-    ctx->save_for_backward({x, w, r[1], r[2]});
-    ctx->saved_data["bias"] = bias.has_value() && bias->defined();
+    const bool has_bias = bias.has_value() && bias->defined();
+    // each operand where the other's gradient is wanted (what is not saved may be changed in place)
+    ctx->save_for_backward({w.requires_grad() || (has_bias && bias->requires_grad()) ? x : torch::Tensor(),
+                            x.requires_grad() ? w : torch::Tensor(), r[1], r[2]});
+    ctx->saved_data["bias"] = has_bias;
+    ctx->saved_data["tot"] = w.size(0);
     ctx->mark_non_differentiable({r[1]});
     ctx->set_materialize_grads(false);
     return {r[0], r[1], r[2]};
@@ -1086,12 +1095,12 @@ class GateLinearTopk : public torch::autograd::Function<GateLinearTopk> {
     const bool has_bias = ctx->saved_data["bias"].toBool();
     const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
     const bool need_db = has_bias && ctx->needs_input_grad(2);
-    if (at::GradMode::is_enabled() && (!grads[2].defined() || s[0].scalar_type() == torch::kFloat)) {
+    if (at::GradMode::is_enabled() && (!grads[2].defined() || s[3].scalar_type() == torch::kFloat)) {
       // a gradient of the gradient is wanted: the linear's, in operations that have one (the scores'
       // counts as a constant)
       torch::Tensor dl = grads[0];
       if (grads[2].defined()) {
-        auto through = gate_topk_softmax_bwd(grads[2].contiguous(), s[2], s[3], s[1].size(0));
+        auto through = gate_topk_softmax_bwd(grads[2].contiguous(), s[2], s[3], ctx->saved_data["tot"].toInt());
         dl = dl.defined() ? dl + through : through;
       }
       return {need_dx ? dl.matmul(s[1]) : torch::Tensor(), need_dw ? dl.t().matmul(s[0]) : torch::Tensor(),
@@ -1101,8 +1110,9 @@ class GateLinearTopk : public torch::autograd::Function<GateLinearTopk> {
       return g.defined() ? c10::optional<torch::Tensor>(g.contiguous()) : c10::nullopt;
     };
     // (at any address: the caller's, or where hooks on saved tensors put them)
-    auto r = gate_linear_topk_bwd(given(grads[2]), s[2], s[3], given(grads[0]), aligned(s[0], 16), aligned(s[1], 16),
-                                  need_dx, need_db);
+    auto rows = [](const torch::Tensor& t) { return t.defined() ? c10::optional<torch::Tensor>(aligned(t, 16)) : c10::nullopt; };
+    auto r = gate_linear_topk_bwd(given(grads[2]), s[2], s[3], given(grads[0]), rows(s[0]), rows(s[1]), need_dx, need_db,
+                                  ctx->saved_data["tot"].toInt());
     return {need_dx ? r[0] : torch::Tensor(), need_dw ? r[1] : torch::Tensor(), need_db ? r[2] : torch::Tensor(),
             torch::Tensor(), torch::Tensor()};
   }
@@ -1196,7 +1206,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gate_fused_supported", &gate_fused_supported);
   m.def("gate_linear_topk", &gate_linear_topk, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("k"),
         py::arg("few") = false, py::arg("zero") = py::none());
-  m.def("gate_linear_topk_bwd", &gate_linear_topk_bwd);
+  m.def("gate_linear_topk_bwd", &gate_linear_topk_bwd, py::arg("dprob"), py::arg("idx"), py::arg("prob"), py::arg("dlogits"),
+        py::arg("x"), py::arg("w"), py::arg("need_dx"), py::arg("need_db"), py::arg("tot") = 0);
   m.def("launch_count", []() { return g_launches.load(); });
   m.def("read_status", &read_status);
   m.def("clear_status", &clear_status);

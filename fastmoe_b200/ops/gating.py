@@ -66,10 +66,12 @@ class _LinearTopkSoftmax(Function):
     @staticmethod
     def forward(ctx, x, weight, bias, k):
         # (the kernels load 16 bytes at a time; saved are the inputs, which a gradient of the gradient goes
-        # on to, and not copies made here)
+        # on to, and not copies made here: each where the other's gradient is wanted, as what is not saved
+        # may be changed in place)
         logits, idx, prob = native.get().gate_linear_topk(gg.aligned(x, 16), gg.aligned(weight, 16), bias, int(k))
-        ctx.save_for_backward(x, weight, idx, prob)
-        ctx.has_bias = bias is not None
+        need_dx, need_dw, need_db = ctx.needs_input_grad[:3]
+        ctx.save_for_backward(x if need_dw or need_db else None, weight if need_dx else None, idx, prob)
+        ctx.has_bias, ctx.tot = bias is not None, weight.shape[0]
         ctx.mark_non_differentiable(idx)
         ctx.set_materialize_grads(False)
         return logits, idx, prob
@@ -79,18 +81,19 @@ class _LinearTopkSoftmax(Function):
         x, weight, idx, prob = ctx.saved_tensors
         if grad_logits is None and grad_prob is None:
             return None, None, None, None
-        if torch.is_grad_enabled() and x.dtype == torch.float32:   # a gradient of the gradient, as in the native node
+        need_dx, need_dw, need_db = ctx.needs_input_grad[:3]
+        if torch.is_grad_enabled() and prob.dtype == torch.float32:   # a gradient of the gradient, as in the native node
             dl = grad_logits
             if grad_prob is not None:
-                through = native.get().gate_topk_softmax_bwd(grad_prob.contiguous(), idx, prob, weight.shape[0])
+                through = native.get().gate_topk_softmax_bwd(grad_prob.contiguous(), idx, prob, ctx.tot)
                 dl = through if dl is None else dl + through
-            return dl.matmul(weight), dl.t().matmul(x), dl.sum(0) if ctx.has_bias else None, None
+            return (dl.matmul(weight) if need_dx else None, dl.t().matmul(x) if need_dw else None,
+                    dl.sum(0) if need_db else None, None)
         dx, dw, db, _dl = native.get().gate_linear_topk_bwd(
             None if grad_prob is None else grad_prob.contiguous(), idx, prob,
             None if grad_logits is None else grad_logits.contiguous(), gg.aligned(x, 16), gg.aligned(weight, 16),
-            ctx.needs_input_grad[0], ctx.has_bias and ctx.needs_input_grad[2])
-        return (dx if ctx.needs_input_grad[0] else None, dw if ctx.needs_input_grad[1] else None,
-                db if ctx.has_bias and ctx.needs_input_grad[2] else None, None)
+            need_dx, need_db, ctx.tot)
+        return dx if need_dx else None, dw if need_dw else None, db if need_db else None, None
 
 
 def _plain(*tensors):

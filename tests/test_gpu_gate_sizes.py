@@ -148,6 +148,32 @@ def test_gate_gradient_of_the_gradient_at_odd_addresses():
             assert torch.allclose(a, b, rtol=1e-3, atol=1e-3 * float(b.abs().max()))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("frozen", ["weight", "weight and bias", "input"])
+def test_gate_saves_what_its_gradients_need(dtype, frozen):
+    r"""With a frozen gate the input may be changed in place afterwards, and the weight where the input
+    needs no gradient, as around ``nn.Linear``; the other gradients are those of all together."""
+    from fastmoe_b200.ops import gating
+    torch.manual_seed(1)
+    base = [torch.randn(100, 64, device=DEV, dtype=dtype), torch.randn(4, 64, device=DEV, dtype=dtype),
+            torch.randn(4, device=DEV, dtype=dtype)]
+    off = {"weight": (1,), "weight and bias": (1, 2), "input": (0,)}[frozen]
+    for gate in (lambda *a: gating.linear_topk_softmax(*a, 2), lambda *a: gating._LinearTopkSoftmax.apply(*a, 2)):
+        results = []
+        for partly in (True, False):
+            t = [b.clone().requires_grad_(not partly or i not in off) for i, b in enumerate(base)]
+            x, w, b = (v * 1 for v in t)   # (not leaves, which nothing may change in place)
+            logits, _idx, prob = gate(x, w, b)
+            if partly and frozen == "weight and bias":
+                x.add_(1.0)
+            elif partly and frozen == "input":
+                w.add_(1.0)
+            torch.autograd.backward([logits, prob], [torch.ones_like(logits), logits.detach()[:, :2] + 1])
+            results.append([v.grad for i, v in enumerate(t) if i not in off])
+        for a, c in zip(*results):
+            assert torch.equal(a, c)
+
+
 def test_fp32_gate_keeps_subclasses_and_autocast_on_the_operations():
     from fastmoe_b200.ops import gating
 
