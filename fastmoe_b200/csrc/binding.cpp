@@ -8,6 +8,7 @@
 // Python exceptions; nothing calls exit().
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -1039,6 +1040,103 @@ std::vector<torch::Tensor> gate_linear_topk_bwd(c10::optional<torch::Tensor> dpr
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
+// The fp32 layer's inputs that its backward does not read, for a gradient of the gradient.  Looked at only
+// there: until then they may be changed in place.
+struct SecondOrder : torch::CustomClassHolder {
+  torch::autograd::SavedVariable x, score, b1, b2;
+};
+
+// The layer behind the gate as operations, experts one after the other.
+torch::Tensor moe_mlp_operations(const torch::Tensor& x, const torch::Tensor& score, const torch::Tensor& w1, const torch::Tensor& b1,
+                                 const torch::Tensor& w2, const torch::Tensor& b2, const torch::Tensor& rank,
+                                 const torch::Tensor& offs, const torch::Tensor& idx, int64_t act) {
+  const torch::Tensor ends = offs.cpu();
+  const int* end = ends.data_ptr<int>();
+  const int64_t groups = w1.size(0), k = idx.numel() / x.size(0), rows = end[groups];
+  const torch::Tensor kept = rank.ge(0).nonzero().squeeze(1), expert = idx.index_select(0, kept);
+  const torch::Tensor row = (offs.index_select(0, expert) + rank.index_select(0, kept)).to(torch::kLong);
+  const torch::Tensor slot = torch::empty({rows}, idx.options()).index_copy_(0, row, kept);
+  const torch::Tensor token = torch::floor_divide(slot, k), xs = x.index_select(0, token);
+  std::vector<torch::Tensor> ys;
+  for (int64_t e = 0; e < groups; ++e) {
+    if (end[e + 1] == end[e]) continue;
+    torch::Tensor hid = torch::linear(xs.slice(0, end[e], end[e + 1]), w1.select(0, e), b1.select(0, e));
+    if (act == fmoe::kActRelu) hid = torch::relu(hid);
+    if (act == fmoe::kActGelu || act == fmoe::kActGeluTanh) hid = at::gelu(hid, act == fmoe::kActGelu ? "none" : "tanh");
+    ys.push_back(torch::linear(hid, w2.select(0, e), b2.select(0, e)));
+  }
+  const torch::Tensor w = score.reshape({-1}).index_select(0, slot).to(x.scalar_type()).unsqueeze(1);
+  return torch::zeros_like(x).index_add(0, token, torch::cat(ys) * w);
+}
+
+struct MoEMLPSaved {
+  torch::Tensor xs, pre, a, ys, rank, offs, score, slots;
+};
+
+// The fp32 layer's backward as a node of its own, for create_graph: its values are the kernels', its derivatives
+// those of the operations.  Outputs: dx where wanted, dscore, dw1 and db1, dw2 and db2 where wanted.
+class MoEMLPGrad : public torch::autograd::Function<MoEMLPGrad> {
+ public:
+  static variable_list forward(AutogradContext* ctx, const torch::Tensor& dout, const torch::Tensor& x, const torch::Tensor& score,
+                               const torch::Tensor& w1, const torch::Tensor& b1, const torch::Tensor& w2, const torch::Tensor& b2,
+                               const MoEMLPSaved* s, int64_t act, bool need_dx, bool need_w1, bool need_w2) {
+    c10::optional<torch::Tensor> pre;
+    if (s->pre.defined()) pre = s->pre;
+    auto r = moe_mlp_backward(dout, s->xs, pre, s->a, s->ys, s->rank, s->offs, s->score, s->slots, w1, w2, act, need_dx,
+                              need_w1, need_w2);
+    variable_list out;
+    std::vector<int64_t> of;   // which input each output is the gradient of (1: x, 2: score, ...)
+    for (int64_t i = 0; i < 6; ++i) {
+      if (!r[i].defined()) continue;
+      out.push_back(r[i]);
+      of.push_back(i + 1);
+    }
+    ctx->save_for_backward({dout, x, score, w1, b1, w2, b2, s->rank, s->offs, s->slots});
+    ctx->saved_data["of"] = of;
+    ctx->saved_data["act"] = act;
+    ctx->set_materialize_grads(false);
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const std::vector<int64_t> of = ctx->saved_data["of"].toIntVector();
+    const bool again = at::GradMode::is_enabled();
+    at::AutoGradMode record(true);
+    at::NoTF32Guard all_bits;
+    variable_list in(s.begin(), s.begin() + 7), result(12);   // dout, x, score, w1, b1, w2, b2
+    // variables of their own: dout depends on the other inputs, and the derivatives wanted are the partial ones
+    for (auto& t : in) t = again ? t.view_as(t) : t.detach().set_requires_grad(true);
+    const torch::Tensor y = moe_mlp_operations(in[1], in[2], in[3], in[4], in[5], in[6], s[7], s[8], s[9],
+                                               ctx->saved_data["act"].toInt());
+    variable_list wrt, seeds;
+    for (size_t i = 0; i < grads.size(); ++i) {
+      const torch::Tensor& t = in[of[i]];
+      if (!grads[i].defined() || !t.requires_grad()) continue;
+      wrt.push_back(t);
+      seeds.push_back(grads[i].reshape(t.sizes()).to(t.scalar_type()));
+    }
+    if (wrt.empty()) return result;
+    const variable_list first = torch::autograd::grad({y}, wrt, {in[0]}, true, true, true);
+    variable_list outs, out_seeds, ins;
+    std::vector<int64_t> at_input;
+    for (size_t i = 0; i < first.size(); ++i) {
+      if (!first[i].defined() || !first[i].requires_grad()) continue;
+      outs.push_back(first[i]);
+      out_seeds.push_back(seeds[i]);
+    }
+    for (int64_t i = 0; i < 7; ++i) {
+      if (!ctx->needs_input_grad(i)) continue;
+      ins.push_back(in[i]);
+      at_input.push_back(i);
+    }
+    if (outs.empty() || ins.empty()) return result;
+    const variable_list second = torch::autograd::grad(outs, ins, out_seeds, true, again, true);
+    for (size_t i = 0; i < ins.size(); ++i) result[at_input[i]] = second[i];
+    return result;
+  }
+};
+
 class MoEMLP : public torch::autograd::Function<MoEMLP> {
  public:
   static torch::Tensor forward(AutogradContext* ctx, const torch::Tensor& x, const torch::Tensor& score,
@@ -1049,6 +1147,14 @@ class MoEMLP : public torch::autograd::Function<MoEMLP> {
     ctx->saved_data["act"] = act;
     ctx->saved_data["shape"] = score.sizes().vec();
     ctx->saved_data["dtype"] = static_cast<int64_t>(score.scalar_type());
+    if (keep && x.scalar_type() == torch::kFloat) {
+      auto second = c10::make_intrusive<SecondOrder>();
+      second->x = torch::autograd::SavedVariable(x, false);
+      second->score = torch::autograd::SavedVariable(score, false);
+      second->b1 = torch::autograd::SavedVariable(b1, false);
+      second->b2 = torch::autograd::SavedVariable(b2, false);
+      ctx->saved_data["second"] = c10::IValue::make_capsule(second);
+    }
     return r[0];
   }
 
@@ -1057,10 +1163,22 @@ class MoEMLP : public torch::autograd::Function<MoEMLP> {
     const bool need_dx = ctx->needs_input_grad(0), need_score = ctx->needs_input_grad(1);
     const bool need_w1 = ctx->needs_input_grad(2) || ctx->needs_input_grad(3);
     const bool need_w2 = ctx->needs_input_grad(4) || ctx->needs_input_grad(5);
-    c10::optional<torch::Tensor> pre;
-    if (s[1].defined()) pre = s[1];
-    auto r = moe_mlp_backward(grads[0], s[0], pre, s[2], s[3], s[4], s[5], s[6], s[7], s[8], s[9],
-                              ctx->saved_data["act"].toInt(), need_dx, need_w1, need_w2);
+    const int64_t act = ctx->saved_data["act"].toInt();
+    variable_list r;   // dx, dscore, dw1, db1, dw2, db2
+    if (at::GradMode::is_enabled() && s[3].scalar_type() == torch::kFloat) {
+      auto second = c10::static_intrusive_pointer_cast<SecondOrder>(ctx->saved_data["second"].toCapsule());
+      const MoEMLPSaved saved{s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7]};
+      const variable_list out = MoEMLPGrad::apply(grads[0], second->x.unpack(), second->score.unpack(), s[8], second->b1.unpack(),
+                                                  s[9], second->b2.unpack(), &saved, act, need_dx, need_w1, need_w2);
+      size_t next = 0;
+      auto take = [&](bool there) { return there ? out[next++] : torch::Tensor(); };
+      for (bool there : {need_dx, true, need_w1, need_w1, need_w2, need_w2}) r.push_back(take(there));
+    } else {
+      c10::optional<torch::Tensor> pre;
+      if (s[1].defined()) pre = s[1];
+      r = moe_mlp_backward(grads[0], s[0], pre, s[2], s[3], s[4], s[5], s[6], s[7], s[8], s[9], act, need_dx, need_w1, need_w2);
+    }
+    if (!torch::autograd::get_current_graph_task_keep_graph()) ctx->saved_data.erase("second");   // as the saved variables
     torch::Tensor dscore;
     if (need_score) {
       dscore = r[1].to(static_cast<torch::ScalarType>(ctx->saved_data["dtype"].toInt()))

@@ -200,3 +200,85 @@ def test_fp32_layer_in_a_graph_and_on_two_streams():
                     outs.append(moe(x))
             torch.cuda.synchronize()
             assert all(torch.equal(a, b) for a, b in zip(outs, want))
+
+
+@pytest.mark.parametrize("act", [nn.GELU(), nn.GELU(approximate="tanh"), nn.ReLU(), nn.Identity()])
+@pytest.mark.parametrize("constant", ["nothing", "scores", "experts", "input"])
+def test_fp32_layer_gradient_of_the_gradient(act, constant):
+    r"""Second and third derivatives against 64 bits; dropped slots, an expert without rows.  fp32 sums of at
+    most 2 * 64 * 96 terms, several of them one after the other."""
+    from fastmoe_b200 import FMoETransformerMLP
+    from fastmoe_b200.ops import fused
+    torch.manual_seed(4)
+    moe = FMoETransformerMLP(num_expert=4, d_model=64, d_hidden=96, activation=act, top_k=2).to(DEV)
+    nn.init.normal_(moe.experts.htoh4.bias)
+    nn.init.normal_(moe.experts.h4toh.bias)
+    base = [torch.randn(64, 64, device=DEV), torch.rand(64, 2, device=DEV)] + [p.detach() for p in moe.experts.parameters()]
+    ids = torch.randint(-1, 3, (64, 2), device=DEV)
+    off = {"nothing": (), "scores": (1,), "experts": (2, 3, 4, 5), "input": (0,)}[constant]
+    names = [n for n, _ in moe.experts.named_parameters()]
+
+    def layer(x, score, *params):
+        p = dict(zip(names, params))
+        if x.dtype == torch.float32:
+            from fastmoe_b200.ops import grouped_gemm as gg, native
+            from fastmoe_b200.transformer import activation_kind
+            return native.get().moe_mlp(x, score, p["htoh4.weight"], p["htoh4.bias"], p["h4toh.weight"], p["h4toh.bias"],
+                                        ids, gg.ACT_CODES[activation_kind(act)], True)
+        rows = torch.stack([act(x @ p["htoh4.weight"][e].t() + p["htoh4.bias"][e]) @ p["h4toh.weight"][e].t()
+                            + p["h4toh.bias"][e] for e in range(4)])
+        picked = rows[ids.clamp(min=0), torch.arange(64, device=DEV)[:, None]]
+        return (picked * (score * (ids >= 0))[..., None]).sum(1)
+
+    assert fused.supports(moe, base[0], ids, base[1])
+    results = []
+    for dtype in (torch.float32, torch.float64):
+        t = [b.to(dtype, copy=True).requires_grad_(i not in off) for i, b in enumerate(base)]
+        wanted = [v for i, v in enumerate(t) if i not in off]
+        y = layer(*t)
+        first = torch.autograd.grad((y.sin() * 0.5).sum(), wanted, create_graph=True)
+        second = torch.autograd.grad(sum(g.square().sum() for g in first), wanted, create_graph=True, allow_unused=True)
+        third = torch.autograd.grad(sum(g.square().sum() for g in second if g is not None), wanted, allow_unused=True)
+        results.append([torch.zeros(()) if g is None else g.detach().double().cpu() for g in first + second + third])
+    for got, want in zip(*results):
+        assert float((got - want).norm()) <= 2e-5 * float(want.norm()) + 1e-12, (got.shape,)
+
+
+def test_fp32_layer_input_changed_in_place_afterwards():
+    r"""The backward does not read the input: with a frozen gate it may be changed, as it may around the general
+    path; a gradient of the gradient does, and notices."""
+    from fastmoe_b200 import FMoETransformerMLP
+    torch.manual_seed(5)
+    moe = FMoETransformerMLP(num_expert=4, d_model=64, d_hidden=96, top_k=2).to(DEV)
+    moe.gate.requires_grad_(False)
+    leaf = torch.randn(64, 64, device=DEV, requires_grad=True)
+    want, = torch.autograd.grad((leaf * 1 + moe(leaf * 1)).sum(), leaf)
+    x = leaf * 1
+    x += moe(x)
+    got, = torch.autograd.grad(x.sum(), leaf)
+    assert torch.allclose(got, want, rtol=0, atol=1e-6)   # (sums of three terms in another order)
+    x = leaf * 1
+    x += moe(x)
+    with pytest.raises(RuntimeError, match="inplace operation"):
+        torch.autograd.grad(x.square().sum(), leaf, create_graph=True)
+
+
+def test_fp32_layer_under_checkpointing_and_offloading():
+    from torch.utils.checkpoint import checkpoint
+    from fastmoe_b200 import FMoETransformerMLP
+    torch.manual_seed(6)
+    moe = FMoETransformerMLP(num_expert=4, d_model=64, d_hidden=96, top_k=2).to(DEV)
+    x = torch.randn(64, 64, device=DEV, requires_grad=True)
+
+    def offloaded(t):
+        with torch.autograd.graph.save_on_cpu():
+            return moe(t)
+    results = []
+    for run in (moe, lambda t: checkpoint(moe, t, use_reentrant=False), offloaded):
+        moe.zero_grad(set_to_none=True)
+        grads = torch.autograd.grad(run(x).square().sum(), [x] + list(moe.parameters()))
+        twice = torch.autograd.grad(torch.autograd.grad(run(x).square().sum(), x, create_graph=True)[0].square().sum(), x)
+        results.append(grads + twice)
+    for other in results[1:]:
+        for a, b in zip(other, results[0]):
+            assert torch.allclose(a, b, rtol=1e-5, atol=1e-5 * float(b.abs().max()))
