@@ -1,16 +1,19 @@
 // fp32 grouped GEMM on the tensor cores.
 //
-// An fp32 value is the sum of three bf16 values h + m + l (8 + 8 + 8 bits, each the rounded rest of
-// the one before; same exponent range), so that a product of two is the sum of nine bf16 products,
-// each exact in fp32.  Six are formed: h h, and the five of the next two orders (h m, m h, m m, h l,
-// l h); what is left out (m l, l m, l l) is below 2^-26 of the product.  tf32, the tensor cores' own
-// fp32 format, would drop 13 bits of the inputs instead.
+// An fp32 value is the sum of three bf16 values, h + m + l (8 + 8 + 8 bits, each the rounded rest of
+// the one before), so that a product of two is the sum of nine bf16 products, each exact in fp32.  Six are
+// formed: h h, and the five of the next two orders (h m, m h, and m m, h l, l h); what is left out (m l,
+// l m, l l) is below 2^-26 of the product.  tf32, the tensor cores' own fp32 format, would drop 13 bits of
+// the inputs instead.  m and l are held as m 2^7 and l 2^14, which keeps them in bf16's range where
+// the value is in fp32's, but for an error of at most 2^-148; unscaled, the rests of a value below 2^-110 fall
+// under the smallest bf16 subnormal, 2^-133 (at 2^-120 6e-5 of the value was lost).  Larger scales would let the
+// small products overflow before the result does.  The three orders have an accumulator each.
 //
 // The tensor cores add with truncation, which over a long sum costs more than the roundings of fp32
 // FMAs.  So h h is accumulated in TMEM over one K block of 64 only (four additions); the epilogue
-// warps take every block's sum into registers and add them in fp32, rounded to nearest.  The five
-// small products have an accumulator of their own for the whole sum: they are 2^-8 of the result.
-// Keeping the two apart also keeps infinities: inf - inf of h l and h m would be NaN where the
+// warps take every block's sum into registers and add them in fp32, rounded to nearest.  The small
+// products are accumulated over the whole sum: they are 2^-8 of the result and less.
+// Keeping them apart also keeps infinities: inf - inf of h l and h m would be NaN where the
 // product is inf, so a total that is not finite is replaced by the sum of h h.
 //
 // Error against 64 bits (2-norm, 8 experts, 4096 rows, 512 -> 2048): forward 7.3e-8, input gradient
@@ -33,7 +36,7 @@
 //   warps 2, 3  weight gradient: column sums of P (the bias gradient) and zeros of experts without
 //               rows; row modes: zeros past the last expert;
 //   warps 4-11  epilogue.
-// TMEM: three accumulators of 128 columns for h h, one for the small products.
+// TMEM: two accumulators of 128 columns for h h in turn, one each for the products of the next two orders.
 #include "split_gemm.cuh"
 
 #include <float.h>
@@ -69,8 +72,11 @@ constexpr int NUM_EPI_WARPS = 8;
 constexpr int FIRST_EPI_WARP = 4;
 constexpr int NUM_THREADS = (FIRST_EPI_WARP + NUM_EPI_WARPS) * 32;
 constexpr int EPI_COLS = TILE_N / 2;             // columns per epilogue warp
-constexpr int MAIN_BUFS = 3;
+constexpr int MAIN_BUFS = 2;
+constexpr int M_COL = MAIN_BUFS * TILE_N;        // TMEM columns of the products with one m, and of the order after
+constexpr int L_COL = M_COL + TILE_N;
 constexpr int TMEM_COLS = 512;
+constexpr float M_SCALE = 128.f, L_SCALE = M_SCALE * M_SCALE;   // (m m is of l's order)
 
 struct Shared {
   uint64_t full[STAGES];          // CTA 0's counts: one arrival and the bytes of each CTA
@@ -135,20 +141,24 @@ __device__ __forceinline__ Tile decode(const Shared* sh, int n_tiles, const Walk
 }
 
 // ------------------------------------------------------------------------------ values
-// h + m + l == x for finite x; the planes of a value that is not finite are (x, 0, 0).
+// h + m / M_SCALE + l / L_SCALE == x for finite x, l exact in bf16 for x of at least 2^-124 and rounded to a
+// multiple of 2^-133 below; the planes of a value that is not finite are (x, 0, 0).
 __device__ __forceinline__ void split1(float x, float& h, float& m, float& l) {
   // 0x7f7f8000 and above would round to infinity: the largest bf16 value is taken instead
   const float mag = fminf(fabsf(x), __uint_as_float(0x7f7f0000u));
   h = __bfloat162float(__float2bfloat16_rn(copysignf(mag, x)));
-  const float r = x - h;
+  const float r = (x - h) * M_SCALE;
   m = __bfloat162float(__float2bfloat16_rn(r));
-  l = r - m;
+  l = (r - m) * (L_SCALE / M_SCALE);
   if (!(fabsf(x) <= FLT_MAX)) {
     h = x;
     m = 0.f;
     l = 0.f;
   }
 }
+
+// The value again; the sum of the two smaller parts is rounded once.
+__device__ __forceinline__ float join3(float h, float m, float l) { return h + fmaf(l, 1.f / L_SCALE, m * (1.f / M_SCALE)); }
 
 __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
   float h0, m0, l0, h1, m1, l1;
@@ -344,7 +354,7 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       while (ok && walk.next(part_of)) {
         const Tile c = decode(sh, n_tiles, part_of);
         const int len = MODE == kWgrad ? c.rows : p.k;
-        const uint32_t d_small = tmem_base + MAIN_BUFS * TILE_N;
+        const uint32_t d_m = tmem_base + M_COL, d_l = tmem_base + L_COL;
         for (int kb = part_of.kb0; kb < part_of.kb1; ++kb) {
           const uint32_t d_main = tmem_base + buf * TILE_N;
           if (!(ok = wait(&sh->main_empty[buf], buf_phase ^ 1) && wait(&sh->full[stage], phase))) break;
@@ -372,11 +382,12 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           for (int k16 = 0; k16 < BK / UMMA_K; ++k16) {
             if (k16 < steps) {
               ptx::umma_f16_pair_collect<ptx::kCollectFill>(d_main, desc_a(0, k16), desc_b(0, k16), idesc, k16 != 0 ? 1u : 0u);
-              ptx::umma_f16_pair_collect<ptx::kCollectUse>(d_small, desc_a(0, k16), desc_b(2, k16), idesc, first && k16 == 0 ? 0u : 1u);
-              ptx::umma_f16_pair_collect<ptx::kCollectLast>(d_small, desc_a(0, k16), desc_b(1, k16), idesc, 1u);
-              ptx::umma_f16_pair_collect<ptx::kCollectFill>(d_small, desc_a(1, k16), desc_b(1, k16), idesc, 1u);
-              ptx::umma_f16_pair_collect<ptx::kCollectLast>(d_small, desc_a(1, k16), desc_b(0, k16), idesc, 1u);
-              ptx::umma_f16_pair(d_small, desc_a(2, k16), desc_b(0, k16), idesc, 1u);
+              const uint32_t on = first && k16 == 0 ? 0u : 1u;
+              ptx::umma_f16_pair_collect<ptx::kCollectUse>(d_l, desc_a(0, k16), desc_b(2, k16), idesc, on);
+              ptx::umma_f16_pair_collect<ptx::kCollectLast>(d_m, desc_a(0, k16), desc_b(1, k16), idesc, on);
+              ptx::umma_f16_pair_collect<ptx::kCollectFill>(d_l, desc_a(1, k16), desc_b(1, k16), idesc, 1u);
+              ptx::umma_f16_pair_collect<ptx::kCollectLast>(d_m, desc_a(1, k16), desc_b(0, k16), idesc, 1u);
+              ptx::umma_f16_pair(d_l, desc_a(2, k16), desc_b(0, k16), idesc, 1u);
             }
           }
           ptx::umma_commit_pair(&sh->main_full[buf]);
@@ -437,8 +448,8 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                   float a[3], b[3];
 #pragma unroll
                   for (int pl = 0; pl < 3; ++pl) gg::Cvt<bf16>::unpack((&v[u][pl].x)[j], a[pl], b[pl]);
-                  sa += a[0] + (a[1] + a[2]);
-                  sb += b[0] + (b[1] + b[2]);
+                  sa += join3(a[0], a[1], a[2]);
+                  sb += join3(b[0], b[1], b[2]);
                 }
                 cs[2 * j] += sa;
                 cs[2 * j + 1] += sb;
@@ -554,20 +565,21 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       small_phase ^= 1;
       ptx::tc_fence_after_sync();
       float v[EPI_COLS];
-      {
-        uint32_t r0[32], r1[32];
-        ptx::tmem_ld_32x32(t_lane + MAIN_BUFS * TILE_N, r0);
-        ptx::tmem_ld_32x32(t_lane + MAIN_BUFS * TILE_N + 32, r1);
-        ptx::tmem_ld_wait();
-        release(&sh->small_empty);
 #pragma unroll
-        for (int j = 0; j < EPI_COLS / 2; ++j) {
+      for (int q = 0; q < 2; ++q) {   // 32 columns at a time: both sums of small products
+        uint32_t rm[32], rl[32];
+        ptx::tmem_ld_32x32(t_lane + M_COL + q * 32, rm);
+        ptx::tmem_ld_32x32(t_lane + L_COL + q * 32, rl);
+        ptx::tmem_ld_wait();
+        if (q == 1) release(&sh->small_empty);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
           float a0, a1;
-          ptx::unpack2(acc[j], a0, a1);
-          const float s0 = a0 + __uint_as_float(j < 16 ? r0[(2 * j) & 31] : r1[(2 * j) & 31]);
-          const float s1 = a1 + __uint_as_float(j < 16 ? r0[(2 * j + 1) & 31] : r1[(2 * j + 1) & 31]);
-          v[2 * j] = fabsf(s0) <= FLT_MAX ? s0 : a0;
-          v[2 * j + 1] = fabsf(s1) <= FLT_MAX ? s1 : a1;
+          ptx::unpack2(acc[q * 16 + j], a0, a1);
+          const float s0 = join3(a0, __uint_as_float(rm[2 * j]), __uint_as_float(rl[2 * j]));
+          const float s1 = join3(a1, __uint_as_float(rm[2 * j + 1]), __uint_as_float(rl[2 * j + 1]));
+          v[q * 32 + 2 * j] = fabsf(s0) <= FLT_MAX ? s0 : a0;
+          v[q * 32 + 2 * j + 1] = fabsf(s1) <= FLT_MAX ? s1 : a1;
         }
       }
       const int ew = warp - FIRST_EPI_WARP;

@@ -5,7 +5,8 @@
 
 namespace fmoe {
 
-// An fp32 matrix as three bf16 planes h, m, l with h + m + l equal to the value, one behind the other.
+// An fp32 matrix as three bf16 planes, one behind the other: h, m 2^7 and l 2^14, where h + m + l is the value (to
+// 2^-148 where it is below 2^-124).
 // Matrices of token rows are padded: rows of expert e begin at split_row(offs[e], e), and the rows
 // from its last one to the next multiple of 64 are zero.
 __host__ __device__ inline long split_row(long off, long e) { return ((off + 63) / 64 + e) * 64; }

@@ -99,6 +99,39 @@ def test_split_gemm_keeps_infinities_large_and_small_values():
     assert bool(((y.double() - ref).abs()[ok] <= _bound(size, k)[ok]).all())
 
 
+@pytest.mark.parametrize("exponent", [-100, -108, -112, -116, -120, -124, -127])
+@pytest.mark.parametrize("which", ["rows", "weights"])
+def test_split_gemm_of_values_near_the_end_of_the_range(exponent, which):
+    r"""As for other values; besides, an operand is held to 2^-148, and a sum below 2^-126 is a multiple of 2^-149."""
+    nat = _native()
+    torch.manual_seed(exponent)
+    counts, k, n = [70, 300], 128, 192
+    offs = _offs(counts)
+    x, dy = torch.randn(370, k, device=DEV), torch.randn(370, n, device=DEV)
+    w = torch.randn(2, n, k, device=DEV)
+    for t in (x, dy) if which == "rows" else (w,):
+        t *= 2.0 ** exponent
+    y, dx, dw, db = (torch.empty(*size, device=DEV) for size in ((370, n), (370, k), (2, n, k), (2, n)))
+    nat.split_grouped_gemm(0, x, w, offs, y, None, None)
+    nat.split_grouped_gemm(1, dy, w, offs, dx, None, None)
+    nat.split_grouped_gemm(2, dy, x if which == "weights" else x * 2.0 ** -exponent, offs, dw, None, db)
+    if which == "rows":
+        x_of_dw = x * 2.0 ** -exponent
+    base = 0
+    for e, c in enumerate(counts):
+        s = slice(base, base + c)
+        base += c
+        X, D, W = x[s].double(), dy[s].double(), w[e].double()
+        V = x_of_dw[s].double() if which == "rows" else X
+        for got, ref, size, small, terms in [
+                (y[s], X @ W.t(), X.abs() @ W.abs().t(), (X if which == "weights" else W).abs().max(), k),
+                (dx[s], D @ W, D.abs() @ W.abs(), (D if which == "weights" else W).abs().max(), n),
+                (dw[e], D.t() @ V, D.abs().t() @ V.abs(), V.abs().max(), c)]:
+            bound = _bound(size, terms) + terms * (2.0 ** -148 * small + 2.0 ** -149)
+            assert bool(((got.double() - ref).abs() <= bound).all()), float(((got.double() - ref).abs() / bound).max())
+        assert bool(((db[e].double() - D.sum(0)).abs() <= D.abs().sum(0) * (24 + c / 256) * 2.0 ** -24 + c * 2.0 ** -148).all())
+
+
 @pytest.mark.parametrize("act", [nn.GELU(), nn.ReLU(), nn.GELU(approximate="tanh"), nn.Identity(),
                                  nn.Sequential(nn.ReLU(), nn.Dropout(0.0))])
 @pytest.mark.parametrize("experts,k,d,h,tokens", [(4, 2, 64, 136, 300), (3, 1, 40, 72, 65), (8, 3, 128, 512, 1000)])
