@@ -92,3 +92,23 @@ def test_naive_gate_under_function_transforms(default):
     assert held.dtype == default and held.requires_grad and held.is_leaf and float(held.detach()) == 0
     with torch.inference_mode():
         gate(x)
+
+
+@pytest.mark.parametrize("how", ["subclass", "instance"])
+def test_naive_gate_with_another_choice(how):
+    from fastmoe_b200.gates import NaiveGate
+
+    class Worst(NaiveGate):
+        def _choose(self, inp):
+            logits, idx, score = super()._choose(inp)
+            return logits, idx.flip(1), score
+    torch.manual_seed(0)
+    plain, x = NaiveGate(16, 4, 1, 2), torch.randn(6, 16)
+    gate = Worst(16, 4, 1, 2) if how == "subclass" else NaiveGate(16, 4, 1, 2)
+    gate.load_state_dict(plain.state_dict())
+    if how == "instance":
+        def choose(inp):
+            logits, idx, score = NaiveGate._choose(gate, inp)
+            return logits, idx.flip(1), score
+        gate._choose = choose
+    assert torch.equal(gate(x)[0], plain(x)[0].flip(1)) and float(gate.get_loss().detach()) == 0
