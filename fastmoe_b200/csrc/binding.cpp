@@ -475,15 +475,15 @@ void split_grouped_gemm(int64_t mode, torch::Tensor a, torch::Tensor b, torch::T
   FMOE_CUDA_CHECK(fmoe::launch_split_gemm(g));
 }
 
-// When one product by itself is faster split than on the FMA units.  Those take the larger of the
-// operations at 47 TFLOP/s and their serial chain (one sum over k, or over an expert's rows: 0.066 us
-// per element).  Split, the operands are read and written first (16 bytes an element in all), the
-// weight gradient is stored by few tiles, and the chain is short.  Taken where the estimate is 25 us
-// lower, which is what issuing the other launches costs an eager program (8 experts, 277 rows each,
-// 160 -> 320, eager, forward and backward: 203 us split, 183 not).  us measured, split against FMA, forward / input gradient / weight gradient: 8
-// experts, 512 rows each, 512 -> 2048: 94, 113, 108 against 203, 220, 177; 16 experts, 64 rows each:
-// 92, 110, 74 against 83, 152, 54; 8 experts, 128 rows each, 128 -> 512: 17, 26, 27 against 12, 37, 12;
-// 4 experts, 7500 rows each, 64 -> 64: 20, 17, 43 against 17, 15, 544.
+// When one product by itself is faster split than on the FMA units.  Those take the larger of the operations
+// at 47 TFLOP/s and their serial chain (one sum over k, or over an expert's rows: 0.066 us per element).
+// Split, the operands are read and written first (16 bytes an element in all), the weight gradient is stored
+// by few tiles, and the chain is short.  Taken where the estimate is 25 us lower, which is what issuing the
+// other launches costs an eager program (8 experts, 277 rows each, 160 -> 320, eager, forward and backward:
+// 203 us split, 183 not).  us measured, split against FMA, forward / input gradient / weight gradient: 8
+// experts, 512 rows each, 512 -> 2048: 94, 113, 108 against 203, 220, 177; 16 experts, 64 rows each: 92, 110,
+// 74 against 83, 152, 54; 8 experts, 128 rows each, 128 -> 512: 17, 26, 27 against 12, 37, 12; 4 experts,
+// 7500 rows each, 64 -> 64: 20, 17, 43 against 17, 15, 544.
 bool split_worth_it(int64_t mode, int64_t rows, const GemmSizes& z) {
   const bool wgrad = mode == fmoe::kWgrad;
   const double r = static_cast<double>(rows), n = z.n, k = wgrad ? z.m : z.k, weights = n * k * z.groups;

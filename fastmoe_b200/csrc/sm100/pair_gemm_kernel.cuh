@@ -388,10 +388,10 @@ __device__ __forceinline__ void epilogue_tile_update(const Params& p, const EpiT
   release_accumulator(et);
 }
 
-// The bias gradient of a grouped linear is the column sum, per expert, of the matrix its weight
-// gradient takes as P.  Either (`side_sums` = 0) on the tiles of the first N column block the epilogue warps, which wait
-// for the main loop then, add up this CTA's 128 columns of P with plain 16-byte loads (the rows
-// pass through the L2 for the TMA loads at the same time).
+// The bias gradient of a grouped linear is the column sum, per expert, of the matrix its weight gradient
+// takes as P.  Either (`side_sums` = 0) on the tiles of the first N column block the epilogue warps, which
+// wait for the main loop then, add up this CTA's 128 columns of P with plain 16-byte loads (the rows pass
+// through the L2 for the TMA loads at the same time).
 template <typename T>
 __device__ __forceinline__ void column_sums(const Params& p, uint8_t* patches, const Tile& c, int col0, int warp, int lane) {
   const int ew = warp - FIRST_EPI_WARP;

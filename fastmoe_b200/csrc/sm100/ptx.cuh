@@ -332,8 +332,6 @@ __device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_a
                : "memory");
 }
 
-__device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
-
 // Tiled load into this CTA's shared memory (no multicast) whose completion is counted on a
 // barrier of either CTA of the pair.
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr,

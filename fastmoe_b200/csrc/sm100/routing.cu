@@ -35,12 +35,11 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // into exclusive prefixes over warps, pass 2 hands every slot its rank.  Within a warp slots
 // are visited in order, 32 at a time.  The chain of these steps is what bounds the kernel (a
 // match of 32 keys and an update of shared memory that the next step waits for), so up to
-// kRouteClusterSlots slots are spread over a cluster of eight CTAs, which exchange their
-// per-expert totals through distributed shared memory in the one launch: 16384 slots on 8 experts
-// 19 -> 6.8 us, 8192 slots on 64 experts 17.9 -> 6.4 us.  For more slots the work is spread over more CTAs and two launches: the first
-// (`part_out`) only writes every CTA's per-expert totals, the second (`part_in`) starts each CTA's
-// prefixes at the sum of the totals of the CTAs before it.  Ranks are always those of a single
-// ordered scan.
+// kRouteClusterSlots slots are spread over a cluster of eight CTAs, which exchange their per-expert totals
+// through distributed shared memory in the one launch: 16384 slots on 8 experts 19 -> 6.8 us, 8192 slots on
+// 64 experts 17.9 -> 6.4 us.  For more slots the work is spread over more CTAs and two launches: the first
+// (`part_out`) only writes every CTA's per-expert totals, the second (`part_in`) starts each CTA's prefixes
+// at the sum of the totals of the CTAs before it.  Ranks are always those of a single ordered scan.
 __global__ void __launch_bounds__(kRouteThreads, 1)
 route_kernel(const int64_t* __restrict__ idx, int n_slots, int tot, int nw, int cta_slots, int in_cluster,
              const int* __restrict__ part_in, int* __restrict__ part_out, int* __restrict__ counts,
@@ -833,7 +832,6 @@ switch_top1_kernel(const T* __restrict__ logits, int n, int tot, int64_t* __rest
   Ld<T>::put(score, t, best_p);
 }
 
-// new_idx[s] = idx[s] when fewer than `cap` slots of its expert come before it, else -1
 // What the tensor-core gate multiplies with when its experts are no multiple of 64: one launch where padding,
 // filling and copying were four (a layer's step, eager, 16 experts, 1237 tokens, d 256: 472 -> 430 us).
 template <typename T>
@@ -864,6 +862,7 @@ __global__ void host_offsets_kernel(const __grid_constant__ HostValues<N> values
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = values.v[i];
 }
 
+// out[s] = idx[s] when fewer than `cap` slots of its expert come before it, else -1
 __global__ void prune_scalar_kernel(const int64_t* __restrict__ idx, const int* __restrict__ rank, int cap, int n_slots,
                                     int tot, int64_t* __restrict__ out) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1443,11 +1442,11 @@ template <> __device__ __forceinline__ void stv<__half>(__half* p, long i, float
   p[i] = __float2half(v);
 }
 
-// Shared-memory tiled SIMT GEMM for fp64, for fp32 with rows that are not 16-byte aligned (split_gemm.cu
-// and sgemm.cu take the others) and for 16-bit shapes the tensor-core kernel does not take.  One CTA of 256 threads computes a 64 x 64 tile
-// of C = A B with a K step of 16; every thread owns a 4 x 4 block of the tile and accumulates in
-// fp32 (fp64 for doubles).  The three products of a grouped linear differ only in where A(i, kk)
-// and B(kk, j) live:
+// Shared-memory tiled SIMT GEMM for fp64, for fp32 with rows that are not 16-byte aligned (split_gemm.cu and
+// sgemm.cu take the others) and for 16-bit shapes the tensor-core kernel does not take.  One CTA of 256
+// threads computes a 64 x 64 tile of C = A B with a K step of 16; every thread owns a 4 x 4 block of the tile
+// and accumulates in fp32 (fp64 for doubles).  The three products of a grouped linear differ only in where
+// A(i, kk) and B(kk, j) live:
 //   mode 0 (NT)   rows of expert g:  A = a[row, kk],   B = b[g, j, kk]
 //   mode 1 (NN)   rows of expert g:  A = a[row, kk],   B = b[g, kk, j]
 //   mode 2 (wgrad) out[g, i, j]:     A = p[r0 + kk, i], B = q[r0 + kk, j], K = rows of expert g

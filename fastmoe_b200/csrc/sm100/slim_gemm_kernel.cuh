@@ -1,15 +1,15 @@
 // Grouped GEMM on CTA pairs, row modes (forward and input gradient): the token rows are the N side of
 // the MMA.
 //
-// With tiles of 256 token rows, as the weight gradient's kernel has them and this one's predecessor
-// had, an expert with 130 rows costs as much as one with 256, the second CTA has next to nothing to
-// store, and half of what is loaded are other experts' rows.  Here a tile is 256 output columns (rows of the weights, M) by as
-// many token rows as the expert has left, in steps of 64 and at most 256 (N, chosen tile by tile in
-// the instruction descriptor), so that both the MMAs and the loads go with the rows there are and the
-// epilogue is shared evenly by the two CTAs.  What bounds it: with up to a hundred rows per expert the
-// weights (64 experts, 64 rows each, 1024 -> 4096, no activation: 100 us, 5.4 TB/s); with many rows
-// the tensor cores (8192 rows, 2 experts, 1024 <-> 4096: 53 and 51 us, 1280 to 1340 TFLOP/s) and, with
-// few K blocks, the epilogue.  Against 256-row tiles: see the rule in grouped_gemm.cu.
+// With tiles of 256 token rows, as the weight gradient's kernel has them and this one's predecessor had, an
+// expert with 130 rows costs as much as one with 256, the second CTA has next to nothing to store, and half
+// of what is loaded are other experts' rows.  Here a tile is 256 output columns (rows of the weights, M) by
+// as many token rows as the expert has left, in steps of 64 and at most 256 (N, chosen tile by tile in the
+// instruction descriptor), so that both the MMAs and the loads go with the rows there are and the epilogue is
+// shared evenly by the two CTAs.  What bounds it: with up to a hundred rows per expert the weights (64
+// experts, 64 rows each, 1024 -> 4096, no activation: 100 us, 5.4 TB/s); with many rows the tensor cores
+// (8192 rows, 2 experts, 1024 <-> 4096: 53 and 51 us, 1280 to 1340 TFLOP/s) and, with few K blocks, the
+// epilogue.  Against 256-row tiles: see the rule in grouped_gemm.cu.
 //
 // The accumulators come out transposed: a TMEM lane is an output column, a TMEM column a token row.  The
 // epilogue loads them as 8 x 8 fragments (tcgen05.ld 16x256b) and transposes them on the way to shared

@@ -26,7 +26,7 @@
 // A pair of CTAs (cta_group::2) works
 // on a 256 x 128 tile, half the width of the 16-bit kernel's: an epilogue warp holds 32 x 64 sums in
 // registers, 64 per thread, and fp32 layers are small (512 outputs of 8 experts with 512 rows are
-// 64 such tiles for 74 pairs).  The tiles of the last rounds are cut along K (tile_walk.cuh): 8
+// 64 such tiles for 74 pairs).  The tiles of the last round are cut along K (tile_walk.cuh): 8
 // experts with 384 to 640 rows, 2048 -> 512, 119 against 141 us, splitting included.
 //
 // Roles of a CTA (384 threads), persistent over the tiles of its pair:

@@ -1,14 +1,15 @@
 // Which parts of which output tiles a CTA pair of a persistent grouped GEMM works on.
 //
 // T tiles on P pairs take ceil(T / P) rounds, and a last round of few tiles leaves most of the chip
-// idle.  So only the rounds before the last full one are dealt out tile by tile, in turn, which keeps
-// tiles that run at the same time next to each other.  The tiles left (P to 2 P of them, or all of
-// T < P) are one sequence of K blocks, cut into equal pieces, one per pair.  A piece begins with the
-// end of one tile and ends with the beginning of another.  The pair that has a tile's first K block
-// owns the tile; the others hand it their sums through global memory.  A pair meets the part it does
-// not own first and the part for which it has to collect the rest last: nobody waits before handing
-// over, so every wait ends whatever order the pairs run in, and an owner hardly waits.  The cut
-// depends on the offsets alone: equal calls add in equal order.
+// idle.  The full rounds are dealt out tile by tile, in turn, which keeps tiles that run at the same time
+// next to each other.  Where cutting pays (dealt_tiles), the T mod P tiles left are one sequence of K
+// blocks, cut into equal pieces, one per pair, but no more pieces than leave each `cost_kb` K blocks on
+// average (at least one per tile).  A piece begins with the end of one tile and ends with the beginning of
+// another, or lies inside one.  The pair that has a tile's first K block owns the tile; the others hand it
+// their sums through global memory.  A pair meets the part it does not own first and the part for which it
+// has to collect the rest last: nobody waits before handing over, so every wait ends whatever order the
+// pairs run in, and an owner hardly waits.  The cut depends on the offsets alone: equal calls add in equal
+// order.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -148,7 +148,8 @@ class _Combine(Function):
 def rows_supported(x, ids, scores):
     r"""Whether the kernels that move and combine rows take a call of the general path."""
     return (torch.is_tensor(x) and x.is_cuda and x.dim() == 2 and x.dtype in _TC + (torch.float32,)
-            and x.shape[1] % 8 == 0 and x.shape[1] > 0 and ids.is_cuda and ids.dtype == torch.int64 and ids.dim() in (1, 2)
+            and x.shape[1] % 8 == 0 and x.shape[1] > 0
+            and ids.is_cuda and ids.dtype == torch.int64 and ids.dim() in (1, 2)
             and ids.device == x.device and scores.device == x.device
             and ids.shape[0] == x.shape[0] and ids.numel() > 0 and ids.numel() < 2 ** 31
             and scores.numel() == ids.numel() and scores.is_floating_point()
@@ -265,7 +266,9 @@ class _MoEMLP(Function):
     r"""The whole single-GPU layer behind the gate as one node: :class:`_Dispatch`,
     :class:`_ExpertMLP` and :class:`_Combine` with their launches issued by one native call per
     direction.  With ``keep`` false (nothing will be differentiated) the pre-activation is not
-    written.  In fp32 ``xs`` and ``a`` are kept as the bf16 parts that the tensor cores multiply.
+    written.  In fp32 ``xs`` and ``a`` are kept as the bf16 parts that the tensor cores multiply, 6
+    bytes an element between forward and backward where fp32 has 4, and beside each GEMM its weights
+    are held in parts too (6 bytes a weight, for the time of the launch).
 
     The native node of the same (``binding.cpp::MoEMLP``) takes all calls but traced ones: its backward
     runs without the interpreter (a small layer's step, 512 tokens, d 256, 4 experts: 429 us of host time

@@ -82,7 +82,8 @@ class _LinearTopkSoftmax(Function):
         if grad_logits is None and grad_prob is None:
             return None, None, None, None
         need_dx, need_dw, need_db = ctx.needs_input_grad[:3]
-        if torch.is_grad_enabled() and prob.dtype == torch.float32:   # a gradient of the gradient, as in the native node
+        if torch.is_grad_enabled() and prob.dtype == torch.float32:
+            # a gradient of the gradient, as in the native node
             dl = grad_logits
             if grad_prob is not None:
                 through = native.get().gate_topk_softmax_bwd(grad_prob.contiguous(), idx, prob, ctx.tot)
@@ -141,10 +142,11 @@ def traced():
 
 class _GateGemm(Function):
     r"""``logits = x W^T + b`` on the tcgen05 grouped-GEMM kernel (one group, whose row count goes
-    with the launch: no offsets on the device), for any number of experts.  The expert dimension is padded to a multiple of 64 — the padding columns get a
-    large negative bias, so a top-k over the padded logits never selects them; 64, 128 ... experts need no
-    copies, others one launch — and the backward products ``dx = dl W`` and ``dW = dl^T x`` (with ``db`` from the same launch) run on
-    the same kernel's input-gradient and weight-gradient modes."""
+    with the launch: no offsets on the device), for any number of experts.  The expert dimension is
+    padded to a multiple of 64 — the padding columns get a large negative bias, so a top-k over the
+    padded logits never selects them; 64, 128 ... experts need no copies, others one launch — and the
+    backward products ``dx = dl W`` and ``dW = dl^T x`` (with ``db`` from the same launch) run on the
+    same kernel's input-gradient and weight-gradient modes."""
 
     @staticmethod
     def forward(ctx, x, weight, bias):
@@ -154,7 +156,8 @@ class _GateGemm(Function):
             wp = weight.contiguous().unsqueeze(0)
             bp = None if bias is None else bias.contiguous().unsqueeze(0)
         else:
-            wp, bp = native.get().gate_pad(gg.aligned(weight, 16), None if bias is None else bias.contiguous(), tot + pad)
+            wp, bp = native.get().gate_pad(gg.aligned(weight, 16), None if bias is None else bias.contiguous(),
+                                           tot + pad)
         logits = gg.forward(x, wp, None, bp)
         ctx.save_for_backward(x, wp)
         ctx.tot = tot
@@ -224,9 +227,8 @@ def linear_topk_softmax(x, weight, bias, k, zero=None):
         return tuple(native.get().gate_linear_topk_node(xc, weight.contiguous(), bias, int(k), zero))
     if _few_tokens_ok(x, weight, bias, k):
         x, weight = gg.aligned(x, 16), gg.aligned(weight, 16)
-        logits, idx, prob = native.get().gate_linear_topk(x, weight, None if bias is None else bias.contiguous(), int(k), True,
-                                                            zero)
-        return logits, idx, prob
+        bias = None if bias is None else bias.contiguous()
+        return tuple(native.get().gate_linear_topk(x, weight, bias, int(k), True, zero))
     if _gate_gemm_ok(x, weight, bias) and k <= MAX_FUSED_K:
         # more experts: tensor-core product on this library's own kernel, then the top-k /
         # softmax kernel over the (padded) logits

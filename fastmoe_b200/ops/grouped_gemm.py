@@ -6,9 +6,9 @@ The three products of a grouped linear — forward ``Y_e = X_e W_e^T (+b_e)``, i
 124-147`` in the reference, one cuBLAS call each per expert) — are single launches of the
 tcgen05 kernel for bf16/fp16 with tensor-core-friendly shapes.  fp32 runs on the tensor cores
 too where there is enough to compute, as six products of bf16 parts that together keep fp32's
-precision; small fp32 calls, fp64 and odd shapes take the reference-precision SIMT kernels.  Row offsets are an int32 device tensor
-``offs[E+1]`` (``None`` for a single group of all rows, tensor-core shapes only); only the
-compatibility entry points below take host counts.
+precision; small fp32 calls, fp64 and odd shapes take the reference-precision SIMT kernels.  Row
+offsets are an int32 device tensor ``offs[E+1]`` (``None`` for a single group of all rows,
+tensor-core shapes only); only the compatibility entry points below take host counts.
 """
 import torch
 

@@ -156,8 +156,8 @@ def test_scores_need_not_lie_next_to_each_other(dtype, kind):
     torch.manual_seed(3)
     x = torch.randn(50, 64, device=DEV, dtype=dtype)
     ids = torch.randint(-1, 3, (50, 1), device=DEV)
-    table = torch.rand(50, 5, device=DEV, dtype=dtype) if kind == "column" else torch.rand(1, 1, device=DEV, dtype=dtype)
-    for run in (general._general_path, lambda *a: between._fused_forward(*a) if dtype != torch.float32 else general._general_path(*a)):
+    table = torch.rand(*((50, 5) if kind == "column" else (1, 1)), device=DEV, dtype=dtype)
+    for run in [general._general_path] + ([between._fused_forward] if dtype != torch.float32 else []):
         results = []
         for apart in (True, False):
             leaf = table.clone().requires_grad_(True)

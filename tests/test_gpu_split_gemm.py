@@ -129,7 +129,8 @@ def test_split_gemm_of_values_near_the_end_of_the_range(exponent, which):
                 (dw[e], D.t() @ V, D.abs().t() @ V.abs(), V.abs().max(), c)]:
             bound = _bound(size, terms) + terms * (2.0 ** -148 * small + 2.0 ** -149)
             assert bool(((got.double() - ref).abs() <= bound).all()), float(((got.double() - ref).abs() / bound).max())
-        assert bool(((db[e].double() - D.sum(0)).abs() <= D.abs().sum(0) * (24 + c / 256) * 2.0 ** -24 + c * 2.0 ** -148).all())
+        bound = D.abs().sum(0) * (24 + c / 256) * 2.0 ** -24 + c * 2.0 ** -148
+        assert bool(((db[e].double() - D.sum(0)).abs() <= bound).all())
 
 
 @pytest.mark.parametrize("act", [nn.GELU(), nn.ReLU(), nn.GELU(approximate="tanh"), nn.Identity(),
@@ -246,7 +247,8 @@ def test_fp32_layer_gradient_of_the_gradient(act, constant):
     moe = FMoETransformerMLP(num_expert=4, d_model=64, d_hidden=96, activation=act, top_k=2).to(DEV)
     nn.init.normal_(moe.experts.htoh4.bias)
     nn.init.normal_(moe.experts.h4toh.bias)
-    base = [torch.randn(64, 64, device=DEV), torch.rand(64, 2, device=DEV)] + [p.detach() for p in moe.experts.parameters()]
+    base = [torch.randn(64, 64, device=DEV), torch.rand(64, 2, device=DEV)]
+    base += [p.detach() for p in moe.experts.parameters()]
     ids = torch.randint(-1, 3, (64, 2), device=DEV)
     off = {"nothing": (), "scores": (1,), "experts": (2, 3, 4, 5), "input": (0,)}[constant]
     names = [n for n, _ in moe.experts.named_parameters()]
@@ -256,8 +258,8 @@ def test_fp32_layer_gradient_of_the_gradient(act, constant):
         if x.dtype == torch.float32:
             from fastmoe_b200.ops import grouped_gemm as gg, native
             from fastmoe_b200.transformer import activation_kind
-            return native.get().moe_mlp(x, score, p["htoh4.weight"], p["htoh4.bias"], p["h4toh.weight"], p["h4toh.bias"],
-                                        ids, gg.ACT_CODES[activation_kind(act)], True)
+            return native.get().moe_mlp(x, score, p["htoh4.weight"], p["htoh4.bias"], p["h4toh.weight"],
+                                        p["h4toh.bias"], ids, gg.ACT_CODES[activation_kind(act)], True)
         rows = torch.stack([act(x @ p["htoh4.weight"][e].t() + p["htoh4.bias"][e]) @ p["h4toh.weight"][e].t()
                             + p["h4toh.bias"][e] for e in range(4)])
         picked = rows[ids.clamp(min=0), torch.arange(64, device=DEV)[:, None]]
@@ -310,7 +312,8 @@ def test_fp32_layer_under_checkpointing_and_offloading():
     for run in (moe, lambda t: checkpoint(moe, t, use_reentrant=False), offloaded):
         moe.zero_grad(set_to_none=True)
         grads = torch.autograd.grad(run(x).square().sum(), [x] + list(moe.parameters()))
-        twice = torch.autograd.grad(torch.autograd.grad(run(x).square().sum(), x, create_graph=True)[0].square().sum(), x)
+        first, = torch.autograd.grad(run(x).square().sum(), x, create_graph=True)
+        twice = torch.autograd.grad(first.square().sum(), x)
         results.append(grads + twice)
     for other in results[1:]:
         for a, b in zip(other, results[0]):
