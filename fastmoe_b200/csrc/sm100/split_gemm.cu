@@ -16,18 +16,17 @@
 // Keeping them apart also keeps infinities: inf - inf of h l and h m would be NaN where the
 // product is inf, so a total that is not finite is replaced by the sum of h h.
 //
-// Error against 64 bits (2-norm, 8 experts, 4096 rows, 512 -> 2048): forward 7.3e-8, input gradient
-// 1.2e-7, weight gradient 9.1e-8, where FMAs in ascending order have 3.1e-7, 8.1e-7 and 4.1e-7.
+// Error against 64 bits (2-norm, 8 experts, 4096 rows, 512 -> 2048): forward 9.0e-8, input gradient
+// 1.1e-7, weight gradient 9.0e-8, where FMAs in ascending order have 4.1e-7, 8.1e-7 and 4.1e-7.
 //
 // What bounds it: the tensor cores, at six times the bf16 work, and the shared memory their operands
-// come from.  4 experts, 16384 rows, 1024 -> 2048: 310 to 330 us = 1250 to 1330 TFLOP/s of bf16
-// products, 208 to 220 of fp32, with the splitting 364 to 418, where the FMA kernel (sgemm.cu) takes
+// come from.  4 experts, 16384 rows, 1024 -> 2048: 307 to 327 us = 1260 to 1340 TFLOP/s of bf16
+// products, 210 to 224 of fp32, with the splitting 355 to 417, where the FMA kernel (sgemm.cu) takes
 // 1290 to 1400.  A plane of A serves all its products in a row out of the operand collector: 4 to 5 %.
-// A pair of CTAs (cta_group::2) works
-// on a 256 x 128 tile, half the width of the 16-bit kernel's: an epilogue warp holds 32 x 64 sums in
-// registers, 64 per thread, and fp32 layers are small (512 outputs of 8 experts with 512 rows are
-// 64 such tiles for 74 pairs).  The tiles of the last round are cut along K (tile_walk.cuh): 8
-// experts with 384 to 640 rows, 2048 -> 512, 119 against 141 us, splitting included.
+// A pair of CTAs (cta_group::2) works on a 256 x 128 tile, half the width of the 16-bit kernel's: an
+// epilogue warp holds 32 x 64 sums in registers, 64 per thread, and fp32 layers are small (512 outputs
+// of 8 experts with 512 rows are 64 such tiles for 74 pairs).  The tiles of the last round are cut along
+// K (tile_walk.cuh): 8 experts with 384 to 640 rows, 2048 -> 512, 121 against 141 us, splitting included.
 //
 // Roles of a CTA (384 threads), persistent over the tiles of its pair:
 //   warp 0      TMA producer, one lane: three planes of this CTA's halves of A and B per K block, 72 KB
@@ -37,6 +36,9 @@
 //               rows; row modes: zeros past the last expert;
 //   warps 4-11  epilogue.
 // TMEM: two accumulators of 128 columns for h h in turn, one each for the products of the next two orders.
+// (One for both of these, unscaled, leaves three for h h: what an epilogue with an activation holds up is a
+// K block less then.  8 experts, 4096 rows, 512 -> 2048: GELU 103 -> 106 us, its derivative 106 -> 116, plain
+// products the same to 3 %; the scales are worth it, see above.)
 #include "split_gemm.cuh"
 
 #include <float.h>
@@ -625,7 +627,8 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       // 16 columns at a time: a lane has a row of its own, so that each store of a warp touches 32 lines
       // whatever its width, and the widest are the fewest (32 bytes to a plane where the rows allow it).
       // With 16-byte stores and loads behind the stores, 8 experts, 4096 rows, 512 -> 2048 took 131 us with
-      // GELU and 115 in its derivative, 104 and 103 now; 16 experts, 8192 rows, 256 -> 1024 110 and 95, 79 and 84.
+      // GELU and 115 in its derivative, 104 and 103 so; 16 experts, 8192 rows, 256 -> 1024 110 and 95, 79 and 84.
+      // (With three accumulators for h h; with the two there are 106, 116, 82 and 90.)
       float x[16];
       auto load_pre = [&](int col, float (&to)[16]) {
 #pragma unroll
