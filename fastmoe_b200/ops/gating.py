@@ -113,21 +113,37 @@ def _single_pass_type(x, weight, bias):
     return x.dtype == torch.float32 and _plain(x, weight, bias)
 
 
+def _wants_grad(*tensors):
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+
+
 def _no_tangent(*tensors):
     r"""Whether no forward-mode derivative passes through: the native calls would drop it."""
     return all(t is None or forward_ad.unpack_dual(t).tangent is None for t in tensors)
 
 
+def _library_linear_better(tokens, d, experts, grads):
+    r"""Whether a Switch layer in 16 bits is faster with the library's linear.  The library has tensor-core
+    kernels for output rows of a multiple of 16 bytes (8 experts); with others it splits K, is slower and
+    rounds twice.  Layers of 8 experts with the kernel / with the linear, us: without gradients d 512: 30.8 / 31.1 at 64
+    tokens, 48.6 / 46.7 at 8192; d 1024: 34.9 / 34.5, 64.0 / 60.7; d 4096: 61.8 / 58.3, 150.9 / 135.0, and 4 us of host
+    time; a step of d 512: 78.7 / 80.3, 138.3 / 151.3; d 1024: 90.4 / 88.4, 121.7 / 119.7 at 2048 tokens, 171.8 /
+    181.5; d 2048: 112.8 / 104.9, 241.3 / 237.4.  (4 experts, d 2048, 64 tokens: 41.4 / 49.8, a step 103.9 / 114.3.)"""
+    return experts % 8 == 0 and not (grads and (d <= 512 or (d <= 1024 and tokens >= 4096)))
+
+
 def linear_logits(x, linear):
     r"""``linear(x)`` of a gate's ``nn.Linear`` in the single-pass kernel, or ``None`` where that does not
-    take the call or somebody watches the module.  It stands for three library products and a column sum
-    (a Switch layer's step, 4096 tokens, d 512, 8 experts: 492 us with those, 446 with this)."""
+    take the call, somebody watches the module or the linear is faster.  It stands for three library products
+    and a column sum (a Switch layer's step, 8192 tokens, d 1024, 2 experts: 216 us with those, 193 with this)."""
     from ..transformer import _hooked, _hooked_globally
     if type(linear) is not torch.nn.Linear:   # the user's own module (a quantised one, an adapter)
         return None
     w, b = linear.weight, linear.bias
     if (w.shape[0] <= MAX_SINGLE_PASS_EXPERTS and x.is_cuda and x.dim() == 2 and x.is_contiguous()
             and x.shape[0] > 0 and _single_pass_type(x, w, b) and not torch.is_autocast_enabled() and not traced()
+            and not (x.element_size() == 2 and _library_linear_better(x.shape[0], x.shape[1], w.shape[0],
+                                                                      _wants_grad(x, w, b)))
             and native.get().gate_fused_supported(w.shape[0], x.shape[1], 1)
             and _plain(x, w, b) and _no_tangent(x, w, b)
             and not _hooked(linear) and not _hooked_globally()):
@@ -193,7 +209,7 @@ def _few_tokens_ok(x, weight, bias, k):
             and x.shape[0] * x.shape[1] * weight.shape[0] <= MAX_FEW_PRODUCTS
             and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype
             and (bias is None or bias.dtype == x.dtype)
-            and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, weight, bias)))
+            and not _wants_grad(x, weight, bias)
             and not torch.is_autocast_enabled() and not traced() and _no_tangent(x, weight, bias)
             and native.get().gate_fused_supported(weight.shape[0], x.shape[1], k))
 

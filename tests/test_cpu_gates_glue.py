@@ -112,3 +112,15 @@ def test_naive_gate_with_another_choice(how):
             return logits, idx.flip(1), score
         gate._choose = choose
     assert torch.equal(gate(x)[0], plain(x)[0].flip(1)) and float(gate.get_loss().detach()) == 0
+
+
+@pytest.mark.parametrize("dtype,experts,tokens,d,grads,kernel", [
+    (torch.bfloat16, 8, 64, 512, False, False), (torch.float16, 8, 8192, 4096, False, False),
+    (torch.bfloat16, 8, 64, 512, True, True), (torch.bfloat16, 8, 4095, 1024, True, False),
+    (torch.float16, 8, 4096, 1024, True, True), (torch.bfloat16, 8, 8192, 2048, True, False),
+    (torch.bfloat16, 7, 64, 4096, False, True), (torch.bfloat16, 2, 1, 256, True, True),
+    (torch.float32, 8, 64, 512, False, True)])
+def test_switch_gate_linear_goes_where_it_is_faster(kernels, dtype, experts, tokens, d, grads, kernel):
+    linear, x = torch.nn.Linear(d, experts).to(dtype), torch.zeros(tokens, d, dtype=dtype)
+    with torch.set_grad_enabled(grads):
+        assert gating.linear_logits(x, linear) == ("kernel" if kernel else None)
